@@ -14,7 +14,7 @@
 // the neighbour's face trace and adds only its own side, so no atomics are
 // needed and results are bitwise reproducible run to run.
 #pragma once
-#include "atm_internal.h"
+#include "device_util.cuh"
 
 namespace atm {
 
@@ -529,40 +529,6 @@ __device__ __forceinline__ QGeoT<T> qgeo(const T *__restrict__ g, int q) {
   return r;
 }
 
-// Values between two cells' A^{-1} blocks ([nc][stride]).  FP64: the full
-// (k+1)^2 x (k+1)^2 block.  FP32 (multigrid levels): A^{-1} is symmetric, so
-// only its lower triangle is stored, row by row ((r, c <= r) at
-// r (r+1)/2 + c), padded to a multiple of 16 bytes: the B kernel stages the
-// blocks of its cells into shared memory with 16-byte cp.async copies, and
-// half the bytes leave more room there.
-template <int K, typename T>
-__host__ __device__ constexpr int ainv_stride() {
-  return sizeof(T) == 4
-             ? ((K + 1) * (K + 1) * ((K + 1) * (K + 1) + 1) / 2 + 3) / 4 * 4
-             : (K + 1) * (K + 1) * (K + 1) * (K + 1);
-}
-inline long ainv_stride_rt(int k, size_t elem) {
-  const long n2 = (long)(k + 1) * (k + 1);
-  return elem == 4 ? (n2 * (n2 + 1) / 2 + 3) / 4 * 4 : n2 * n2;
-}
-
-// 16-byte asynchronous global -> shared copies (cp.async, bypassing L1) and
-// the wait for all of this thread's outstanding copies
-__device__ __forceinline__ void cp_async16(void *smem, const void *gmem) {
-  const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async4(void *smem, const void *gmem) {
-  const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(s), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() {
-  asm volatile("cp.async.commit_group;\n" ::: "memory");
-}
-__device__ __forceinline__ void cp_async_wait_all() {
-  asm volatile("cp.async.wait_all;\n" ::: "memory");
-}
-
 // Quadrature-point geometry of cell c along the column of Gauss points
 // (g_col, g_qz), qz = 0..NQ-1, as the Schur kernels consume it.  FP64 reads
 // the stored table qgeo.  FP32 (multigrid levels) forms it from the cell's
@@ -661,28 +627,6 @@ struct GeoCol<K, float> {
     get = xxi * w;
   }
 };
-
-// Let kernel `fn` use up to the device's opt-in maximum of dynamic shared
-// memory when a launch needs more than the default 48 KB.  The limit is set
-// to that maximum, always the same value: host threads launching the same
-// kernel with different block shapes (serving members, the autotuner) must
-// never lower each other's limit between setting it and launching.
-template <typename F>
-inline cudaError_t allow_smem(F fn, size_t bytes) {
-  if (bytes <= 48 * 1024) return cudaSuccess;
-  static int cap[64] = {0};  // per device; a benign race writes the same value
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  int mx = dev >= 0 && dev < 64 ? cap[dev] : 0;
-  if (mx == 0) {
-    e = cudaDeviceGetAttribute(&mx, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    if (e != cudaSuccess) return e;
-    if (dev >= 0 && dev < 64) cap[dev] = mx;
-  }
-  if (bytes > (size_t)mx) return cudaErrorInvalidValue;
-  return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
-}
 
 // tiles, x-contraction exchange, face values [, subface-1 face values]
 template <int K, typename T = double>

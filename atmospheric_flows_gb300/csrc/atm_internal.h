@@ -64,6 +64,8 @@ template <typename T>
 struct MeshT {
   int nc = 0, k = 0, nn = 0, nq = 0, nn2 = 0, nq2 = 0;
   T *qgeo = nullptr;   // [nc][5][nq2]: dxi/dx*JxW, dxi/dz*JxW, deta/dx*JxW, deta/dz*JxW, JxW
+  T *jw = nullptr;     // JxW at the (2k+1)^2 points of cell c: jw + c * jw_stride (in qgeo,
+  long jw_stride = 0;  // or an array of its own on levels that have no qgeo)
   T *fgeo = nullptr;   // [nc][4][3][nq]: n_x, n_z, JxW (own-side, outward)
   int *nbr = nullptr;  // [nc][4] neighbour cell, -1 at a wall (hanging index h, code 3)
   int *nbrf = nullptr; // [nc][4] neighbour's local face | code << 2 (see below)
@@ -88,6 +90,17 @@ struct MeshT {
   // quadrature-point geometry from it in the Schur kernels instead of
   // reading qgeo (null on the FP64 operator mesh).
   T *map2 = nullptr;
+  // Tables of the Schur kernels for mapping degree <= 2 (schur_exact.cuh;
+  // `exact` when they are there), n = k+1, c = floor((3k+3)/2), q = 2k+1:
+  //   gB [nc][n][n][4]  -cofactors x weight at the k+1 Gauss points ([qx][qz])
+  //   fB [nc][4][n][2]  half outward normal x weight at the k+1 face points
+  //   gC [nc][c][c][4], gJ [nc][c][c]  cofactors and det J / (gamma-1) x weight
+  //   fC [nc][4][q][2]  outward normal x weight at the 2k+1 face points, times
+  //   half gamma/(gamma-1) (as gC holds gamma/(gamma-1))
+  //   hB [2 nhang][n][2], hC [2 nhang][q][2]  the coarse side's subfaces
+  bool exact = false;
+  T *gB = nullptr, *fB = nullptr, *gC = nullptr, *gJ = nullptr, *fC = nullptr;
+  T *hB = nullptr, *hC = nullptr;
 };
 using Mesh = MeshT<double>;
 
@@ -130,6 +143,7 @@ struct atm_ctx {
   // host copy of the operator mesh's mapping at degree 2 (MeshT::map2
   // layout): the geometry of the FP32 multigrid level 0
   std::vector<double> map2;
+  std::vector<int> hcf;  // host copy of HostMesh::hcf
   long n_scalar() const { return (long)nc * nn2; }
   long n_vector() const { return 2L * nc * nn2; }
 };
@@ -169,6 +183,7 @@ struct HostBasis {
 };
 HostBasis make_basis(int k);
 std::vector<double> gll_nodes(int k);
+void gauss_nodes(int n, std::vector<double> &x, std::vector<double> &w);  // on [0, 1]
 void lagrange_eval(const std::vector<double> &nodes, double x, double *val, double *der);
 // upload S/D tables of every degree to each translation unit's constant bank
 int upload_basis_all();
@@ -181,9 +196,11 @@ int launch_rhs_vel(const atm_ctx &c, int stage, double *dst, const double *const
                    const StageCoef &co);
 int launch_rhs_pres(const atm_ctx &c, int stage, double *dst, const double *const *src,
                     const StageCoef &co);
-// B p -> dst (velocity); mode 0: dst = B p; 1: dst -= B p;
-// 2: dst = A^{-1} B p (uses c.ainv)
-int launch_B(const atm_ctx &c, double *dst, const double *p, double coeff, int mode);
+// B p -> dst (velocity); mode 0: dst = cB B p; 1: dst -= cB B p;
+// 2: dst = A^{-1} B p as the C/D modes 1 and 2 take it (uses c.ainv): times
+// cB cC on meshes with `exact` tables, times cB otherwise
+int launch_B(const atm_ctx &c, double *dst, const double *p, double cB, int mode,
+             double cC = 1.0);
 // C/D family on pressure space:
 //   mode 0: dst = C w
 //   mode 1: dst = sD*D p - C w
@@ -263,7 +280,22 @@ struct LevelViewT {
   const T *pfix = nullptr, *pfq = nullptr, *pff = nullptr;  // level p_fix (+ prepared)
 };
 template <typename T>
-int level_B(const LevelViewT<T> &v, T *dst, const T *p, T cB, int mode);
+using OpView = LevelViewT<T>;
+inline OpView<double> schur_view(const atm_ctx &c) {
+  return OpView<double>{c.k, c.nc, c.mesh, c.ainv, c.invdiag_D, c.stream,
+                        c.autotune && !c.capturing, c.pres_fix, c.pfq, c.pff};
+}
+#define ATM_DISPATCH_K(kk, call)          \
+  switch (kk) {                           \
+    case 1: { constexpr int K = 1; return call; } \
+    case 2: { constexpr int K = 2; return call; } \
+    case 3: { constexpr int K = 3; return call; } \
+    case 4: { constexpr int K = 4; return call; } \
+    case 5: { constexpr int K = 5; return call; } \
+    default: return ATM_BAD_ARG;          \
+  }
+template <typename T>
+int level_B(const LevelViewT<T> &v, T *dst, const T *p, T cB, T cC);
 template <typename T>
 int level_CD(const LevelViewT<T> &v, T *dst, const T *w, const T *p, T cC, int mode);
 // Chebyshev update fused into the C/D epilogue (multigrid smoother): with
@@ -278,6 +310,22 @@ struct ChebArgs {
 };
 template <typename T>
 int level_CD_cheb(const LevelViewT<T> &v, const T *w, T cC, const ChebArgs<T> &ch);
+// Schur kernels on meshes with `exact` tables (schur_exact*.cu): modes as
+// launch_B and launch_CD, and 4 for the Chebyshev update
+int exact_B(const OpView<double> &o, double *dst, const double *p, double cB, double cC, int mode);
+int exact_B(const OpView<float> &o, float *dst, const float *p, float cB, float cC, int mode);
+int exact_CD(const OpView<double> &o, double *dst, const double *w, const double *p, double cC,
+             int mode, const ChebArgs<double> *ch);
+int exact_CD(const OpView<float> &o, float *dst, const float *w, const float *p, float cC,
+             int mode, const ChebArgs<float> *ch);
+int exact_pfix(const OpView<double> &o);
+int exact_pfix(const OpView<float> &o);
+int upload_exact_all();
+template <typename T>
+int exact_mesh_build(MeshT<T> &m, const double *map2, const std::vector<int> &hcf,
+                     cudaStream_t st);
+template <typename T>
+void exact_mesh_free(MeshT<T> &m);
 template <typename T>
 int level_pfix_prep(const LevelViewT<T> &v);
 template <typename T>
@@ -319,9 +367,11 @@ struct HostMesh {
   std::vector<double> qgeo, fgeo;
   std::vector<int> nbr, nbrf;
   std::vector<int> hnb;      // [nhang][2]
+  std::vector<int> hcf;      // [nhang] 4 cell + face of the coarse side
   std::vector<double> hgeo;  // [nhang][2][3][nq]
   std::vector<double> map2;  // [nc][3][3][2] the mapping at degree 2 (MeshT::map2)
   int nhang = 0;
+  bool exact = false;  // mapping degree <= 2: the degree-2 mapping is the mapping
 };
 int build_mesh_tables(int k, int nc, int mapdeg, const double *nodes, int n_inner,
                       const int *inner, int n_bdry, const int *bdry, HostMesh &out);

@@ -139,7 +139,8 @@ int atm_ctx_create(int dim, int degree, int n_cells, int mapping_degree,
   } while (0)
   ALLOC(c->rho_fix, ns);
   ALLOC(c->pres_fix, ns);
-  ALLOC(c->pfq, (long)n_cells * c->nq2);
+  const long ncp = (3 * degree + 3) / 2;  // H of the exact Schur kernels, or pfq
+  ALLOC(c->pfq, (long)n_cells * 4 * ncp * ncp);
   ALLOC(c->pff, (long)n_cells * 4 * c->nq);
   ALLOC(c->u_fix, nv);
   ALLOC(c->ainv, blk);

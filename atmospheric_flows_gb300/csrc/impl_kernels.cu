@@ -55,14 +55,14 @@ __global__ void __launch_bounds__(Cfg<K>::THREADS)
     const T *tl = tiles + lc * NT * NN2;
     T wv[NQ];
     if (WEIGHTED) eval_col<K>(tl + NCOMP * NN2, Sx, wv);
-    const T *G = mesh.qgeo + (long)c * 5 * NQ2;
+    const T *G = mesh.jw + c * mesh.jw_stride;
 #pragma unroll
     for (int comp = 0; comp < NCOMP; ++comp) {
       T v[NQ], V[NQ];
       eval_col<K>(tl + comp * NN2, Sx, v);
 #pragma unroll
       for (int qz = 0; qz < NQ; ++qz) {
-        const T jxw = G[4 * NQ2 + qz * NQ + col];
+        const T jxw = G[qz * NQ + col];
         V[qz] = (WEIGHTED ? wv[qz] * v[qz] : scale * v[qz]) * jxw;
       }
       integrate_col_z<K, true, false>(V, V, V, xab + (lc * NCOMP + comp) * NN * NQ, (T *)nullptr,
@@ -107,14 +107,14 @@ __global__ void __launch_bounds__(Cfg<K>::THREADS)
   if (active) {
     T wv[NQ];
     if (WEIGHTED) eval_col<K>(tiles + lc * NN2, Sx, wv);
-    const T *G = mesh.qgeo + (long)c * 5 * NQ2;
+    const T *G = mesh.jw + c * mesh.jw_stride;
 #pragma unroll
     for (int iz = 0; iz < NN; ++iz) {
       T s = T(0.0);
 #pragma unroll
       for (int qz = 0; qz < NQ; ++qz) {
         const T b = bS<K, T>(qz, iz);
-        const T wj = (WEIGHTED ? wv[qz] : scale) * G[4 * NQ2 + qz * NQ + col];
+        const T wj = (WEIGHTED ? wv[qz] : scale) * G[qz * NQ + col];
         s = fma(b * b, wj, s);
       }
       xab[lc * NN * NQ + iz * NQ + col] = s;
@@ -202,7 +202,7 @@ __global__ void __launch_bounds__(32 * BI_WARPS)
   T *colk = M + NTRI;            // [NN2] pivot column
   T *cd = colk + NN2;            // [NN2] pivot column / pivot
   T *tx = cd + NN2;              // [NN][NQ] x-contracted weight field
-  const T *G = mesh.qgeo + (long)c * 5 * NQ2;
+  const T *G = mesh.jw + c * mesh.jw_stride;
   if (weight) {
     const T *wt = weight + (long)c * NN2;
     for (int e = lane; e < NN * NQ; e += 32) {
@@ -218,10 +218,10 @@ __global__ void __launch_bounds__(32 * BI_WARPS)
       T s = T(0.0);
 #pragma unroll
       for (int iz = 0; iz < NN; ++iz) s = fma(bS<K, T>(qz, iz), tx[iz * NQ + qx], s);
-      wq[q] = s * G[4 * NQ2 + q];
+      wq[q] = s * G[q];
     }
   } else {
-    for (int q = lane; q < NQ2; q += 32) wq[q] = G[4 * NQ2 + q];
+    for (int q = lane; q < NQ2; q += 32) wq[q] = G[q];
   }
   __syncwarp();
   for (int e = lane; e < NQ * NP; e += 32) {
@@ -339,7 +339,7 @@ int block_apply_launch(const OpView<T> &v, T *dst, const T *src, const T *binv, 
   return ATM_OK;
 }
 }  // namespace
-int launch_B(const atm_ctx &c, double *dst, const double *p, double coeff, int mode) {
+int launch_B(const atm_ctx &c, double *dst, const double *p, double cB, int mode, double cC) {
   const double ns = (double)c.nc * c.nn2;
   // p read; B p written (2 comps); mode 1 reads dst too; mode 2 reads A^{-1}
   const double bytes = 8.0 * ns * (1 + 2 + (mode == 1 ? 2 : 0)) +
@@ -348,8 +348,9 @@ int launch_B(const atm_ctx &c, double *dst, const double *p, double coeff, int m
                                4.0 * (2 * fl_face(c.k) + 2 * fl_face(c.k)) +
                                (mode == 2 ? 4.0 * c.nn2 * c.nn2 : 0.0));
   TimedRegion tr(c, KF_B, bytes, flops);
-  if (c.mesh.nhang > 0) return launch_B_hang(c, dst, p, coeff, mode);
-  ATM_DISPATCH_K(c.k, (B_launch<K, double, false>(schur_view(c), dst, p, coeff, mode)));
+  if (c.mesh.exact) return exact_B(schur_view(c), dst, p, cB, cC, mode);
+  if (c.mesh.nhang > 0) return launch_B_hang(c, dst, p, cB, mode);
+  ATM_DISPATCH_K(c.k, (B_launch<K, double, false>(schur_view(c), dst, p, cB, mode)));
 }
 int launch_CD(const atm_ctx &c, double *dst, const double *w, const double *p, double coeff,
               int mode) {
@@ -360,6 +361,7 @@ int launch_CD(const atm_ctx &c, double *dst, const double *w, const double *p, d
   const double flops = c.nc * ((wd ? 4 : 3) * fl_eval(c.k) + fl_integrate(c.k, true) +
                                4.0 * (2 * 3 * fl_face(c.k) + fl_face(c.k)));
   TimedRegion tr(c, KF_CD, bytes, flops);
+  if (c.mesh.exact) return exact_CD(schur_view(c), dst, w, p, coeff, mode, nullptr);
   if (c.mesh.nhang > 0) return launch_CD_hang(c, dst, w, p, coeff, mode);
   ATM_DISPATCH_K(c.k, (CD_launch<K, double, false>(schur_view(c), dst, w, p, coeff, mode)));
 }
@@ -368,6 +370,7 @@ int launch_pfix_prep(const atm_ctx &c) {
   const double bytes = 8.0 * c.nc * (c.nn2 + c.nq2 + 4.0 * c.nq);
   const double flops = c.nc * (fl_eval(c.k) + 4.0 * fl_face(c.k));
   TimedRegion tr(c, KF_PFIX_PREP, bytes, flops);
+  if (c.mesh.exact) return exact_pfix(schur_view(c));
   ATM_DISPATCH_K(c.k, (pfix_prep_launch<K, double>(schur_view(c))));
 }
 int launch_mass(const atm_ctx &c, double *dst, const double *src, int ncomp,
@@ -403,40 +406,38 @@ int launch_block_apply(const atm_ctx &c, double *dst, const double *src, const d
 
 // ---- launchers on a multigrid level (untimed; float or double) -----------
 template <typename T>
-int level_B(const LevelViewT<T> &v, T *dst, const T *p, T cB, int mode) {
-  OpView<T> o{v.k, v.nc, v.mesh, v.ainv, v.invd, v.st, v.tune, v.pfix, v.pfq, v.pff};
-  if (v.mesh.nhang > 0) return level_B_hang<T>(o, dst, p, cB, mode);
-  ATM_DISPATCH_K(v.k, (B_launch<K, T, false>(o, dst, p, cB, mode)));
+int level_B(const LevelViewT<T> &v, T *dst, const T *p, T cB, T cC) {
+  if (v.mesh.exact) return exact_B(v, dst, p, cB, cC, 2);
+  if (v.mesh.nhang > 0) return level_B_hang<T>(v, dst, p, cB, 2);
+  ATM_DISPATCH_K(v.k, (B_launch<K, T, false>(v, dst, p, cB, 2)));
 }
 template <typename T>
 int level_CD(const LevelViewT<T> &v, T *dst, const T *w, const T *p, T cC, int mode) {
-  OpView<T> o{v.k, v.nc, v.mesh, v.ainv, v.invd, v.st, v.tune, v.pfix, v.pfq, v.pff};
-  if (v.mesh.nhang > 0) return level_CD_hang<T>(o, dst, w, p, cC, mode, nullptr);
-  ATM_DISPATCH_K(v.k, (CD_launch<K, T, false>(o, dst, w, p, cC, mode)));
+  if (v.mesh.exact) return exact_CD(v, dst, w, p, cC, mode, nullptr);
+  if (v.mesh.nhang > 0) return level_CD_hang<T>(v, dst, w, p, cC, mode, nullptr);
+  ATM_DISPATCH_K(v.k, (CD_launch<K, T, false>(v, dst, w, p, cC, mode)));
 }
 template <typename T>
 int level_CD_cheb(const LevelViewT<T> &v, const T *w, T cC, const ChebArgs<T> &ch) {
-  OpView<T> o{v.k, v.nc, v.mesh, v.ainv, v.invd, v.st, v.tune, v.pfix, v.pfq, v.pff};
-  if (v.mesh.nhang > 0) return level_CD_hang<T>(o, nullptr, w, ch.x, cC, 4, &ch);
-  ATM_DISPATCH_K(v.k, (CD_launch<K, T, false>(o, nullptr, w, ch.x, cC, 4, &ch)));
+  if (v.mesh.exact) return exact_CD(v, (T *)nullptr, w, ch.x, cC, 4, &ch);
+  if (v.mesh.nhang > 0) return level_CD_hang<T>(v, nullptr, w, ch.x, cC, 4, &ch);
+  ATM_DISPATCH_K(v.k, (CD_launch<K, T, false>(v, nullptr, w, ch.x, cC, 4, &ch)));
 }
 template <typename T>
 int level_pfix_prep(const LevelViewT<T> &v) {
-  OpView<T> o{v.k, v.nc, v.mesh, v.ainv, v.invd, v.st, v.tune, v.pfix, v.pfq, v.pff};
-  ATM_DISPATCH_K(v.k, (pfix_prep_launch<K, T>(o)));
+  if (v.mesh.exact) return exact_pfix(v);
+  ATM_DISPATCH_K(v.k, (pfix_prep_launch<K, T>(v)));
 }
 template <typename T>
 int level_inv_diag(const LevelViewT<T> &v, T *out, T scale) {
-  OpView<T> o{v.k, v.nc, v.mesh, v.ainv, v.invd, v.st, v.tune, v.pfix, v.pfq, v.pff};
-  ATM_DISPATCH_K(v.k, (invdiag_launch<K, T>(o, out, 1, (const T *)nullptr, scale)));
+  ATM_DISPATCH_K(v.k, (invdiag_launch<K, T>(v, out, 1, (const T *)nullptr, scale)));
 }
 template <typename T>
 int level_block_inverse(const LevelViewT<T> &v, T *out, const T *weight) {
-  OpView<T> o{v.k, v.nc, v.mesh, v.ainv, v.invd, v.st, v.tune, v.pfix, v.pfq, v.pff};
-  ATM_DISPATCH_K(v.k, (block_inverse_launch<K, T>(o, out, weight)));
+  ATM_DISPATCH_K(v.k, (block_inverse_launch<K, T>(v, out, weight)));
 }
 #define ATM_LEVEL_INST(T)                                                                   \
-  template int level_B<T>(const LevelViewT<T> &, T *, const T *, T, int);                   \
+  template int level_B<T>(const LevelViewT<T> &, T *, const T *, T, T);                     \
   template int level_CD<T>(const LevelViewT<T> &, T *, const T *, const T *, T, int);       \
   template int level_pfix_prep<T>(const LevelViewT<T> &);                                   \
   template int level_CD_cheb<T>(const LevelViewT<T> &, const T *, T, const ChebArgs<T> &);   \

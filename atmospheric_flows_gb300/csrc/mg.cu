@@ -287,6 +287,7 @@ MGHier<double> &hier<double>(MG &mg) { return mg.d; }
 
 template <typename T>
 void level_free(MGLevelT<T> &L) {
+  exact_mesh_free(L.mesh);
   cudaFree(L.mesh.qgeo); cudaFree(L.mesh.fgeo); cudaFree(L.mesh.nbr); cudaFree(L.mesh.nbrf);
   cudaFree(L.mesh.hnb); cudaFree(L.mesh.hgeo); cudaFree(L.mesh.dts); cudaFree(L.mesh.map2);
   cudaFree(L.parent); cudaFree(L.ppos); cudaFree(L.children);
@@ -339,34 +340,41 @@ int level_alloc(atm_ctx &c, MGLevelT<T> &L, const HostMesh &hm) {
   const long ns = (long)L.nc * nn2;
   L.mesh.nc = L.nc; L.mesh.k = c.k; L.mesh.nn = c.nn; L.mesh.nq = nq;
   L.mesh.nn2 = nn2; L.mesh.nq2 = nq2;
-  std::vector<T> qf(hm.qgeo.begin(), hm.qgeo.end()), ff(hm.fgeo.begin(), hm.fgeo.end());
   if (hm.map2.size() != (size_t)L.nc * 18) {
     set_error("multigrid level: missing degree-2 mapping table");
     return ATM_BAD_ARG;
   }
-  if (sizeof(T) == 4) {  // the FP32 Schur kernels form their geometry from it
-    std::vector<T> m2(hm.map2.begin(), hm.map2.end());
-    ATM_CUDA(cudaMalloc(&L.mesh.map2, m2.size() * sizeof(T)));
-    ATM_CUDA(cudaMemcpyAsync(L.mesh.map2, m2.data(), m2.size() * sizeof(T), cudaMemcpyHostToDevice, c.stream));
-    ATM_CUDA(cudaStreamSynchronize(c.stream));  // pageable source
+  if (!hm.exact) {  // the general Schur kernels' geometry
+    std::vector<T> qf(hm.qgeo.begin(), hm.qgeo.end()), ff(hm.fgeo.begin(), hm.fgeo.end());
+    if (sizeof(T) == 4) {  // their FP32 form builds the volume geometry from it
+      std::vector<T> m2(hm.map2.begin(), hm.map2.end());
+      ATM_CUDA(cudaMalloc(&L.mesh.map2, m2.size() * sizeof(T)));
+      ATM_CUDA(cudaMemcpyAsync(L.mesh.map2, m2.data(), m2.size() * sizeof(T), cudaMemcpyHostToDevice, c.stream));
+      ATM_CUDA(cudaStreamSynchronize(c.stream));  // pageable source
+    }
+    ATM_CUDA(cudaMalloc(&L.mesh.qgeo, qf.size() * sizeof(T)));
+    L.mesh.jw = L.mesh.qgeo + 4 * nq2;
+    L.mesh.jw_stride = 5 * nq2;
+    ATM_CUDA(cudaMalloc(&L.mesh.fgeo, ff.size() * sizeof(T)));
+    ATM_CUDA(cudaMemcpyAsync(L.mesh.qgeo, qf.data(), qf.size() * sizeof(T), cudaMemcpyHostToDevice, c.stream));
+    ATM_CUDA(cudaMemcpyAsync(L.mesh.fgeo, ff.data(), ff.size() * sizeof(T), cudaMemcpyHostToDevice, c.stream));
+    ATM_CUDA(cudaStreamSynchronize(c.stream));  // pageable sources
   }
-  ATM_CUDA(cudaMalloc(&L.mesh.qgeo, qf.size() * sizeof(T)));
-  ATM_CUDA(cudaMalloc(&L.mesh.fgeo, ff.size() * sizeof(T)));
   ATM_CUDA(cudaMalloc(&L.mesh.nbr, hm.nbr.size() * sizeof(int)));
   ATM_CUDA(cudaMalloc(&L.mesh.nbrf, hm.nbrf.size() * sizeof(int)));
-  ATM_CUDA(cudaMemcpyAsync(L.mesh.qgeo, qf.data(), qf.size() * sizeof(T), cudaMemcpyHostToDevice, c.stream));
-  ATM_CUDA(cudaMemcpyAsync(L.mesh.fgeo, ff.data(), ff.size() * sizeof(T), cudaMemcpyHostToDevice, c.stream));
   ATM_CUDA(cudaMemcpyAsync(L.mesh.nbr, hm.nbr.data(), hm.nbr.size() * sizeof(int), cudaMemcpyHostToDevice, c.stream));
   ATM_CUDA(cudaMemcpyAsync(L.mesh.nbrf, hm.nbrf.data(), hm.nbrf.size() * sizeof(int), cudaMemcpyHostToDevice, c.stream));
   L.mesh.nhang = hm.nhang;
   if (hm.nhang > 0) {
-    std::vector<T> hg(hm.hgeo.begin(), hm.hgeo.end());
     ATM_CUDA(cudaMalloc(&L.mesh.hnb, hm.hnb.size() * sizeof(int)));
-    ATM_CUDA(cudaMalloc(&L.mesh.hgeo, hg.size() * sizeof(T)));
     ATM_CUDA(cudaMemcpyAsync(L.mesh.hnb, hm.hnb.data(), hm.hnb.size() * sizeof(int), cudaMemcpyHostToDevice, c.stream));
-    ATM_CUDA(cudaMemcpyAsync(L.mesh.hgeo, hg.data(), hg.size() * sizeof(T), cudaMemcpyHostToDevice, c.stream));
-    // the host copies above are pageable: finish them before `hg` goes away
-    ATM_CUDA(cudaStreamSynchronize(c.stream));
+    if (!hm.exact) {
+      std::vector<T> hg(hm.hgeo.begin(), hm.hgeo.end());
+      ATM_CUDA(cudaMalloc(&L.mesh.hgeo, hg.size() * sizeof(T)));
+      ATM_CUDA(cudaMemcpyAsync(L.mesh.hgeo, hg.data(), hg.size() * sizeof(T), cudaMemcpyHostToDevice, c.stream));
+      // the host copy is pageable: finish it before `hg` goes away
+      ATM_CUDA(cudaStreamSynchronize(c.stream));
+    }
   }
   T **vecs[] = {&L.invd, &L.rho, &L.pfix, &L.x, &L.b, &L.r, &L.t, &L.d};
   for (T **v : vecs) {
@@ -378,7 +386,10 @@ int level_alloc(atm_ctx &c, MGLevelT<T> &L, const HostMesh &hm) {
   // the padding after each FP32 triangle is copied but never used
   ATM_CUDA(cudaMemsetAsync(L.ainv, 0, (size_t)L.nc * ainv_stride_rt(c.k, sizeof(T)) * sizeof(T),
                            c.stream));
-  ATM_CUDA(cudaMalloc(&L.pfq, (size_t)L.nc * c.nq2 * sizeof(T)));
+  if (hm.exact)
+    if (int rc = exact_mesh_build(L.mesh, hm.map2.data(), hm.hcf, c.stream)) return rc;
+  const size_t ncp = (3 * c.k + 3) / 2;  // H of the exact Schur kernels, or pfq
+  ATM_CUDA(cudaMalloc(&L.pfq, (size_t)L.nc * 4 * ncp * ncp * sizeof(T)));
   ATM_CUDA(cudaMalloc(&L.pff, (size_t)L.nc * 4 * c.nq * sizeof(T)));
   return level_inv_diag<T>(lview(c, L), L.invd, (T)(1.0 / (GAS_GAMMA - 1.0)));
 }
@@ -457,7 +468,7 @@ int level_apply(atm_ctx &c, MGLevelT<T> &L, T *out, const T *x) {
                                4.0 * c.nn2 * c.nn2 + 4 * fl_eval(c.k) + fl_integrate(c.k, true) +
                                4.0 * 7 * fl_face(c.k));
   TimedRegion tr(c, KF_MG_APPLY, bytes, flops);
-  int rc = level_B<T>(v, L.wv, x, (T)(co * c.dt / (c.Ma * c.Ma)), 2);
+  int rc = level_B<T>(v, L.wv, x, (T)(co * c.dt / (c.Ma * c.Ma)), (T)(co * c.dt));
   if (rc) return rc;
   return level_CD<T>(v, out, L.wv, x, (T)(co * c.dt), 1);
 }
@@ -476,7 +487,7 @@ int level_apply_cheb(atm_ctx &c, MGLevelT<T> &L, double a, double b_coef, bool f
                                4.0 * c.nn2 * c.nn2 + 4 * fl_eval(c.k) + fl_integrate(c.k, true) +
                                4.0 * 7 * fl_face(c.k));
   TimedRegion tr(c, KF_MG_APPLY, bytes, flops);
-  int rc = level_B<T>(v, L.wv, L.x, (T)(co * c.dt / (c.Ma * c.Ma)), 2);
+  int rc = level_B<T>(v, L.wv, L.x, (T)(co * c.dt / (c.Ma * c.Ma)), (T)(co * c.dt));
   if (rc) return rc;
   ChebArgs<T> ch;
   ch.x = L.x;
@@ -740,21 +751,26 @@ int mg_add_level(atm_ctx &c, int n_cells, int mapdeg, const double *nodes, int n
   if (!c.mg) {
     MG *mg = new MG();
     HostMesh hm;
-    hm.qgeo.resize((size_t)c.nc * 5 * c.nq2);
-    hm.fgeo.resize((size_t)c.nc * 4 * 3 * c.nq);
     hm.nbr.resize((size_t)c.nc * 4);
     hm.nbrf.resize((size_t)c.nc * 4);
     hm.nhang = c.mesh.nhang;
     hm.hnb.resize((size_t)c.mesh.nhang * 2);
-    hm.hgeo.resize((size_t)c.mesh.nhang * 2 * 3 * c.nq);
     hm.map2 = c.map2;
-    ATM_CUDA(cudaMemcpyAsync(hm.qgeo.data(), c.mesh.qgeo, hm.qgeo.size() * 8, cudaMemcpyDeviceToHost, c.stream));
-    ATM_CUDA(cudaMemcpyAsync(hm.fgeo.data(), c.mesh.fgeo, hm.fgeo.size() * 8, cudaMemcpyDeviceToHost, c.stream));
+    hm.hcf = c.hcf;
+    hm.exact = c.mesh.exact;
     ATM_CUDA(cudaMemcpyAsync(hm.nbr.data(), c.mesh.nbr, hm.nbr.size() * 4, cudaMemcpyDeviceToHost, c.stream));
     ATM_CUDA(cudaMemcpyAsync(hm.nbrf.data(), c.mesh.nbrf, hm.nbrf.size() * 4, cudaMemcpyDeviceToHost, c.stream));
-    if (hm.nhang > 0) {
+    if (hm.nhang > 0)
       ATM_CUDA(cudaMemcpyAsync(hm.hnb.data(), c.mesh.hnb, hm.hnb.size() * 4, cudaMemcpyDeviceToHost, c.stream));
-      ATM_CUDA(cudaMemcpyAsync(hm.hgeo.data(), c.mesh.hgeo, hm.hgeo.size() * 8, cudaMemcpyDeviceToHost, c.stream));
+    if (!hm.exact) {  // the general Schur kernels' geometry
+      hm.qgeo.resize((size_t)c.nc * 5 * c.nq2);
+      hm.fgeo.resize((size_t)c.nc * 4 * 3 * c.nq);
+      ATM_CUDA(cudaMemcpyAsync(hm.qgeo.data(), c.mesh.qgeo, hm.qgeo.size() * 8, cudaMemcpyDeviceToHost, c.stream));
+      ATM_CUDA(cudaMemcpyAsync(hm.fgeo.data(), c.mesh.fgeo, hm.fgeo.size() * 8, cudaMemcpyDeviceToHost, c.stream));
+      if (hm.nhang > 0) {
+        hm.hgeo.resize((size_t)c.mesh.nhang * 2 * 3 * c.nq);
+        ATM_CUDA(cudaMemcpyAsync(hm.hgeo.data(), c.mesh.hgeo, hm.hgeo.size() * 8, cudaMemcpyDeviceToHost, c.stream));
+      }
     }
     ATM_CUDA(cudaStreamSynchronize(c.stream));
     mg->hm.push_back(std::move(hm));

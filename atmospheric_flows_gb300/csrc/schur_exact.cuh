@@ -1,0 +1,775 @@
+// Schur-complement kernels for mappings of degree <= 2 (MappingQ(2),
+// equation_data.h:43): B (then optionally the exact cell-wise A^{-1}) and C/D.
+//   B   euler_operator.h:1512-1617
+//   C   euler_operator.h:1413-1507
+//   D   euler_operator.h:1386-1408
+//
+// The FP64 pipe of sm_103a issues two lanes per clock and SM, so a kernel
+// here costs what its FP64 instructions cost; everything else hides behind
+// them.  Two things set that count.
+//   * Quadrature.  The reference integrates everything with QGauss(2k+1).  On
+//     a degree-2 mapping the cofactors of the Jacobian have degree <= 2 along
+//     their own reference direction and <= 1 along the other one, so the
+//     integrands of B (p cof grad v) have degree 2k+1 and those of C
+//     (w p_fix cof grad q) degree 3k+1 in each direction: k+1 and
+//     NC = floor((3k+3)/2) Gauss points integrate them exactly, as the 2k+1
+//     points do (D, degree 2k+3, is exact on the NC points too).  The results
+//     agree to rounding with 25 and 49 points instead of 81 at k = 4.  The face
+//     terms of C hold the upwind speed max |w.n|, which is no polynomial: they
+//     keep the 2k+1 points.  The face terms of B (degree 2k+1) take k+1.
+//   * Idle lanes cost as much as busy ones.  Every 1D contraction is done for
+//     a whole row, column or face by one thread, with the even-odd split of
+//     the symmetric point sets and compile-time coefficients, and the tasks of
+//     a phase are dealt out over the threads of the block so that warps are
+//     full: (cell, row), (cell, column), (cell, face), (cell, row of A^{-1}).
+//
+// Geometry enters as products tabulated once per mesh (k_exact_tables): the
+// cofactors times the quadrature weight per point, four values together, and
+// the outward normal times the face weight, each with the equation's constant
+// factors.  p_fix enters C as H = gamma/(gamma-1) p_fix cof per point and as
+// its face traces, prepared when p_fix is set.
+//
+// Measured on GB300 at 51,200 cells, k = 4, FP64 (before: the kernels of
+// schur_kernels.cuh, 2k+1 points everywhere, 9 threads per cell): B with A^{-1}
+// 0.56 -> 0.28 ms, C/D 0.55 -> 0.33 ms, the FP64 pipe busy 83-86% in both; the
+// FP32 V-cycle 1.53 -> 0.97 ms.
+//
+// In the Schur apply, B stores w = cB cC A^{-1} B p and C/D applies C with unit
+// coefficient: C is homogeneous of degree one in w for the positive cC
+// (the upwind speed scales with w).
+#pragma once
+#include "device_util.cuh"
+
+namespace atm {
+
+template <int K>
+struct Ex {
+  static constexpr int NN = K + 1, NN2 = NN * NN;
+  static constexpr int NQ = 2 * K + 1;         // face points of C
+  static constexpr int NC = (3 * K + 3) / 2;   // volume points per direction of C and D
+  static constexpr int NC2 = NC * NC;
+};
+
+// Even-odd halves of the 1D tables of one point set: [kind][q][i] for
+// q < ceil(NP/2), i < ceil(NN/2), kind 0 E_S, 1 O_S, 2 E_D, 3 O_D with
+// E = (M(q,i) + M(q,k-i)) / 2 and O = (M(q,i) - M(q,k-i)) / 2.  Sets: 0 the
+// k+1, 1 the NC, 2 the 2k+1 Gauss points.
+constexpr int EO_Q = 6, EO_I = 3, EO_SETS = 3;
+static __constant__ double c_eo[KMAX + 1][EO_SETS][4][EO_Q][EO_I];
+static __constant__ float c_eo_f[KMAX + 1][EO_SETS][4][EO_Q][EO_I];
+// basis values at the subface points (g_q + s)/2 of hanging faces:
+// [k][0: the k+1 points, 1: the 2k+1 points][s][q][i]
+static __constant__ double c_sub[KMAX + 1][2][2][NQ_MAX][NN_MAX];
+static __constant__ float c_sub_f[KMAX + 1][2][2][NQ_MAX][NN_MAX];
+constexpr int EO_DOUBLES = (KMAX + 1) * EO_SETS * 4 * EO_Q * EO_I;
+constexpr int SUB_DOUBLES = (KMAX + 1) * 4 * NQ_MAX * NN_MAX;
+
+// `table`: c_eo followed by c_sub (make_exact_basis)
+static inline int upload_exact_here(const double *table) {
+  std::vector<float> f(table, table + EO_DOUBLES + SUB_DOUBLES);
+  if (cudaMemcpyToSymbol(c_eo, table, sizeof(c_eo)) != cudaSuccess) return 1;
+  if (cudaMemcpyToSymbol(c_sub, table + EO_DOUBLES, sizeof(c_sub)) != cudaSuccess) return 1;
+  if (cudaMemcpyToSymbol(c_eo_f, f.data(), sizeof(c_eo_f)) != cudaSuccess) return 1;
+  return cudaMemcpyToSymbol(c_sub_f, f.data() + EO_DOUBLES, sizeof(c_sub_f)) == cudaSuccess ? 0 : 1;
+}
+
+template <typename T>
+struct CEo;
+template <>
+struct CEo<double> {
+  static __device__ __forceinline__ double get(int k, int s, int w, int q, int i) {
+    return c_eo[k][s][w][q][i];
+  }
+  static __device__ __forceinline__ double sub(int k, int p, int s, int q, int i) {
+    return c_sub[k][p][s][q][i];
+  }
+};
+template <>
+struct CEo<float> {
+  static __device__ __forceinline__ float get(int k, int s, int w, int q, int i) {
+    return c_eo_f[k][s][w][q][i];
+  }
+  static __device__ __forceinline__ float sub(int k, int p, int s, int q, int i) {
+    return c_sub_f[k][p][s][q][i];
+  }
+};
+
+// v_q = sum_i S(q,i) t_i
+template <int K, int SET, int NP, typename T>
+__device__ __forceinline__ void eo_interp(const T (&t)[K + 1], T (&v)[NP]) {
+  constexpr int H = (K + 1) / 2, P = NP / 2;
+  constexpr bool MI = ((K + 1) & 1) != 0, MQ = (NP & 1) != 0;
+  T te[H], to[H];
+#pragma unroll
+  for (int i = 0; i < H; ++i) {
+    te[i] = t[i] + t[K - i];
+    to[i] = t[i] - t[K - i];
+  }
+#pragma unroll
+  for (int q = 0; q < P; ++q) {
+    T e = CEo<T>::get(K, SET, 0, q, 0) * te[0], o = CEo<T>::get(K, SET, 1, q, 0) * to[0];
+#pragma unroll
+    for (int i = 1; i < H; ++i) {
+      e = fma(CEo<T>::get(K, SET, 0, q, i), te[i], e);
+      o = fma(CEo<T>::get(K, SET, 1, q, i), to[i], o);
+    }
+    if (MI) e = fma(CEo<T>::get(K, SET, 0, q, H), t[H], e);
+    v[q] = e + o;
+    v[NP - 1 - q] = e - o;
+  }
+  if (MQ) {
+    T e = CEo<T>::get(K, SET, 0, P, 0) * te[0];
+#pragma unroll
+    for (int i = 1; i < H; ++i) e = fma(CEo<T>::get(K, SET, 0, P, i), te[i], e);
+    if (MI) e = fma(CEo<T>::get(K, SET, 0, P, H), t[H], e);
+    v[P] = e;
+  }
+}
+
+// out_i = sum_q S(q,i) V_q + D(q,i) G_q
+template <int K, int SET, int NP, bool HAS_V, bool HAS_G, typename T>
+__device__ __forceinline__ void eo_integ(const T (&V)[NP], const T (&G)[NP], T (&out)[K + 1]) {
+  static_assert(HAS_V || HAS_G, "nothing to integrate");
+  constexpr int H = (K + 1) / 2, P = NP / 2;
+  constexpr bool MI = ((K + 1) & 1) != 0, MQ = (NP & 1) != 0;
+  T ve[P], vo[P], ge[P], go[P];
+#pragma unroll
+  for (int q = 0; q < P; ++q) {
+    if (HAS_V) {
+      ve[q] = V[q] + V[NP - 1 - q];
+      vo[q] = V[q] - V[NP - 1 - q];
+    }
+    if (HAS_G) {
+      ge[q] = G[q] + G[NP - 1 - q];
+      go[q] = G[q] - G[NP - 1 - q];
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < H; ++i) {
+    T e = HAS_V ? CEo<T>::get(K, SET, 0, 0, i) * ve[0] : CEo<T>::get(K, SET, 2, 0, i) * go[0];
+    T o = HAS_V ? CEo<T>::get(K, SET, 1, 0, i) * vo[0] : CEo<T>::get(K, SET, 3, 0, i) * ge[0];
+    if (HAS_V && HAS_G) {
+      e = fma(CEo<T>::get(K, SET, 2, 0, i), go[0], e);
+      o = fma(CEo<T>::get(K, SET, 3, 0, i), ge[0], o);
+    }
+#pragma unroll
+    for (int q = 1; q < P; ++q) {
+      if (HAS_V) {
+        e = fma(CEo<T>::get(K, SET, 0, q, i), ve[q], e);
+        o = fma(CEo<T>::get(K, SET, 1, q, i), vo[q], o);
+      }
+      if (HAS_G) {
+        e = fma(CEo<T>::get(K, SET, 2, q, i), go[q], e);
+        o = fma(CEo<T>::get(K, SET, 3, q, i), ge[q], o);
+      }
+    }
+    if (MQ && HAS_V) e = fma(CEo<T>::get(K, SET, 0, P, i), V[P], e);
+    if (MQ && HAS_G) o = fma(CEo<T>::get(K, SET, 3, P, i), G[P], o);
+    out[i] = e + o;
+    out[K - i] = e - o;
+  }
+  if (MI) {  // i = k/2: O_S = O_D = 0 and D(mid, k/2) = 0
+    T e = HAS_V ? CEo<T>::get(K, SET, 0, 0, H) * ve[0] : CEo<T>::get(K, SET, 2, 0, H) * go[0];
+    if (HAS_V && HAS_G) e = fma(CEo<T>::get(K, SET, 2, 0, H), go[0], e);
+#pragma unroll
+    for (int q = 1; q < P; ++q) {
+      if (HAS_V) e = fma(CEo<T>::get(K, SET, 0, q, H), ve[q], e);
+      if (HAS_G) e = fma(CEo<T>::get(K, SET, 2, q, H), go[q], e);
+    }
+    if (MQ && HAS_V) e = fma(CEo<T>::get(K, SET, 0, P, H), V[P], e);
+    out[H] = e;
+  }
+}
+
+// max(|a|, |b|) on the integer pipe for doubles (a double comparison takes an
+// FP64 issue slot); a NaN on either side gives a NaN
+__device__ __forceinline__ double abs_max(double a, double b) {
+  const long long m = 0x7fffffffffffffffll;
+  const long long x = __double_as_longlong(a) & m, y = __double_as_longlong(b) & m;
+  return __longlong_as_double(x > y ? x : y);
+}
+__device__ __forceinline__ float abs_max(float a, float b) {
+  const int m = 0x7fffffff;
+  const int x = __float_as_int(a) & m, y = __float_as_int(b) & m;
+  return __int_as_float(x > y ? x : y);
+}
+
+template <typename T>
+struct Vec4;
+template <>
+struct Vec4<float> {
+  float v[4];
+  __device__ __forceinline__ explicit Vec4(const float *p) {  // 16-byte aligned
+    const float4 a = __ldg(reinterpret_cast<const float4 *>(p));
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+  }
+  __device__ __forceinline__ void store(float *p) const {
+    *reinterpret_cast<float4 *>(p) = make_float4(v[0], v[1], v[2], v[3]);
+  }
+};
+template <>
+struct Vec4<double> {
+  double v[4];
+  __device__ __forceinline__ explicit Vec4(const double *p) {  // 16-byte aligned
+    const double2 a = __ldg(reinterpret_cast<const double2 *>(p));
+    const double2 b = __ldg(reinterpret_cast<const double2 *>(p) + 1);
+    v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
+  }
+  __device__ __forceinline__ void store(double *p) const {
+    reinterpret_cast<double2 *>(p)[0] = make_double2(v[0], v[1]);
+    reinterpret_cast<double2 *>(p)[1] = make_double2(v[2], v[3]);
+  }
+};
+__device__ __forceinline__ void load2(const float *p, float &a, float &b) {  // 8-byte aligned
+  const float2 x = __ldg(reinterpret_cast<const float2 *>(p));
+  a = x.x; b = x.y;
+}
+__device__ __forceinline__ void load2(const double *p, double &a, double &b) {  // 16-byte
+  const double2 x = __ldg(reinterpret_cast<const double2 *>(p));
+  a = x.x; b = x.y;
+}
+
+// nodal trace of a cell's field on face f
+template <int K, typename T>
+__device__ __forceinline__ void trace(const T *__restrict__ cell, int f, T (&t)[K + 1]) {
+  constexpr int NN = K + 1;
+  const T *b = cell + (f == 1 ? K : f == 3 ? K * NN : 0);
+  const int st = f < 2 ? NN : 1;
+#pragma unroll
+  for (int i = 0; i < NN; ++i) t[i] = __ldg(b + i * st);
+}
+// the same trace at the points of subface s (point set PS: 0 k+1, 1 2k+1)
+template <int K, int PS, int NP, typename T>
+__device__ __forceinline__ void sub_interp(const T (&t)[K + 1], int s, T (&v)[NP]) {
+  for (int q = 0; q < NP; ++q) {
+    T a = CEo<T>::sub(K, PS, s, q, 0) * t[0];
+#pragma unroll
+    for (int i = 1; i <= K; ++i) a = fma(CEo<T>::sub(K, PS, s, q, i), t[i], a);
+    v[q] = a;
+  }
+}
+template <int K, int PS, int NP, typename T>
+__device__ __forceinline__ void sub_integ_add(const T (&F)[NP], int s, T (&out)[K + 1]) {
+#pragma unroll
+  for (int i = 0; i <= K; ++i)
+    for (int q = 0; q < NP; ++q) out[i] = fma(CEo<T>::sub(K, PS, s, q, i), F[q], out[i]);
+}
+
+// trace of a cell's field at the 2k+1 points of face f (sub < 0) or of its
+// subface `sub`
+template <int K, int NP, typename T>
+__device__ __forceinline__ void own_or_sub(const T *__restrict__ cell, int f, int sub, T (&v)[NP]) {
+  T t[K + 1];
+  trace<K>(cell, f, t);
+  if (sub < 0) eo_interp<K, 2>(t, v);
+  else sub_interp<K, 1>(t, sub, v);
+}
+
+// flux of C at a face point, times the face weight: half gamma/(gamma-1)
+// (a un+ + b un-) plus the upwind jump max |un| (a - b) / (2 (gamma-1)), with
+// a, b the p_fix traces and g the normal times the weight times half
+// gamma/(gamma-1)
+template <typename T>
+__device__ __forceinline__ T flux_C(const T *__restrict__ g, T wx, T wz, T vx, T vz, T a, T b) {
+  T n0, n1;
+  load2(g, n0, n1);
+  const T up = fma(wx, n0, wz * n1), um = fma(vx, n0, vz * n1);
+  return fma(abs_max(up, um), (a - b) * T(1.0 / GAS_GAMMA), fma(a, up, b * um));
+}
+
+// face contributions of the output row iz: faces x = 0, 1 add to the row's
+// ends, faces z = 0, 1 to the whole first and last row.  F: [4][NN]
+template <int K, typename T>
+__device__ __forceinline__ void face_rows(const T *__restrict__ F, int iz, T (&add)[K + 1]) {
+  constexpr int NN = K + 1;
+  const T *Fz = iz == 0 ? F + 2 * NN : F + 3 * NN;
+  const bool edge = iz == 0 || iz == K;
+#pragma unroll
+  for (int i = 0; i < NN; ++i) add[i] = edge ? Fz[i] : T(0);
+  add[0] += F[iz];
+  add[K] += F[NN + iz];
+}
+
+// ====================================================================== B ===
+// MODE 0: dst = cB B p ; 1: dst -= cB B p ; 2: dst = cB cC A^{-1} B p
+// (with a per-cell time-step multiplier d: cB d and cC d).
+// Threads (cell, j), j < k+1; `cpb` cells per block.
+template <int K, int MODE, typename T, bool HG>
+__global__ void __launch_bounds__(192)
+    k_exact_B(T *__restrict__ dst, const T *__restrict__ p, T cB, T cC,
+              const T *__restrict__ ainv, MeshT<T> mesh, int cpb) {
+  constexpr int NN = K + 1, NN2 = NN * NN;
+  constexpr bool STAGE = MODE == 2 && sizeof(T) == 4;
+  constexpr int AS = ainv_stride<K, T>();
+  extern __shared__ __align__(16) unsigned char sm_raw[];
+  T *sm = reinterpret_cast<T *>(sm_raw);
+  T *as = sm;                                  // [cpb][AS] staged A^{-1} (STAGE)
+  T *Xs = sm + (STAGE ? cpb * AS : 0);         // [cpb][NN2] x-interpolated p
+  T *Y = Xs + cpb * NN2;                       // [cpb][2 comp][2][NN2]
+  T *Fs = Y + cpb * 4 * NN2;                   // [cpb][2 comp][4][NN]
+  const int tid = threadIdx.x, lc = tid / NN, j = tid - lc * NN;
+  const int c0 = blockIdx.x * cpb;
+  const int cnt = min(cpb, mesh.nc - c0);
+  if constexpr (STAGE) {
+    // cells c0 .. c0+cnt-1: cnt * AS values, 16-byte aligned (AS % 4 == 0);
+    // they arrive while B is computed
+    const T *src = ainv + (long)c0 * AS;
+    const int n16 = cnt * AS / 4;
+    for (int e = tid; e < n16; e += blockDim.x) cp_async16(as + 4 * e, src + 4 * e);
+    cp_async_commit();
+  }
+  const bool active = lc < cnt;
+  const int c = c0 + lc;
+  if (active) {
+    // row j: x-interpolation to the k+1 Gauss points
+    {
+      T t[NN], v[NN];
+      const T *row = p + (long)c * NN2 + j * NN;
+#pragma unroll
+      for (int i = 0; i < NN; ++i) t[i] = __ldg(row + i);
+      eo_interp<K, 0>(t, v);
+#pragma unroll
+      for (int i = 0; i < NN; ++i) Xs[lc * NN2 + j * NN + i] = v[i];
+    }
+    // faces j, j + NN, ...: fB holds half the outward normal times the weight
+    for (int f = j; f < 4; f += NN) {
+      const int nb = mesh.nbr[c * 4 + f], nfc = mesh.nbrf[c * 4 + f];
+      const int code = HG && nb >= 0 ? nfc >> 2 : 0;
+      T own[NN], o0[NN], o1[NN];
+      trace<K>(p + (long)c * NN2, f, own);
+      if (!HG || code < 3) {
+        T nbt[NN], s[NN], F0[NN], F1[NN];
+        if (nb >= 0) {
+          trace<K>(p + (long)nb * NN2, nfc & 3, nbt);
+        } else {  // wall, p_D = p
+#pragma unroll
+          for (int i = 0; i < NN; ++i) nbt[i] = own[i];
+        }
+        if (!HG || code == 0) {
+#pragma unroll
+          for (int i = 0; i < NN; ++i) nbt[i] += own[i];
+          eo_interp<K, 0>(nbt, s);
+        } else {  // fine side: the coarse neighbour at the shifted points
+          T sn[NN];
+          eo_interp<K, 0>(own, s);
+          sub_interp<K, 0>(nbt, code - 1, sn);
+#pragma unroll
+          for (int q = 0; q < NN; ++q) s[q] += sn[q];
+        }
+        const T *g = mesh.fB + ((long)c * 4 + f) * 2 * NN;
+#pragma unroll
+        for (int q = 0; q < NN; ++q) {
+          T n0, n1;
+          load2(g + 2 * q, n0, n1);
+          F0[q] = n0 * s[q];
+          F1[q] = n1 * s[q];
+        }
+        eo_integ<K, 0, NN, true, false>(F0, F0, o0);
+        eo_integ<K, 0, NN, true, false>(F1, F1, o1);
+      } else {  // coarse side: two subfaces
+#pragma unroll
+        for (int i = 0; i < NN; ++i) o0[i] = o1[i] = T(0);
+        for (int h = 0; h < 2; ++h) {
+          T nbt[NN], s[NN], sn[NN], F0[NN], F1[NN];
+          trace<K>(p + (long)mesh.hnb[nb * 2 + h] * NN2, nfc & 3, nbt);
+          sub_interp<K, 0>(own, h, s);
+          eo_interp<K, 0>(nbt, sn);
+          const T *g = mesh.hB + ((long)nb * 2 + h) * 2 * NN;
+#pragma unroll
+          for (int q = 0; q < NN; ++q) {
+            T n0, n1;
+            load2(g + 2 * q, n0, n1);
+            s[q] += sn[q];
+            F0[q] = n0 * s[q];
+            F1[q] = n1 * s[q];
+          }
+          sub_integ_add<K, 0>(F0, h, o0);
+          sub_integ_add<K, 0>(F1, h, o1);
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < NN; ++i) {
+        Fs[((lc * 2 + 0) * 4 + f) * NN + i] = o0[i];
+        Fs[((lc * 2 + 1) * 4 + f) * NN + i] = o1[i];
+      }
+    }
+  }
+  __syncthreads();
+  if (active) {
+    // column j: z-interpolation, fluxes, z-integration
+    T t[NN], v[NN];
+#pragma unroll
+    for (int i = 0; i < NN; ++i) t[i] = Xs[lc * NN2 + i * NN + j];
+    eo_interp<K, 0>(t, v);
+    const T *g = mesh.gB + ((long)c * NN + j) * NN * 4;
+    T G[4][NN];
+#pragma unroll
+    for (int q = 0; q < NN; ++q) {
+      const Vec4<T> w(g + 4 * q);  // -cof of (xi, eta) for x, then for z
+#pragma unroll
+      for (int d = 0; d < 4; ++d) G[d][q] = w.v[d] * v[q];
+    }
+#pragma unroll
+    for (int comp = 0; comp < 2; ++comp) {
+      T a[NN], b[NN];
+      eo_integ<K, 0, NN, false, true>(G[2 * comp + 1], G[2 * comp + 1], a);
+      eo_integ<K, 0, NN, true, false>(G[2 * comp], G[2 * comp], b);
+      T *y = Y + (lc * 2 + comp) * 2 * NN2 + j;
+#pragma unroll
+      for (int i = 0; i < NN; ++i) {
+        y[i * NN] = a[i];
+        y[NN2 + i * NN] = b[i];
+      }
+    }
+  }
+  __syncthreads();
+  if (active) {
+    // output row j; MODE 2 leaves it in place of its own Y row (nobody else
+    // reads that row)
+    T s = MODE == 2 ? cB * cC : cB;
+    if (mesh.dts) {
+      const T d = mesh.dts[c];
+      s *= MODE == 2 ? d * d : d;
+    }
+#pragma unroll
+    for (int comp = 0; comp < 2; ++comp) {
+      T *y = Y + (lc * 2 + comp) * 2 * NN2 + j * NN;
+      T a[NN], b[NN], out[NN], add[NN];
+#pragma unroll
+      for (int i = 0; i < NN; ++i) {
+        a[i] = y[i];
+        b[i] = y[NN2 + i];
+      }
+      eo_integ<K, 0, NN, true, true>(a, b, out);
+      face_rows<K>(Fs + (lc * 2 + comp) * 4 * NN, j, add);
+      T *d = dst + ((long)c * 2 + comp) * NN2 + j * NN;
+#pragma unroll
+      for (int i = 0; i < NN; ++i) {
+        const T o = s * (out[i] + add[i]);
+        if (MODE == 2) y[i] = o;
+        else if (MODE == 1) d[i] -= o;
+        else d[i] = o;
+      }
+    }
+  }
+  if constexpr (MODE == 2) {
+    if constexpr (STAGE) cp_async_wait_all();
+    __syncthreads();
+    // rows (cell, i) of A^{-1}, NN per thread: consecutive threads read
+    // consecutive values of the cell's (symmetric) block
+    for (int e = tid; e < cnt * NN2; e += blockDim.x) {
+      const int l = e / NN2, i = e - l * NN2;
+      const T *b0 = Y + l * 4 * NN2, *b1 = b0 + 2 * NN2;
+      T s0 = T(0), s1 = T(0);
+      if constexpr (STAGE) {
+        // packed lower triangle: A_ij at i(i+1)/2 + j (j <= i), else j(j+1)/2 + i
+        const T *Ab = as + l * AS;
+        const int ri = i * (i + 1) / 2;
+#pragma unroll
+        for (int jj = 0; jj < NN2; ++jj) {
+          const T a = jj <= i ? Ab[ri + jj] : Ab[jj * (jj + 1) / 2 + i];
+          s0 = fma(a, b0[jj], s0);
+          s1 = fma(a, b1[jj], s1);
+        }
+      } else {
+        const T *Ab = ainv + (long)(c0 + l) * AS + i;
+#pragma unroll
+        for (int jj = 0; jj < NN2; ++jj) {
+          const T a = __ldg(Ab + jj * NN2);
+          s0 = fma(a, b0[jj], s0);
+          s1 = fma(a, b1[jj], s1);
+        }
+      }
+      T *d = dst + (long)(c0 + l) * 2 * NN2 + i;
+      d[0] = s0;
+      d[NN2] = s1;
+    }
+  }
+}
+
+// ===================================================================== CD ===
+// MODE 0: dst = cC C w ; 3: dst -= cC C w
+// MODE 1: dst = D p - C w ; 2: dst = invd .* (D p - C w)
+// MODE 4: t = D p - C w with p = ch.x, then the Chebyshev update of ch
+// Threads (cell, column), column < NC; `cpb` cells per block, a multiple of 8.
+template <int K, int MODE, typename T, bool HG>
+__global__ void __launch_bounds__(288)
+    k_exact_CD(T *__restrict__ dst, const T *__restrict__ w, const T *__restrict__ p,
+               const T *__restrict__ pfix, const T *__restrict__ hq, const T *__restrict__ pff,
+               T cC, const T *__restrict__ invd, MeshT<T> mesh, ChebArgs<T> ch, int cpb) {
+  using E = Ex<K>;
+  constexpr int NN = E::NN, NN2 = E::NN2, NC = E::NC, NC2 = E::NC2, NQ = E::NQ;
+  constexpr bool WITH_D = MODE == 1 || MODE == 2 || MODE == 4;
+  constexpr int NF = WITH_D ? 3 : 2;
+  constexpr int XS = NN * NC;
+  extern __shared__ __align__(16) unsigned char sm_raw[];
+  T *X = reinterpret_cast<T *>(sm_raw);  // [cpb][NF][NN][NC] x-interpolated w, p; then xa, xb
+  T *Fs = X + cpb * NF * XS;             // [cpb][4][NN] face integrals of C w
+  const int tid = threadIdx.x, nt = blockDim.x;
+  const int c0 = blockIdx.x * cpb;
+  const int cnt = min(cpb, mesh.nc - c0);
+  // faces: one thread per (cell, face); with NC > 4 the first 4 cpb threads
+  // (whole warps) take them while the others interpolate the rows
+  for (int e = tid; e < 4 * cnt; e += nt) {
+    const int l = e >> 2, f = e & 3, c = c0 + l;
+    const int nb = mesh.nbr[c * 4 + f], nfc = mesh.nbrf[c * 4 + f];
+    const int code = HG && nb >= 0 ? nfc >> 2 : 0;
+    const T *wc = w + (long)c * 2 * NN2;
+    T o[NN];
+    if (nb < 0) {
+#pragma unroll
+      for (int i = 0; i < NN; ++i) o[i] = T(0);
+    } else if (!HG || code == 0) {
+      T t[NN], wx[NQ], wz[NQ], vx[NQ], vz[NQ], F[NQ];
+      const T *wn = w + (long)nb * 2 * NN2;
+      trace<K>(wc, f, t);
+      eo_interp<K, 2>(t, wx);
+      trace<K>(wc + NN2, f, t);
+      eo_interp<K, 2>(t, wz);
+      trace<K>(wn, nfc & 3, t);
+      eo_interp<K, 2>(t, vx);
+      trace<K>(wn + NN2, nfc & 3, t);
+      eo_interp<K, 2>(t, vz);
+      const T *hp = pff + ((long)c * 4 + f) * NQ, *hm = pff + ((long)nb * 4 + (nfc & 3)) * NQ;
+      const T *g = mesh.fC + ((long)c * 4 + f) * 2 * NQ;
+#pragma unroll
+      for (int q = 0; q < NQ; ++q)
+        F[q] = flux_C(g + 2 * q, wx[q], wz[q], vx[q], vz[q], __ldg(hp + q), __ldg(hm + q));
+      eo_integ<K, 2, NQ, true, false>(F, F, o);
+    } else {
+#pragma unroll
+      for (int i = 0; i < NN; ++i) o[i] = T(0);
+      // fine side (code 1, 2): one face, the neighbour at the shifted points;
+      // coarse side (code 3): two subfaces, this cell at the shifted points
+      for (int h = 0; h < (code == 3 ? 2 : 1); ++h) {
+        const int nc = code == 3 ? mesh.hnb[nb * 2 + h] : nb;
+        const T *wn = w + (long)nc * 2 * NN2;
+        T wx[NQ], wz[NQ], vx[NQ], vz[NQ], a[NQ], b[NQ], F[NQ];
+        own_or_sub<K>(wc, f, code == 3 ? h : -1, wx);
+        own_or_sub<K>(wc + NN2, f, code == 3 ? h : -1, wz);
+        own_or_sub<K>(pfix + (long)c * NN2, f, code == 3 ? h : -1, a);
+        own_or_sub<K>(wn, nfc & 3, code == 3 ? -1 : code - 1, vx);
+        own_or_sub<K>(wn + NN2, nfc & 3, code == 3 ? -1 : code - 1, vz);
+        own_or_sub<K>(pfix + (long)nc * NN2, nfc & 3, code == 3 ? -1 : code - 1, b);
+        const T *g = code == 3 ? mesh.hC + ((long)nb * 2 + h) * 2 * NQ
+                               : mesh.fC + ((long)c * 4 + f) * 2 * NQ;
+#pragma unroll
+        for (int q = 0; q < NQ; ++q)
+          F[q] = flux_C(g + 2 * q, wx[q], wz[q], vx[q], vz[q], a[q], b[q]);
+        if (code == 3) {
+          sub_integ_add<K, 1>(F, h, o);
+        } else {
+          eo_integ<K, 2, NQ, true, false>(F, F, o);
+        }
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < NN; ++i) Fs[(l * 4 + f) * NN + i] = o[i];
+  }
+  // rows (cell, field, iz): x-interpolation to the NC points
+  {
+    constexpr bool SPLIT = NC > 4;
+    const int first = SPLIT ? 4 * cpb : 0, stride = nt - first;
+    for (int e = tid - first; e >= 0 && e < cnt * NF * NN; e += stride) {
+      const int l = e / (NF * NN), r = e - l * (NF * NN);
+      const T *row = r < 2 * NN ? w + ((long)(c0 + l) * 2 * NN + r) * NN
+                                : p + ((long)(c0 + l) * NN + (r - 2 * NN)) * NN;
+      T t[NN], v[NC];
+#pragma unroll
+      for (int i = 0; i < NN; ++i) t[i] = row[i];
+      eo_interp<K, 1>(t, v);
+#pragma unroll
+      for (int q = 0; q < NC; ++q) X[l * NF * XS + r * NC + q] = v[q];
+    }
+  }
+  __syncthreads();
+  // columns: z-interpolation, fluxes, z-integration; xa and xb replace the
+  // column's own x-interpolated values
+  {
+    const int l = tid / NC, j = tid - l * NC;
+    if (l < cnt) {
+      T *x = X + l * NF * XS + j;
+      T t[NN], wx[NC], wz[NC], V[NC], Gx[NC], Ge[NC];
+#pragma unroll
+      for (int i = 0; i < NN; ++i) t[i] = x[i * NC];
+      eo_interp<K, 1>(t, wx);
+#pragma unroll
+      for (int i = 0; i < NN; ++i) t[i] = x[XS + i * NC];
+      eo_interp<K, 1>(t, wz);
+      if (WITH_D) {
+        const T *jx = mesh.gJ + ((long)(c0 + l) * NC + j) * NC;
+#pragma unroll
+        for (int i = 0; i < NN; ++i) t[i] = x[2 * XS + i * NC];
+        eo_interp<K, 1>(t, V);
+#pragma unroll
+        for (int q = 0; q < NC; ++q) V[q] *= __ldg(jx + q);
+      }
+      const T *h = hq + ((long)(c0 + l) * NC + j) * NC * 4;
+#pragma unroll
+      for (int q = 0; q < NC; ++q) {
+        const Vec4<T> H(h + 4 * q);  // (xi, eta) from w_x, then from w_z
+        Gx[q] = fma(H.v[0], wx[q], H.v[2] * wz[q]);
+        Ge[q] = fma(H.v[1], wx[q], H.v[3] * wz[q]);
+      }
+      T a[NN], b[NN];
+      eo_integ<K, 1, NC, WITH_D, true>(V, Ge, a);
+      eo_integ<K, 1, NC, true, false>(Gx, Gx, b);
+#pragma unroll
+      for (int i = 0; i < NN; ++i) {
+        x[i * NC] = a[i];
+        x[XS + i * NC] = b[i];
+      }
+    }
+  }
+  __syncthreads();
+  // output rows: D p - C w
+  for (int e = tid; e < cnt * NN; e += nt) {
+    const int l = e / NN, iz = e - l * NN;
+    const T *x = X + l * NF * XS + iz * NC;
+    T a[NC], b[NC], out[NN], add[NN];
+#pragma unroll
+    for (int q = 0; q < NC; ++q) {
+      a[q] = x[q];
+      b[q] = x[XS + q];
+    }
+    eo_integ<K, 1, NC, true, true>(a, b, out);
+    face_rows<K>(Fs + l * 4 * NN, iz, add);
+    const long g0 = (long)(c0 + l) * NN2 + iz * NN;
+    T s = cC;
+    if (!WITH_D && mesh.dts) s *= mesh.dts[c0 + l];
+#pragma unroll
+    for (int i = 0; i < NN; ++i) {
+      const T r = out[i] - add[i];
+      const long g = g0 + i;
+      if (MODE == 0) dst[g] = -s * r;
+      else if (MODE == 1) dst[g] = r;
+      else if (MODE == 2) dst[g] = invd[g] * r;
+      else if (MODE == 3) dst[g] += s * r;
+      else {
+        const T res = ch.rhs[g] - r;
+        const T dk = (ch.first ? T(0) : ch.a * ch.d[g]) + ch.b * invd[g] * res;
+        ch.d[g] = dk;
+        ch.x[g] += dk;
+      }
+    }
+  }
+}
+
+// ========================================================== p_fix prep ===
+// H = gamma/(gamma-1) p_fix cof at the NC x NC points ([c][qx][qz][4]) and the
+// face traces of p_fix at the 2k+1 points.  Threads (cell, column).  Bound by
+// its stores at large meshes (1,568 + 288 bytes per cell at k = 4 in FP64).
+template <int K, typename T>
+__global__ void __launch_bounds__(32 * Ex<K>::NC)
+    k_exact_pfix(T *__restrict__ hq, T *__restrict__ pff, const T *__restrict__ pfix,
+                 MeshT<T> mesh, int cpb) {
+  using E = Ex<K>;
+  constexpr int NN = E::NN, NN2 = E::NN2, NC = E::NC, NQ = E::NQ;
+  extern __shared__ __align__(16) unsigned char sm_raw[];
+  T *X = reinterpret_cast<T *>(sm_raw);  // [cpb][NN][NC]
+  const int tid = threadIdx.x, nt = blockDim.x;
+  const int c0 = blockIdx.x * cpb;
+  const int cnt = min(cpb, mesh.nc - c0);
+  for (int e = tid; e < cnt * NN; e += nt) {
+    T t[NN], v[NC];
+#pragma unroll
+    for (int i = 0; i < NN; ++i) t[i] = __ldg(pfix + ((long)c0 * NN + e) * NN + i);
+    eo_interp<K, 1>(t, v);
+#pragma unroll
+    for (int q = 0; q < NC; ++q) X[e * NC + q] = v[q];
+  }
+  for (int e = tid; e < cnt * 4; e += nt) {
+    T t[NN], v[NQ];
+    trace<K>(pfix + (long)(c0 + (e >> 2)) * NN2, e & 3, t);
+    eo_interp<K, 2>(t, v);
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) pff[((long)c0 * 4 + e) * NQ + q] = v[q];
+  }
+  __syncthreads();
+  const int l = tid / NC, j = tid - l * NC;
+  if (l >= cnt) return;
+  T t[NN], v[NC];
+#pragma unroll
+  for (int i = 0; i < NN; ++i) t[i] = X[(l * NN + i) * NC + j];
+  eo_interp<K, 1>(t, v);
+  const long o = ((long)(c0 + l) * NC + j) * NC * 4;
+#pragma unroll
+  for (int q = 0; q < NC; ++q) {
+    Vec4<T> g(mesh.gC + o + 4 * q);
+#pragma unroll
+    for (int d = 0; d < 4; ++d) g.v[d] *= v[q];
+    g.store(hq + o + 4 * q);
+  }
+}
+
+// ============================================================ launchers ===
+// The autotuner's cells per block, rounded up to a multiple of 8 so that the
+// face threads of C/D fill whole warps.
+inline int exact_cells(int cpb) { return (cpb + 7) / 8 * 8; }
+
+template <int K, typename T, bool HG>
+int exact_B_launch(const OpView<T> &v, T *dst, const T *p, T cB, T cC, int mode) {
+  constexpr int NN = K + 1, NN2 = NN * NN;
+  auto launch = [&](int tuned) -> cudaError_t {
+    int cpb = exact_cells(tuned);
+    if (cpb * NN > 192) cpb = 192 / NN / 8 * 8;
+    const size_t sm = sizeof(T) * (size_t)cpb *
+                      (5 * NN2 + 8 * NN + (mode == 2 && sizeof(T) == 4 ? ainv_stride<K, T>() : 0));
+    void (*fn)(T *, const T *, T, T, const T *, MeshT<T>, int) =
+        mode == 0 ? k_exact_B<K, 0, T, HG>
+                  : (mode == 1 ? k_exact_B<K, 1, T, HG> : k_exact_B<K, 2, T, HG>);
+    if (cudaError_t e = allow_smem(fn, sm); e != cudaSuccess) return e;
+    fn<<<(v.nc + cpb - 1) / cpb, cpb * NN, sm, v.st>>>(dst, p, cB, cC, v.ainv, v.mesh, cpb);
+    return cudaGetLastError();
+  };
+  // mode 1 (dst -= B p) is not idempotent: it uses the choice made for mode 0
+  const int cpb = tuned_cpb(v.tune, v.st, TF_B, K, mode == 1 ? 0 : mode, HG, (int)sizeof(T),
+                            v.nc, mode != 1 && dst != p, launch);
+  ATM_CUDA(launch(cpb));
+  g_kernel_launches.fetch_add(1);
+  return ATM_OK;
+}
+
+template <int K, typename T, bool HG>
+int exact_CD_launch(const OpView<T> &v, T *dst, const T *w, const T *p, T cC, int mode,
+                    const ChebArgs<T> *cheb) {
+  using E = Ex<K>;
+  const T *pfix = v.pfix;
+  const ChebArgs<T> ch = cheb ? *cheb : ChebArgs<T>{};
+  auto launch = [&](int tuned) -> cudaError_t {
+    int cpb = exact_cells(tuned);
+    if (cpb * E::NC > 288) cpb = 288 / E::NC / 8 * 8;
+    const size_t sm =
+        sizeof(T) * (size_t)cpb * ((mode == 0 || mode == 3 ? 2 : 3) * E::NN * E::NC + 4 * E::NN);
+    void (*fn)(T *, const T *, const T *, const T *, const T *, const T *, T, const T *, MeshT<T>,
+               ChebArgs<T>, int) = mode == 0   ? k_exact_CD<K, 0, T, HG>
+                                   : mode == 1 ? k_exact_CD<K, 1, T, HG>
+                                   : mode == 2 ? k_exact_CD<K, 2, T, HG>
+                                   : mode == 3 ? k_exact_CD<K, 3, T, HG>
+                                               : k_exact_CD<K, 4, T, HG>;
+    if (cudaError_t e = allow_smem(fn, sm); e != cudaSuccess) return e;
+    fn<<<(v.nc + cpb - 1) / cpb, cpb * E::NC, sm, v.st>>>(dst, w, p, pfix, v.pfq, v.pff, cC,
+                                                        v.invd, v.mesh, ch, cpb);
+    return cudaGetLastError();
+  };
+  // modes 3 (dst -= C w) and 4 (x += d) are not idempotent: they use the
+  // choices made for modes 0 and 1
+  const bool idem = mode < 3 && dst != w && dst != p && dst != pfix;
+  const int key = mode == 3 ? 0 : (mode == 4 ? 1 : mode);
+  const int cpb = tuned_cpb(v.tune, v.st, TF_CD, K, key, HG, (int)sizeof(T), v.nc, idem, launch);
+  ATM_CUDA(launch(cpb));
+  g_kernel_launches.fetch_add(1);
+  return ATM_OK;
+}
+
+template <int K, typename T>
+int exact_pfix_launch(const OpView<T> &v) {
+  using E = Ex<K>;
+  const int cpb = v.nc < 4096 ? 8 : 32;
+  k_exact_pfix<K, T><<<(v.nc + cpb - 1) / cpb, cpb * E::NC, sizeof(T) * cpb * E::NN * E::NC, v.st>>>(
+      const_cast<T *>(v.pfq), const_cast<T *>(v.pff), v.pfix, v.mesh, cpb);
+  ATM_CHECK_LAUNCH("k_exact_pfix");
+  return ATM_OK;
+}
+
+}  // namespace atm

@@ -5,6 +5,10 @@
 //   C   euler_operator.h:1413-1507
 //   D   euler_operator.h:1386-1408
 // HG selects the face loop with hanging faces (2:1 adaptive meshes).
+// These kernels integrate with 2k+1 points whatever the geometry; they serve
+// mappings of degree 3 and higher (and FP32 levels of such meshes), where no
+// smaller point set gives the same integrals.  Degree <= 2 runs
+// schur_exact.cuh.
 // Included by impl_kernels.cu (HG = false) and hang_rhs_*.cu / hang_schur.cu (HG = true).
 #pragma once
 #include "atm_device.cuh"
@@ -340,22 +344,6 @@ __global__ void __launch_bounds__(Cfg<K>::THREADS)
 }
 
 // ============================================================ launchers ===
-template <typename T>
-struct OpView {
-  int k, nc;
-  MeshT<T> mesh;
-  const T *ainv;
-  const T *invd;
-  cudaStream_t st;
-  bool tune;  // the autotuner may time tile shapes on this stream
-  const T *pfix, *pfq, *pff;  // frozen p_fix and its prepared values (C/D)
-};
-
-inline OpView<double> schur_view(const atm_ctx &c) {
-  return OpView<double>{c.k, c.nc, c.mesh, c.ainv, c.invdiag_D, c.stream,
-                        c.autotune && !c.capturing, c.pres_fix, c.pfq, c.pff};
-}
-
 template <int K, typename T, bool HG>
 int B_launch(const OpView<T> &v, T *dst, const T *p, T cB, int mode) {
   using C = Cfg<K>;
@@ -421,16 +409,5 @@ int CD_launch(const OpView<T> &v, T *dst, const T *w, const T *p, T cC, int mode
   g_kernel_launches.fetch_add(1);
   return ATM_OK;
 }
-
-#define ATM_DISPATCH_K(kk, call)          \
-  switch (kk) {                           \
-    case 1: { constexpr int K = 1; return call; } \
-    case 2: { constexpr int K = 2; return call; } \
-    case 3: { constexpr int K = 3; return call; } \
-    case 4: { constexpr int K = 4; return call; } \
-    case 5: { constexpr int K = 5; return call; } \
-    default: return ATM_BAD_ARG;          \
-  }
-
 
 }  // namespace atm

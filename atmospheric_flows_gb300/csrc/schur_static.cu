@@ -81,7 +81,7 @@ extern "C" int atm_schur_vmult_static_scratch(atm_handle h, double *dst, const d
   // earlier calls are used, otherwise the default blocks
   const bool tune = h->autotune;
   h->autotune = false;
-  rc = launch_B(*h, scratch, src, co * h->dt / (h->Ma * h->Ma), 2);
+  rc = launch_B(*h, scratch, src, co * h->dt / (h->Ma * h->Ma), 2, co * h->dt);
   if (rc == ATM_OK) rc = launch_CD(*h, dst, scratch, src, co * h->dt, 1);
   h->autotune = tune;
   return rc;

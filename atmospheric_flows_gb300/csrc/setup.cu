@@ -57,7 +57,7 @@ std::vector<double> gll_nodes(int k) {
   return x;
 }
 
-static void gauss_nodes(int n, std::vector<double> &x, std::vector<double> &w) {
+void gauss_nodes(int n, std::vector<double> &x, std::vector<double> &w) {
   x.resize(n);
   w.resize(n);
   for (int i = 0; i < n; ++i) {
@@ -158,7 +158,7 @@ int upload_basis_all() {
   if (upload_basis_rhs(tab.data()) || upload_basis_impl(tab.data()) ||
       upload_basis_hang_rho(tab.data()) || upload_basis_hang_vel(tab.data()) ||
       upload_basis_hang_pres(tab.data()) || upload_basis_hang_schur(tab.data()) ||
-      upload_basis_hang_schur_f(tab.data())) {
+      upload_basis_hang_schur_f(tab.data()) || upload_exact_all()) {
     set_error("failed to upload basis tables to constant memory");
     return ATM_CUDA_ERROR;
   }
@@ -167,6 +167,7 @@ int upload_basis_all() {
 }
 
 void mesh_free(Mesh &m) {
+  exact_mesh_free(m);
   cudaFree(m.qgeo);
   cudaFree(m.fgeo);
   cudaFree(m.nbr);
@@ -195,6 +196,8 @@ int build_mesh_tables(int k, int nc, int mapdeg, const double *nodes, int n_inne
   nbrf.assign((size_t)nc * 4, -1);
   std::vector<int> hidx((size_t)nc * 4, -1);
   out.hnb.clear();
+  out.hcf.clear();
+  out.exact = mapdeg <= 2;
   for (int f = 0; f < n_inner; ++f) {
     const int *e = inner + 5L * f;
     if (e[0] < 0 || e[0] >= nc || e[2] < 0 || e[2] >= nc || e[1] < 0 || e[1] > 3 ||
@@ -234,6 +237,7 @@ int build_mesh_tables(int k, int nc, int mapdeg, const double *nodes, int n_inne
           return ATM_BAD_ARG;
         }
         hidx[b] = (int)(out.hnb.size() / 2);
+        out.hcf.push_back((int)b);
         out.hnb.push_back(-1);
         out.hnb.push_back(-1);
         nbr[b] = hidx[b];
@@ -394,6 +398,8 @@ int mesh_upload(atm_ctx &c, int mapdeg, const double *nodes, int n_inner, const 
   Mesh &m = c.mesh;
   m.nc = nc; m.k = k; m.nn = nn; m.nq = nq; m.nn2 = nn * nn; m.nq2 = nq2;
   ATM_CUDA(cudaMalloc(&m.qgeo, hm.qgeo.size() * sizeof(double)));
+  m.jw = m.qgeo + 4 * nq2;
+  m.jw_stride = 5 * nq2;
   ATM_CUDA(cudaMalloc(&m.fgeo, hm.fgeo.size() * sizeof(double)));
   ATM_CUDA(cudaMalloc(&m.nbr, hm.nbr.size() * sizeof(int)));
   ATM_CUDA(cudaMalloc(&m.nbrf, hm.nbrf.size() * sizeof(int)));
@@ -411,10 +417,14 @@ int mesh_upload(atm_ctx &c, int mapdeg, const double *nodes, int n_inner, const 
   m.nhang = hm.nhang;
   c.mapdeg = mapdeg;
   c.map2 = std::move(hm.map2);
+  c.hcf = std::move(hm.hcf);
+  if (hm.exact && (rc = exact_mesh_build(m, c.map2.data(), c.hcf, c.stream))) return rc;
   rc = launch_block_inverse(c, m.minv, nullptr);
   if (rc) return rc;
   rc = launch_inv_diag(c, c.invdiag_D, 1, nullptr, 1.0 / (GAS_GAMMA - 1.0));
   if (rc) return rc;
+  // what C keeps of p_fix holds geometry: prepare it again on the new mesh
+  if ((rc = launch_pfix_prep(c))) return rc;
   ATM_CUDA(cudaStreamSynchronize(c.stream));
   return ATM_OK;
 }

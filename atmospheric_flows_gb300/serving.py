@@ -103,7 +103,9 @@ def member_bytes(p: HillParams, precision: int = 1) -> int:
     k = p.degree
     nn2, nq, nc = (k + 1) ** 2, 2 * k + 1, p.nx * p.nz
     ns = nc * nn2
-    geo = nc * (5 * nq * nq + 12 * nq) * 8 + nc * 8 * 4 * 2
+    ncp = (3 * k + 3) // 2  # Schur kernels: geometry products and prepared p_fix per cell
+    schur = 4 * nn2 + 8 * (k + 1) + 9 * ncp * ncp + 12 * nq
+    geo = nc * (5 * nq * nq + 12 * nq + schur) * 8 + nc * 8 * 4 * 2
     blocks = 2 * nc * nn2 * nn2 * 8           # M^{-1}, A^{-1}
     ctx_vec = (4 + 4 + 2 + 1 + 29) * ns * 8   # frozen fields, work, GMRES basis
     solver_vec = (12 + 14) * ns * 8
@@ -111,7 +113,7 @@ def member_bytes(p: HillParams, precision: int = 1) -> int:
     if precision in (1, 2):
         w = 4 if precision == 1 else 8
         # FGMRES basis + levels (geometry, A^{-1}, vectors) over a 4/3 series
-        lv = (nc * (5 * nq * nq + 12 * nq) * w + nc * nn2 * nn2 * w + 10 * ns * w) * 4 // 3
+        lv = (nc * (5 * nq * nq + 12 * nq + schur) * w + nc * nn2 * nn2 * w + 10 * ns * w) * 4 // 3
         total += 16 * ns * 8 + lv
     return int(total * 1.15) + (16 << 20)
 
