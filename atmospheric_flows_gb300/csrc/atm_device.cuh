@@ -88,10 +88,6 @@ __device__ __forceinline__ T bH(int s, int q, int i) {
   return CBasis<T>::get(K, 2 + s, q * (K + 1) + i);
 }
 
-struct SrcPtrs {
-  const double *p[12];
-};
-
 // local node index of node i (0..k) on face f: 0 x=0, 1 x=1, 2 z=0, 3 z=1
 template <int K>
 __device__ __forceinline__ int face_node(int f, int i) {

@@ -120,6 +120,7 @@ struct atm_ctx {
   double *ainv = nullptr;       // [nc][nn2*nn2] inverse of rho_fix-weighted mass
   double *invdiag_D = nullptr;  // inverse diagonal of D (Schur Jacobi)
   // workspace
+  double *fbuf = nullptr;  // [nc][4][2][nn] face integrals of the explicit right-hand sides
   double *wv1 = nullptr, *wv2 = nullptr;  // velocity-sized
   double *ws1 = nullptr, *ws2 = nullptr;  // scalar-sized
   double *red = nullptr;                  // reduction partials (device)

@@ -80,6 +80,7 @@ static void ctx_free(atm_ctx *c) {
   cudaFree(c->u_fix);
   cudaFree(c->ainv);
   cudaFree(c->invdiag_D);
+  cudaFree(c->fbuf);
   cudaFree(c->wv1);
   cudaFree(c->wv2);
   cudaFree(c->ws1);
@@ -145,6 +146,7 @@ int atm_ctx_create(int dim, int degree, int n_cells, int mapping_degree,
   ALLOC(c->u_fix, nv);
   ALLOC(c->ainv, blk);
   ALLOC(c->invdiag_D, ns);
+  ALLOC(c->fbuf, (long)n_cells * 8 * c->nn);
   ALLOC(c->wv1, nv);
   ALLOC(c->wv2, nv);
   ALLOC(c->ws1, ns);

@@ -5,6 +5,11 @@
 
 namespace atm {
 
+// source vectors of a right-hand side, in the operator's positional order
+struct SrcPtrs {
+  const double *p[12];
+};
+
 // Values between two cells' A^{-1} blocks ([nc][stride]).  FP64: the full
 // (k+1)^2 x (k+1)^2 block.  FP32 (multigrid levels): A^{-1} is symmetric, so
 // only its lower triangle is stored, row by row ((r, c <= r) at

@@ -1,45 +1,85 @@
-// Explicit IMEX stage right-hand sides: conforming-mesh instantiations and
-// the public launchers (the kernels are in rhs_kernels.cuh).
+// Explicit IMEX stage right-hand sides: the cell kernels, the face kernels of
+// conforming meshes and the public launchers (rhs_kernels.cuh).
 #include "rhs_kernels.cuh"
 
 namespace atm {
 
-int upload_basis_rhs(const double *t) { return upload_basis_here(t); }
+int upload_contract_rhs(const double *t) { return upload_exact_here(t); }
 
-// hanging-face instantiations, one translation unit per equation
-int rhs_dispatch_hang_rho(const atm_ctx &c, int stage, double *dst, const double *const *src,
-                          const StageCoef &co);
-int rhs_dispatch_hang_vel(const atm_ctx &c, int stage, double *dst, const double *const *src,
-                          const StageCoef &co);
-int rhs_dispatch_hang_pres(const atm_ctx &c, int stage, double *dst, const double *const *src,
-                           const StageCoef &co);
+// face kernels of meshes with hanging faces (hang_rhs.cu)
+int rhs_face_hang(const atm_ctx &c, int kind, int stage, const SrcPtrs &sp, const StageCoef &co);
 
 namespace {
-int rhs_dispatch(const atm_ctx &c, int kind, int stage, double *dst, const double *const *src,
-                 const StageCoef &co) {
-  const bool hg = c.mesh.nhang > 0;
-  switch (kind) {
-    case 0: return hg ? rhs_dispatch_hang_rho(c, stage, dst, src, co)
-                      : rhs_dispatch_kind<false, 0>(c, stage, dst, src, co);
-    case 1: return hg ? rhs_dispatch_hang_vel(c, stage, dst, src, co)
-                      : rhs_dispatch_kind<false, 1>(c, stage, dst, src, co);
-    default: return hg ? rhs_dispatch_hang_pres(c, stage, dst, src, co)
-                       : rhs_dispatch_kind<false, 2>(c, stage, dst, src, co);
+template <int K, int KIND>
+int rhs_cell_launch(const atm_ctx &c, int stage, double *dst, const SrcPtrs &sp,
+                    const StageCoef &co, bool idem) {
+  using E = Ex<K>;
+  const bool ex = KIND == 0 && c.mesh.exact;
+  const int np = ex ? E::NC : E::NQ;
+  void (*fn)(double *, SrcPtrs, StageCoef, Mesh, const double *, int);
+  if (ex) {
+    constexpr bool X = KIND == 0;
+    fn = stage == 1 ? k_rhs_cell<K, 1, KIND, X>
+                    : (stage == 2 ? k_rhs_cell<K, 2, KIND, X> : k_rhs_cell<K, 3, KIND, X>);
+  } else {
+    fn = stage == 1 ? k_rhs_cell<K, 1, KIND, false>
+                    : (stage == 2 ? k_rhs_cell<K, 2, KIND, false> : k_rhs_cell<K, 3, KIND, false>);
   }
+  auto launch = [&](int tuned) -> cudaError_t {
+    // below 2048 cells the tuner has no say: small blocks reach more SMs
+    int cpb = c.nc < 2048 ? 8 : (tuned + 7) / 8 * 8;
+    if (cpb * np > 288) cpb = 288 / np / 8 * 8;
+    const size_t sm = sizeof(double) * (size_t)cpb * RhsKind<KIND>::NF * E::NN * np;
+    if (cudaError_t e = allow_smem(fn, sm); e != cudaSuccess) return e;
+    fn<<<(c.nc + cpb - 1) / cpb, cpb * np, sm, c.stream>>>(dst, sp, co, c.mesh, c.fbuf, cpb);
+    return cudaGetLastError();
+  };
+  const int cpb = tuned_cpb(c.autotune && !c.capturing, c.stream, TF_RHS_RHO + KIND, K, stage,
+                            c.mesh.nhang > 0, 8, c.nc, idem, launch);
+  ATM_CUDA(launch(cpb));
+  g_kernel_launches.fetch_add(1);
+  return ATM_OK;
+}
+
+template <int KIND>
+int rhs_launch(const atm_ctx &c, int stage, double *dst, const double *const *src,
+               const StageCoef &co) {
+  if (stage < 1 || stage > 3) return ATM_BAD_ARG;
+  SrcPtrs sp{};
+  int nsrc;
+  rhs_sources(sp, nsrc, KIND, stage, src);
+  bool idem = true;  // the kernel only writes dst: safe to run repeatedly
+  for (int i = 0; i < nsrc; ++i) idem = idem && src[i] != dst;
+  // algorithmic bytes: every source field read once, the result written once
+  const int k = c.k, nout = KIND == 1 ? 2 : 1;
+  const int nfields =
+      KIND == 0 ? 3 * stage : (KIND == 1 ? 4 * stage + (stage < 3) : 4 * stage + 3);
+  const double bytes = 8.0 * c.nc * c.nn2 * (nfields + nout);
+  // contractions: evaluate every source field, integrate values and gradients
+  // per output component, the traces of both sides and the integration of two
+  // faces per cell
+  const int ntrace = (KIND == 0 ? 3 : 4) * stage;
+  const double flops = c.nc * (nfields * fl_eval(k) + nout * fl_integrate(k, true) +
+                               2.0 * (2 * ntrace * fl_face(k) + nout * fl_face(k)));
+  TimedRegion tr(c, KF_RHS_RHO + KIND, bytes, flops);
+  if (int rc = c.mesh.nhang > 0 ? rhs_face_hang(c, KIND, stage, sp, co)
+                                : rhs_face_dispatch<KIND, false>(c, stage, sp, co))
+    return rc;
+  ATM_DISPATCH_K(k, (rhs_cell_launch<K, KIND>(c, stage, dst, sp, co, idem)));
 }
 }  // namespace
 
 int launch_rhs_rho(const atm_ctx &c, int stage, double *dst, const double *const *src,
                    const StageCoef &co) {
-  return rhs_dispatch(c, 0, stage, dst, src, co);
+  return rhs_launch<0>(c, stage, dst, src, co);
 }
 int launch_rhs_vel(const atm_ctx &c, int stage, double *dst, const double *const *src,
                    const StageCoef &co) {
-  return rhs_dispatch(c, 1, stage, dst, src, co);
+  return rhs_launch<1>(c, stage, dst, src, co);
 }
 int launch_rhs_pres(const atm_ctx &c, int stage, double *dst, const double *const *src,
                     const StageCoef &co) {
-  return rhs_dispatch(c, 2, stage, dst, src, co);
+  return rhs_launch<2>(c, stage, dst, src, co);
 }
 
 }  // namespace atm

@@ -1,475 +1,452 @@
-// Explicit IMEX stage right-hand sides (FP64), one kernel per equation,
-// templated on the polynomial degree K, the IMEX stage ST and HG (mesh with
-// hanging faces).  Included by rhs_kernels.cu (HG = false) and
-// hang_rhs_*.cu / hang_schur.cu (HG = true), so the two families compile in parallel.
-//
-//   rho      : euler_operator.h:344-473 (cell), 478-692 (face), no boundary
-//   momentum : euler_operator.h:1622-1886 (cell), 1891-2184 (face),
-//              2189-2305 (wall, p_D = p)
-//   energy   : euler_operator.h:745-1007 (cell), 1012-1361 (face), no boundary
+// Explicit IMEX stage right-hand sides (FP64), templated on the polynomial
+// degree K, the IMEX stage ST and the equation KIND:
+//   0 rho      : euler_operator.h:344-473 (cell), 478-692 (face), no boundary
+//   1 momentum : euler_operator.h:1622-1886 (cell), 1891-2184 (face),
+//                2189-2305 (wall, p_D = p)
+//   2 energy   : euler_operator.h:745-1007 (cell), 1012-1361 (face), no boundary
 //
 // 2D form of the reference's 3D operators: gravity acts along -e_z with the
 // factor a^2/r^2 = 1 (euler_operator.h:790-811 on a Cartesian domain).
-// The face formulas are evaluated from each cell's own side (element-centric):
-// the reference's "+" and "-" contributions are the same expression with
-// own/neighbour swapped and n -> -n, so every cell adds
-//   -F(own, neighbour, n_own)
-// for the explicit operators.
+//
+// Each right-hand side is two kernels, bound by their FP64 instructions:
+//   * k_rhs_face integrates the numerical flux of every face once.  The fluxes
+//     are conservative (the reference's "+" and "-" contributions are one
+//     expression with the sides swapped and n -> -n), so of the two sides of a
+//     conforming face only the odd local face (1: x = 1, 3: z = 1) is
+//     integrated and the cell on the other side adds the same nodal integrals
+//     with the opposite sign.  Walls and hanging faces are integrated from
+//     each of their sides, with that side's geometry.
+//   * k_rhs_cell evaluates the fields row by row and column by column (one
+//     thread per 1D contraction, contract.cuh), forms the cell integrals and
+//     adds the face integrals.
+// A face trace takes 35 FP64 instructions per field and stage state, a face
+// point about 20: integrating a face from both cells would cost a quarter of
+// the whole right-hand side.  No atomics; runs are bitwise reproducible.
+// Measured on GB300, the three right-hand sides of the last stage at 51,200
+// cells, k = 4: 5.82 -> 4.20 ms against one kernel per equation with every
+// face integrated twice and the x-contractions done point by point (the energy
+// cell kernel keeps the FP64 pipe 82-85% busy); 3239 cells, k = 3, second
+// stage: 232 -> 214 us.
+//
+// The reference integrates with 2k+1 points.  The momentum flux (degree 4k+1
+// on a degree-2 mapping) needs them all, the energy flux more; the density
+// flux rho u cof grad v has degree 3k+1 and takes floor((3k+3)/2) points where
+// the mesh has the tables of that set (`exact`, mapping degree <= 2).
 #pragma once
-#include "atm_device.cuh"
+#include "contract.cuh"
 
 namespace atm {
 
-// ============================================================== rho rhs ===
-template <int K, int ST, bool HG>
-__global__ void __launch_bounds__(Cfg<K>::MAX_THREADS)
-    k_rhs_rho(double *__restrict__ dst, SrcPtrs src, StageCoef co, Mesh mesh) {
-  using C = Cfg<K>;
-  constexpr int NN = C::NN, NQ = C::NQ, NN2 = C::NN2, NQ2 = C::NQ2;
-  const int CPB = blockDim.x / NQ;  // cells per block, chosen by the autotuner
-  constexpr int NT = 3 * ST;
-  extern __shared__ double sm[];
-  double *tiles = sm;
-  double *xab = tiles + CPB * NT * NN2;
-  double *fb = xab + CPB * 2 * NN * NQ;
-  double *fh = fb + CPB * 4 * NQ;  // subface-1 values (HG)
-  const int tid = threadIdx.x, lc = tid / NQ, col = tid - lc * NQ;
-  const int c0 = blockIdx.x * CPB;
-  const int cnt = min(CPB, mesh.nc - c0);
-#pragma unroll
-  for (int j = 0; j < ST; ++j) {
-    load_tiles<K>(tiles, NT, 3 * j, src.p[2 * j], 1, c0, cnt);
-    load_tiles<K>(tiles, NT, 3 * j + 1, src.p[2 * j + 1], 2, c0, cnt);
-  }
-  __syncthreads();
-  const bool active = lc < cnt;
-  const int c = c0 + lc;
-  if (mesh.dts && active) co.dt *= mesh.dts[c];  // per-member time step
-  double Sx[NN], Dx[NN];
-  load_rows<K>(col, Sx, Dx);
-  if (active) {
-    const double *T = tiles + lc * NT * NN2;
-    double gx[NQ], gz[NQ], v0[NQ];
-#pragma unroll
-    for (int q = 0; q < NQ; ++q) gx[q] = gz[q] = 0.0;
-#pragma unroll
-    for (int j = 0; j < ST; ++j) {
-      double r[NQ], ux[NQ], uz[NQ];
-      eval_col<K>(T + (3 * j) * NN2, Sx, r);
-      eval_col<K>(T + (3 * j + 1) * NN2, Sx, ux);
-      eval_col<K>(T + (3 * j + 2) * NN2, Sx, uz);
-      const double w = co.ca[j] * co.dt;
-#pragma unroll
-      for (int q = 0; q < NQ; ++q) {
-        if (j == 0) v0[q] = r[q];
-        gx[q] += w * r[q] * ux[q];
-        gz[q] += w * r[q] * uz[q];
-      }
-    }
-    const double *G = mesh.qgeo + (long)c * 5 * NQ2;
-    double V[NQ], Gxi[NQ], Get[NQ];
-#pragma unroll
-    for (int qz = 0; qz < NQ; ++qz) {
-      const QGeo g = qgeo<K>(G, qz * NQ + col);
-      V[qz] = v0[qz] * g.jxw;
-      Gxi[qz] = g.xx * gx[qz] + g.xz * gz[qz];
-      Get[qz] = g.ex * gx[qz] + g.ez * gz[qz];
-    }
-    double *xa = xab + lc * 2 * NN * NQ;
-    integrate_col_z<K, true, true>(V, Gxi, Get, xa, xa + NN * NQ, col);
-    // faces
-    face_terms<K, 1, HG>(mesh, c, col, Sx, fb + lc * 4 * NQ, fh + lc * 4 * NQ,
-                         [&](int f, int nb, int nf, double n0, double n1, double jxw,
-                             const auto &Ro, const auto &Rn, auto &val) {
-      double flux = 0.0;
-      if (nb >= 0) {
-#pragma unroll
-        for (int j = 0; j < ST; ++j) {
-          const double rp = face_val<K>(T + (3 * j) * NN2, f, Ro);
-          const double uxp = face_val<K>(T + (3 * j + 1) * NN2, f, Ro);
-          const double uzp = face_val<K>(T + (3 * j + 2) * NN2, f, Ro);
-          const double rm = face_val<K>(src.p[2 * j] + (long)nb * NN2, nf, Rn);
-          const double uxm = face_val<K>(src.p[2 * j + 1] + (long)nb * 2 * NN2, nf, Rn);
-          const double uzm = face_val<K>(src.p[2 * j + 1] + ((long)nb * 2 + 1) * NN2, nf, Rn);
-          const double avg0 = 0.5 * (rp * uxp + rm * uxm);
-          const double avg1 = 0.5 * (rp * uzp + rm * uzm);
-          const double lam = fmax(fabs(uxp * n0 + uzp * n1), fabs(uxm * n0 + uzm * n1));
-          flux += co.ca[j] * co.dt * ((avg0 * n0 + avg1 * n1) + 0.5 * lam * (rp - rm));
-        }
-      }
-      val[0] = nb >= 0 ? -flux * jxw : 0.0;
-    });
-  }
-  __syncthreads();
-  if (active && col < NN) {
-    double St[NQ], Dt[NQ], out[NN];
-    load_cols<K>(col, St, Dt);
-    const double *xa = xab + lc * 2 * NN * NQ;
-    output_phase<K, HG>(mesh, c, xa, xa + NN * NQ, fb + lc * 4 * NQ, fh + lc * 4 * NQ, col, St, Dt,
-                        out);
-    double *d = dst + (long)c * NN2;
-#pragma unroll
-    for (int iz = 0; iz < NN; ++iz) d[out_node<K, HG>(col, iz)] = out[iz];
-  }
-}
+template <int KIND>
+struct RhsKind {
+  static constexpr int NF = KIND == 0 ? 3 : 4;     // fields of a stage state: rho, u, [p]
+  static constexpr int PER = KIND == 0 ? 2 : 3;    // source vectors of a stage state
+  static constexpr int NCOMP = KIND == 1 ? 2 : 1;  // output components
+};
 
-// ========================================================= momentum rhs ===
-template <int K, int ST, bool HG>
-__global__ void __launch_bounds__(Cfg<K>::MAX_THREADS)
-    k_rhs_vel(double *__restrict__ dst, SrcPtrs src, StageCoef co, Mesh mesh) {
-  using C = Cfg<K>;
-  constexpr int NN = C::NN, NQ = C::NQ, NN2 = C::NN2, NQ2 = C::NQ2;
-  const int CPB = blockDim.x / NQ;  // cells per block, chosen by the autotuner
-  constexpr int NG = (ST == 1) ? 2 : 3;             // gravity terms
-  constexpr int NT = 4 * ST + (ST < 3 ? 1 : 0);     // tiles
-  extern __shared__ double sm[];
-  double *tiles = sm;
-  double *xab = tiles + CPB * NT * NN2;             // [CPB][2 comp][2][NN*NQ]
-  double *fb = xab + CPB * 4 * NN * NQ;             // [CPB][2 comp][4][NQ]
-  double *fh = fb + CPB * 8 * NQ;                   // subface-1 values (HG)
-  const int tid = threadIdx.x, lc = tid / NQ, col = tid - lc * NQ;
-  const int c0 = blockIdx.x * CPB;
-  const int cnt = min(CPB, mesh.nc - c0);
+// =============================================================== faces ===
+// F[comp][q] += numerical flux of all stage states at the points of one face,
+// outward of cell c, times the face weight.  n0, n1: normal times weight.
+// sub_o / sub_n >= 0: this cell's / the neighbour's trace on that subface.
+template <int K, int ST, int KIND, bool HG>
+__device__ __forceinline__ void face_flux(const SrcPtrs &src, const StageCoef &co, int c, int f,
+                                          int sub_o, int nb, int nf, int sub_n,
+                                          const double (&n0)[2 * K + 1],
+                                          const double (&n1)[2 * K + 1],
+                                          double (&F)[RhsKind<KIND>::NCOMP][2 * K + 1]) {
+  constexpr int NN2 = (K + 1) * (K + 1), NQ = 2 * K + 1, PER = RhsKind<KIND>::PER;
+  constexpr double IG = 1.0 / (GAS_GAMMA - 1.0), HGF = GAS_GAMMA * IG;
+  constexpr bool MIXED = KIND == 2 && ST == 2;  // stage 2 mixes the states' velocities
+  if (!HG) sub_o = sub_n = -1;
+  double xo[MIXED ? NQ : 1], zo[MIXED ? NQ : 1], xn[MIXED ? NQ : 1], zn[MIXED ? NQ : 1];
 #pragma unroll
   for (int j = 0; j < ST; ++j) {
-    load_tiles<K>(tiles, NT, 4 * j, src.p[3 * j], 1, c0, cnt);
-    load_tiles<K>(tiles, NT, 4 * j + 1, src.p[3 * j + 1], 2, c0, cnt);
-    load_tiles<K>(tiles, NT, 4 * j + 3, src.p[3 * j + 2], 1, c0, cnt);
-  }
-  if (ST < 3) load_tiles<K>(tiles, NT, 4 * ST, src.p[3 * ST], 1, c0, cnt);
-  __syncthreads();
-  const bool active = lc < cnt;
-  const int c = c0 + lc;
-  if (mesh.dts && active) co.dt *= mesh.dts[c];  // per-member time step
-  double Sx[NN], Dx[NN];
-  load_rows<K>(col, Sx, Dx);
-  const double dtM2 = co.dt / (co.Ma * co.Ma);
-  if (active) {
-    const double *T = tiles + lc * NT * NN2;
-    double v0[NQ], v1[NQ], g00[NQ], g01[NQ], g10[NQ], g11[NQ];
+    const double *sr = src.p[PER * j], *su = src.p[PER * j + 1];
+    double r[NQ], ux[NQ], uz[NQ], p[NQ], un[NQ];
+    own_or_sub<K>(sr + (long)c * NN2, f, sub_o, r);
+    own_or_sub<K>(su + (long)c * 2 * NN2, f, sub_o, ux);
+    own_or_sub<K>(su + ((long)c * 2 + 1) * NN2, f, sub_o, uz);
+    if (KIND > 0) own_or_sub<K>(src.p[PER * j + 2] + (long)c * NN2, f, sub_o, p);
+    double vr[NQ], vx[NQ], vz[NQ], vp[NQ];
+    own_or_sub<K>(sr + (long)nb * NN2, nf, sub_n, vr);
+    own_or_sub<K>(su + (long)nb * 2 * NN2, nf, sub_n, vx);
+    own_or_sub<K>(su + ((long)nb * 2 + 1) * NN2, nf, sub_n, vz);
+    if (KIND > 0) own_or_sub<K>(src.p[PER * j + 2] + (long)nb * NN2, nf, sub_n, vp);
 #pragma unroll
-    for (int q = 0; q < NQ; ++q) g00[q] = g01[q] = g10[q] = g11[q] = 0.0;
-#pragma unroll
-    for (int j = 0; j < ST; ++j) {
-      double r[NQ], ux[NQ], uz[NQ], p[NQ];
-      eval_col<K>(T + (4 * j) * NN2, Sx, r);
-      eval_col<K>(T + (4 * j + 1) * NN2, Sx, ux);
-      eval_col<K>(T + (4 * j + 2) * NN2, Sx, uz);
-      eval_col<K>(T + (4 * j + 3) * NN2, Sx, p);
-      const double wa = co.ca[j] * co.dt, wp = co.ct[j] * dtM2;
-      const double wg = co.cg[j] * co.dt / (co.Fr * co.Fr);
+    for (int q = 0; q < NQ; ++q) un[q] = fma(ux[q], n0[q], uz[q] * n1[q]);
+    if constexpr (KIND == 0) {
+      const double h = 0.5 * co.ca[j] * co.dt;
 #pragma unroll
       for (int q = 0; q < NQ; ++q) {
-        if (j == 0) {
-          v0[q] = r[q] * ux[q];
-          v1[q] = r[q] * uz[q];
-        }
-        v1[q] -= wg * r[q];
-        const double ru0 = wa * r[q] * ux[q], ru1 = wa * r[q] * uz[q];
-        const double pp = wp * p[q];
-        g00[q] += ru0 * ux[q] + pp;
-        g01[q] += ru0 * uz[q];
-        g10[q] += ru1 * ux[q];
-        g11[q] += ru1 * uz[q] + pp;
+        const double um = fma(vx[q], n0[q], vz[q] * n1[q]);
+        const double t = fma(abs_max(un[q], um), r[q] - vr[q], fma(r[q], un[q], vr[q] * um));
+        F[0][q] = fma(h, t, F[0][q]);
       }
-    }
-    if (NG > ST) {  // implicit gravity term of the density being solved for
-      double r[NQ];
-      eval_col<K>(T + (4 * ST) * NN2, Sx, r);
-      const double wg = co.cg[ST] * co.dt / (co.Fr * co.Fr);
+    } else if constexpr (KIND == 1) {
+      const double h = 0.5 * co.ca[j] * co.dt, hp = 0.5 * co.ct[j] * co.dt / (co.Ma * co.Ma);
 #pragma unroll
-      for (int q = 0; q < NQ; ++q) v1[q] -= wg * r[q];
-    }
-    const double *G = mesh.qgeo + (long)c * 5 * NQ2;
-    double V[NQ], Gxi[NQ], Get[NQ];
-    double *xa0 = xab + (lc * 2 + 0) * 2 * NN * NQ;
-    double *xa1 = xab + (lc * 2 + 1) * 2 * NN * NQ;
-#pragma unroll
-    for (int qz = 0; qz < NQ; ++qz) {
-      const QGeo g = qgeo<K>(G, qz * NQ + col);
-      V[qz] = v0[qz] * g.jxw;
-      Gxi[qz] = g.xx * g00[qz] + g.xz * g01[qz];
-      Get[qz] = g.ex * g00[qz] + g.ez * g01[qz];
-    }
-    integrate_col_z<K, true, true>(V, Gxi, Get, xa0, xa0 + NN * NQ, col);
-#pragma unroll
-    for (int qz = 0; qz < NQ; ++qz) {
-      const QGeo g = qgeo<K>(G, qz * NQ + col);
-      V[qz] = v1[qz] * g.jxw;
-      Gxi[qz] = g.xx * g10[qz] + g.xz * g11[qz];
-      Get[qz] = g.ex * g10[qz] + g.ez * g11[qz];
-    }
-    integrate_col_z<K, true, true>(V, Gxi, Get, xa1, xa1 + NN * NQ, col);
-    // faces
-    face_terms<K, 2, HG>(mesh, c, col, Sx, fb + lc * 2 * 4 * NQ, fh + lc * 2 * 4 * NQ,
-                         [&](int f, int nb, int nf, double n0, double n1, double jxw,
-                             const auto &Ro, const auto &Rn, auto &val) {
-      double f0 = 0.0, f1 = 0.0;
-      if (nb >= 0) {
-#pragma unroll
-        for (int j = 0; j < ST; ++j) {
-          const double rp = face_val<K>(T + (4 * j) * NN2, f, Ro);
-          const double uxp = face_val<K>(T + (4 * j + 1) * NN2, f, Ro);
-          const double uzp = face_val<K>(T + (4 * j + 2) * NN2, f, Ro);
-          const double pp = face_val<K>(T + (4 * j + 3) * NN2, f, Ro);
-          const double rm = face_val<K>(src.p[3 * j] + (long)nb * NN2, nf, Rn);
-          const double uxm = face_val<K>(src.p[3 * j + 1] + (long)nb * 2 * NN2, nf, Rn);
-          const double uzm = face_val<K>(src.p[3 * j + 1] + ((long)nb * 2 + 1) * NN2, nf, Rn);
-          const double pm = face_val<K>(src.p[3 * j + 2] + (long)nb * NN2, nf, Rn);
-          const double unp = uxp * n0 + uzp * n1, unm = uxm * n0 + uzm * n1;
-          const double at0 = 0.5 * (rp * uxp * unp + rm * uxm * unm);
-          const double at1 = 0.5 * (rp * uzp * unp + rm * uzm * unm);
-          const double avgp = 0.5 * (pp + pm);
-          const double lam = fmax(fabs(unp), fabs(unm));
-          const double wa = co.ca[j] * co.dt, wp = co.ct[j] * dtM2;
-          f0 += wa * at0 + wp * avgp * n0 + wa * 0.5 * lam * (rp * uxp - rm * uxm);
-          f1 += wa * at1 + wp * avgp * n1 + wa * 0.5 * lam * (rp * uzp - rm * uzm);
-        }
-      } else {
-        // no-flux wall: only the pressure term with p_D = p
-#pragma unroll
-        for (int j = 0; j < ST; ++j) {
-          const double pp = face_val<K>(T + (4 * j + 3) * NN2, f, Ro);
-          const double avg = 0.5 * (pp + pp);
-          f0 += co.ct[j] * dtM2 * avg * n0;
-          f1 += co.ct[j] * dtM2 * avg * n1;
-        }
+      for (int q = 0; q < NQ; ++q) {
+        const double um = fma(vx[q], n0[q], vz[q] * n1[q]);
+        const double lam = abs_max(un[q], um);
+        const double a0 = r[q] * ux[q], a1 = r[q] * uz[q], b0 = vr[q] * vx[q], b1 = vr[q] * vz[q];
+        const double t0 = fma(lam, a0 - b0, fma(a0, un[q], b0 * um));
+        const double t1 = fma(lam, a1 - b1, fma(a1, un[q], b1 * um));
+        const double ps = hp * (p[q] + vp[q]);
+        F[0][q] = fma(h, t0, fma(ps, n0[q], F[0][q]));
+        F[1][q] = fma(h, t1, fma(ps, n1[q], F[1][q]));
       }
-      val[0] = -f0 * jxw;
-      val[1] = -f1 * jxw;
-    });
-  }
-  __syncthreads();
-  if (active && col < NN) {
-    double St[NQ], Dt[NQ];
-    load_cols<K>(col, St, Dt);
+    } else {
+      // per side s = k1 rho |u|^2 + k2 p (the flux over u.n) and t = k1 rho
+      // |u|^2 + k3 p (what jumps); stage 3 jumps the total rho E
+      // (euler_operator.h:1290,1313,1336), where the enthalpy carries the
+      // explicit weight; the division by rho in the reference's E cancels
+      const double wa = co.ca[j] * co.dt, we = ST == 3 ? wa : co.ct[j] * co.dt;
+      const double k1 = 0.25 * wa * co.Ma * co.Ma, k2 = 0.5 * HGF * we, k3 = 0.5 * IG * we;
 #pragma unroll
-    for (int comp = 0; comp < 2; ++comp) {
-      double out[NN];
-      const double *xa = xab + (lc * 2 + comp) * 2 * NN * NQ;
-      output_phase<K, HG>(mesh, c, xa, xa + NN * NQ, fb + (lc * 2 + comp) * 4 * NQ, fh + (lc * 2 + comp) * 4 * NQ, col, St, Dt,
-                          out);
-      double *d = dst + ((long)c * 2 + comp) * NN2;
-#pragma unroll
-      for (int iz = 0; iz < NN; ++iz) d[out_node<K, HG>(col, iz)] = out[iz];
+      for (int q = 0; q < NQ; ++q) {
+        const double um = fma(vx[q], n0[q], vz[q] * n1[q]);
+        const double lam = abs_max(un[q], um);
+        const double a = k1 * r[q], b = k1 * vr[q];
+        const double ka = a * fma(ux[q], ux[q], uz[q] * uz[q]);
+        const double kb = b * fma(vx[q], vx[q], vz[q] * vz[q]);
+        double ja = ka, jb = kb;
+        if constexpr (MIXED) {
+          if (j == 0) {
+            xo[q] = ux[q]; zo[q] = uz[q]; xn[q] = vx[q]; zn[q] = vz[q];
+          } else {  // the reference's mixed kinetic jump (euler_operator.h:1182-1183)
+            ja = a * fma(ux[q], xo[q], uz[q] * zo[q]);
+            jb = b * fma(vx[q], xn[q], vz[q] * zn[q]);
+          }
+        }
+        F[0][q] = fma(fma(k2, p[q], ka), un[q], F[0][q]);
+        F[0][q] = fma(fma(k2, vp[q], kb), um, F[0][q]);
+        F[0][q] = fma(lam, fma(k3, p[q], ja) - fma(k3, vp[q], jb), F[0][q]);
+      }
     }
   }
 }
 
-// ======================================================== energy rhs (p) ===
-template <int K, int ST, bool HG>
-__global__ void __launch_bounds__(Cfg<K>::MAX_THREADS)
-    k_rhs_pres(double *__restrict__ dst, SrcPtrs src, StageCoef co, Mesh mesh) {
-  using C = Cfg<K>;
-  constexpr int NN = C::NN, NQ = C::NQ, NN2 = C::NN2, NQ2 = C::NQ2;
-  const int CPB = blockDim.x / NQ;  // cells per block, chosen by the autotuner
-  constexpr int NG = (ST == 1) ? 2 : 3;
-  constexpr int NT = 4 * ST + 3;
-  constexpr double GM1 = GAS_GAMMA - 1.0;
-  // The reference forms E = p / ((gamma-1) rho) + Ma^2 |u|^2 / 2 and then
-  // only uses rho E and rho (E - Ma^2 |u|^2 / 2) + p.  Those are
-  // p / (gamma-1) + rho Ma^2 |u|^2 / 2 and gamma / (gamma-1) p: the division
-  // by rho cancels, and the kernel forms the products directly (no FP64
-  // division per point; the values agree to rounding).
-  constexpr double IG = 1.0 / GM1, HGF = GAS_GAMMA / GM1;
-  extern __shared__ double sm[];
-  double *tiles = sm;
-  double *xab = tiles + CPB * NT * NN2;
-  double *fb = xab + CPB * 2 * NN * NQ;
-  double *fh = fb + CPB * 4 * NQ;  // subface-1 values (HG)
-  const int tid = threadIdx.x, lc = tid / NQ, col = tid - lc * NQ;
-  const int c0 = blockIdx.x * CPB;
-  const int cnt = min(CPB, mesh.nc - c0);
+// Fb[c][f][comp][k+1]: nodal integrals of the outward flux; one thread per
+// face, the odd local faces first, then (`all`) the even ones that are not
+// the other side of a conforming face.
+template <int K, int ST, int KIND, bool HG>
+__global__ void __launch_bounds__(64)
+    k_rhs_face(double *__restrict__ Fb, SrcPtrs src, StageCoef co, Mesh mesh) {
+  constexpr int NN = K + 1, NN2 = NN * NN, NQ = 2 * K + 1, NCOMP = RhsKind<KIND>::NCOMP;
+  const long g = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  const bool even = g >= 2L * mesh.nc;
+  const long e = even ? g - 2L * mesh.nc : g;
+  if (e >= 2L * mesh.nc) return;
+  const int c = (int)(e >> 1), f = (int)(e & 1) * 2 + (even ? 0 : 1);
+  const int nb = mesh.nbr[c * 4 + f], nfc = mesh.nbrf[c * 4 + f], nf = nfc & 3;
+  if (nb < 0 && KIND != 1) return;
+  const int code = HG && nb >= 0 ? nfc >> 2 : 0;
+  if (even && nb >= 0 && code == 0) return;  // the neighbour's odd face
+  if (mesh.dts) co.dt *= mesh.dts[c];  // per-member time step
+  double o[NCOMP][NN];
+  double n0[NQ], n1[NQ], F[NCOMP][NQ];
+  if (!HG || code < 3) {
+    const double *fg = mesh.fgeo + ((long)c * 4 + f) * 3 * NQ;
 #pragma unroll
-  for (int j = 0; j < ST; ++j) {
-    load_tiles<K>(tiles, NT, 4 * j, src.p[3 * j], 1, c0, cnt);
-    load_tiles<K>(tiles, NT, 4 * j + 1, src.p[3 * j + 1], 2, c0, cnt);
-    load_tiles<K>(tiles, NT, 4 * j + 3, src.p[3 * j + 2], 1, c0, cnt);
-  }
-  load_tiles<K>(tiles, NT, 4 * ST, src.p[3 * ST], 1, c0, cnt);
-  load_tiles<K>(tiles, NT, 4 * ST + 1, src.p[3 * ST + 1], 2, c0, cnt);
-  __syncthreads();
-  const bool active = lc < cnt;
-  const int c = c0 + lc;
-  if (mesh.dts && active) co.dt *= mesh.dts[c];  // per-member time step
-  double Sx[NN], Dx[NN];
-  load_rows<K>(col, Sx, Dx);
-  const double M2 = co.Ma * co.Ma;
-  if (active) {
-    const double *T = tiles + lc * NT * NN2;
-    double v[NQ], gx[NQ], gz[NQ];
+    for (int q = 0; q < NQ; ++q) {
+      n0[q] = fg[q] * fg[2 * NQ + q];
+      n1[q] = fg[NQ + q] * fg[2 * NQ + q];
 #pragma unroll
-    for (int q = 0; q < NQ; ++q) v[q] = gx[q] = gz[q] = 0.0;
-#pragma unroll
-    for (int j = 0; j < ST; ++j) {
-      double r[NQ], ux[NQ], uz[NQ], p[NQ];
-      eval_col<K>(T + (4 * j) * NN2, Sx, r);
-      eval_col<K>(T + (4 * j + 1) * NN2, Sx, ux);
-      eval_col<K>(T + (4 * j + 2) * NN2, Sx, uz);
-      eval_col<K>(T + (4 * j + 3) * NN2, Sx, p);
-      const double wgrav = co.cg[j] * co.dt * M2 / (co.Fr * co.Fr);
-      const double wk = 0.5 * co.ca[j] * co.dt * M2;
-      const double we = co.ct[j] * co.dt;
-#pragma unroll
-      for (int q = 0; q < NQ; ++q) {
-        const double uu = ux[q] * ux[q] + uz[q] * uz[q];
-        if (j == 0) v[q] += IG * p[q] + 0.5 * M2 * uu * r[q];  // rho E
-        v[q] -= wgrav * r[q] * uz[q];
-        const double kin = wk * uu * r[q];
-        const double ent = we * HGF * p[q];  // rho (E - Ma^2 |u|^2 / 2) + p
-        gx[q] += kin * ux[q] + ent * ux[q];
-        gz[q] += kin * uz[q] + ent * uz[q];
-      }
+      for (int d = 0; d < NCOMP; ++d) F[d][q] = 0.0;
     }
-    {
-      // kinetic energy of the fixed-point velocity, and the implicit gravity
-      // work of the density being solved for (stages 1, 2)
-      double r[NQ], ux[NQ], uz[NQ];
-      eval_col<K>(T + (4 * ST) * NN2, Sx, r);
-      eval_col<K>(T + (4 * ST + 1) * NN2, Sx, ux);
-      eval_col<K>(T + (4 * ST + 2) * NN2, Sx, uz);
-      const double wgrav = (NG > ST) ? co.cg[ST] * co.dt * M2 / (co.Fr * co.Fr) : 0.0;
-#pragma unroll
-      for (int q = 0; q < NQ; ++q) {
-        v[q] -= 0.5 * r[q] * M2 * (ux[q] * ux[q] + uz[q] * uz[q]);
-        if (NG > ST) v[q] -= wgrav * r[q] * uz[q];
-      }
-    }
-    const double *G = mesh.qgeo + (long)c * 5 * NQ2;
-    double V[NQ], Gxi[NQ], Get[NQ];
-#pragma unroll
-    for (int qz = 0; qz < NQ; ++qz) {
-      const QGeo g = qgeo<K>(G, qz * NQ + col);
-      V[qz] = v[qz] * g.jxw;
-      Gxi[qz] = g.xx * gx[qz] + g.xz * gz[qz];
-      Get[qz] = g.ex * gx[qz] + g.ez * gz[qz];
-    }
-    double *xa = xab + lc * 2 * NN * NQ;
-    integrate_col_z<K, true, true>(V, Gxi, Get, xa, xa + NN * NQ, col);
-    // faces
-    face_terms<K, 1, HG>(mesh, c, col, Sx, fb + lc * 4 * NQ, fh + lc * 4 * NQ,
-                         [&](int f, int nb, int nf, double n0, double n1, double jxw,
-                             const auto &Ro, const auto &Rn, auto &val) {
-      if (nb < 0) {
-        val[0] = 0.0;
-        return;
-      }
-      double flux = 0.0;
-      double ux0p = 0.0, uz0p = 0.0, ux0m = 0.0, uz0m = 0.0;  // state-0 velocity traces
+    if (KIND == 1 && nb < 0) {  // no-flux wall: only the pressure term with p_D = p
 #pragma unroll
       for (int j = 0; j < ST; ++j) {
-        const double rp = face_val<K>(T + (4 * j) * NN2, f, Ro);
-        const double uxp = face_val<K>(T + (4 * j + 1) * NN2, f, Ro);
-        const double uzp = face_val<K>(T + (4 * j + 2) * NN2, f, Ro);
-        const double pp = face_val<K>(T + (4 * j + 3) * NN2, f, Ro);
-        const double rm = face_val<K>(src.p[3 * j] + (long)nb * NN2, nf, Rn);
-        const double uxm = face_val<K>(src.p[3 * j + 1] + (long)nb * 2 * NN2, nf, Rn);
-        const double uzm = face_val<K>(src.p[3 * j + 1] + ((long)nb * 2 + 1) * NN2, nf, Rn);
-        const double pm = face_val<K>(src.p[3 * j + 2] + (long)nb * NN2, nf, Rn);
-        if (j == 0) { ux0p = uxp; uz0p = uzp; ux0m = uxm; uz0m = uzm; }
-        const double uup = uxp * uxp + uzp * uzp, uum = uxm * uxm + uzm * uzm;
-        const double unp = uxp * n0 + uzp * n1, unm = uxm * n0 + uzm * n1;
-        const double akin = 0.5 * (0.5 * uup * rp * unp + 0.5 * uum * rm * unm);
-        // enthalpy rho (E - Ma^2 |u|^2 / 2) + p of each side
-        const double hp = HGF * pp, hm = HGF * pm;
-        const double aent = 0.5 * (hp * unp + hm * unm);
-        const double lam = fmax(fabs(unp), fabs(unm));
-        const double wa = co.ca[j] * co.dt;
-        if (ST == 3) {
-          // stage 3 jumps the total rho E (euler_operator.h:1290,1313,1336)
-          const double jE = IG * (pp - pm) + 0.5 * M2 * (rp * uup - rm * uum);
-          flux += wa * M2 * akin + wa * aent + wa * 0.5 * lam * jE;
-        } else {
-          // stage 2 keeps the reference's mixed kinetic jump for tmp_2
-          // (euler_operator.h:1182-1183)
-          const double jkin = (ST == 2 && j == 1)
-                                  ? rp * 0.5 * (uxp * ux0p + uzp * uz0p) -
-                                        rm * 0.5 * (uxm * ux0m + uzm * uz0m)
-                                  : rp * 0.5 * uup - rm * 0.5 * uum;
-          const double je = IG * (pp - pm);  // jump of rho (E - Ma^2 |u|^2 / 2)
-          flux += wa * M2 * (akin + 0.5 * lam * jkin) +
-                  co.ct[j] * co.dt * (aent + 0.5 * lam * je);
+        double p[NQ];
+        own_or_sub<K>(src.p[RhsKind<KIND>::PER * j + 2] + (long)c * NN2, f, -1, p);
+        const double w = co.ct[j] * co.dt / (co.Ma * co.Ma);
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) {
+          F[0][q] = fma(w * p[q], n0[q], F[0][q]);
+          F[NCOMP - 1][q] = fma(w * p[q], n1[q], F[NCOMP - 1][q]);
         }
       }
-      val[0] = -flux * jxw;
-    });
+    } else {
+      face_flux<K, ST, KIND, HG>(src, co, c, f, -1, nb, nf, code - 1, n0, n1, F);
+    }
+#pragma unroll
+    for (int d = 0; d < NCOMP; ++d) eo_integ<K, 2, NQ, true, false>(F[d], F[d], o[d]);
+  } else {
+#pragma unroll
+    for (int d = 0; d < NCOMP; ++d)
+#pragma unroll
+      for (int i = 0; i < NN; ++i) o[d][i] = 0.0;
+    for (int h = 0; h < 2; ++h) {
+      const double *fg = mesh.hgeo + ((long)nb * 2 + h) * 3 * NQ;
+#pragma unroll
+      for (int q = 0; q < NQ; ++q) {
+        n0[q] = fg[q] * fg[2 * NQ + q];
+        n1[q] = fg[NQ + q] * fg[2 * NQ + q];
+#pragma unroll
+        for (int d = 0; d < NCOMP; ++d) F[d][q] = 0.0;
+      }
+      face_flux<K, ST, KIND, HG>(src, co, c, f, h, mesh.hnb[nb * 2 + h], nf, -1, n0, n1, F);
+#pragma unroll
+      for (int d = 0; d < NCOMP; ++d) sub_integ_add<K, 1>(F[d], h, o[d]);
+    }
+  }
+  double *out = Fb + ((long)c * 4 + f) * NCOMP * NN;
+#pragma unroll
+  for (int d = 0; d < NCOMP; ++d)
+#pragma unroll
+    for (int i = 0; i < NN; ++i) out[d * NN + i] = o[d][i];
+}
+
+// =============================================================== cells ===
+// x-interpolation of NF fields (rho; rho, u; or rho, u, p) of the block's
+// cells: X[l][field][iz][NP], one row per thread
+template <int K, int SET, int NP, int NF>
+__device__ __forceinline__ void rhs_rows(double *__restrict__ X, int per, const double *r,
+                                         const double *u, const double *p, int c0, int cnt) {
+  constexpr int NN = K + 1;
+  for (int e = threadIdx.x; e < cnt * NF * NN; e += blockDim.x) {
+    const int l = e / (NF * NN), i = e - l * (NF * NN);
+    const long c = c0 + l;
+    const double *row = i < NN ? r + (c * NN + i) * NN
+                        : i < 3 * NN ? u + (c * 2 * NN + (i - NN)) * NN
+                                     : p + (c * NN + (i - 3 * NN)) * NN;
+    double t[NN], v[NP];
+#pragma unroll
+    for (int a = 0; a < NN; ++a) t[a] = __ldg(row + a);
+    eo_interp<K, SET>(t, v);
+#pragma unroll
+    for (int q = 0; q < NP; ++q) X[l * per + i * NP + q] = v[q];
+  }
+}
+// z-interpolation of one field's column
+template <int K, int SET, int NP>
+__device__ __forceinline__ void rhs_col(const double *__restrict__ x, double (&v)[NP]) {
+  double t[K + 1];
+#pragma unroll
+  for (int i = 0; i <= K; ++i) t[i] = x[i * NP];
+  eo_interp<K, SET>(t, v);
+}
+
+// face integrals of component `comp` that output row iz adds
+template <int K, int KIND>
+__device__ __forceinline__ void rhs_face_rows(const double *__restrict__ Fb, const Mesh &mesh,
+                                              long c, int comp, int iz, double (&add)[K + 1]) {
+  constexpr int NN = K + 1, NCOMP = RhsKind<KIND>::NCOMP;
+  const int4 nb4 = *reinterpret_cast<const int4 *>(mesh.nbr + c * 4);
+  const int4 nf4 = *reinterpret_cast<const int4 *>(mesh.nbrf + c * 4);
+  const int nb[4] = {nb4.x, nb4.y, nb4.z, nb4.w}, nf[4] = {nf4.x, nf4.y, nf4.z, nf4.w};
+#pragma unroll
+  for (int i = 0; i < NN; ++i) add[i] = 0.0;
+#pragma unroll
+  for (int f = 0; f < 4; ++f) {
+    if (f == 2 ? iz != 0 : f == 3 ? iz != K : false) continue;
+    if (nb[f] < 0 && KIND != 1) continue;
+    // even conforming faces: the neighbour's integrals, as they are; the
+    // others: this cell's own with the sign flipped (on the integer pipe)
+    const bool theirs = !(f & 1) && nb[f] >= 0 && (nf[f] >> 2) == 0;
+    const double *F =
+        Fb + (theirs ? (long)nb[f] * 4 + (nf[f] & 3) : c * 4 + f) * NCOMP * NN + comp * NN;
+    const long long flip = theirs ? 0 : (long long)0x8000000000000000ull;
+    if (f < 2) {
+      const double v = __longlong_as_double(__double_as_longlong(F[iz]) ^ flip);
+      if (f == 0) add[0] += v;
+      else add[K] += v;
+    } else {
+#pragma unroll
+      for (int i = 0; i < NN; ++i)
+        add[i] += __longlong_as_double(__double_as_longlong(F[i]) ^ flip);
+    }
+  }
+}
+
+// Threads (cell, column); `cpb` cells per block.
+template <int K, int ST, int KIND, bool EX>
+__global__ void __launch_bounds__(288)
+    k_rhs_cell(double *__restrict__ dst, SrcPtrs src, StageCoef co, Mesh mesh,
+               const double *__restrict__ Fb, int cpb) {
+  using E = Ex<K>;
+  using R = RhsKind<KIND>;
+  constexpr int NN = E::NN, NN2 = E::NN2, NCOMP = R::NCOMP, PER = R::PER;
+  constexpr int SET = EX ? 1 : 2, NP = EX ? E::NC : E::NQ, XS = NN * NP, XC = R::NF * XS;
+  constexpr double IG = 1.0 / (GAS_GAMMA - 1.0), HGF = GAS_GAMMA * IG;
+  extern __shared__ double sm[];  // [cpb][NF][NN][NP]
+  const int tid = threadIdx.x, l = tid / NP, col = tid - l * NP;
+  const int c0 = blockIdx.x * cpb, cnt = min(cpb, mesh.nc - c0);
+  const bool active = l < cnt;
+  const long c = c0 + l;
+  if (mesh.dts && active) co.dt *= mesh.dts[c];  // per-member time step
+  const double M2 = co.Ma * co.Ma;
+  double *x = sm + l * XC + col;
+  // momentum: g00, g01 = g10, g11 and v0, v1; the others: gx, gz and v0
+  double ga[NP], gb[NP], gc[KIND == 1 ? NP : 1], v0[NP], v1[KIND == 1 ? NP : 1];
+#pragma unroll
+  for (int q = 0; q < NP; ++q) {
+    ga[q] = gb[q] = v0[q] = 0.0;
+    if (KIND == 1) gc[q] = v1[q] = 0.0;
+  }
+#pragma unroll
+  for (int j = 0; j < ST; ++j) {
+    rhs_rows<K, SET, NP, R::NF>(sm, XC, src.p[PER * j], src.p[PER * j + 1],
+                                KIND > 0 ? src.p[PER * j + 2] : nullptr, c0, cnt);
+    __syncthreads();
+    if (active) {
+      double r[NP], ux[NP], uz[NP], p[NP];
+      rhs_col<K, SET>(x, r);
+      rhs_col<K, SET>(x + XS, ux);
+      rhs_col<K, SET>(x + 2 * XS, uz);
+      if (KIND > 0) rhs_col<K, SET>(x + 3 * XS, p);
+      const double wa = co.ca[j] * co.dt;
+      if constexpr (KIND == 0) {
+        // the tables of the smaller point set carry gamma/(gamma-1)
+        const double w = EX ? wa / HGF : wa;
+#pragma unroll
+        for (int q = 0; q < NP; ++q) {
+          if (j == 0) v0[q] = r[q];
+          const double wr = w * r[q];
+          ga[q] = fma(wr, ux[q], ga[q]);
+          gb[q] = fma(wr, uz[q], gb[q]);
+        }
+      } else if constexpr (KIND == 1) {
+        const double wp = co.ct[j] * co.dt / M2, wg = co.cg[j] * co.dt / (co.Fr * co.Fr);
+#pragma unroll
+        for (int q = 0; q < NP; ++q) {
+          if (j == 0) {
+            v0[q] = r[q] * ux[q];
+            v1[q] = r[q] * uz[q];
+          }
+          v1[q] = fma(-wg, r[q], v1[q]);
+          const double wr = wa * r[q], rx = wr * ux[q], rz = wr * uz[q];
+          const double pp = wp * p[q];
+          ga[q] += fma(rx, ux[q], pp);
+          gb[q] = fma(rx, uz[q], gb[q]);
+          gc[q] += fma(rz, uz[q], pp);
+        }
+      } else {
+        // the reference forms E = p / ((gamma-1) rho) + Ma^2 |u|^2 / 2 and
+        // uses rho E and rho (E - Ma^2 |u|^2 / 2) + p: the division cancels
+        const double wgrav = co.cg[j] * co.dt * M2 / (co.Fr * co.Fr);
+        const double wk = 0.5 * wa * M2, we = co.ct[j] * co.dt * HGF;
+#pragma unroll
+        for (int q = 0; q < NP; ++q) {
+          const double k = r[q] * fma(ux[q], ux[q], uz[q] * uz[q]);
+          if (j == 0) v0[q] = fma(IG, p[q], 0.5 * M2 * k);  // rho E
+          v0[q] = fma(-wgrav * r[q], uz[q], v0[q]);
+          const double s = fma(wk, k, we * p[q]);
+          ga[q] = fma(s, ux[q], ga[q]);
+          gb[q] = fma(s, uz[q], gb[q]);
+        }
+      }
+    }
+    __syncthreads();
+  }
+  if constexpr (KIND == 1 && ST < 3) {  // implicit gravity of the density being solved for
+    rhs_rows<K, SET, NP, 1>(sm, XC, src.p[PER * ST], nullptr, nullptr, c0, cnt);
+    __syncthreads();
+    if (active) {
+      double r[NP];
+      rhs_col<K, SET>(x, r);
+      const double wg = co.cg[ST] * co.dt / (co.Fr * co.Fr);
+#pragma unroll
+      for (int q = 0; q < NP; ++q) v1[q] = fma(-wg, r[q], v1[q]);
+    }
+    __syncthreads();
+  }
+  if constexpr (KIND == 2) {
+    if (src.p[PER * ST + 1]) {  // kinetic energy and gravity work of the fixed-point velocity
+      rhs_rows<K, SET, NP, 3>(sm, XC, src.p[PER * ST], src.p[PER * ST + 1], nullptr, c0, cnt);
+      __syncthreads();
+      if (active) {
+        double r[NP], ux[NP], uz[NP];
+        rhs_col<K, SET>(x, r);
+        rhs_col<K, SET>(x + XS, ux);
+        rhs_col<K, SET>(x + 2 * XS, uz);
+        const double wgrav = ST < 3 ? co.cg[ST < 3 ? ST : 0] * co.dt * M2 / (co.Fr * co.Fr) : 0.0;
+#pragma unroll
+        for (int q = 0; q < NP; ++q) {
+          double t = 0.5 * M2 * fma(ux[q], ux[q], uz[q] * uz[q]);
+          if (ST < 3) t = fma(wgrav, uz[q], t);
+          v0[q] = fma(-t, r[q], v0[q]);
+        }
+      }
+      __syncthreads();
+    }
+  }
+  // fluxes to reference directions, z-integration; the results replace the
+  // column's own values
+  if (active) {
+    double V[NP], Gx[NP], Ge[NP], a[NN], b[NN];
+#pragma unroll
+    for (int comp = 0; comp < NCOMP; ++comp) {
+      if constexpr (EX) {
+        const double *g = mesh.gC + (c * NP + col) * NP * 4, *jw = mesh.gJ + (c * NP + col) * NP;
+#pragma unroll
+        for (int q = 0; q < NP; ++q) {
+          const Vec4<double> w(g + 4 * q);
+          V[q] = (GAS_GAMMA - 1.0) * v0[q] * __ldg(jw + q);  // gJ carries 1/(gamma-1)
+          Gx[q] = fma(w.v[0], ga[q], w.v[2] * gb[q]);
+          Ge[q] = fma(w.v[1], ga[q], w.v[3] * gb[q]);
+        }
+      } else {
+        constexpr int NQ2 = NP * NP;
+        const double *g = mesh.qgeo + c * 5 * NQ2 + col;
+#pragma unroll
+        for (int q = 0; q < NP; ++q) {
+          const double hx = comp == 0 ? ga[q] : gb[q];
+          const double hz = KIND == 1 && comp == 1 ? gc[q] : gb[q];
+          V[q] = (KIND == 1 && comp == 1 ? v1[q] : v0[q]) * __ldg(g + 4 * NQ2 + q * NP);
+          Gx[q] = fma(__ldg(g + q * NP), hx, __ldg(g + NQ2 + q * NP) * hz);
+          Ge[q] = fma(__ldg(g + 2 * NQ2 + q * NP), hx, __ldg(g + 3 * NQ2 + q * NP) * hz);
+        }
+      }
+      eo_integ<K, SET, NP, true, true>(V, Ge, a);
+      eo_integ<K, SET, NP, true, false>(Gx, Gx, b);
+#pragma unroll
+      for (int i = 0; i < NN; ++i) {
+        x[2 * comp * XS + i * NP] = a[i];
+        x[(2 * comp + 1) * XS + i * NP] = b[i];
+      }
+    }
   }
   __syncthreads();
-  if (active && col < NN) {
-    double St[NQ], Dt[NQ], out[NN];
-    load_cols<K>(col, St, Dt);
-    const double *xa = xab + lc * 2 * NN * NQ;
-    output_phase<K, HG>(mesh, c, xa, xa + NN * NQ, fb + lc * 4 * NQ, fh + lc * 4 * NQ, col, St, Dt,
-                        out);
-    double *d = dst + (long)c * NN2;
+  for (int e = tid; e < cnt * NCOMP * NN; e += blockDim.x) {
+    const int lo = e / (NCOMP * NN), i = e - lo * (NCOMP * NN), comp = i / NN, iz = i - comp * NN;
+    const double *y = sm + lo * XC + 2 * comp * XS + iz * NP;
+    double a[NP], b[NP], out[NN], add[NN];
 #pragma unroll
-    for (int iz = 0; iz < NN; ++iz) d[out_node<K, HG>(col, iz)] = out[iz];
+    for (int q = 0; q < NP; ++q) {
+      a[q] = y[q];
+      b[q] = y[XS + q];
+    }
+    rhs_face_rows<K, KIND>(Fb, mesh, c0 + lo, comp, iz, add);
+    eo_integ<K, SET, NP, true, true>(a, b, out);
+    double *d = dst + ((long)(c0 + lo) * NCOMP + comp) * NN2 + iz * NN;
+#pragma unroll
+    for (int q = 0; q < NN; ++q) d[q] = out[q] + add[q];
   }
 }
 
 // ============================================================ launchers ===
-// KIND 0 density, 1 momentum, 2 energy (a template parameter, so each kind's
-// kernels can be instantiated in a translation unit of its own)
-template <int K, bool HG, int KIND>
-int rhs_launch(const atm_ctx &c, int stage, double *dst, const double *const *src,
-               const StageCoef &co) {
-  using C = Cfg<K>;
-  constexpr int kind = KIND;
-  SrcPtrs sp{};
+inline void rhs_sources(SrcPtrs &sp, int &nsrc, int kind, int stage, const double *const *src) {
   const int nsrc_tab[3][3] = {{2, 4, 6}, {4, 7, 9}, {5, 8, 11}};
-  const int nsrc = nsrc_tab[kind][stage - 1];
+  nsrc = nsrc_tab[kind][stage - 1];
   for (int i = 0; i < nsrc; ++i) sp.p[i] = src[i];
-  int ntile;
-  void (*fn)(double *, SrcPtrs, StageCoef, Mesh) = nullptr;
-  if constexpr (KIND == 0) {
-    ntile = 3 * stage;
-    fn = stage == 1 ? k_rhs_rho<K, 1, HG> : (stage == 2 ? k_rhs_rho<K, 2, HG> : k_rhs_rho<K, 3, HG>);
-  } else if constexpr (KIND == 1) {
-    ntile = 4 * stage + (stage < 3 ? 1 : 0);
-    fn = stage == 1 ? k_rhs_vel<K, 1, HG> : (stage == 2 ? k_rhs_vel<K, 2, HG> : k_rhs_vel<K, 3, HG>);
-  } else {
-    ntile = 4 * stage + 3;
-    fn = stage == 1 ? k_rhs_pres<K, 1, HG> : (stage == 2 ? k_rhs_pres<K, 2, HG> : k_rhs_pres<K, 3, HG>);
-  }
-  const int ncomp = kind == 1 ? 2 : 1;
-  auto launch = [&](int cpb) -> cudaError_t {
-    const size_t sm = smem_bytes<K>(cpb, ntile, ncomp, HG);
-    if (cudaError_t e = allow_smem(fn, sm); e != cudaSuccess) return e;
-    fn<<<(c.nc + cpb - 1) / cpb, cpb * C::NQ, sm, c.stream>>>(dst, sp, co, c.mesh);
-    return cudaGetLastError();
-  };
-  bool idem = true;  // the kernel only writes dst: safe to run repeatedly
-  for (int i = 0; i < nsrc; ++i) idem = idem && src[i] != dst;
-  const int cpb = tuned_cpb(c.autotune && !c.capturing, c.stream, TF_RHS_RHO + kind, K, stage,
-                            HG, 8, c.nc, idem, launch);
-  // algorithmic bytes: every source field read once, the result written once
-  const double ns = (double)c.nc * C::NN2;
-  const int nfields = (kind == 0) ? 3 * stage : (kind == 1 ? 4 * stage + (stage < 3) : 4 * stage + 3);
-  const int nout = kind == 1 ? 2 : 1;
-  const double bytes = 8.0 * ns * (nfields + nout);
-  // contractions: evaluate every source tile, integrate values+gradients per
-  // output component, face traces of both sides (4 faces) and face integration
-  const int ntrace = (kind == 0) ? 3 * stage : 4 * stage;
-  const double flops = c.nc * (nfields * fl_eval(K) + nout * fl_integrate(K, true) +
-                               4.0 * (2 * ntrace * fl_face(K) + nout * fl_face(K)));
-  TimedRegion tr(c, KF_RHS_RHO + kind, bytes, flops);
-  ATM_CUDA(launch(cpb));
-  g_kernel_launches.fetch_add(1);
+}
+
+template <int K, int KIND, bool HG>
+int rhs_face_launch(const atm_ctx &c, int stage, const SrcPtrs &sp, const StageCoef &co) {
+  // even faces: the momentum walls, and hanging faces
+  const long n = (long)c.nc * (HG || KIND == 1 ? 4 : 2);
+  void (*fn)(double *, SrcPtrs, StageCoef, Mesh) =
+      stage == 1 ? k_rhs_face<K, 1, KIND, HG>
+                 : (stage == 2 ? k_rhs_face<K, 2, KIND, HG> : k_rhs_face<K, 3, KIND, HG>);
+  fn<<<(unsigned)((n + 63) / 64), 64, 0, c.stream>>>(c.fbuf, sp, co, c.mesh);
+  ATM_CHECK_LAUNCH("k_rhs_face");
   return ATM_OK;
 }
 
-template <bool HG, int KIND>
-int rhs_dispatch_kind(const atm_ctx &c, int stage, double *dst, const double *const *src,
-                      const StageCoef &co) {
-  if (stage < 1 || stage > 3) return ATM_BAD_ARG;
-  switch (c.k) {
-    case 1: return rhs_launch<1, HG, KIND>(c, stage, dst, src, co);
-    case 2: return rhs_launch<2, HG, KIND>(c, stage, dst, src, co);
-    case 3: return rhs_launch<3, HG, KIND>(c, stage, dst, src, co);
-    case 4: return rhs_launch<4, HG, KIND>(c, stage, dst, src, co);
-    case 5: return rhs_launch<5, HG, KIND>(c, stage, dst, src, co);
-    default: return ATM_BAD_ARG;
-  }
+template <int KIND, bool HG>
+int rhs_face_dispatch(const atm_ctx &c, int stage, const SrcPtrs &sp, const StageCoef &co) {
+  ATM_DISPATCH_K(c.k, (rhs_face_launch<K, KIND, HG>(c, stage, sp, co)));
 }
 
 }  // namespace atm

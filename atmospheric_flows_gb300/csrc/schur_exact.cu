@@ -6,6 +6,8 @@
 namespace atm {
 
 int upload_exact_f(const double *t);
+int upload_contract_rhs(const double *t);
+int upload_contract_hang_rhs(const double *t);
 int upload_exact_hang(const double *t);
 int upload_exact_hang_f(const double *t);
 
@@ -135,7 +137,8 @@ __global__ void k_exact_hang_tables(MeshT<T> m, const double *__restrict__ map2,
 }
 }  // namespace
 
-// 1D tables of every degree to the constant banks of the four translation units
+// 1D tables of every degree to the constant banks of the translation units that
+// contract with them
 int upload_exact_all() {
   std::vector<double> t(EO_DOUBLES + SUB_DOUBLES, 0.0);
   for (int k = 1; k <= KMAX; ++k) {
@@ -163,7 +166,8 @@ int upload_exact_all() {
     }
   }
   return upload_exact_here(t.data()) || upload_exact_f(t.data()) || upload_exact_hang(t.data()) ||
-         upload_exact_hang_f(t.data());
+         upload_exact_hang_f(t.data()) || upload_contract_rhs(t.data()) ||
+         upload_contract_hang_rhs(t.data());
 }
 
 template <typename T>

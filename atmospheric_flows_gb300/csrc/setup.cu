@@ -16,11 +16,7 @@
 
 namespace atm {
 
-int upload_basis_rhs(const double *t);
 int upload_basis_impl(const double *t);
-int upload_basis_hang_rho(const double *t);
-int upload_basis_hang_vel(const double *t);
-int upload_basis_hang_pres(const double *t);
 int upload_basis_hang_schur(const double *t);
 int upload_basis_hang_schur_f(const double *t);
 
@@ -155,9 +151,7 @@ int upload_basis_all() {
         }
     }
   }
-  if (upload_basis_rhs(tab.data()) || upload_basis_impl(tab.data()) ||
-      upload_basis_hang_rho(tab.data()) || upload_basis_hang_vel(tab.data()) ||
-      upload_basis_hang_pres(tab.data()) || upload_basis_hang_schur(tab.data()) ||
+  if (upload_basis_impl(tab.data()) || upload_basis_hang_schur(tab.data()) ||
       upload_basis_hang_schur_f(tab.data()) || upload_exact_all()) {
     set_error("failed to upload basis tables to constant memory");
     return ATM_CUDA_ERROR;
