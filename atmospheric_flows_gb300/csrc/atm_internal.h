@@ -197,6 +197,11 @@ int launch_rhs_vel(const atm_ctx &c, int stage, double *dst, const double *const
                    const StageCoef &co);
 int launch_rhs_pres(const atm_ctx &c, int stage, double *dst, const double *const *src,
                     const StageCoef &co);
+// The energy right-hand side in two parts: launch_rhs_pres with a null last
+// source (the fixed-point velocity) gives the base, and this adds the
+// velocity's part: dst = base + ...
+int launch_rhs_kinetic(const atm_ctx &c, int stage, double *dst, const double *base,
+                       const double *rho, const double *u, const StageCoef &co);
 // B p -> dst (velocity); mode 0: dst = cB B p; 1: dst -= cB B p;
 // 2: dst = A^{-1} B p as the C/D modes 1 and 2 take it (uses c.ainv): times
 // cB cC on meshes with `exact` tables, times cB otherwise
@@ -424,6 +429,7 @@ struct Solver {
   double *rho_old, *rho_tmp_2, *rho_tmp_3, *rho_curr, *rhs_rho;
   double *u_old, *u_tmp_2, *u_tmp_3, *u_curr, *u_fixed, *rhs_u, *tmp_1;
   double *pres_old, *pres_tmp_2, *pres_tmp_3, *pres_fixed, *pres_fixed_old, *rhs_pres;
+  double *rhs_u0, *rhs_pres0;  // the parts of a stage's right-hand sides that Picard keeps
   double *alpha;
   double *pool = nullptr;
 };

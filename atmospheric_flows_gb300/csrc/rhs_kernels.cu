@@ -82,4 +82,28 @@ int launch_rhs_pres(const atm_ctx &c, int stage, double *dst, const double *cons
   return rhs_launch<2>(c, stage, dst, src, co);
 }
 
+namespace {
+template <int K>
+int rhs_kinetic_launch(const atm_ctx &c, double *dst, const double *base, const double *rho,
+                       const double *u, double wgrav, double M2) {
+  constexpr int NP = 2 * K + 1;
+  const int cpb = c.nc < 2048 ? 8 : 16;
+  const size_t sm = sizeof(double) * (size_t)cpb * 3 * (K + 1) * NP;
+  ATM_CUDA(allow_smem(k_rhs_kinetic<K>, sm));
+  k_rhs_kinetic<K><<<(c.nc + cpb - 1) / cpb, cpb * NP, sm, c.stream>>>(dst, base, rho, u, wgrav, M2,
+                                                                     c.mesh, cpb);
+  ATM_CHECK_LAUNCH("k_rhs_kinetic");
+  return ATM_OK;
+}
+}  // namespace
+
+int launch_rhs_kinetic(const atm_ctx &c, int stage, double *dst, const double *base,
+                       const double *rho, const double *u, const StageCoef &co) {
+  const double M2 = co.Ma * co.Ma;
+  const double wgrav = stage < 3 ? co.cg[stage] * co.dt * M2 / (co.Fr * co.Fr) : 0.0;
+  TimedRegion tr(c, KF_RHS_PRES, 8.0 * c.nc * c.nn2 * 5,
+                 c.nc * (3 * fl_eval(c.k) + fl_integrate(c.k, false)));
+  ATM_DISPATCH_K(c.k, (rhs_kinetic_launch<K>(c, dst, base, rho, u, wgrav, M2)));
+}
+
 }  // namespace atm

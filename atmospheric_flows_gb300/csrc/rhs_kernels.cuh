@@ -352,7 +352,7 @@ __global__ void __launch_bounds__(288)
     __syncthreads();
   }
   if constexpr (KIND == 2) {
-    if (src.p[PER * ST + 1]) {  // kinetic energy and gravity work of the fixed-point velocity
+    if (src.p[PER * ST + 1]) {  // (not in a Picard loop's base) kinetic energy and gravity work of the fixed-point velocity
       rhs_rows<K, SET, NP, 3>(sm, XC, src.p[PER * ST], src.p[PER * ST + 1], nullptr, c0, cnt);
       __syncthreads();
       if (active) {
@@ -422,6 +422,53 @@ __global__ void __launch_bounds__(288)
     double *d = dst + ((long)(c0 + lo) * NCOMP + comp) * NN2 + iz * NN;
 #pragma unroll
     for (int q = 0; q < NN; ++q) d[q] = out[q] + add[q];
+  }
+}
+
+// dst = base - integrals of rho (Ma^2 |u|^2 / 2 + wgrav u_z) phi: what the
+// energy right-hand side takes from the fixed-point velocity, the only part of
+// it that changes from one Picard iteration to the next
+// (Atmospheric_Flow.cc:1135-1153).  At 51,200 cells, k = 4 it takes a seventh
+// of the time of the whole right-hand side.  Threads (cell, column).
+template <int K>
+__global__ void __launch_bounds__(288)
+    k_rhs_kinetic(double *__restrict__ dst, const double *__restrict__ base,
+                  const double *__restrict__ rho, const double *__restrict__ u, double wgrav,
+                  double M2, Mesh mesh, int cpb) {
+  constexpr int NN = K + 1, NP = 2 * K + 1, XS = NN * NP, XC = 3 * XS;
+  extern __shared__ double sm[];  // [cpb][3][NN][NP]
+  const int tid = threadIdx.x, l = tid / NP, col = tid - l * NP;
+  const int c0 = blockIdx.x * cpb, cnt = min(cpb, mesh.nc - c0);
+  rhs_rows<K, 2, NP, 3>(sm, XC, rho, u, nullptr, c0, cnt);
+  __syncthreads();
+  if (l < cnt) {
+    const long c = c0 + l;
+    if (mesh.dts) wgrav *= mesh.dts[c];  // per-member time step
+    double *x = sm + l * XC + col;
+    double r[NP], ux[NP], uz[NP], a[NN];
+    rhs_col<K, 2>(x, r);
+    rhs_col<K, 2>(x + XS, ux);
+    rhs_col<K, 2>(x + 2 * XS, uz);
+    const double *jw = mesh.jw + c * mesh.jw_stride + col;
+#pragma unroll
+    for (int q = 0; q < NP; ++q) {
+      const double t = fma(0.5 * M2, fma(ux[q], ux[q], uz[q] * uz[q]), wgrav * uz[q]);
+      r[q] = -t * r[q] * __ldg(jw + q * NP);
+    }
+    eo_integ<K, 2, NP, true, false>(r, r, a);
+#pragma unroll
+    for (int i = 0; i < NN; ++i) x[i * NP] = a[i];
+  }
+  __syncthreads();
+  for (int e = tid; e < cnt * NN; e += blockDim.x) {
+    const int lo = e / NN, iz = e - lo * NN;
+    double a[NP], out[NN];
+#pragma unroll
+    for (int q = 0; q < NP; ++q) a[q] = sm[lo * XC + iz * NP + q];
+    eo_integ<K, 2, NP, true, false>(a, a, out);
+    const long g = ((long)(c0 + lo) * NN + iz) * NN;
+#pragma unroll
+    for (int q = 0; q < NN; ++q) dst[g + q] = base[g + q] + out[q];
   }
 }
 

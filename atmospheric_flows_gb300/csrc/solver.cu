@@ -23,7 +23,7 @@ namespace atm {
 
 int solver_alloc(atm_ctx &c, Solver &s) {
   const long ns = c.n_scalar(), nv = c.n_vector();
-  const long total = 12 * ns + 7 * nv;
+  const long total = 13 * ns + 8 * nv;
   ATM_CUDA(cudaMalloc(&s.pool, total * sizeof(double)));
   ATM_CUDA(cudaMemsetAsync(s.pool, 0, total * sizeof(double), c.stream));
   ATM_CUDA(cudaStreamSynchronize(c.stream));
@@ -33,9 +33,10 @@ int solver_alloc(atm_ctx &c, Solver &s) {
   s.rho_curr = take(ns); s.rhs_rho = take(ns);
   s.pres_old = take(ns); s.pres_tmp_2 = take(ns); s.pres_tmp_3 = take(ns);
   s.pres_fixed = take(ns); s.pres_fixed_old = take(ns); s.rhs_pres = take(ns);
-  s.alpha = take(ns);
+  s.alpha = take(ns); s.rhs_pres0 = take(ns);
   s.u_old = take(nv); s.u_tmp_2 = take(nv); s.u_tmp_3 = take(nv); s.u_curr = take(nv);
   s.u_fixed = take(nv); s.rhs_u = take(nv); s.tmp_1 = take(nv);
+  s.rhs_u0 = take(nv);
   return ATM_OK;
 }
 
@@ -86,8 +87,11 @@ void member_fill(atm_ctx &c, Solver &s, int m) {
   const Members &M = *c.mem;
   const long a = (long)M.off[m] * c.nn2, len = (long)(M.off[m + 1] - M.off[m]) * c.nn2;
   double *ones[] = {s.rho_old, s.rho_tmp_2, s.rho_tmp_3, s.rho_curr, s.pres_old, s.pres_tmp_2,
-                    s.pres_tmp_3, s.pres_fixed, s.pres_fixed_old, c.rho_fix, c.pres_fix};
-  double *zeros[] = {s.u_old, s.u_tmp_2, s.u_tmp_3, s.u_curr, s.u_fixed, c.u_fix};
+                    s.pres_tmp_3, s.pres_fixed, s.pres_fixed_old, c.rho_fix, c.pres_fix,
+                    s.rhs_pres0};
+  // with the parts of the right-hand sides that a Picard loop keeps
+  double *zeros[] = {s.u_old, s.u_tmp_2, s.u_tmp_3, s.u_curr, s.u_fixed, c.u_fix,
+                     s.rhs_u0, s.tmp_1};
   for (double *v : ones) vec_fill(c.stream, v + a, 1.0, len);
   for (double *v : zeros) vec_fill(c.stream, v + 2 * a, 0.0, 2 * len);
 }
@@ -141,27 +145,37 @@ int schur_solve_members(atm_ctx &c, Solver &s) {
   return ATM_OK;
 }
 
+// What the iterations of one Picard loop share: the momentum right-hand side
+// and tmp_1 = A^{-1} of it, and the energy right-hand side without the
+// fixed-point velocity's part.  Their sources (the old and the stage states,
+// rho_fix) do not change in the loop.
+int picard_prepare(atm_ctx &c, Solver &s) {
+  const StageCoef co = stage_coef_flux(c, c.hstage);
+  if (c.hstage == 1) {
+    const double *sp[] = {s.rho_old, s.u_old, s.pres_old, s.rho_tmp_2, nullptr};
+    TRY(launch_rhs_pres(c, 1, s.rhs_pres0, sp, co));
+    const double *su[] = {s.rho_old, s.u_old, s.pres_old, s.rho_tmp_2};
+    TRY(launch_rhs_vel(c, 1, s.rhs_u0, su, co));
+  } else {
+    const double *sp[] = {s.rho_old, s.u_old, s.pres_old, s.rho_tmp_2, s.u_tmp_2,
+                          s.pres_tmp_2, s.rho_tmp_3, nullptr};
+    TRY(launch_rhs_pres(c, 2, s.rhs_pres0, sp, co));
+    const double *su[] = {s.rho_old, s.u_old, s.pres_old, s.rho_tmp_2, s.u_tmp_2,
+                          s.pres_tmp_2, s.rho_tmp_3};
+    TRY(launch_rhs_vel(c, 2, s.rhs_u0, su, co));
+  }
+  return launch_block_apply(c, s.tmp_1, s.rhs_u0, c.ainv, 2, 1.0);
+}
+
 // Atmospheric_Flow.cc:544-673
 int pressure_fixed_point(atm_ctx &c, Solver &s) {
   const long ns = c.n_scalar();
   TRY(vec_copy(c.stream, c.pres_fix, s.pres_fixed_old, ns));  // set_pres_fixed
   TRY(launch_pfix_prep(c));
   const StageCoef co = stage_coef_flux(c, c.hstage);
-  if (c.hstage == 1) {
-    const double *sp[] = {s.rho_old, s.u_old, s.pres_old, s.rho_tmp_2, s.u_fixed};
-    TRY(launch_rhs_pres(c, 1, s.rhs_pres, sp, co));
-    const double *su[] = {s.rho_old, s.u_old, s.pres_old, s.rho_tmp_2};
-    TRY(launch_rhs_vel(c, 1, s.rhs_u, su, co));
-  } else {
-    const double *sp[] = {s.rho_old, s.u_old, s.pres_old, s.rho_tmp_2, s.u_tmp_2,
-                          s.pres_tmp_2, s.rho_tmp_3, s.u_fixed};
-    TRY(launch_rhs_pres(c, 2, s.rhs_pres, sp, co));
-    const double *su[] = {s.rho_old, s.u_old, s.pres_old, s.rho_tmp_2, s.u_tmp_2,
-                          s.pres_tmp_2, s.rho_tmp_3};
-    TRY(launch_rhs_vel(c, 2, s.rhs_u, su, co));
-  }
-  // tmp_1 = A^{-1} rhs_u ; rhs_pres -= C tmp_1
-  TRY(launch_block_apply(c, s.tmp_1, s.rhs_u, c.ainv, 2, 1.0));
+  TRY(launch_rhs_kinetic(c, c.hstage, s.rhs_pres, s.rhs_pres0,
+                         c.hstage == 1 ? s.rho_tmp_2 : s.rho_tmp_3, s.u_fixed, co));
+  // rhs_pres -= C A^{-1} rhs_u
   const double cc = implicit_coeff(c);
   TRY(launch_CD(c, s.rhs_pres, s.tmp_1, nullptr, cc * c.dt, 3));
   if (c.mem) return schur_solve_members(c, s);
@@ -193,6 +207,7 @@ int pressure_fixed_point(atm_ctx &c, Solver &s) {
 int update_velocity(atm_ctx &c, Solver &s) {
   if (c.hstage == 1 || c.hstage == 2) {
     const double co = implicit_coeff(c);
+    TRY(vec_copy(c.stream, s.rhs_u, s.rhs_u0, c.n_vector()));
     TRY(launch_B(c, s.rhs_u, s.pres_fixed, co * c.dt / (c.Ma * c.Ma), 1));
     return launch_block_apply(c, s.u_fixed, s.rhs_u, c.ainv, 2, 1.0);
   }
@@ -222,6 +237,7 @@ int picard_members(atm_ctx &c, Solver &s, int which) {
   const long ns = c.n_scalar();
   std::vector<int> iters(M.n, 0);
   for (int m = 0; m < M.n; ++m) M.active[m] = M.status[m] == ATM_OK;
+  TRY(picard_prepare(c, s));
   for (int iter = 0; iter < 100; ++iter) {
     TRY(pressure_fixed_point(c, s));
     TRY(update_velocity(c, s));
@@ -254,6 +270,7 @@ int picard(atm_ctx &c, Solver &s, int which) {
   if (c.mem) return picard_members(c, s, which);
   const long ns = c.n_scalar();
   int iters = 0;
+  TRY(picard_prepare(c, s));
   for (int iter = 0; iter < 100; ++iter) {
     TRY(pressure_fixed_point(c, s));
     TRY(update_velocity(c, s));

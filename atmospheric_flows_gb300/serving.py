@@ -108,7 +108,7 @@ def member_bytes(p: HillParams, precision: int = 1) -> int:
     geo = nc * (5 * nq * nq + 12 * nq + schur) * 8 + nc * 8 * 4 * 2
     blocks = 2 * nc * nn2 * nn2 * 8           # M^{-1}, A^{-1}
     ctx_vec = (4 + 4 + 2 + 1 + 29) * ns * 8 + nc * 8 * (k + 1) * 8  # frozen fields, work, GMRES basis, face integrals
-    solver_vec = (12 + 14) * ns * 8
+    solver_vec = (13 + 16) * ns * 8
     total = geo + blocks + ctx_vec + solver_vec
     if precision in (1, 2):
         w = 4 if precision == 1 else 8
