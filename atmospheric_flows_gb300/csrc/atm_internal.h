@@ -92,7 +92,7 @@ struct MeshT {
   T *map2 = nullptr;
   // Tables of the Schur kernels for mapping degree <= 2 (schur_exact.cuh;
   // `exact` when they are there), n = k+1, c = floor((3k+3)/2), q = 2k+1:
-  //   gB [nc][n][n][4]  -cofactors x weight at the k+1 Gauss points ([qx][qz])
+  //   gB [nc][n][n][4]  cofactors x weight at the k+1 Gauss points ([qx][qz])
   //   fB [nc][4][n][2]  half outward normal x weight at the k+1 face points
   //   gC [nc][c][c][4], gJ [nc][c][c]  cofactors and det J / (gamma-1) x weight
   //   fC [nc][4][q][2]  outward normal x weight at the 2k+1 face points, times

@@ -94,6 +94,42 @@ __device__ __forceinline__ void eo_interp(const T (&t)[K + 1], T (&v)[NP]) {
   }
 }
 
+// v_q = sum_i S(q,i) t_i and d_q = sum_i D(q,i) t_i
+template <int K, int SET, int NP, typename T>
+__device__ __forceinline__ void eo_interp_d(const T (&t)[K + 1], T (&v)[NP], T (&d)[NP]) {
+  constexpr int H = (K + 1) / 2, P = NP / 2;
+  constexpr bool MI = ((K + 1) & 1) != 0, MQ = (NP & 1) != 0;
+  eo_interp<K, SET>(t, v);
+  T te[H], to[H];
+#pragma unroll
+  for (int i = 0; i < H; ++i) {
+    te[i] = t[i] + t[K - i];
+    to[i] = t[i] - t[K - i];
+  }
+#pragma unroll
+  for (int q = 0; q < P + (MQ ? 1 : 0); ++q) {
+    T b = CEo<T>::get(K, SET, 3, q, 0) * to[0];
+#pragma unroll
+    for (int i = 1; i < H; ++i) b = fma(CEo<T>::get(K, SET, 3, q, i), to[i], b);
+    if (MQ && q == P) {  // E_D = 0 at the middle point
+      d[P] = b;
+    } else {
+      T a = CEo<T>::get(K, SET, 2, q, 0) * te[0];
+#pragma unroll
+      for (int i = 1; i < H; ++i) a = fma(CEo<T>::get(K, SET, 2, q, i), te[i], a);
+      if (MI) a = fma(CEo<T>::get(K, SET, 2, q, H), t[H], a);
+      d[q] = b + a;
+      d[NP - 1 - q] = b - a;
+    }
+  }
+}
+// d_q = sum_i D(q,i) t_i alone
+template <int K, int SET, int NP, typename T>
+__device__ __forceinline__ void eo_deriv(const T (&t)[K + 1], T (&d)[NP]) {
+  T v[NP];
+  eo_interp_d<K, SET>(t, v, d);  // the unused values are dropped by the compiler
+}
+
 // out_i = sum_q S(q,i) V_q + D(q,i) G_q
 template <int K, int SET, int NP, bool HAS_V, bool HAS_G, typename T>
 __device__ __forceinline__ void eo_integ(const T (&V)[NP], const T (&G)[NP], T (&out)[K + 1]) {
@@ -167,8 +203,10 @@ struct Vec4;
 template <>
 struct Vec4<float> {
   float v[4];
-  __device__ __forceinline__ explicit Vec4(const float *p) {  // 16-byte aligned
-    const float4 a = __ldg(reinterpret_cast<const float4 *>(p));
+  // 16-byte aligned, in global memory or (shared) in shared memory
+  __device__ __forceinline__ explicit Vec4(const float *p, bool shared = false) {
+    const float4 *s = reinterpret_cast<const float4 *>(p);
+    const float4 a = shared ? *s : __ldg(s);
     v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
   }
   __device__ __forceinline__ void store(float *p) const {
@@ -178,7 +216,7 @@ struct Vec4<float> {
 template <>
 struct Vec4<double> {
   double v[4];
-  __device__ __forceinline__ explicit Vec4(const double *p) {  // 16-byte aligned
+  __device__ __forceinline__ explicit Vec4(const double *p, bool = false) {  // 16-byte aligned
     const double2 a = __ldg(reinterpret_cast<const double2 *>(p));
     const double2 b = __ldg(reinterpret_cast<const double2 *>(p) + 1);
     v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;

@@ -12,19 +12,43 @@ struct SrcPtrs {
 
 // Values between two cells' A^{-1} blocks ([nc][stride]).  FP64: the full
 // (k+1)^2 x (k+1)^2 block.  FP32 (multigrid levels): A^{-1} is symmetric, so
-// only its lower triangle is stored, row by row ((r, c <= r) at
-// r (r+1)/2 + c), padded to a multiple of 16 bytes: the B kernel stages the
-// blocks of its cells into shared memory with 16-byte cp.async copies, and
-// half the bytes leave more room there.
+// only its lower triangle of (k+1) x (k+1) tiles is stored: tile (a, b), b <= a,
+// couples the node rows iz = a and iz = b.  Off-diagonal tiles come first
+// (row by row, each padded to a multiple of four values), then the diagonal
+// ones as packed lower triangles.  The B kernel stages the blocks of its cells
+// into shared memory with 16-byte copies and reads tiles in 16-byte loads; the
+// stride is 4 mod 8 values, so that eight cells' equal offsets fall into
+// eight different groups of four banks.
+template <int K>
+struct ATile {
+  static constexpr int NN = K + 1;
+  static constexpr int OFF = (NN * NN + 3) / 4 * 4;               // an off-diagonal tile
+  static constexpr int DIA = (NN * (NN + 1) / 2 + 3) / 4 * 4;     // a diagonal tile
+  static constexpr int D0 = NN * (NN - 1) / 2 * OFF;              // first diagonal tile
+  static constexpr int USED = D0 + NN * DIA;
+  static constexpr int STRIDE = USED % 8 == 4 ? USED : USED + 4;
+};
 template <int K, typename T>
 __host__ __device__ constexpr int ainv_stride() {
-  return sizeof(T) == 4
-             ? ((K + 1) * (K + 1) * ((K + 1) * (K + 1) + 1) / 2 + 3) / 4 * 4
-             : (K + 1) * (K + 1) * (K + 1) * (K + 1);
+  return sizeof(T) == 4 ? ATile<K>::STRIDE : (K + 1) * (K + 1) * (K + 1) * (K + 1);
+}
+// offset of entry (i, j), i >= j, in the FP32 tiles
+template <int K>
+__device__ __forceinline__ int atile_index(int i, int j) {
+  constexpr int NN = K + 1;
+  const int a = i / NN, b = j / NN, r = i - a * NN, c = j - b * NN;
+  if (a == b) return ATile<K>::D0 + a * ATile<K>::DIA + r * (r + 1) / 2 + c;
+  return (a * (a - 1) / 2 + b) * ATile<K>::OFF + r * NN + c;
 }
 inline long ainv_stride_rt(int k, size_t elem) {
-  const long n2 = (long)(k + 1) * (k + 1);
-  return elem == 4 ? (n2 * (n2 + 1) / 2 + 3) / 4 * 4 : n2 * n2;
+  if (elem != 4) return (long)(k + 1) * (k + 1) * (k + 1) * (k + 1);
+  switch (k) {
+    case 1: return ATile<1>::STRIDE;
+    case 2: return ATile<2>::STRIDE;
+    case 3: return ATile<3>::STRIDE;
+    case 4: return ATile<4>::STRIDE;
+    default: return ATile<5>::STRIDE;
+  }
 }
 
 // 16-byte asynchronous global -> shared copies (cp.async, bypassing L1) and

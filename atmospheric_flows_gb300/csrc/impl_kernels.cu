@@ -261,8 +261,8 @@ __global__ void __launch_bounds__(32 * BI_WARPS)
     __syncwarp();
   }
   T *o = out + (long)c * ainv_stride<K, T>();
-  if constexpr (sizeof(T) == 4) {  // packed lower triangle (ainv_stride)
-    for (int e = lane; e < NTRI; e += 32) o[e] = -M[e];
+  if constexpr (sizeof(T) == 4) {  // lower triangle of tiles (ATile)
+    for (int e = lane; e < NTRI; e += 32) o[atile_index<K>(ti[e], tj[e])] = -M[e];
   } else {
     for (int e = lane; e < NN2 * NN2; e += 32) {
       const int j = e / NN2, i = e - j * NN2;

@@ -100,7 +100,7 @@ __global__ void k_exact_tables(MeshT<T> m, const double *__restrict__ map2, Exac
     const long o = (c * np * np + e) * 4;
     for (int d = 0; d < 4; ++d) {
       if (s) m.gC[o + d] = (T)(GAS_GAMMA / (GAS_GAMMA - 1.0) * cof[d]);
-      else m.gB[o + d] = (T)(-cof[d]);
+      else m.gB[o + d] = (T)cof[d];
     }
     if (s) m.gJ[c * np * np + e] = (T)((J[0] * J[3] - J[1] * J[2]) * w / (GAS_GAMMA - 1.0));
   } else {

@@ -29,10 +29,10 @@
 // factors.  p_fix enters C as H = gamma/(gamma-1) p_fix cof per point and as
 // its face traces, prepared when p_fix is set.
 //
-// Measured on GB300 at 51,200 cells, k = 4, FP64 (before: the kernels of
-// schur_kernels.cuh, 2k+1 points everywhere, 9 threads per cell): B with A^{-1}
-// 0.56 -> 0.28 ms, C/D 0.55 -> 0.33 ms, the FP64 pipe busy 83-86% in both; the
-// FP32 V-cycle 1.53 -> 0.97 ms.
+// Measured on GB300 at 51,200 cells, k = 4 (before: the kernels of
+// schur_kernels.cuh, 2k+1 points everywhere, 9 threads per cell): FP64 B with
+// A^{-1} 0.56 -> 0.26 ms, C/D 0.55 -> 0.33 ms, the FP64 pipe busy 83-86% in
+// both; the FP32 V-cycle 1.54 -> 0.84 ms.
 //
 // In the Schur apply, B stores w = cB cC A^{-1} B p and C/D applies C with unit
 // coefficient: C is homogeneous of degree one in w for the positive cC
@@ -54,6 +54,13 @@ __device__ __forceinline__ T flux_C(const T *__restrict__ g, T wx, T wz, T vx, T
   return fma(abs_max(up, um), (a - b) * T(1.0 / GAS_GAMMA), fma(a, up, b * um));
 }
 
+// asynchronous copy of n contiguous values into shared memory by the block;
+// both addresses 16-byte aligned (blocks start at multiples of 8 cells)
+__device__ __forceinline__ void stage(float *s, const float *g, int n) {
+  for (int e = threadIdx.x; e < n / 4; e += blockDim.x) cp_async16(s + 4 * e, g + 4 * e);
+  for (int e = n / 4 * 4 + threadIdx.x; e < n; e += blockDim.x) cp_async4(s + e, g + e);
+}
+
 // face contributions of the output row iz: faces x = 0, 1 add to the row's
 // ends, faces z = 0, 1 to the whole first and last row.  F: [4][NN]
 template <int K, typename T>
@@ -67,24 +74,100 @@ __device__ __forceinline__ void face_rows(const T *__restrict__ F, int iz, T (&a
   add[K] += F[NN + iz];
 }
 
+// (rows NN of A^{-1}) x (b0, b1) of one cell, FP32 tiles: thread (cell, a) owns
+// the node row iz = a, s0/s1[r] for the nodes (a, r).  b holds (b0, b1) pairs.
+template <int K>
+__device__ __forceinline__ void atile_apply(const float *__restrict__ A,
+                                            const float2 *__restrict__ b, int a,
+                                            float (&s0)[K + 1], float (&s1)[K + 1]) {
+  using L = ATile<K>;
+  constexpr int NN = K + 1;
+#pragma unroll
+  for (int r = 0; r < NN; ++r) s0[r] = s1[r] = 0.0f;
+#pragma unroll
+  for (int t = 0; t < NN; ++t) {
+    float2 v[NN];
+#pragma unroll
+    for (int j = 0; j < NN; ++j) v[j] = b[t * NN + j];
+    if (t == a) {
+      float d[L::DIA];
+#pragma unroll
+      for (int i = 0; i < L::DIA; i += 4)
+        *reinterpret_cast<float4 *>(d + i) =
+            *reinterpret_cast<const float4 *>(A + L::D0 + t * L::DIA + i);
+#pragma unroll
+      for (int r = 0; r < NN; ++r)
+#pragma unroll
+        for (int j = 0; j < NN; ++j) {
+          const float x = d[r >= j ? r * (r + 1) / 2 + j : j * (j + 1) / 2 + r];
+          s0[r] = fmaf(x, v[j].x, s0[r]);
+          s1[r] = fmaf(x, v[j].y, s1[r]);
+        }
+    } else {
+      const int hi = max(a, t), lo = min(a, t);
+      const float *T = A + (hi * (hi - 1) / 2 + lo) * L::OFF;
+      float d[L::OFF];
+#pragma unroll
+      for (int i = 0; i < L::OFF; i += 4)
+        *reinterpret_cast<float4 *>(d + i) = *reinterpret_cast<const float4 *>(T + i);
+      if (a > t) {
+#pragma unroll
+        for (int r = 0; r < NN; ++r)
+#pragma unroll
+          for (int j = 0; j < NN; ++j) {
+            s0[r] = fmaf(d[r * NN + j], v[j].x, s0[r]);
+            s1[r] = fmaf(d[r * NN + j], v[j].y, s1[r]);
+          }
+      } else {  // the transposed tile
+#pragma unroll
+        for (int r = 0; r < NN; ++r)
+#pragma unroll
+          for (int j = 0; j < NN; ++j) {
+            s0[r] = fmaf(d[j * NN + r], v[j].x, s0[r]);
+            s1[r] = fmaf(d[j * NN + r], v[j].y, s1[r]);
+          }
+      }
+    }
+  }
+}
+
 // ====================================================================== B ===
 // MODE 0: dst = cB B p ; 1: dst -= cB B p ; 2: dst = cB cC A^{-1} B p
 // (with a per-cell time-step multiplier d: cB d and cC d).
-// Threads (cell, j), j < k+1; `cpb` cells per block.
+//
+// B is evaluated in its strong form: with exact quadrature
+//   -int p d(phi) + oint p* n phi = int d(p) phi - oint (p - p*) n phi,
+// which takes one derivative of p (six percent fewer FP64 instructions than
+// testing with the gradients of both components) and has no wall term (p* = p
+// there).  p - p* is half the jump of p.
+//
+// The first 4 cpb threads take the faces, the next (k+1) cpb the rows, then
+// the columns and the output rows; A^{-1} is dealt out over all of them.
+// `cpb` cells per block, a multiple of 8 (whole warps of face threads).
+template <int K>
+struct ExB {
+  static constexpr int TPC = K + 5;         // threads per cell
+  static constexpr int XV = 2 * (K + 1) * (K + 1), FV = 8 * (K + 1);
+  template <typename T>
+  static constexpr int values(bool stage) {  // shared-memory values per cell
+    return 2 * XV + FV + (stage ? ainv_stride<K, T>() : 0);
+  }
+};
+
 template <int K, int MODE, typename T, bool HG>
-__global__ void __launch_bounds__(192)
+__global__ void __launch_bounds__(320)
     k_exact_B(T *__restrict__ dst, const T *__restrict__ p, T cB, T cC,
               const T *__restrict__ ainv, MeshT<T> mesh, int cpb) {
-  constexpr int NN = K + 1, NN2 = NN * NN;
+  constexpr int NN = K + 1, NN2 = NN * NN, XV = ExB<K>::XV, FV = ExB<K>::FV;
   constexpr bool STAGE = MODE == 2 && sizeof(T) == 4;
   constexpr int AS = ainv_stride<K, T>();
   extern __shared__ __align__(16) unsigned char sm_raw[];
   T *sm = reinterpret_cast<T *>(sm_raw);
-  T *as = sm;                                  // [cpb][AS] staged A^{-1} (STAGE)
-  T *Xs = sm + (STAGE ? cpb * AS : 0);         // [cpb][NN2] x-interpolated p
-  T *Y = Xs + cpb * NN2;                       // [cpb][2 comp][2][NN2]
-  T *Fs = Y + cpb * 4 * NN2;                   // [cpb][2 comp][4][NN]
-  const int tid = threadIdx.x, lc = tid / NN, j = tid - lc * NN;
+  T *as = sm;                                // [cpb][AS] staged A^{-1} (STAGE)
+  T *Xs = sm + (STAGE ? cpb * AS : 0);       // [cpb][2][NN2] p, d_xi p at (iz, qx); then B p pairs
+  T *Y = Xs + cpb * XV;                      // [cpb][2 comp][NN2]; then the result
+  T *Fs = Y + cpb * XV;                      // [cpb][2 comp][4][NN]
+  const int tid = threadIdx.x;
   const int c0 = blockIdx.x * cpb;
   const int cnt = min(cpb, mesh.nc - c0);
   if constexpr (STAGE) {
@@ -95,45 +178,49 @@ __global__ void __launch_bounds__(192)
     for (int e = tid; e < n16; e += blockDim.x) cp_async16(as + 4 * e, src + 4 * e);
     cp_async_commit();
   }
-  const bool active = lc < cnt;
+  const int rt = tid - 4 * cpb;             // row/column threads: rt >= 0
+  const int lc = rt / NN, j = rt - lc * NN;
+  const bool active = rt >= 0 && lc < cnt;
   const int c = c0 + lc;
   if (active) {
-    // row j: x-interpolation to the k+1 Gauss points
-    {
-      T t[NN], v[NN];
-      const T *row = p + (long)c * NN2 + j * NN;
+    // row j: values and xi-derivatives at the k+1 Gauss points
+    T t[NN], v[NN], d[NN];
+    const T *row = p + (long)c * NN2 + j * NN;
 #pragma unroll
-      for (int i = 0; i < NN; ++i) t[i] = __ldg(row + i);
-      eo_interp<K, 0>(t, v);
+    for (int i = 0; i < NN; ++i) t[i] = __ldg(row + i);
+    eo_interp_d<K, 0>(t, v, d);
+    T *x = Xs + lc * XV + j * NN;
 #pragma unroll
-      for (int i = 0; i < NN; ++i) Xs[lc * NN2 + j * NN + i] = v[i];
+    for (int i = 0; i < NN; ++i) {
+      x[i] = v[i];
+      x[NN2 + i] = d[i];
     }
-    // faces j, j + NN, ...: fB holds half the outward normal times the weight
-    for (int f = j; f < 4; f += NN) {
-      const int nb = mesh.nbr[c * 4 + f], nfc = mesh.nbrf[c * 4 + f];
-      const int code = HG && nb >= 0 ? nfc >> 2 : 0;
-      T own[NN], o0[NN], o1[NN];
-      trace<K>(p + (long)c * NN2, f, own);
+  } else if (rt < 0 && tid < 4 * cnt) {
+    // fB, hB hold half the outward normal times the weight; what is added to
+    // the rows is half the jump times it
+    const int l = tid >> 2, f = tid & 3, cf = c0 + l;
+    const int nb = mesh.nbr[cf * 4 + f], nfc = mesh.nbrf[cf * 4 + f];
+    const int code = HG && nb >= 0 ? nfc >> 2 : 0;
+    T own[NN], o0[NN], o1[NN];
+#pragma unroll
+    for (int i = 0; i < NN; ++i) o0[i] = o1[i] = T(0);
+    if (nb >= 0) {
+      trace<K>(p + (long)cf * NN2, f, own);
       if (!HG || code < 3) {
         T nbt[NN], s[NN], F0[NN], F1[NN];
-        if (nb >= 0) {
-          trace<K>(p + (long)nb * NN2, nfc & 3, nbt);
-        } else {  // wall, p_D = p
-#pragma unroll
-          for (int i = 0; i < NN; ++i) nbt[i] = own[i];
-        }
+        trace<K>(p + (long)nb * NN2, nfc & 3, nbt);
         if (!HG || code == 0) {
 #pragma unroll
-          for (int i = 0; i < NN; ++i) nbt[i] += own[i];
+          for (int i = 0; i < NN; ++i) nbt[i] -= own[i];
           eo_interp<K, 0>(nbt, s);
         } else {  // fine side: the coarse neighbour at the shifted points
           T sn[NN];
-          eo_interp<K, 0>(own, s);
-          sub_interp<K, 0>(nbt, code - 1, sn);
+          eo_interp<K, 0>(own, sn);
+          sub_interp<K, 0>(nbt, code - 1, s);
 #pragma unroll
-          for (int q = 0; q < NN; ++q) s[q] += sn[q];
+          for (int q = 0; q < NN; ++q) s[q] -= sn[q];
         }
-        const T *g = mesh.fB + ((long)c * 4 + f) * 2 * NN;
+        const T *g = mesh.fB + ((long)cf * 4 + f) * 2 * NN;
 #pragma unroll
         for (int q = 0; q < NN; ++q) {
           T n0, n1;
@@ -144,19 +231,17 @@ __global__ void __launch_bounds__(192)
         eo_integ<K, 0, NN, true, false>(F0, F0, o0);
         eo_integ<K, 0, NN, true, false>(F1, F1, o1);
       } else {  // coarse side: two subfaces
-#pragma unroll
-        for (int i = 0; i < NN; ++i) o0[i] = o1[i] = T(0);
         for (int h = 0; h < 2; ++h) {
           T nbt[NN], s[NN], sn[NN], F0[NN], F1[NN];
           trace<K>(p + (long)mesh.hnb[nb * 2 + h] * NN2, nfc & 3, nbt);
-          sub_interp<K, 0>(own, h, s);
-          eo_interp<K, 0>(nbt, sn);
+          sub_interp<K, 0>(own, h, sn);
+          eo_interp<K, 0>(nbt, s);
           const T *g = mesh.hB + ((long)nb * 2 + h) * 2 * NN;
 #pragma unroll
           for (int q = 0; q < NN; ++q) {
             T n0, n1;
             load2(g + 2 * q, n0, n1);
-            s[q] += sn[q];
+            s[q] -= sn[q];
             F0[q] = n0 * s[q];
             F1[q] = n1 * s[q];
           }
@@ -164,45 +249,43 @@ __global__ void __launch_bounds__(192)
           sub_integ_add<K, 0>(F1, h, o1);
         }
       }
+    }
+    T *F = Fs + l * FV + f * NN;
 #pragma unroll
-      for (int i = 0; i < NN; ++i) {
-        Fs[((lc * 2 + 0) * 4 + f) * NN + i] = o0[i];
-        Fs[((lc * 2 + 1) * 4 + f) * NN + i] = o1[i];
-      }
+    for (int i = 0; i < NN; ++i) {
+      F[i] = o0[i];
+      F[4 * NN + i] = o1[i];
     }
   }
   __syncthreads();
   if (active) {
-    // column j: z-interpolation, fluxes, z-integration
-    T t[NN], v[NN];
+    // column j: gradient at the points, z-integration of both components
+    T t[NN], px[NN], pe[NN], G0[NN], G1[NN], b[NN];
+    const T *x = Xs + lc * XV + j;
 #pragma unroll
-    for (int i = 0; i < NN; ++i) t[i] = Xs[lc * NN2 + i * NN + j];
-    eo_interp<K, 0>(t, v);
+    for (int i = 0; i < NN; ++i) t[i] = x[NN2 + i * NN];
+    eo_interp<K, 0>(t, px);
+#pragma unroll
+    for (int i = 0; i < NN; ++i) t[i] = x[i * NN];
+    eo_deriv<K, 0>(t, pe);
     const T *g = mesh.gB + ((long)c * NN + j) * NN * 4;
-    T G[4][NN];
 #pragma unroll
     for (int q = 0; q < NN; ++q) {
-      const Vec4<T> w(g + 4 * q);  // -cof of (xi, eta) for x, then for z
-#pragma unroll
-      for (int d = 0; d < 4; ++d) G[d][q] = w.v[d] * v[q];
+      const Vec4<T> w(g + 4 * q);  // cofactors of (xi, eta) for d/dx, then for d/dz
+      G0[q] = fma(w.v[0], px[q], w.v[1] * pe[q]);
+      G1[q] = fma(w.v[2], px[q], w.v[3] * pe[q]);
     }
+    T *y = Y + lc * XV + j;
+    eo_integ<K, 0, NN, true, false>(G0, G0, b);
 #pragma unroll
-    for (int comp = 0; comp < 2; ++comp) {
-      T a[NN], b[NN];
-      eo_integ<K, 0, NN, false, true>(G[2 * comp + 1], G[2 * comp + 1], a);
-      eo_integ<K, 0, NN, true, false>(G[2 * comp], G[2 * comp], b);
-      T *y = Y + (lc * 2 + comp) * 2 * NN2 + j;
+    for (int i = 0; i < NN; ++i) y[i * NN] = b[i];
+    eo_integ<K, 0, NN, true, false>(G1, G1, b);
 #pragma unroll
-      for (int i = 0; i < NN; ++i) {
-        y[i * NN] = a[i];
-        y[NN2 + i * NN] = b[i];
-      }
-    }
+    for (int i = 0; i < NN; ++i) y[NN2 + i * NN] = b[i];
   }
   __syncthreads();
   if (active) {
-    // output row j; MODE 2 leaves it in place of its own Y row (nobody else
-    // reads that row)
+    // output row j; MODE 2 leaves (B p)_x, (B p)_z pairs in Xs
     T s = MODE == 2 ? cB * cC : cB;
     if (mesh.dts) {
       const T d = mesh.dts[c];
@@ -210,20 +293,17 @@ __global__ void __launch_bounds__(192)
     }
 #pragma unroll
     for (int comp = 0; comp < 2; ++comp) {
-      T *y = Y + (lc * 2 + comp) * 2 * NN2 + j * NN;
-      T a[NN], b[NN], out[NN], add[NN];
+      const T *y = Y + lc * XV + comp * NN2 + j * NN;
+      T a[NN], out[NN], add[NN];
 #pragma unroll
-      for (int i = 0; i < NN; ++i) {
-        a[i] = y[i];
-        b[i] = y[NN2 + i];
-      }
-      eo_integ<K, 0, NN, true, true>(a, b, out);
-      face_rows<K>(Fs + (lc * 2 + comp) * 4 * NN, j, add);
+      for (int i = 0; i < NN; ++i) a[i] = y[i];
+      eo_integ<K, 0, NN, true, false>(a, a, out);
+      face_rows<K>(Fs + lc * FV + comp * 4 * NN, j, add);
       T *d = dst + ((long)c * 2 + comp) * NN2 + j * NN;
 #pragma unroll
       for (int i = 0; i < NN; ++i) {
         const T o = s * (out[i] + add[i]);
-        if (MODE == 2) y[i] = o;
+        if (MODE == 2) Xs[lc * XV + 2 * (j * NN + i) + comp] = o;
         else if (MODE == 1) d[i] -= o;
         else d[i] = o;
       }
@@ -232,34 +312,41 @@ __global__ void __launch_bounds__(192)
   if constexpr (MODE == 2) {
     if constexpr (STAGE) cp_async_wait_all();
     __syncthreads();
-    // rows (cell, i) of A^{-1}, NN per thread: consecutive threads read
-    // consecutive values of the cell's (symmetric) block
-    for (int e = tid; e < cnt * NN2; e += blockDim.x) {
-      const int l = e / NN2, i = e - l * NN2;
-      const T *b0 = Y + l * 4 * NN2, *b1 = b0 + 2 * NN2;
-      T s0 = T(0), s1 = T(0);
-      if constexpr (STAGE) {
-        // packed lower triangle: A_ij at i(i+1)/2 + j (j <= i), else j(j+1)/2 + i
-        const T *Ab = as + l * AS;
-        const int ri = i * (i + 1) / 2;
+    if constexpr (STAGE) {
+      // thread (a, cell): the node row a of the cell, then one coalesced copy
+      for (int e = tid; e < NN * cpb; e += blockDim.x) {
+        const int a = e / cpb, l = e - a * cpb;
+        if (l >= cnt) continue;
+        T s0[NN], s1[NN];
+        atile_apply<K>(as + l * AS, reinterpret_cast<const float2 *>(Xs + l * XV), a, s0, s1);
+        T *y = Y + l * XV + a * NN;
 #pragma unroll
-        for (int jj = 0; jj < NN2; ++jj) {
-          const T a = jj <= i ? Ab[ri + jj] : Ab[jj * (jj + 1) / 2 + i];
-          s0 = fma(a, b0[jj], s0);
-          s1 = fma(a, b1[jj], s1);
+        for (int r = 0; r < NN; ++r) {
+          y[r] = s0[r];
+          y[NN2 + r] = s1[r];
         }
-      } else {
+      }
+      __syncthreads();
+      T *d = dst + (long)c0 * XV;
+      for (int e = tid; e < cnt * XV; e += blockDim.x) d[e] = Y[e];
+    } else {
+      // rows (cell, i) of A^{-1}: consecutive threads read consecutive values
+      // of the cell's (symmetric) block
+      for (int e = tid; e < cnt * NN2; e += blockDim.x) {
+        const int l = e / NN2, i = e - l * NN2;
+        const T *b = Xs + l * XV;
+        T s0 = T(0), s1 = T(0);
         const T *Ab = ainv + (long)(c0 + l) * AS + i;
 #pragma unroll
         for (int jj = 0; jj < NN2; ++jj) {
           const T a = __ldg(Ab + jj * NN2);
-          s0 = fma(a, b0[jj], s0);
-          s1 = fma(a, b1[jj], s1);
+          s0 = fma(a, b[2 * jj], s0);
+          s1 = fma(a, b[2 * jj + 1], s1);
         }
+        T *d = dst + (long)(c0 + l) * 2 * NN2 + i;
+        d[0] = s0;
+        d[NN2] = s1;
       }
-      T *d = dst + (long)(c0 + l) * 2 * NN2 + i;
-      d[0] = s0;
-      d[NN2] = s1;
     }
   }
 }
@@ -280,11 +367,30 @@ __global__ void __launch_bounds__(288)
   constexpr int NF = WITH_D ? 3 : 2;
   constexpr int XS = NN * NC;
   extern __shared__ __align__(16) unsigned char sm_raw[];
-  T *X = reinterpret_cast<T *>(sm_raw);  // [cpb][NF][NN][NC] x-interpolated w, p; then xa, xb
-  T *Fs = X + cpb * NF * XS;             // [cpb][4][NN] face integrals of C w
+  // FP32 (multigrid levels, latency bound): H, det J and the Chebyshev vectors
+  // of the block's cells are contiguous and arrive in shared memory while the
+  // faces and rows are computed (V-cycle of 320x160, k = 4: 0.90 -> 0.84 ms)
+  constexpr bool STG = sizeof(T) == 4;
+  constexpr int NV = MODE == 4 ? 4 : 0;
+  T *sH = reinterpret_cast<T *>(sm_raw);       // [cpb][NC][NC][4] (STG)
+  T *sJ = sH + (STG ? cpb * 4 * NC2 : 0);      // [cpb][NC][NC]
+  T *sV = sJ + (STG ? cpb * NC2 : 0);          // [NV][cpb][NN2]: rhs, invd, d, x
+  T *X = sV + (STG ? NV * cpb * NN2 : 0);      // [cpb][NF][NN][NC] x-interpolated w, p; then xa, xb
+  T *Fs = X + cpb * NF * XS;                   // [cpb][4][NN] face integrals of C w
   const int tid = threadIdx.x, nt = blockDim.x;
   const int c0 = blockIdx.x * cpb;
   const int cnt = min(cpb, mesh.nc - c0);
+  if constexpr (STG) {
+    stage(sH, hq + (long)c0 * 4 * NC2, cnt * 4 * NC2);
+    if (WITH_D) stage(sJ, mesh.gJ + (long)c0 * NC2, cnt * NC2);
+    if constexpr (NV > 0) {
+      stage(sV, ch.rhs + (long)c0 * NN2, cnt * NN2);
+      stage(sV + cpb * NN2, invd + (long)c0 * NN2, cnt * NN2);
+      stage(sV + 2 * cpb * NN2, ch.d + (long)c0 * NN2, cnt * NN2);
+      stage(sV + 3 * cpb * NN2, p + (long)c0 * NN2, cnt * NN2);
+    }
+    cp_async_commit();
+  }
   // faces: one thread per (cell, face); with NC > 4 the first 4 cpb threads
   // (whole warps) take them while the others interpolate the rows
   for (int e = tid; e < 4 * cnt; e += nt) {
@@ -359,6 +465,7 @@ __global__ void __launch_bounds__(288)
       for (int q = 0; q < NC; ++q) X[l * NF * XS + r * NC + q] = v[q];
     }
   }
+  if constexpr (STG) cp_async_wait_all();
   __syncthreads();
   // columns: z-interpolation, fluxes, z-integration; xa and xb replace the
   // column's own x-interpolated values
@@ -374,17 +481,17 @@ __global__ void __launch_bounds__(288)
       for (int i = 0; i < NN; ++i) t[i] = x[XS + i * NC];
       eo_interp<K, 1>(t, wz);
       if (WITH_D) {
-        const T *jx = mesh.gJ + ((long)(c0 + l) * NC + j) * NC;
+        const T *jx = STG ? sJ + (l * NC + j) * NC : mesh.gJ + ((long)(c0 + l) * NC + j) * NC;
 #pragma unroll
         for (int i = 0; i < NN; ++i) t[i] = x[2 * XS + i * NC];
         eo_interp<K, 1>(t, V);
 #pragma unroll
-        for (int q = 0; q < NC; ++q) V[q] *= __ldg(jx + q);
+        for (int q = 0; q < NC; ++q) V[q] *= jx[q];
       }
-      const T *h = hq + ((long)(c0 + l) * NC + j) * NC * 4;
+      const T *h = STG ? sH + (l * NC + j) * NC * 4 : hq + ((long)(c0 + l) * NC + j) * NC * 4;
 #pragma unroll
       for (int q = 0; q < NC; ++q) {
-        const Vec4<T> H(h + 4 * q);  // (xi, eta) from w_x, then from w_z
+        const Vec4<T> H(h + 4 * q, STG);  // (xi, eta) from w_x, then from w_z
         Gx[q] = fma(H.v[0], wx[q], H.v[2] * wz[q]);
         Ge[q] = fma(H.v[1], wx[q], H.v[3] * wz[q]);
       }
@@ -423,10 +530,22 @@ __global__ void __launch_bounds__(288)
       else if (MODE == 2) dst[g] = invd[g] * r;
       else if (MODE == 3) dst[g] += s * r;
       else {
-        const T res = ch.rhs[g] - r;
-        const T dk = (ch.first ? T(0) : ch.a * ch.d[g]) + ch.b * invd[g] * res;
+        T rh, iv, dd, xx;
+        if constexpr (STG) {
+          const T *v = sV + e * NN + i;
+          rh = v[0];
+          iv = v[cpb * NN2];
+          dd = v[2 * cpb * NN2];
+          xx = v[3 * cpb * NN2];
+        } else {
+          rh = ch.rhs[g];
+          iv = invd[g];
+          dd = ch.d[g];
+          xx = ch.x[g];
+        }
+        const T dk = (ch.first ? T(0) : ch.a * dd) + ch.b * iv * (rh - r);
         ch.d[g] = dk;
-        ch.x[g] += dk;
+        ch.x[g] = xx + dk;
       }
     }
   }
@@ -486,17 +605,17 @@ inline int exact_cells(int cpb) { return (cpb + 7) / 8 * 8; }
 
 template <int K, typename T, bool HG>
 int exact_B_launch(const OpView<T> &v, T *dst, const T *p, T cB, T cC, int mode) {
-  constexpr int NN = K + 1, NN2 = NN * NN;
   auto launch = [&](int tuned) -> cudaError_t {
-    int cpb = exact_cells(tuned);
-    if (cpb * NN > 192) cpb = 192 / NN / 8 * 8;
-    const size_t sm = sizeof(T) * (size_t)cpb *
-                      (5 * NN2 + 8 * NN + (mode == 2 && sizeof(T) == 4 ? ainv_stride<K, T>() : 0));
+    int cpb = v.nc < 2048 ? 8 : exact_cells(tuned);
+    if (cpb * ExB<K>::TPC > 320) cpb = 320 / ExB<K>::TPC / 8 * 8;
+    const size_t sm =
+        sizeof(T) * (size_t)cpb * ExB<K>::template values<T>(mode == 2 && sizeof(T) == 4);
     void (*fn)(T *, const T *, T, T, const T *, MeshT<T>, int) =
         mode == 0 ? k_exact_B<K, 0, T, HG>
                   : (mode == 1 ? k_exact_B<K, 1, T, HG> : k_exact_B<K, 2, T, HG>);
     if (cudaError_t e = allow_smem(fn, sm); e != cudaSuccess) return e;
-    fn<<<(v.nc + cpb - 1) / cpb, cpb * NN, sm, v.st>>>(dst, p, cB, cC, v.ainv, v.mesh, cpb);
+    fn<<<(v.nc + cpb - 1) / cpb, cpb * ExB<K>::TPC, sm, v.st>>>(dst, p, cB, cC, v.ainv, v.mesh,
+                                                              cpb);
     return cudaGetLastError();
   };
   // mode 1 (dst -= B p) is not idempotent: it uses the choice made for mode 0
@@ -514,10 +633,11 @@ int exact_CD_launch(const OpView<T> &v, T *dst, const T *w, const T *p, T cC, in
   const T *pfix = v.pfix;
   const ChebArgs<T> ch = cheb ? *cheb : ChebArgs<T>{};
   auto launch = [&](int tuned) -> cudaError_t {
-    int cpb = exact_cells(tuned);
+    int cpb = v.nc < 2048 ? 8 : exact_cells(tuned);
     if (cpb * E::NC > 288) cpb = 288 / E::NC / 8 * 8;
-    const size_t sm =
-        sizeof(T) * (size_t)cpb * ((mode == 0 || mode == 3 ? 2 : 3) * E::NN * E::NC + 4 * E::NN);
+    const int staged = sizeof(T) == 4 ? 5 * E::NC2 + (mode == 4 ? 4 * E::NN2 : 0) : 0;
+    const size_t sm = sizeof(T) * (size_t)cpb *
+                      ((mode == 0 || mode == 3 ? 2 : 3) * E::NN * E::NC + 4 * E::NN + staged);
     void (*fn)(T *, const T *, const T *, const T *, const T *, const T *, T, const T *, MeshT<T>,
                ChebArgs<T>, int) = mode == 0   ? k_exact_CD<K, 0, T, HG>
                                    : mode == 1 ? k_exact_CD<K, 1, T, HG>

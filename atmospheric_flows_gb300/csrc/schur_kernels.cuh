@@ -124,12 +124,10 @@ __global__ void __launch_bounds__(Cfg<K>::MAX_THREADS)
       for (int i = col; i < NN2; i += NQ) {
         T s0 = T(0.0), s1 = T(0.0);
         if constexpr (STAGE) {
-          // packed lower triangle: A_ij at i(i+1)/2 + j (j <= i), else
-          // j(j+1)/2 + i; the same values in the same order as the full block
-          const int ri = i * (i + 1) / 2;
-#pragma unroll
+          // lower triangle of tiles (ATile); the same values in the same
+          // order as the full block
           for (int j = 0; j < NN2; ++j) {
-            const T a = j <= i ? Ab[ri + j] : Ab[j * (j + 1) / 2 + i];
+            const T a = Ab[j <= i ? atile_index<K>(i, j) : atile_index<K>(j, i)];
             s0 = fma(a, b0[j], s0);
             s1 = fma(a, b1[j], s1);
           }
