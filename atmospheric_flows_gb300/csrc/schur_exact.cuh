@@ -170,6 +170,7 @@ __global__ void __launch_bounds__(320)
   const int tid = threadIdx.x;
   const int c0 = blockIdx.x * cpb;
   const int cnt = min(cpb, mesh.nc - c0);
+  pdl_trigger();
   if constexpr (STAGE) {
     // cells c0 .. c0+cnt-1: cnt * AS values, 16-byte aligned (AS % 4 == 0);
     // they arrive while B is computed
@@ -178,6 +179,8 @@ __global__ void __launch_bounds__(320)
     for (int e = tid; e < n16; e += blockDim.x) cp_async16(as + 4 * e, src + 4 * e);
     cp_async_commit();
   }
+  // up to here only A^{-1}, which no kernel of the overlapping chain writes
+  pdl_wait();
   const int rt = tid - 4 * cpb;             // row/column threads: rt >= 0
   const int lc = rt / NN, j = rt - lc * NN;
   const bool active = rt >= 0 && lc < cnt;
@@ -380,9 +383,14 @@ __global__ void __launch_bounds__(288)
   const int tid = threadIdx.x, nt = blockDim.x;
   const int c0 = blockIdx.x * cpb;
   const int cnt = min(cpb, mesh.nc - c0);
+  pdl_trigger();
   if constexpr (STG) {
+    // no kernel of the overlapping chain writes these two
     stage(sH, hq + (long)c0 * 4 * NC2, cnt * 4 * NC2);
     if (WITH_D) stage(sJ, mesh.gJ + (long)c0 * NC2, cnt * NC2);
+  }
+  pdl_wait();
+  if constexpr (STG) {
     if constexpr (NV > 0) {
       stage(sV, ch.rhs + (long)c0 * NN2, cnt * NN2);
       stage(sV + cpb * NN2, invd + (long)c0 * NN2, cnt * NN2);
@@ -605,6 +613,7 @@ inline int exact_cells(int cpb) { return (cpb + 7) / 8 * 8; }
 
 template <int K, typename T, bool HG>
 int exact_B_launch(const OpView<T> &v, T *dst, const T *p, T cB, T cC, int mode) {
+  bool overlap = false;  // not while the tuner times the kernel
   auto launch = [&](int tuned) -> cudaError_t {
     int cpb = v.nc < 2048 ? 8 : exact_cells(tuned);
     if (cpb * ExB<K>::TPC > 320) cpb = 320 / ExB<K>::TPC / 8 * 8;
@@ -614,13 +623,13 @@ int exact_B_launch(const OpView<T> &v, T *dst, const T *p, T cB, T cC, int mode)
         mode == 0 ? k_exact_B<K, 0, T, HG>
                   : (mode == 1 ? k_exact_B<K, 1, T, HG> : k_exact_B<K, 2, T, HG>);
     if (cudaError_t e = allow_smem(fn, sm); e != cudaSuccess) return e;
-    fn<<<(v.nc + cpb - 1) / cpb, cpb * ExB<K>::TPC, sm, v.st>>>(dst, p, cB, cC, v.ainv, v.mesh,
-                                                              cpb);
-    return cudaGetLastError();
+    return launch_overlapped(overlap, fn, (v.nc + cpb - 1) / cpb, cpb * ExB<K>::TPC, sm, v.st, dst, p, cB,
+                             cC, v.ainv, v.mesh, cpb);
   };
   // mode 1 (dst -= B p) is not idempotent: it uses the choice made for mode 0
   const int cpb = tuned_cpb(v.tune, v.st, TF_B, K, mode == 1 ? 0 : mode, HG, (int)sizeof(T),
                             v.nc, mode != 1 && dst != p, launch);
+  overlap = !HG;
   ATM_CUDA(launch(cpb));
   g_kernel_launches.fetch_add(1);
   return ATM_OK;
@@ -632,6 +641,7 @@ int exact_CD_launch(const OpView<T> &v, T *dst, const T *w, const T *p, T cC, in
   using E = Ex<K>;
   const T *pfix = v.pfix;
   const ChebArgs<T> ch = cheb ? *cheb : ChebArgs<T>{};
+  bool overlap = false;  // not while the tuner times the kernel
   auto launch = [&](int tuned) -> cudaError_t {
     int cpb = v.nc < 2048 ? 8 : exact_cells(tuned);
     if (cpb * E::NC > 288) cpb = 288 / E::NC / 8 * 8;
@@ -645,15 +655,15 @@ int exact_CD_launch(const OpView<T> &v, T *dst, const T *w, const T *p, T cC, in
                                    : mode == 3 ? k_exact_CD<K, 3, T, HG>
                                                : k_exact_CD<K, 4, T, HG>;
     if (cudaError_t e = allow_smem(fn, sm); e != cudaSuccess) return e;
-    fn<<<(v.nc + cpb - 1) / cpb, cpb * E::NC, sm, v.st>>>(dst, w, p, pfix, v.pfq, v.pff, cC,
-                                                        v.invd, v.mesh, ch, cpb);
-    return cudaGetLastError();
+    return launch_overlapped(overlap, fn, (v.nc + cpb - 1) / cpb, cpb * E::NC, sm, v.st, dst, w, p, pfix,
+                             v.pfq, v.pff, cC, v.invd, v.mesh, ch, cpb);
   };
   // modes 3 (dst -= C w) and 4 (x += d) are not idempotent: they use the
   // choices made for modes 0 and 1
   const bool idem = mode < 3 && dst != w && dst != p && dst != pfix;
   const int key = mode == 3 ? 0 : (mode == 4 ? 1 : mode);
   const int cpb = tuned_cpb(v.tune, v.st, TF_CD, K, key, HG, (int)sizeof(T), v.nc, idem, launch);
+  overlap = !HG;
   ATM_CUDA(launch(cpb));
   g_kernel_launches.fetch_add(1);
   return ATM_OK;
