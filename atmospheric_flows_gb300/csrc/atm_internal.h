@@ -245,19 +245,27 @@ int vec_dot(cudaStream_t st, const double *x, const double *y, long n, double *r
             double *out);  // out[0] = x.y (device)
 // One Arnoldi orthogonalisation of the new direction w against V_0..V_j,
 // all of length n with stride n: classical Gram-Schmidt with one
-// re-orthogonalisation pass (CGS2), then V_{j+1} = w / |w| when |w| is
-// nonzero (w is overwritten by the unscaled result), in three sweeps over V:
-// project; subtract and project again; subtract and take the norm (the
-// arithmetic of five separate kernels, the same bits).  hcol[0..j] gets the projection
-// coefficients, *hn the remaining norm.  `dsmall` is device scratch of >= 65
-// values (dsmall[64] ends as |V_{j+1}|^2 before the scaling), `h_pinned` a
-// pinned host mirror of >= 65; one stream synchronisation.  (A second pass
+// re-orthogonalisation pass (CGS2), then V_{j+1} = w / |w| (w is overwritten by
+// the unscaled result), in three sweeps over V: project; subtract and
+// project again; subtract and take the norm.  hcol[0..j] gets the projection
+// coefficients, *hn the remaining norm.  `dsmall` is device scratch of 256
+// values whose last eight are zero between calls (dsmall[64] ends as |V_{j+1}|^2
+// before the scaling), `h_pinned` a pinned host mirror of >= 65; one stream
+// synchronisation.  (A second pass
 // only when the first cancels, by the criterion of Daniel, Gragg, Kaufman
 // and Stewart, saves nothing here: with the Jacobi-scaled Schur operator
 // close to the identity the first pass always cancels, and the extra
 // synchronisation made the step slower.)
 int arnoldi_step(cudaStream_t st, double *V, long n, int j, double *w, double *red,
                  double *dsmall, double *h_pinned, double *hcol, double *hn);
+// The three sweeps alone, on `segments` ranges eoff[s]..eoff[s+1] of the
+// vectors (eoff null: one range of n): coefficients h1, h2 and |w|^2 at rows 0,
+// 32 and 64 of coef and of the pinned `host` ([row][segment]).  `red` holds
+// 32 * segments * arnoldi_blocks() values, `ticket` one zero per segment.  No
+// synchronisation.
+int arnoldi_blocks(long n, int m, int segments);
+int arnoldi_sweeps(cudaStream_t st, double *V, long n, int j, double *w, const long *eoff,
+                   int segments, double *red, double *coef, unsigned *ticket, double *host);
 int vec_multidot(cudaStream_t st, const double *V, long ldv, int m, const double *w, long n,
                  double *red, double *out);  // out[l] = V_l . w, l < m
 // w += sign * sum_l h[l] V_l  (h device)
@@ -450,6 +458,7 @@ struct Members {
   long *eoff = nullptr;        // [n+1] first scalar-vector element of each member
   double *dts = nullptr;       // [nc] dt multiplier (device; mesh.dts points here)
   double *red = nullptr;       // partial sums [rows][n][sb] (device)
+  unsigned *ticket = nullptr;  // [n] block counters of the Arnoldi sweeps (device)
   double *out = nullptr;       // reduced values [rows][n] (device)
   double *h_out = nullptr;     // pinned host mirror of out
   double *coef = nullptr;      // coefficients [cols][n] (device)

@@ -65,9 +65,14 @@ __global__ void k_xmy_scaled(double *__restrict__ d, const double *__restrict__ 
 }
 __global__ void k_scale_inv_norm(double *__restrict__ d, const double *__restrict__ s,
                                  const double *__restrict__ nsq, long n) {
-  const double inv = 1.0 / sqrt(*nsq);
+  // one root and division per block: per thread they cost more FP64 time than
+  // the vector takes to move
+  __shared__ double inv;
+  if (threadIdx.x == 0) inv = 1.0 / sqrt(*nsq);
+  __syncthreads();
+  const double a = inv;
   for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
-    d[i] = s[i] * inv;
+    d[i] = s[i] * a;
 }
 
 __global__ void k_dot_partial(const double *__restrict__ x, const double *__restrict__ y, long n,
@@ -138,54 +143,129 @@ __global__ void k_multiaxpy(double *__restrict__ w, const double *__restrict__ V
   }
 }
 
-// w <- w - sum_l h[l] V_l over all m vectors, then the first M dot products
-// V_l . w with the updated w: "subtract, then project again" of CGS2 in one
-// sweep over V.  The per-element sums, the element-to-thread map and the
-// summation order are those of k_multiaxpy and k_multidot_partial, so the
-// results are the same bits as the two separate kernels.
-template <int M>
-__global__ void k_axpy_multidot(double *__restrict__ w, const double *__restrict__ V, long ldv,
-                                int m, const double *__restrict__ h, long n,
-                                double *__restrict__ red) {
-  __shared__ double sh[RT / 32];
-  double acc[M];
+// ------------------------------------------------------ Arnoldi sweeps --
+// One sweep over the basis V_0..V_{M-1} and the new direction w:
+//   MODE 0: out_l = V_l . w
+//   MODE 1: w -= sum_l h_l V_l, then out_l = V_l . w
+//   MODE 2: w -= sum_l h_l V_l, then out_0 = w . w
+// Block (b, s) works on its share of segment s (the whole vector, or one
+// member's range eoff[s]..eoff[s+1]); h and out are [row][segment].  All M dot
+// products stay in registers, so V is read once per sweep, and M is a template
+// parameter so that an element's M loads are in flight together.
+//
+// Bound by FP64 instructions at small vectors (n = 320,000: 28 vectors fit L2):
+// reducing M sums over a warp value by value takes 5 M additions per warp, as
+// much as the elements of a short thread.  The warp instead halves the set of
+// values it carries at each exchange (31 additions for 32 sums), and a thread
+// takes at least four elements.  The last block of a segment to finish sums the
+// partials in block order, which needs no second launch and never depends on
+// scheduling.  In MODE 2 it also writes all coefficients to the pinned
+// mirror `host` (rows 0.. h1, 32.. h2, 64 |w|^2), which saves the copy.
+// At n = 320,000, m = 8 / 20: 12 / 28 us (MODE 0), 17 / 34 us (MODE 1); before,
+// a kernel per eight vectors and one for the sum took 25-41 us each.
+template <int M, int MODE>
+__global__ void __launch_bounds__(RT, 1)
+    k_arnoldi(double *__restrict__ w, const double *__restrict__ V, long ldv,
+              const double *__restrict__ h, const long *__restrict__ eoff, long n,
+              double *__restrict__ red, double *__restrict__ out, unsigned *__restrict__ ticket,
+              const double *__restrict__ h1, double *__restrict__ host) {
+  constexpr int NS = MODE == 2 ? 1 : M;  // sums, and the power of two above
+  constexpr int NV = NS <= 1 ? 1 : NS <= 2 ? 2 : NS <= 4 ? 4 : NS <= 8 ? 8 : NS <= 16 ? 16 : 32;
+  __shared__ double sh[NV][RT / 32];
+  __shared__ bool last;
+  const int seg = blockIdx.y, ns = gridDim.y, b = blockIdx.x, nb = gridDim.x;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const long lo = eoff ? eoff[seg] : 0, hi = eoff ? eoff[seg + 1] : n;
+  double hc[MODE ? M : 1], acc[NV];
 #pragma unroll
-  for (int l = 0; l < M; ++l) acc[l] = 0.0;
-  for (long i = (long)blockIdx.x * RT + threadIdx.x; i < n; i += (long)RED_BLOCKS * RT) {
-    double v[M], s = 0.0;
+  for (int l = 0; l < NV; ++l) acc[l] = 0.0;
+  if (MODE) {
 #pragma unroll
-    for (int l = 0; l < M; ++l) {
-      v[l] = V[l * ldv + i];
-      s = fma(h[l], v[l], s);
+    for (int l = 0; l < M; ++l) hc[MODE ? l : 0] = h[(long)l * ns + seg];
+  }
+  for (long i = lo + (long)b * RT + threadIdx.x; i < hi; i += (long)nb * RT) {
+    double v[M], wi = w[i];
+#pragma unroll
+    for (int l = 0; l < M; ++l) v[l] = V[l * ldv + i];
+    if (MODE) {
+      double s = 0.0;
+#pragma unroll
+      for (int l = 0; l < M; ++l) s = fma(hc[MODE ? l : 0], v[l], s);
+      wi -= s;
+      w[i] = wi;
     }
-    for (int l = M; l < m; ++l) s = fma(h[l], V[l * ldv + i], s);
-    const double wi = w[i] + -1.0 * s;
-    w[i] = wi;
+    if (MODE == 2) {
+      acc[0] = fma(wi, wi, acc[0]);
+    } else {
 #pragma unroll
-    for (int l = 0; l < M; ++l) acc[l] = fma(v[l], wi, acc[l]);
+      for (int l = 0; l < NS; ++l) acc[l] = fma(v[l], wi, acc[l]);
+    }
   }
+  // after the exchanges the lane holds the sum of value lane / (32 / NV)
+  int s = NV;
 #pragma unroll
-  for (int l = 0; l < M; ++l) {
-    const double t = block_reduce<0>(acc[l], sh);
-    if (threadIdx.x == 0) red[(long)l * RED_BLOCKS + blockIdx.x] = t;
+  for (int off = 16; off > 0; off >>= 1) {
+    if (s > 1) {
+      const bool up = lane & off;
+#pragma unroll
+      for (int l = 0; l < NV / 2; ++l)
+        if (l < s / 2) {
+          const double give = up ? acc[l] : acc[l + s / 2], keep = up ? acc[l + s / 2] : acc[l];
+          acc[l] = keep + __shfl_xor_sync(0xffffffffu, give, off);
+        }
+      s /= 2;
+    } else {
+      acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], off);
+    }
   }
+  if (lane % (32 / NV) == 0) sh[lane / (32 / NV)][wid] = acc[0];
+  __syncthreads();
+  double *part = red + (long)seg * 32 * nb;
+  if (threadIdx.x < NS) {
+    double t = 0.0;
+#pragma unroll
+    for (int k = 0; k < RT / 32; ++k) t += sh[threadIdx.x][k];
+    part[(long)threadIdx.x * nb + b] = t;
+    __threadfence();
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(ticket + seg, 1u) == (unsigned)nb - 1;
+  __syncthreads();
+  if (!last) return;
+  for (int l = wid; l < NS; l += RT / 32) {
+    double t = 0.0;
+    for (int k = lane; k < nb; k += 32) t += __ldcg(part + (long)l * nb + k);
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) t += __shfl_xor_sync(0xffffffffu, t, off);
+    if (lane == 0) {
+      out[(long)l * ns + seg] = t;
+      if (MODE == 2) host[64L * ns + seg] = t;
+    }
+  }
+  if (MODE == 2)
+    for (int l = threadIdx.x; l < M; l += RT) {
+      host[(long)l * ns + seg] = h1[(long)l * ns + seg];
+      host[(32L + l) * ns + seg] = h[(long)l * ns + seg];
+    }
+  if (threadIdx.x == 0) ticket[seg] = 0;
 }
 
-// w <- w - sum_l h[l] V_l, then |w|^2 (k_multiaxpy followed by k_dot_partial
-// on w, in one sweep, same bits)
-__global__ void k_axpy_dot(double *__restrict__ w, const double *__restrict__ V, long ldv, int m,
-                           const double *__restrict__ h, long n, double *__restrict__ red) {
-  __shared__ double sh[RT / 32];
-  double acc = 0.0;
-  for (long i = (long)blockIdx.x * RT + threadIdx.x; i < n; i += (long)RED_BLOCKS * RT) {
-    double s = 0.0;
-    for (int l = 0; l < m; ++l) s = fma(h[l], V[l * ldv + i], s);
-    const double wi = w[i] + -1.0 * s;
-    w[i] = wi;
-    acc = fma(wi, wi, acc);
+template <int MODE>
+void arnoldi_sweep(cudaStream_t st, dim3 grid, double *w, const double *V, long n, int m,
+                   const double *h, const long *eoff, double *red, double *out, unsigned *ticket,
+                   const double *h1, double *host) {
+  switch (m) {
+#define ARNOLDI_M(M)                                                                        \
+  case M:                                                                                   \
+    k_arnoldi<M, MODE><<<grid, RT, 0, st>>>(w, V, n, h, eoff, n, red, out, ticket, h1, host); \
+    break;
+#define ARNOLDI_M4(M) ARNOLDI_M(M) ARNOLDI_M(M + 1) ARNOLDI_M(M + 2) ARNOLDI_M(M + 3)
+    ARNOLDI_M4(1) ARNOLDI_M4(5) ARNOLDI_M4(9) ARNOLDI_M4(13)
+    ARNOLDI_M4(17) ARNOLDI_M4(21) ARNOLDI_M4(25) ARNOLDI_M4(29)
+#undef ARNOLDI_M4
+#undef ARNOLDI_M
   }
-  acc = block_reduce<0>(acc, sh);
-  if (threadIdx.x == 0) red[blockIdx.x] = acc;
+  g_kernel_launches.fetch_add(1);
 }
 
 __global__ void k_maxdiff_partial(const double *__restrict__ a, const double *__restrict__ b,
@@ -307,47 +387,43 @@ int vec_multiaxpy(cudaStream_t st, double *w, const double *V, long ldv, int m,
   ATM_CHECK_LAUNCH("k_multiaxpy");
   return ATM_OK;
 }
-int arnoldi_step(cudaStream_t st, double *V, long n, int j, double *w, double *red,
-                 double *dsmall, double *h_pinned, double *hcol, double *hn) {
-  double *h1 = dsmall, *h2 = dsmall + 32, *nsq = dsmall + 64;
+int arnoldi_blocks(long n, int m, int segments) {
+  // at least four elements per thread; one block per SM where the kernel's
+  // registers (m > 8) leave room for one, two otherwise
+  const long most = (m > 8 ? 152L : 304L) / (segments < 1 ? 1 : segments);
+  long g = n / (4L * RT * (segments < 1 ? 1 : segments));
+  if (g > most) g = most;
+  return (int)(g < 1 ? 1 : g);
+}
+int arnoldi_sweeps(cudaStream_t st, double *V, long n, int j, double *w, const long *eoff,
+                   int segments, double *red, double *coef, unsigned *ticket, double *host) {
   const int m = j + 1;
   if (m > MAXM) {
     set_error("Arnoldi step: more basis vectors than the reduction buffer holds");
     return ATM_BAD_ARG;
   }
+  double *h1 = coef, *h2 = coef + 32L * segments, *nsq = coef + 64L * segments;
+  const dim3 grid(arnoldi_blocks(n, m, segments), segments);
+  arnoldi_sweep<0>(st, grid, w, V, n, m, nullptr, eoff, red, h1, ticket, nullptr, nullptr);
+  ATM_CUDA(cudaGetLastError());
+  arnoldi_sweep<1>(st, grid, w, V, n, m, h1, eoff, red, h2, ticket, nullptr, nullptr);
+  ATM_CUDA(cudaGetLastError());
+  arnoldi_sweep<2>(st, grid, w, V, n, m, h2, eoff, red, nsq, ticket, h1, host);
+  ATM_CUDA(cudaGetLastError());
+  return ATM_OK;
+}
+int arnoldi_step(cudaStream_t st, double *V, long n, int j, double *w, double *red,
+                 double *dsmall, double *h_pinned, double *hcol, double *hn) {
   int rc;
-  // h1 = V^T w
-  if ((rc = vec_multidot(st, V, n, m, w, n, red, h1))) return rc;
-  // w -= V h1 and h2 = V^T w, fused over the first 8 vectors
-  const int m0 = m < 8 ? m : 8;
-  switch (m0) {
-    case 1: k_axpy_multidot<1><<<RED_BLOCKS, RT, 0, st>>>(w, V, n, m, h1, n, red); break;
-    case 2: k_axpy_multidot<2><<<RED_BLOCKS, RT, 0, st>>>(w, V, n, m, h1, n, red); break;
-    case 3: k_axpy_multidot<3><<<RED_BLOCKS, RT, 0, st>>>(w, V, n, m, h1, n, red); break;
-    case 4: k_axpy_multidot<4><<<RED_BLOCKS, RT, 0, st>>>(w, V, n, m, h1, n, red); break;
-    case 5: k_axpy_multidot<5><<<RED_BLOCKS, RT, 0, st>>>(w, V, n, m, h1, n, red); break;
-    case 6: k_axpy_multidot<6><<<RED_BLOCKS, RT, 0, st>>>(w, V, n, m, h1, n, red); break;
-    case 7: k_axpy_multidot<7><<<RED_BLOCKS, RT, 0, st>>>(w, V, n, m, h1, n, red); break;
-    default: k_axpy_multidot<8><<<RED_BLOCKS, RT, 0, st>>>(w, V, n, m, h1, n, red); break;
-  }
-  g_kernel_launches.fetch_add(1);
-  for (int l0 = 8; l0 < m; l0 += 8) {
-    const int mm = m - l0 < 8 ? m - l0 : 8;
-    multidot_chunk(st, V + (long)l0 * n, n, mm, w, n, red + (long)l0 * RED_BLOCKS);
-  }
-  k_finalize<0><<<m, RT, 0, st>>>(red, h2);
-  ATM_CHECK_LAUNCH("k_axpy_multidot");
-  // w -= V h2 and |w|^2
-  k_axpy_dot<<<RED_BLOCKS, RT, 0, st>>>(w, V, n, m, h2, n, red);
-  g_kernel_launches.fetch_add(1);
-  k_finalize<0><<<1, RT, 0, st>>>(red, nsq);
-  ATM_CHECK_LAUNCH("k_axpy_dot");
-  ATM_CUDA(cudaMemcpyAsync(h_pinned, dsmall, 65 * sizeof(double), cudaMemcpyDeviceToHost, st));
+  if ((rc = arnoldi_sweeps(st, V, n, j, w, nullptr, 1, red, dsmall,
+                           reinterpret_cast<unsigned *>(dsmall + 248), h_pinned)))
+    return rc;
+  // scaled while the host waits; a zero or non-finite norm ends the cycle and
+  // nobody reads V_{j+1}
+  if ((rc = vec_scale_by_inv_norm(st, V + (long)(j + 1) * n, w, dsmall + 64, n))) return rc;
   ATM_CUDA(cudaStreamSynchronize(st));
   for (int l = 0; l <= j; ++l) hcol[l] = h_pinned[l] + h_pinned[32 + l];
   *hn = std::sqrt(h_pinned[64]);
-  if (*hn > 0.0 && std::isfinite(*hn))
-    if ((rc = vec_scale_by_inv_norm(st, V + (long)(j + 1) * n, w, nsq, n))) return rc;
   return ATM_OK;
 }
 int vec_maxdiff(cudaStream_t st, const double *a, const double *b, long n, double *red,

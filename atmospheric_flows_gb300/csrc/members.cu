@@ -165,6 +165,7 @@ void members_free(atm_ctx &c) {
   cudaFree(M.eoff);
   cudaFree(M.dts);
   cudaFree(M.red);
+  cudaFree(M.ticket);
   cudaFree(M.out);
   cudaFree(M.coef);
   if (M.h_out) cudaFreeHost(M.h_out);
@@ -248,7 +249,12 @@ int members_set(atm_ctx &c, int n, const int *cell_off, const double *dt) {
     if ((e = cudaMalloc(&M->cell_mem, c.nc * sizeof(int)))) return fail(e, "cudaMalloc members");
     if ((e = cudaMalloc(&M->eoff, (n + 1) * sizeof(long)))) return fail(e, "cudaMalloc members");
     if ((e = cudaMalloc(&M->dts, c.nc * sizeof(double)))) return fail(e, "cudaMalloc members");
-    if ((e = cudaMalloc(&M->red, (size_t)8 * n * M->sb * sizeof(double))))
+    // 8 columns of sb blocks, or the Arnoldi sweeps' 32
+    const size_t nred = (size_t)n * std::max(8 * M->sb, 32 * 304);
+    if ((e = cudaMalloc(&M->red, nred * sizeof(double))))
+      return fail(e, "cudaMalloc members");
+    if ((e = cudaMalloc(&M->ticket, n * sizeof(unsigned))) ||
+        (e = cudaMemsetAsync(M->ticket, 0, n * sizeof(unsigned), c.stream)))
       return fail(e, "cudaMalloc members");
     if ((e = cudaMalloc(&M->out, (size_t)MEM_ROWS * n * sizeof(double))))
       return fail(e, "cudaMalloc members");
@@ -324,13 +330,12 @@ int seg_multiaxpy(atm_ctx &c, double *w, const double *V, long ldv, int cols, do
 }
 
 int seg_scale(atm_ctx &c, double *d, const double *s) {
+  // the kernel reads the pinned coefficients in place: the host writes them
+  // again only after a synchronisation that follows it
   Members &M = *c.mem;
-  ATM_CUDA(cudaMemcpyAsync(M.coef, M.h_coef, (size_t)M.n * sizeof(double),
-                           cudaMemcpyHostToDevice, c.stream));
   const long n = c.n_scalar();
-  k_seg_scale<<<gs(n), 256, 0, c.stream>>>(d, s, M.coef, M.cell_mem, c.nn2, n);
+  k_seg_scale<<<gs(n), 256, 0, c.stream>>>(d, s, M.h_coef, M.cell_mem, c.nn2, n);
   ATM_CHECK_LAUNCH("k_seg_scale");
-  ATM_CUDA(cudaStreamSynchronize(c.stream));
   return ATM_OK;
 }
 
@@ -411,16 +416,12 @@ int krylov_members(atm_ctx &c, int precision, double *x, const double *b,
       } else if ((rc = schur_apply(c, w, Vj, true))) {
         return rc;
       }
-      // classical Gram-Schmidt, twice, with member-wise coefficients
-      if ((rc = seg_multidot(c, V, n, j + 1, w)) || (rc = seg_read(c, j + 1))) return rc;
-      std::vector<double> h1(M.h_out, M.h_out + (size_t)(j + 1) * nm);
-      for (size_t q = 0; q < h1.size(); ++q) hc[q] = h1[q];
-      if ((rc = seg_multiaxpy(c, w, V, n, j + 1, -1.0))) return rc;
-      if ((rc = seg_multidot(c, V, n, j + 1, w)) || (rc = seg_read(c, j + 1))) return rc;
-      std::vector<double> h2(M.h_out, M.h_out + (size_t)(j + 1) * nm);
-      for (size_t q = 0; q < h2.size(); ++q) hc[q] = h2[q];
-      if ((rc = seg_multiaxpy(c, w, V, n, j + 1, -1.0))) return rc;
-      if ((rc = seg_multidot(c, w, n, 1, w)) || (rc = seg_read(c, 1))) return rc;
+      // classical Gram-Schmidt, twice, with member-wise coefficients (a member
+      // that has stopped has a zero V_j and ends in exact zeros below)
+      if ((rc = arnoldi_sweeps(c.stream, V, n, j, w, M.eoff, nm, M.red, M.out, M.ticket, M.h_out)))
+        return rc;
+      ATM_CUDA(cudaStreamSynchronize(c.stream));
+      const double *h1 = M.h_out, *h2 = M.h_out + 32L * nm, *nsq = M.h_out + 64L * nm;
       bool more = false;
       for (int m = 0; m < nm; ++m) {
         hc[m] = 0.0;
@@ -429,7 +430,7 @@ int krylov_members(atm_ctx &c, int precision, double *x, const double *b,
         double *Hm = &H[(size_t)m * MR1 * mr], *gm = &g[(size_t)m * MR1];
         double *csm = &cs[(size_t)m * mr], *snm = &sn[(size_t)m * mr];
         for (int l = 0; l <= j; ++l) Hm[l * mr + j] = h1[(size_t)l * nm + m] + h2[(size_t)l * nm + m];
-        const double hn = std::sqrt(M.h_out[m]);
+        const double hn = std::sqrt(nsq[m]);
         if (!std::isfinite(hn)) {  // the member fails; its x is left as it was
           state[m] = ATM_NONFINITE;
           pending[m] = 0;
@@ -463,7 +464,7 @@ int krylov_members(atm_ctx &c, int precision, double *x, const double *b,
         }
       }
       if (!more) break;
-      if ((rc = seg_scale(c, V + (long)(j + 1) * n, w))) return rc;
+      if (j + 1 < mr && (rc = seg_scale(c, V + (long)(j + 1) * n, w))) return rc;
     }
     // x += sum_l y_l V_l (or Z_l) with each member's own y
     int cols = 0;
