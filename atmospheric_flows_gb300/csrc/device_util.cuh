@@ -74,10 +74,13 @@ __device__ __forceinline__ void cp_async_wait_all() {
 // pdl_trigger() (its own successor may do the same) and must call pdl_wait()
 // before it touches anything that an earlier kernel writes or reads: the wait
 // returns when the predecessor, and with it everything before, has completed.
-// Not inside a stream capture (replayed V-cycle graphs got 7% slower with
-// programmatic edges) and not for the hanging-face kernels (S apply of 6300
-// cells, k = 3: 84 -> 144 us); elsewhere S takes 18.8 instead of 22.5 us at 800
-// cells, k = 2, and 577 instead of 582 us at 51,200, k = 4.
+// A kernel triggers only if its successor's blocks then spread well: early
+// blocks of a grid that fits the GPU in a wave pack the SMs that are free first.
+// C/D does not trigger: the next operator's B packed itself that way and S took
+// 307 instead of 249 us at 11,781 cells, k = 5.  Not inside a stream capture
+// (replayed V-cycle graphs got 7% slower with programmatic edges) and not for
+// the hanging-face kernels (6300 cells, k = 3: 84 -> 88 us).  Elsewhere S takes
+// 18.4 instead of 22.5 us at 800 cells, k = 2, 249 instead of 252 at 11,781, k = 5.
 __device__ __forceinline__ void pdl_trigger() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }

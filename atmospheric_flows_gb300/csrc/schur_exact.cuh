@@ -170,7 +170,7 @@ __global__ void __launch_bounds__(320)
   const int tid = threadIdx.x;
   const int c0 = blockIdx.x * cpb;
   const int cnt = min(cpb, mesh.nc - c0);
-  pdl_trigger();
+  pdl_trigger();  // C/D may take the slots that the tail of this grid leaves
   if constexpr (STAGE) {
     // cells c0 .. c0+cnt-1: cnt * AS values, 16-byte aligned (AS % 4 == 0);
     // they arrive while B is computed
@@ -358,9 +358,11 @@ __global__ void __launch_bounds__(320)
 // MODE 0: dst = cC C w ; 3: dst -= cC C w
 // MODE 1: dst = D p - C w ; 2: dst = invd .* (D p - C w)
 // MODE 4: t = D p - C w with p = ch.x, then the Chebyshev update of ch
-// Threads (cell, column), column < NC; `cpb` cells per block, a multiple of 8.
+// Threads (cell, column), column < NC; `cpb` cells per block, a multiple of 8, at
+// most 32.  Three blocks per SM in FP64 (80 registers, k = 4): two leave the
+// SM's quarters with 4, 4, 3 and 3 warps (51,200 cells: S apply 577 -> 572 us).
 template <int K, int MODE, typename T, bool HG>
-__global__ void __launch_bounds__(288)
+__global__ void __launch_bounds__(32 * Ex<K>::NC, sizeof(T) == 8 ? 3 : 1)
     k_exact_CD(T *__restrict__ dst, const T *__restrict__ w, const T *__restrict__ p,
                const T *__restrict__ pfix, const T *__restrict__ hq, const T *__restrict__ pff,
                T cC, const T *__restrict__ invd, MeshT<T> mesh, ChebArgs<T> ch, int cpb) {
@@ -383,7 +385,6 @@ __global__ void __launch_bounds__(288)
   const int tid = threadIdx.x, nt = blockDim.x;
   const int c0 = blockIdx.x * cpb;
   const int cnt = min(cpb, mesh.nc - c0);
-  pdl_trigger();
   if constexpr (STG) {
     // no kernel of the overlapping chain writes these two
     stage(sH, hq + (long)c0 * 4 * NC2, cnt * 4 * NC2);
@@ -644,7 +645,7 @@ int exact_CD_launch(const OpView<T> &v, T *dst, const T *w, const T *p, T cC, in
   bool overlap = false;  // not while the tuner times the kernel
   auto launch = [&](int tuned) -> cudaError_t {
     int cpb = v.nc < 2048 ? 8 : exact_cells(tuned);
-    if (cpb * E::NC > 288) cpb = 288 / E::NC / 8 * 8;
+    if (cpb > 32) cpb = 32;
     const int staged = sizeof(T) == 4 ? 5 * E::NC2 + (mode == 4 ? 4 * E::NN2 : 0) : 0;
     const size_t sm = sizeof(T) * (size_t)cpb *
                       ((mode == 0 || mode == 3 ? 2 : 3) * E::NN * E::NC + 4 * E::NN + staged);
