@@ -138,26 +138,38 @@ __global__ void __launch_bounds__(Cfg<K>::THREADS)
 }
 
 // ================================================= exact block inverse ===
-// One warp per cell.  The (weighted) cell mass matrix
+// G lanes per cell (32 / G cells per warp).  The (weighted) cell mass matrix
 //   M[(iz,ix),(jz,jx)] = sum_q S(qz,iz)S(qz,jz) S(qx,ix)S(qx,jx) w(q) JxW(q)
-// is symmetric positive definite: only its lower triangle is assembled, in
-// packed storage, by sum factorisation over the symmetric 1D index pairs
-// (a <= b) with the products S(q,a)S(q,b) tabulated once per block.  It is
-// then inverted in place by the symmetric sweep operator (Gauss-Jordan
-// restricted to the lower triangle; SPD, no pivoting), which leaves -M^{-1}.
-// The inverse is written out in full, transposed (it is symmetric).
-constexpr int BI_WARPS = 2;
+// is symmetric positive definite and depends only on the two unordered 1D
+// index pairs {iz,jz} and {ix,jx}: 225 sums at k = 4, each stored in one or two
+// places of the packed lower triangle, by sum factorisation over the pairs with
+// the products S(q,a)S(q,b) tabulated once per block.  It is then inverted in
+// place by the symmetric sweep operator (Gauss-Jordan restricted to the
+// lower triangle; SPD, no pivoting), which leaves -M^{-1}.  The inverse is
+// written out in full, transposed (it is symmetric).
+//
+// Bound by FP64 instructions, which cost a warp the same with one useful lane
+// as with 32: with a warp per cell the pivots' divisions were a third of the
+// kernel and 325 triangle entries left 8% of the lanes idle.  Four cells per
+// warp share the division's instructions and fill the lanes.  Fewer than 4096
+// cells leave SMs without warps; there a warp per cell is the shorter chain.
+constexpr int BI_WARPS = 4;
 
 template <int K>
 struct BlockInvCfg {
   static constexpr int NN = K + 1, NQ = 2 * K + 1, NN2 = NN * NN, NQ2 = NQ * NQ;
   static constexpr int NP = NN * (NN + 1) / 2;        // 1D pairs a <= b
   static constexpr int NTRI = NN2 * (NN2 + 1) / 2;    // packed lower triangle
-  static constexpr int PER = NQ2 + NQ * NP + NTRI + 2 * NN2 + NN * NQ;  // per warp
-  // block tables: S products [NQ][NP], then byte tables of pair/triangle indices
+  // per cell: the triangle, the quadrature weights, and the x-contracted
+  // weights, whose space first holds the x-contracted weight field; the pivot
+  // columns reuse the space of the last two.  8 mod 16 values: two groups'
+  // equal offsets fall into different halves of the banks
+  static constexpr int TBX = NQ * (NP > NN ? NP : NN);
+  static constexpr int PER = (NTRI + NQ2 + TBX + 7) / 16 * 16 + 8;
+  // block tables: S products [NQ][NP], then byte tables of triangle indices
   static constexpr int TAB_BYTES = ((NQ * NP) * 8 + 2 * NTRI + 7) / 8 * 8;
   template <typename T>
-  static size_t smem() { return TAB_BYTES + sizeof(T) * (size_t)BI_WARPS * PER; }
+  static size_t smem(int cells) { return TAB_BYTES + sizeof(T) * (size_t)cells * PER; }
 };
 
 __device__ __forceinline__ int tri_index(int i, int j) {  // i >= j
@@ -167,12 +179,12 @@ __device__ __forceinline__ int sym_index(int i, int j) {
   return i >= j ? tri_index(i, j) : tri_index(j, i);
 }
 
-template <int K, typename T>
+template <int K, typename T, int G>
 __global__ void __launch_bounds__(32 * BI_WARPS)
     k_block_inverse(T *__restrict__ out, const T *__restrict__ weight, MeshT<T> mesh) {
   using B = BlockInvCfg<K>;
   constexpr int NN = B::NN, NQ = B::NQ, NN2 = B::NN2, NQ2 = B::NQ2, NP = B::NP;
-  constexpr int NTRI = B::NTRI;
+  constexpr int NTRI = B::NTRI, CPW = 32 / G;
   extern __shared__ __align__(16) unsigned char sm_raw[];
   T *ss = reinterpret_cast<T *>(sm_raw);                              // [NQ][NP]
   unsigned char *ti = sm_raw + (size_t)NQ * NP * sizeof(T);           // [NTRI] row
@@ -193,19 +205,20 @@ __global__ void __launch_bounds__(32 * BI_WARPS)
     tj[e] = (unsigned char)(e - i * (i + 1) / 2);
   }
   __syncthreads();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int c = blockIdx.x * BI_WARPS + warp;
-  if (c >= mesh.nc) return;  // warp-uniform; only warp-level barriers below
-  T *wq = wsm + warp * B::PER;   // [NQ2] w JxW at the quadrature points
+  const int warp = threadIdx.x >> 5, wl = threadIdx.x & 31, grp = wl / G, lane = wl & (G - 1);
+  const int cw = (blockIdx.x * BI_WARPS + warp) * CPW;  // first cell of the warp
+  if (cw >= mesh.nc) return;  // warp-uniform; only warp-level barriers below
+  const int c = min(cw + grp, mesh.nc - 1);  // a spare group repeats the last cell
+  T *M = wsm + (warp * CPW + grp) * B::PER;  // [NTRI] packed lower triangle
+  T *wq = M + NTRI;              // [NQ2] w JxW at the quadrature points
   T *Tb = wq + NQ2;              // [NQ][NP] x-contracted weights
-  T *M = Tb + NQ * NP;           // [NTRI] packed lower triangle
-  T *colk = M + NTRI;            // [NN2] pivot column
-  T *cd = colk + NN2;            // [NN2] pivot column / pivot
-  T *tx = cd + NN2;              // [NN][NQ] x-contracted weight field
-  const T *G = mesh.jw + c * mesh.jw_stride;
+  T *tx = Tb;                    // [NN][NQ] x-contracted weight field, before Tb
+  T *colk = wq, *cd = colk + NN2;  // [NN2] pivot column, and it over the pivot
+  static_assert(2 * NN2 <= NQ2 + NQ * NP, "pivot columns fit the assembly's space");
+  const T *J = mesh.jw + c * mesh.jw_stride;
   if (weight) {
     const T *wt = weight + (long)c * NN2;
-    for (int e = lane; e < NN * NQ; e += 32) {
+    for (int e = lane; e < NN * NQ; e += G) {
       const int iz = e / NQ, qx = e - iz * NQ;
       T s = T(0.0);
 #pragma unroll
@@ -213,18 +226,18 @@ __global__ void __launch_bounds__(32 * BI_WARPS)
       tx[e] = s;
     }
     __syncwarp();
-    for (int q = lane; q < NQ2; q += 32) {
+    for (int q = lane; q < NQ2; q += G) {
       const int qz = q / NQ, qx = q - qz * NQ;
       T s = T(0.0);
 #pragma unroll
       for (int iz = 0; iz < NN; ++iz) s = fma(bS<K, T>(qz, iz), tx[iz * NQ + qx], s);
-      wq[q] = s * G[q];
+      wq[q] = s * J[q];
     }
   } else {
-    for (int q = lane; q < NQ2; q += 32) wq[q] = G[q];
+    for (int q = lane; q < NQ2; q += G) wq[q] = J[q];
   }
   __syncwarp();
-  for (int e = lane; e < NQ * NP; e += 32) {
+  for (int e = lane; e < NQ * NP; e += G) {
     const int qz = e / NP, p = e - qz * NP;
     T s = T(0.0);
 #pragma unroll
@@ -232,41 +245,45 @@ __global__ void __launch_bounds__(32 * BI_WARPS)
     Tb[e] = s;
   }
   __syncwarp();
-  for (int e = lane; e < NTRI; e += 32) {
-    const int I = ti[e], J = tj[e];
-    const int iz = I / NN, ix = I - iz * NN, jz = J / NN, jx = J - jz * NN;
-    const int pz = sym_index(iz, jz), px = sym_index(ix, jx);
+  for (int e = lane; e < NP * NP; e += G) {
+    const int pz = e / NP, px = e - pz * NP;
     T s = T(0.0);
 #pragma unroll
     for (int qz = 0; qz < NQ; ++qz) s = fma(ss[qz * NP + pz], Tb[qz * NP + px], s);
-    M[e] = s;
+    const int zb = ti[pz], za = tj[pz], xb = ti[px], xa = tj[px];  // a <= b
+    M[tri_index(zb * NN + xb, za * NN + xa)] = s;
+    if (zb != za) M[tri_index(zb * NN + xa, za * NN + xb)] = s;
   }
   __syncwarp();
   // symmetric sweep on pivots k = 0..NN2-1:
   //   a_ij -= a_ik a_kj / a_kk (i, j != k);  a_ik = a_ik / a_kk;  a_kk = -1 / a_kk
   for (int k = 0; k < NN2; ++k) {
     const T d = T(1.0) / M[tri_index(k, k)];
-    for (int i = lane; i < NN2; i += 32) {  // NN2 = 36 > 32 for k = 5
+    for (int i = lane; i < NN2; i += G) {
       const T a = M[sym_index(i, k)];
       colk[i] = a;
       cd[i] = a * d;
     }
     __syncwarp();
-    for (int e = lane; e < NTRI; e += 32) {
+#pragma unroll 4
+    for (int e = lane; e < NTRI; e += G) {
       const int i = ti[e], j = tj[e];
       if (i != k && j != k) M[e] = fma(-cd[i], colk[j], M[e]);
     }
     __syncwarp();
-    for (int i = lane; i < NN2; i += 32) M[sym_index(i, k)] = i == k ? -d : cd[i];
+    for (int i = lane; i < NN2; i += G) M[sym_index(i, k)] = i == k ? -d : cd[i];
     __syncwarp();
   }
-  T *o = out + (long)c * ainv_stride<K, T>();
-  if constexpr (sizeof(T) == 4) {  // lower triangle of tiles (ATile)
-    for (int e = lane; e < NTRI; e += 32) o[atile_index<K>(ti[e], tj[e])] = -M[e];
-  } else {
-    for (int e = lane; e < NN2 * NN2; e += 32) {
-      const int j = e / NN2, i = e - j * NN2;
-      o[e] = -M[sym_index(i, j)];
+  for (int g = 0; g < CPW && cw + g < mesh.nc; ++g) {
+    T *o = out + (long)(cw + g) * ainv_stride<K, T>();
+    const T *Mg = wsm + (warp * CPW + g) * B::PER;
+    if constexpr (sizeof(T) == 4) {  // lower triangle of tiles (ATile)
+      for (int e = wl; e < NTRI; e += 32) o[atile_index<K>(ti[e], tj[e])] = -Mg[e];
+    } else {
+      for (int e = wl; e < NN2 * NN2; e += 32) {
+        const int j = e / NN2, i = e - j * NN2;
+        o[e] = -Mg[sym_index(i, j)];
+      }
     }
   }
 }
@@ -319,10 +336,12 @@ int invdiag_launch(const OpView<T> &v, T *out, int ncomp, const T *weight, T sca
 
 template <int K, typename T>
 int block_inverse_launch(const OpView<T> &v, T *out, const T *weight) {
-  const size_t sm = BlockInvCfg<K>::template smem<T>();
-  ATM_CUDA(allow_smem(k_block_inverse<K, T>, sm));
-  const int grid = (v.nc + BI_WARPS - 1) / BI_WARPS;
-  k_block_inverse<K, T><<<grid, 32 * BI_WARPS, sm, v.st>>>(out, weight, v.mesh);
+  const bool one = v.nc < 4096;  // a warp per cell, or four cells per warp
+  const int cells = BI_WARPS * (one ? 1 : 4);
+  const size_t sm = BlockInvCfg<K>::template smem<T>(cells);
+  void (*fn)(T *, const T *, MeshT<T>) = one ? k_block_inverse<K, T, 32> : k_block_inverse<K, T, 8>;
+  ATM_CUDA(allow_smem(fn, sm));
+  fn<<<(v.nc + cells - 1) / cells, 32 * BI_WARPS, sm, v.st>>>(out, weight, v.mesh);
   ATM_CHECK_LAUNCH("k_block_inverse");
   return ATM_OK;
 }
