@@ -26,9 +26,10 @@ int rhs_cell_launch(const atm_ctx &c, int stage, double *dst, const SrcPtrs &sp,
                     : (stage == 2 ? k_rhs_cell<K, 2, KIND, false> : k_rhs_cell<K, 3, KIND, false>);
   }
   auto launch = [&](int tuned) -> cudaError_t {
-    // below 2048 cells the tuner has no say: small blocks reach more SMs
-    int cpb = c.nc < 2048 ? 8 : (tuned + 7) / 8 * 8;
-    if (cpb * np > 288) cpb = 288 / np / 8 * 8;
+    // the tuner's candidates are 64, 128 and 256 threads' worth of columns;
+    // below 2048 cells it has no say: small blocks reach more SMs
+    const int threads = tuned >= 256 / E::NQ ? 256 : (tuned >= 128 / E::NQ ? 128 : 64);
+    const int cpb = (c.nc < 2048 ? 64 : threads) / np;
     const size_t sm = sizeof(double) * (size_t)cpb * RhsKind<KIND>::NF * E::NN * np;
     if (cudaError_t e = allow_smem(fn, sm); e != cudaSuccess) return e;
     fn<<<(c.nc + cpb - 1) / cpb, cpb * np, sm, c.stream>>>(dst, sp, co, c.mesh, c.fbuf, cpb);
@@ -87,7 +88,7 @@ template <int K>
 int rhs_kinetic_launch(const atm_ctx &c, double *dst, const double *base, const double *rho,
                        const double *u, double wgrav, double M2) {
   constexpr int NP = 2 * K + 1;
-  const int cpb = c.nc < 2048 ? 8 : 16;
+  const int cpb = (c.nc < 2048 ? 64 : 128) / NP;
   const size_t sm = sizeof(double) * (size_t)cpb * 3 * (K + 1) * NP;
   ATM_CUDA(allow_smem(k_rhs_kinetic<K>, sm));
   k_rhs_kinetic<K><<<(c.nc + cpb - 1) / cpb, cpb * NP, sm, c.stream>>>(dst, base, rho, u, wgrav, M2,

@@ -261,7 +261,7 @@ __device__ __forceinline__ void rhs_face_rows(const double *__restrict__ Fb, con
 
 // Threads (cell, column); `cpb` cells per block.
 template <int K, int ST, int KIND, bool EX>
-__global__ void __launch_bounds__(288)
+__global__ void __launch_bounds__(256)
     k_rhs_cell(double *__restrict__ dst, SrcPtrs src, StageCoef co, Mesh mesh,
                const double *__restrict__ Fb, int cpb) {
   using E = Ex<K>;
@@ -431,7 +431,7 @@ __global__ void __launch_bounds__(288)
 // (Atmospheric_Flow.cc:1135-1153).  At 51,200 cells, k = 4 it takes a seventh
 // of the time of the whole right-hand side.  Threads (cell, column).
 template <int K>
-__global__ void __launch_bounds__(288)
+__global__ void __launch_bounds__(256)
     k_rhs_kinetic(double *__restrict__ dst, const double *__restrict__ base,
                   const double *__restrict__ rho, const double *__restrict__ u, double wgrav,
                   double M2, Mesh mesh, int cpb) {
