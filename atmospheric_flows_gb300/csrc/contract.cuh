@@ -185,19 +185,6 @@ __device__ __forceinline__ void eo_integ(const T (&V)[NP], const T (&G)[NP], T (
   }
 }
 
-// max(|a|, |b|) on the integer pipe for doubles (a double comparison takes an
-// FP64 issue slot); a NaN on either side gives a NaN
-__device__ __forceinline__ double abs_max(double a, double b) {
-  const long long m = 0x7fffffffffffffffll;
-  const long long x = __double_as_longlong(a) & m, y = __double_as_longlong(b) & m;
-  return __longlong_as_double(x > y ? x : y);
-}
-__device__ __forceinline__ float abs_max(float a, float b) {
-  const int m = 0x7fffffff;
-  const int x = __float_as_int(a) & m, y = __float_as_int(b) & m;
-  return __int_as_float(x > y ? x : y);
-}
-
 template <typename T>
 struct Vec4;
 template <>

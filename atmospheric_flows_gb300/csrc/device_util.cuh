@@ -10,6 +10,19 @@ struct SrcPtrs {
   const double *p[12];
 };
 
+// max(|a|, |b|) on the integer pipe for doubles (a double comparison takes an
+// FP64 issue slot); a NaN on either side gives a NaN
+__device__ __forceinline__ double abs_max(double a, double b) {
+  const long long m = 0x7fffffffffffffffll;
+  const long long x = __double_as_longlong(a) & m, y = __double_as_longlong(b) & m;
+  return __longlong_as_double(x > y ? x : y);
+}
+__device__ __forceinline__ float abs_max(float a, float b) {
+  const int m = 0x7fffffff;
+  const int x = __float_as_int(a) & m, y = __float_as_int(b) & m;
+  return __int_as_float(x > y ? x : y);
+}
+
 // Values between two cells' A^{-1} blocks ([nc][stride]).  FP64: the full
 // (k+1)^2 x (k+1)^2 block.  FP32 (multigrid levels): A^{-1} is symmetric, so
 // only its lower triangle of (k+1) x (k+1) tiles is stored: tile (a, b), b <= a,

@@ -8,14 +8,9 @@
 // + 4 iz on the cell's vertices (Gauss-Lobatto points of degree 1).  Cell
 // geometry at the 27 Gauss points: dxi_e/dx_i * JxW (9 values), JxW, and the
 // gravity direction e_r a^2/r^2 (3); face geometry at the 9 points of each
-// local face: outward normal (3) and JxW.  Faces are element-centric: every
-// cell adds its own side of each of its six faces, reading the neighbour's
-// trace at the matching point (the face-point permutation handles the rotated
-// and flipped parameterisations where cubed-sphere patches meet), so no
-// atomics are needed.
-//
-// One thread per cell: the shell is the known-answer regression of the
-// reference, a few thousand cells, not a throughput path.
+// local face: outward normal (3) and JxW.  The face-point permutation handles
+// the rotated and flipped parameterisations where cubed-sphere patches meet.
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <vector>
@@ -33,6 +28,8 @@ constexpr double EARTH_A = 6.37122e6;  // equation_data.h:26
 __constant__ double c_phi[NQ][NN];      // basis values at the cell points
 __constant__ double c_dphi[NQ][NN][3];  // reference derivatives at the cell points
 __constant__ double c_fphi[6][NF][NN];  // basis values at the face points
+__constant__ double c_psi[NF][4];       // bilinear basis at the face points (any face)
+__constant__ double c_line[2];          // 1 - g_0 and g_0 of the three-point rule
 
 struct Geo3 {
   int nc;
@@ -41,6 +38,8 @@ struct Geo3 {
   const int *nbr;      // [nc][6]: neighbour or -1 (wall)
   const int *nbf;      // [nc][6]: neighbour's local face
   const int *nperm;    // [nc][6][9]: neighbour's point of each own face point
+  int nfaces = 0;      // faces in `own`
+  const int *own;      // cell * 6 + face of every face's owner: the inner faces, then the walls
 };
 
 struct Coef3 {
@@ -62,528 +61,568 @@ __device__ __forceinline__ double at_q(const double *t, int q) {
 }
 // k-th (k < 4) vertex of local face f, in increasing vertex order: the
 // vertices whose bit f/2 equals f%2.  The other four basis functions vanish
-// on the face exactly, so the face sums below skip them.
+// on the face exactly.
 __device__ __forceinline__ int fnode(int f, int k) {
   const int a = f >> 1, lo = k & ((1 << a) - 1);
   return lo | ((f & 1) << a) | ((k >> a) << (a + 1));
 }
-// the neighbour across face f of cell c at own face point q: its cell, its
-// local face and the matching point there (loaded once per face point)
-struct NbPt {
-  int nb, nf, qn;
-};
-__device__ __forceinline__ NbPt nb_point(const Geo3 &g, int c, int f, int q) {
-  return NbPt{g.nbr[c * 6 + f], g.nbf[c * 6 + f], g.nperm[(c * 6 + f) * NF + q]};
+
+// The kernels below are bound by their FP64 instructions (two lanes per clock
+// and SM; an instruction costs the same with few active lanes as with 32), so
+// their tasks are dealt out over all threads of a block and every quantity is
+// computed once:
+//   * a face is integrated once, by its owner (the "+" side of the face list),
+//     and its nodal integrals are stored for both cells.  On a face the four
+//     basis functions are the bilinear ones, the same table for every face;
+//     the neighbour's point and basis row come from the face's permutation;
+//   * a field is interpolated along x on the four edges first, then at each
+//     point by the bilinear weights of the other two directions (5 instead of 8
+//     FMAs a point), and cell integrals contract z, y, x in turn (372 instead
+//     of 864 FMAs per component; the derivative of the degree-1 basis is -1, +1);
+//   * what is linear with fixed coefficients is a dense table: B of the cell's
+//     own and its neighbours' vertices (20 FMAs per output), D, and the volume
+//     part of C for the current p_fix.
+// Measured on GB300 at 6144 cells against a warp per cell with every face from
+// both sides and dense point sums: B with A^{-1} 94 -> 15 us, C/D 99 -> 35 us
+// (25 of them the faces), the second stage's three right-hand sides together
+// 865 -> 335 us; the FP64 pipe is 64-84% busy.
+constexpr int FPB = 32;  // faces per block of the face kernels, 9 threads each
+
+// interpolation of degree-1 values to the three points, and its transpose
+__device__ __forceinline__ void line3(double a, double b, double s, double t, double (&v)[3]) {
+  v[0] = fma(s, a, t * b);  // s = 1 - g_0, t = g_0 (g_2 = 1 - g_0)
+  v[1] = 0.5 * (a + b);
+  v[2] = fma(t, a, s * b);
 }
-// The basis tables staged in a block's shared memory.  The warp-per-cell
-// kernels index them by lane (point, face, vertex): from constant memory,
-// whose cache serves one address per cycle, those divergent reads would be
-// serialised.
-constexpr int TAB3 = NQ * NN + NQ * NN * 3 + 6 * NF * NN;
-struct Tab3S {
-  const double (*phi)[NN];
-  const double (*dphi)[NN][3];
-  const double (*fphi)[NF][NN];
+__device__ __forceinline__ void line3_t(double v0, double v1, double v2, double s, double t,
+                                        double &a, double &b) {
+  const double h = 0.5 * v1;
+  a = fma(s, v0, fma(t, v2, h));
+  b = fma(t, v0, fma(s, v2, h));
+}
+
+// ---------------------------------------------------------- face tables --
+// A face kernel's view of one face point: own cell and face, neighbour (-1: a
+// wall), the two bilinear rows and the normal times the face weight
+struct FacePt {
+  int c, f, nb, nf;
+  double w[4], v[4], n[3];
 };
-__device__ __forceinline__ Tab3S stage_tab3(double *buf) {
-  const double *src[3] = {&c_phi[0][0], &c_dphi[0][0][0], &c_fphi[0][0][0]};
-  const int len[3] = {NQ * NN, NQ * NN * 3, 6 * NF * NN};
-  double *dst = buf;
+__device__ __forceinline__ FacePt face_point(const Geo3 &g, int e, int q) {
+  FacePt P;
+  P.c = e / 6;
+  P.f = e - P.c * 6;
+  P.nb = g.nbr[e];
+  P.nf = g.nbf[e];
+  const int qn = g.nperm[e * NF + q];
+  const double *fq = g.fg + ((long)e * NF + q) * 4;
 #pragma unroll
-  for (int t = 0; t < 3; ++t) {
-    for (int e = threadIdx.x; e < len[t]; e += blockDim.x) dst[e] = src[t][e];
-    dst += len[t];
+  for (int k = 0; k < 4; ++k) {
+    P.w[k] = c_psi[q][k];
+    P.v[k] = c_psi[qn][k];
   }
-  return Tab3S{reinterpret_cast<const double (*)[NN]>(buf),
-               reinterpret_cast<const double (*)[NN][3]>(buf + NQ * NN),
-               reinterpret_cast<const double (*)[NF][NN]>(buf + NQ * NN * 4)};
-}
-// value of the vertex field t at cell point q
-__device__ __forceinline__ double at_qs(const double *t, int q, const Tab3S &T) {
-  double s = 0.0;
 #pragma unroll
-  for (int i = 0; i < NN; ++i) s = fma(T.phi[q][i], t[i], s);
-  return s;
+  for (int d = 0; d < 3; ++d) P.n[d] = fq[d] * fq[3];
+  return P;
 }
-// trace of t at point q of local face f (the face's four vertices)
-__device__ __forceinline__ double at_faces(const double *t, int f, int q, const Tab3S &T) {
-  double s = 0.0;
-#pragma unroll
-  for (int k = 0; k < 4; ++k) s = fma(T.fphi[f][q][fnode(f, k)], t[fnode(f, k)], s);
-  return s;
-}
-// the neighbour's trace of component comp of a field with ncomp components
-__device__ __forceinline__ double nb_vals(const NbPt &n, const double *v, int ncomp, int comp,
-                                          const Tab3S &T) {
-  const double *s = v + ((long)n.nb * ncomp + comp) * NN;
+// traces of component comp of a field with ncomp components
+__device__ __forceinline__ double own_tr(const FacePt &P, const double *v, int ncomp, int comp) {
+  const double *s = v + ((long)P.c * ncomp + comp) * NN;
   double r = 0.0;
 #pragma unroll
-  for (int k = 0; k < 4; ++k) r = fma(T.fphi[n.nf][n.qn][fnode(n.nf, k)], s[fnode(n.nf, k)], r);
+  for (int k = 0; k < 4; ++k) r = fma(P.w[k], __ldg(s + fnode(P.f, k)), r);
   return r;
 }
-// physical vector P (x JxW already) -> reference components Gr[e] = sum_i G[e][i] P_i
-__device__ __forceinline__ void to_ref(const double *cgq, const double *P, double *Gr) {
+__device__ __forceinline__ double nb_tr(const FacePt &P, const double *v, int ncomp, int comp) {
+  const double *s = v + ((long)P.nb * ncomp + comp) * NN;
+  double r = 0.0;
 #pragma unroll
-  for (int e = 0; e < 3; ++e) Gr[e] = cgq[3 * e] * P[0] + cgq[3 * e + 1] * P[1] + cgq[3 * e + 2] * P[2];
+  for (int k = 0; k < 4; ++k) r = fma(P.v[k], __ldg(s + fnode(P.nf, k)), r);
+  return r;
 }
-
-// Every face-integral kernel runs one warp per cell (CELLS3 cells per
-// block): lanes take the 27 quadrature points and the 54 face points of the
-// cell, write their integrands to shared memory, and one lane per output
-// node and component sums them against the basis.  One thread per cell
-// would leave 6144 cells on a third of the SMs with long serial chains.
-constexpr int CELLS3 = 4;
-
-// Copy n values per cell of a field with ncomp components into shared memory:
-// dst[comp][i] for the cell's components comp < ncomp (lanes of one warp).
-__device__ __forceinline__ void tile3(double *dst, const double *src, int c, int ncomp,
-                                      int lane) {
-  for (int e = lane; e < ncomp * NN; e += 32) dst[e] = src[(long)c * ncomp * NN + e];
-}
-
-// For vertex i = lane % 8: the sum over the cell's points of
-// V_q phi_i + Gr_q . grad phi_i and over the points of the three faces that
-// hold the vertex of F_fq phi_i.  The four lanes of each vertex take every
-// fourth term and the partial sums are combined by shuffles, so that all 32
-// lanes work (an FP64 warp instruction costs the same with 8 active lanes as
-// with 32).  Every lane of the warp must call it; lanes 0..7 hold the result
-// of their vertex (all lanes do).
-__device__ __forceinline__ double gather3(const double (*sv)[4], const double (*sf)[NF],
-                                          int lane, const Tab3S &T) {
-  const int i = lane & 7, part = lane >> 3;
-  double o = 0.0;
-  for (int q = part; q < NQ; q += 4)
-    o += sv[q][0] * T.phi[q][i] + sv[q][1] * T.dphi[q][i][0] + sv[q][2] * T.dphi[q][i][1] +
-         sv[q][3] * T.dphi[q][i][2];
-  for (int t = part; t < 3 * NF; t += 4) {
-    const int a = t / NF, q = t - a * NF, f = 2 * a + ((i >> a) & 1);
-    o += sf[f][q] * T.fphi[f][q][i];
-  }
-  o += __shfl_xor_sync(0xffffffffu, o, 8);
-  o += __shfl_xor_sync(0xffffffffu, o, 16);
-  return o;
-}
-
-// The same sums for vertex i by one lane alone (three components at once
-// keep 24 of the 32 lanes busy without the shuffles)
-__device__ __forceinline__ double gather3_one(const double (*sv)[4], const double (*sf)[NF],
-                                              int i, const Tab3S &T) {
-  double o = 0.0;
-  for (int q = 0; q < NQ; ++q)
-    o += sv[q][0] * T.phi[q][i] + sv[q][1] * T.dphi[q][i][0] + sv[q][2] * T.dphi[q][i][1] +
-         sv[q][3] * T.dphi[q][i][2];
-  for (int a = 0; a < 3; ++a) {  // the faces holding vertex i, in increasing order
-    const int f = 2 * a + ((i >> a) & 1);
+// nodal integrals of the block's face values F[face][comp][9]: minus for the
+// owner, plus for the neighbour, Fb[cell][face][comp][4]
+template <int NC>
+__device__ __forceinline__ void face_store(const double *F, const Geo3 &g, int f0, int nf,
+                                           double *__restrict__ Fb) {
+  for (int t = threadIdx.x; t < nf * 2 * NC * 4; t += blockDim.x) {
+    const int lf = t / (8 * NC), r = t - lf * 8 * NC, side = r / (4 * NC);
+    const int comp = (r - side * 4 * NC) >> 2, k = r & 3;
+    const int e = g.own[f0 + lf], nb = g.nbr[e];
+    if (side && nb < 0) continue;
+    const double *v = F + (lf * NC + comp) * NF;
+    double o = 0.0;
 #pragma unroll
-    for (int q = 0; q < NF; ++q) o += sf[f][q] * T.fphi[f][q][i];
+    for (int q = 0; q < NF; ++q)
+      o = fma(c_psi[side ? g.nperm[e * NF + q] : q][k], v[q], o);
+    const long to = side ? (long)nb * 6 + g.nbf[e] : e;
+    Fb[(to * NC + comp) * 4 + k] = side ? o : -o;
   }
-  return o;
 }
 
-// ------------------------------------------------------------- rho rhs --
-// euler_operator.h:344-712; src = (rho^(j), u^(j)) for j < nst
-__global__ void __launch_bounds__(32 * CELLS3)
-    k3_rhs_rho(double *__restrict__ dst, SrcPtrs src, Coef3 co, Geo3 g) {
-  __shared__ double srt[CELLS3][3][NN], sut[CELLS3][3][3][NN];
-  __shared__ double sv[CELLS3][NQ][4], sf[CELLS3][6][NF];
-  const int lc = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int c = blockIdx.x * CELLS3 + lc;
-  const bool active = c < g.nc;
-  __shared__ double stab[TAB3];
-  const Tab3S T = stage_tab3(stab);  // read after the first barrier
-  if (active)
-    for (int j = 0; j < co.nst; ++j) {
-      tile3(srt[lc][j], src.p[2 * j], c, 1, lane);
-      tile3(&sut[lc][j][0][0], src.p[2 * j + 1], c, 3, lane);
-    }
-  __syncthreads();
-  if (active) {
-    if (lane < NQ) {
-      const int q = lane;
-      const double *cq = g.cg + ((long)c * NQ + q) * 13;
-      sv[lc][q][0] = at_qs(srt[lc][0], q, T) * cq[9];
-      double P[3] = {0, 0, 0};
-      for (int j = 0; j < co.nst; ++j) {
-        const double r = at_qs(srt[lc][j], q, T), w = co.ca[j] * co.dt * r;
-        for (int d = 0; d < 3; ++d) P[d] += w * at_qs(sut[lc][j][d], q, T);
-      }
-      to_ref(cq, P, &sv[lc][q][1]);
-    }
-    for (int e = lane; e < 6 * NF; e += 32) {
-      const int f = e / NF, q = e - f * NF;
-      double F = 0.0;
-      if (g.nbr[c * 6 + f] >= 0) {  // no boundary term (euler_operator.h:111-114)
-        const double *fq = g.fg + (((long)c * 6 + f) * NF + q) * 4;
-        double flux = 0.0;
-        const NbPt np = nb_point(g, c, f, q);
+// ------------------------------------------------- explicit rhs, faces --
+// KIND 0 density (euler_operator.h:478-692, no boundary term), 1 momentum
+// (:1891-2305, walls with p_D = p), 2 energy (:1012-1361, the stage-2 kinetic
+// jump mixing in u_old :1182-1183 and the stage-3 total rho E jump
+// :1290-1336; the division by rho in the reference's E cancels).
+// src = (rho, u, [p])^(j) for j < nst.
+template <int KIND>
+__global__ void __launch_bounds__(NF * FPB, 2)
+    k3_rhs_face(double *__restrict__ Fb, SrcPtrs src, Coef3 co, int hstage, Geo3 g) {
+  constexpr int NC = KIND == 1 ? 3 : 1, PER = KIND == 0 ? 2 : 3;
+  constexpr double ig = 1.0 / (GAS_GAMMA - 1.0), hgf = GAS_GAMMA * ig;
+  __shared__ double sF[FPB][NC][NF];
+  const int f0 = blockIdx.x * FPB, nf = min(FPB, g.nfaces - f0);
+  const int lf = threadIdx.x / NF, q = threadIdx.x - lf * NF;
+  if (lf < nf) {
+    const FacePt P = face_point(g, g.own[f0 + lf], q);
+    double F[NC];
+#pragma unroll
+    for (int d = 0; d < NC; ++d) F[d] = 0.0;
+    double xo[3], xn[3];  // state 0's velocity traces (stage 2, energy)
+    if (P.nb < 0) {
+      if constexpr (KIND == 1)
         for (int j = 0; j < co.nst; ++j) {
-          const double ro = at_faces(srt[lc][j], f, q, T), rn = nb_vals(np, src.p[2 * j], 1, 0, T);
-          double avg = 0.0, uno = 0.0, unn = 0.0;
-          for (int d = 0; d < 3; ++d) {
-            const double uo = at_faces(sut[lc][j][d], f, q, T);
-            const double un = nb_vals(np, src.p[2 * j + 1], 3, d, T);
-            avg += 0.5 * (ro * uo + rn * un) * fq[d];
-            uno += uo * fq[d];
-            unn += un * fq[d];
-          }
-          flux += co.ca[j] * co.dt * (avg + 0.5 * fmax(fabs(uno), fabs(unn)) * (ro - rn));
+          const double w = co.ct[j] * co.dt / (co.Ma * co.Ma) * own_tr(P, src.p[PER * j + 2], 1, 0);
+#pragma unroll
+          for (int d = 0; d < 3; ++d) F[d] = fma(w, P.n[d], F[d]);
         }
-        F = -flux * fq[3];
-      }
-      sf[lc][f][q] = F;
-    }
-  }
-  __syncthreads();
-  if (active) {  // warp-uniform: every lane of the cell's warp takes part
-    const double o = gather3(sv[lc], sf[lc], lane, T);
-    if (lane < NN) dst[(long)c * NN + lane] = o;
-  }
-}
-
-// ------------------------------------------------------------ momentum --
-// euler_operator.h:1622-2305; src = (rho, u, p)^(j) for j < nst, then the
-// densities of the gravity terms at gsrc[0..ng)
-__global__ void __launch_bounds__(32 * CELLS3)
-    k3_rhs_vel(double *__restrict__ dst, SrcPtrs src, SrcPtrs gsrc, Coef3 co, Geo3 g) {
-  __shared__ double srt[CELLS3][3][NN], sut[CELLS3][3][3][NN], spt[CELLS3][3][NN];
-  __shared__ double sgt[CELLS3][3][NN];
-  __shared__ double sv[CELLS3][3][NQ][4], sf[CELLS3][3][6][NF];  // per component d
-  const int lc = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int c = blockIdx.x * CELLS3 + lc;
-  const bool active = c < g.nc;
-  __shared__ double stab[TAB3];
-  const Tab3S T = stage_tab3(stab);  // read after the first barrier
-  const double iM2 = 1.0 / (co.Ma * co.Ma), iF2 = 1.0 / (co.Fr * co.Fr);
-  if (active) {
-    for (int j = 0; j < co.nst; ++j) {
-      tile3(srt[lc][j], src.p[3 * j], c, 1, lane);
-      tile3(&sut[lc][j][0][0], src.p[3 * j + 1], c, 3, lane);
-      tile3(spt[lc][j], src.p[3 * j + 2], c, 1, lane);
-    }
-    for (int j = 0; j < co.ng; ++j) tile3(sgt[lc][j], gsrc.p[j], c, 1, lane);
-  }
-  __syncthreads();
-  if (active) {
-    if (lane < NQ) {
-      const int q = lane;
-      const double *cq = g.cg + ((long)c * NQ + q) * 13;
-      for (int d = 0; d < 3; ++d) {
-        double v = at_qs(srt[lc][0], q, T) * at_qs(sut[lc][0][d], q, T);
-        for (int j = 0; j < co.ng; ++j)
-          v -= co.cg[j] * co.dt * iF2 * at_qs(sgt[lc][j], q, T) * cq[10 + d];
-        sv[lc][d][q][0] = v * cq[9];
-        double P[3] = {0, 0, 0};
-        for (int j = 0; j < co.nst; ++j) {
-          const double ru = co.ca[j] * co.dt * at_qs(srt[lc][j], q, T) * at_qs(sut[lc][j][d], q, T);
-          for (int k = 0; k < 3; ++k) P[k] += ru * at_qs(sut[lc][j][k], q, T);
-          P[d] += co.ct[j] * co.dt * iM2 * at_qs(spt[lc][j], q, T);
-        }
-        to_ref(cq, P, &sv[lc][d][q][1]);  // the geometry factors carry JxW
-      }
-    }
-    for (int e = lane; e < 6 * NF; e += 32) {
-      const int f = e / NF, q = e - f * NF;
-      const NbPt np = nb_point(g, c, f, q);
-      const bool wall = np.nb < 0;
-      const double *fq = g.fg + (((long)c * 6 + f) * NF + q) * 4;
-      double fl[3] = {0, 0, 0};
+    } else {
       for (int j = 0; j < co.nst; ++j) {
-        const double po = at_faces(spt[lc][j], f, q, T);
-        if (wall) {  // p_D = p (euler_operator.h:2189-2305)
-          for (int d = 0; d < 3; ++d) fl[d] += co.ct[j] * co.dt * iM2 * 0.5 * (po + po) * fq[d];
-          continue;
-        }
-        const double ro = at_faces(srt[lc][j], f, q, T), rn = nb_vals(np, src.p[3 * j], 1, 0, T);
-        const double pn = nb_vals(np, src.p[3 * j + 2], 1, 0, T);
-        double uo[3], un[3], uno = 0.0, unn = 0.0;
-        for (int k = 0; k < 3; ++k) {
-          uo[k] = at_faces(sut[lc][j][k], f, q, T);
-          un[k] = nb_vals(np, src.p[3 * j + 1], 3, k, T);
-          uno += uo[k] * fq[k];
-          unn += un[k] * fq[k];
-        }
-        const double lam = fmax(fabs(uno), fabs(unn));
-        for (int d = 0; d < 3; ++d)
-          fl[d] += co.ca[j] * co.dt * 0.5 * (ro * uo[d] * uno + rn * un[d] * unn) +
-                   co.ct[j] * co.dt * iM2 * 0.5 * (po + pn) * fq[d] +
-                   co.ca[j] * co.dt * 0.5 * lam * (ro * uo[d] - rn * un[d]);
-      }
-      for (int d = 0; d < 3; ++d) sf[lc][d][f][q] = -fl[d] * fq[3];
-    }
-  }
-  __syncthreads();
-  if (active && lane < 3 * NN) {
-    const int d = lane / NN, i = lane - d * NN;
-    dst[((long)c * 3 + d) * NN + i] = gather3_one(sv[lc][d], sf[lc][d], i, T);
-  }
-}
-
-// -------------------------------------------------------------- energy --
-// euler_operator.h:745-1381 with the radial gravity work (:790-811), the
-// stage-2 kinetic jump mixing in u_old (:1182-1183) and the stage-3 total
-// rho E jump (:1290-1336).  src = (rho, u, p)^(j); gsrc = gravity densities
-// and velocities (rho, u)^(j) for j < ng, then the kinetic (rho, u).  The
-// reference's E = p / ((gamma-1) rho) + Ma^2 |u|^2 / 2 only enters as rho E
-// and rho (E - Ma^2 |u|^2 / 2) + p, where the division by rho cancels: the
-// kernel forms p / (gamma-1) + rho Ma^2 |u|^2 / 2 and gamma p / (gamma-1).
-__global__ void __launch_bounds__(32 * CELLS3)
-    k3_rhs_pres(double *__restrict__ dst, SrcPtrs src, SrcPtrs gsrc, Coef3 co, int hstage,
-                Geo3 g) {
-  __shared__ double srt[CELLS3][3][NN], sut[CELLS3][3][3][NN], spt[CELLS3][3][NN];
-  __shared__ double sgr[CELLS3][4][NN], sgu[CELLS3][4][3][NN];  // gravity j < ng, kinetic
-  __shared__ double sv[CELLS3][NQ][4], sf[CELLS3][6][NF];
-  const int lc = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int c = blockIdx.x * CELLS3 + lc;
-  const bool active = c < g.nc;
-  __shared__ double stab[TAB3];
-  const Tab3S T = stage_tab3(stab);  // read after the first barrier
-  const double ig = 1.0 / (GAS_GAMMA - 1.0), hgf = GAS_GAMMA / (GAS_GAMMA - 1.0);
-  const double M2 = co.Ma * co.Ma, iF2 = 1.0 / (co.Fr * co.Fr);
-  if (active) {
-    for (int j = 0; j < co.nst; ++j) {
-      tile3(srt[lc][j], src.p[3 * j], c, 1, lane);
-      tile3(&sut[lc][j][0][0], src.p[3 * j + 1], c, 3, lane);
-      tile3(spt[lc][j], src.p[3 * j + 2], c, 1, lane);
-    }
-    for (int j = 0; j <= co.ng; ++j) {  // j = ng: the kinetic (rho, u)
-      tile3(sgr[lc][j], gsrc.p[2 * j], c, 1, lane);
-      tile3(&sgu[lc][j][0][0], gsrc.p[2 * j + 1], c, 3, lane);
-    }
-  }
-  __syncthreads();
-  if (active) {
-    if (lane < NQ) {
-      const int q = lane;
-      const double *cq = g.cg + ((long)c * NQ + q) * 13;
-      const double r0 = at_qs(srt[lc][0], q, T), p0 = at_qs(spt[lc][0], q, T);
-      double uu0 = 0.0;
-      for (int d = 0; d < 3; ++d) {
-        const double u = at_qs(sut[lc][0][d], q, T);
-        uu0 += u * u;
-      }
-      const double kr = at_qs(sgr[lc][co.ng], q, T);
-      double kk = 0.0;
-      for (int d = 0; d < 3; ++d) {
-        const double kv = at_qs(sgu[lc][co.ng][d], q, T);
-        kk += kv * kv;
-      }
-      double v = ig * p0 + 0.5 * M2 * uu0 * r0 - 0.5 * kr * M2 * kk;  // rho E - kinetic
-      for (int j = 0; j < co.ng; ++j) {
-        const double gr = at_qs(sgr[lc][j], q, T);
-        double ue = 0.0;
-        for (int d = 0; d < 3; ++d) ue += at_qs(sgu[lc][j][d], q, T) * cq[10 + d];  // u . e_r a^2/r^2
-        v -= co.cg[j] * co.dt * M2 * iF2 * gr * ue;
-      }
-      sv[lc][q][0] = v * cq[9];
-      double P[3] = {0, 0, 0};
-      for (int j = 0; j < co.nst; ++j) {
-        const double r = at_qs(srt[lc][j], q, T), p = at_qs(spt[lc][j], q, T);
-        double u[3], uu = 0.0;
+        const double ro = own_tr(P, src.p[PER * j], 1, 0), rn = nb_tr(P, src.p[PER * j], 1, 0);
+        double uo[3], un[3], a = 0.0, b = 0.0;
+#pragma unroll
         for (int d = 0; d < 3; ++d) {
-          u[d] = at_qs(sut[lc][j][d], q, T);
-          uu += u[d] * u[d];
+          uo[d] = own_tr(P, src.p[PER * j + 1], 3, d);
+          un[d] = nb_tr(P, src.p[PER * j + 1], 3, d);
+          a = fma(uo[d], P.n[d], a);
+          b = fma(un[d], P.n[d], b);
         }
-        const double w = 0.5 * co.ca[j] * co.dt * M2 * uu * r + co.ct[j] * co.dt * hgf * p;
-        for (int d = 0; d < 3; ++d) P[d] += w * u[d];
-      }
-      to_ref(cq, P, &sv[lc][q][1]);
-    }
-    for (int e = lane; e < 6 * NF; e += 32) {
-      const int f = e / NF, q = e - f * NF;
-      double F = 0.0;
-      if (g.nbr[c * 6 + f] >= 0) {  // no boundary term
-        const double *fq = g.fg + (((long)c * 6 + f) * NF + q) * 4;
-        const NbPt np = nb_point(g, c, f, q);
-        double uo[3][3], un[3][3];
-        for (int j = 0; j < co.nst; ++j)
-          for (int d = 0; d < 3; ++d) {
-            uo[j][d] = at_faces(sut[lc][j][d], f, q, T);
-            un[j][d] = nb_vals(np, src.p[3 * j + 1], 3, d, T);
-          }
-        double flux = 0.0;
-        for (int j = 0; j < co.nst; ++j) {
-          const double ro = at_faces(srt[lc][j], f, q, T), rn = nb_vals(np, src.p[3 * j], 1, 0, T);
-          const double po = at_faces(spt[lc][j], f, q, T), pn = nb_vals(np, src.p[3 * j + 2], 1, 0, T);
-          double uuo = 0, uun = 0, uno = 0, unn = 0;
-          for (int d = 0; d < 3; ++d) {
-            uuo += uo[j][d] * uo[j][d]; uun += un[j][d] * un[j][d];
-            uno += uo[j][d] * fq[d]; unn += un[j][d] * fq[d];
-          }
-          const double akin = 0.5 * (0.5 * uuo * ro * uno + 0.5 * uun * rn * unn);
-          const double aent = 0.5 * (hgf * po * uno + hgf * pn * unn);
-          const double lam = fmax(fabs(uno), fabs(unn));
-          if (hstage == 3) {  // jump of the total rho E
-            const double jE = ig * (po - pn) + 0.5 * M2 * (ro * uuo - rn * uun);
-            flux += co.ca[j] * co.dt * M2 * akin + co.ca[j] * co.dt * aent +
-                    co.ca[j] * co.dt * 0.5 * lam * jE;
-          } else {
-            double jk;
-            if (hstage == 2 && j == 1) {
-              double ko = 0, kn = 0;
-              for (int d = 0; d < 3; ++d) { ko += uo[1][d] * uo[0][d]; kn += un[1][d] * un[0][d]; }
-              jk = ro * 0.5 * ko - rn * 0.5 * kn;
-            } else {
-              jk = ro * 0.5 * uuo - rn * 0.5 * uun;
+        const double lam = abs_max(a, b), wa = co.ca[j] * co.dt;
+        if constexpr (KIND == 0) {
+          F[0] = fma(0.5 * wa, fma(lam, ro - rn, fma(ro, a, rn * b)), F[0]);
+        } else {
+          const double po = own_tr(P, src.p[PER * j + 2], 1, 0);
+          const double pn = nb_tr(P, src.p[PER * j + 2], 1, 0);
+          if constexpr (KIND == 1) {
+            const double ps = 0.5 * co.ct[j] * co.dt / (co.Ma * co.Ma) * (po + pn);
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+              const double mo = ro * uo[d], mn = rn * un[d];
+              const double t = fma(lam, mo - mn, fma(mo, a, mn * b));
+              F[d] = fma(0.5 * wa, t, fma(ps, P.n[d], F[d]));
             }
-            const double je = ig * (po - pn);  // jump of rho (E - Ma^2 |u|^2 / 2)
-            flux += co.ca[j] * co.dt * M2 * (akin + 0.5 * lam * jk) +
-                    co.ct[j] * co.dt * (aent + 0.5 * lam * je);
+          } else {
+            // per side: k rho |u|^2 + k2 p over the flux, + k3 p in the jump
+            const double we = hstage == 3 ? wa : co.ct[j] * co.dt;
+            const double k1 = 0.25 * wa * co.Ma * co.Ma, k2 = 0.5 * hgf * we, k3 = 0.5 * ig * we;
+            double so = 0.0, sn = 0.0;
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+              so = fma(uo[d], uo[d], so);
+              sn = fma(un[d], un[d], sn);
+            }
+            const double ko = k1 * ro * so, kn = k1 * rn * sn;
+            double jo = ko, jn = kn;
+            if (hstage == 2) {
+              if (j == 0) {
+#pragma unroll
+                for (int d = 0; d < 3; ++d) {
+                  xo[d] = uo[d];
+                  xn[d] = un[d];
+                }
+              } else {
+                so = sn = 0.0;
+#pragma unroll
+                for (int d = 0; d < 3; ++d) {
+                  so = fma(uo[d], xo[d], so);
+                  sn = fma(un[d], xn[d], sn);
+                }
+                jo = k1 * ro * so;
+                jn = k1 * rn * sn;
+              }
+            }
+            F[0] = fma(fma(k2, po, ko), a, F[0]);
+            F[0] = fma(fma(k2, pn, kn), b, F[0]);
+            F[0] = fma(lam, fma(k3, po, jo) - fma(k3, pn, jn), F[0]);
           }
         }
-        F = -flux * fq[3];
       }
-      sf[lc][f][q] = F;
+    }
+#pragma unroll
+    for (int d = 0; d < NC; ++d) sF[lf][d][q] = F[d];
+  }
+  __syncthreads();
+  face_store<NC>(&sF[0][0][0], g, f0, nf, Fb);
+}
+
+// -------------------------------------------------- explicit rhs, cells --
+// euler_operator.h:344-473 (density), 1622-1886 (momentum), 745-1007 (energy,
+// with the radial gravity work :790-811), plus the face integrals Fb.
+// `cpb` cells per block, 27 threads each.  `fields` counts the scalar fields
+// that the block interpolates: (rho, u, [p])^(j), then KIND 1: the density
+// being solved for (stages 1, 2), KIND 2: the kinetic (rho, u).
+template <int KIND>
+__global__ void __launch_bounds__(27 * 14)
+    k3_rhs_cell(double *__restrict__ dst, SrcPtrs src, Coef3 co, int hstage, int fields, Geo3 g,
+                const double *__restrict__ Fb, int cpb) {
+  constexpr int NC = KIND == 1 ? 3 : 1, PER = KIND == 0 ? 2 : 3, SF = KIND == 0 ? 4 : 5;
+  constexpr double ig = 1.0 / (GAS_GAMMA - 1.0), hgf = GAS_GAMMA * ig;
+  extern __shared__ double sm[];  // [cpb][fields][4][3], then [cpb][NC][4][27]
+  __shared__ double spsi[NF][4];
+  const int per = max(fields * 12, NC * 4 * NQ);
+  const int c0 = blockIdx.x * cpb, cnt = min(cpb, g.nc - c0);
+  const double s = c_line[0], t = c_line[1];
+  const int tid = threadIdx.x, nt = blockDim.x;
+  for (int e = tid; e < NF * 4; e += nt) spsi[e >> 2][e & 3] = c_psi[e >> 2][e & 3];
+  // x-lines: (cell, field, edge)
+  for (int e = tid; e < cnt * fields * 4; e += nt) {
+    const int l = e / (fields * 4), r = e - l * fields * 4, fd = r >> 2, m = r & 3;
+    const long c = c0 + l;
+    const int j = fd / SF, k = fd - j * SF;  // state and its field
+    const double *v;
+    if (j < co.nst) {
+      v = k == 0 ? src.p[PER * j] + c * NN
+                 : k < 4 ? src.p[PER * j + 1] + (c * 3 + k - 1) * NN : src.p[PER * j + 2] + c * NN;
+    } else {
+      v = k == 0 ? src.p[PER * co.nst] + c * NN : src.p[PER * co.nst + 1] + (c * 3 + k - 1) * NN;
+    }
+    double o[3];
+    line3(__ldg(v + 2 * m), __ldg(v + 2 * m + 1), s, t, o);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) sm[l * per + r * 3 + i] = o[i];
+  }
+  __syncthreads();
+  const int l = tid / NQ, q = tid - l * NQ;
+  double V[NC], G[NC][3];
+  if (l < cnt) {
+    const double *X = sm + l * per + q % 3;
+    double w[4];
+#pragma unroll
+    for (int m = 0; m < 4; ++m) w[m] = spsi[q / 3][m];
+    const double *cq = g.cg + ((long)(c0 + l) * NQ + q) * 13;
+    auto val = [&](int fd) {
+      double r = 0.0;
+#pragma unroll
+      for (int m = 0; m < 4; ++m) r = fma(w[m], X[(fd * 4 + m) * 3], r);
+      return r;
+    };
+    double P[NC][3], gr = 0.0;  // physical fluxes; gravity's density / work
+#pragma unroll
+    for (int d = 0; d < NC; ++d) {
+      V[d] = 0.0;
+#pragma unroll
+      for (int i = 0; i < 3; ++i) P[d][i] = 0.0;
+    }
+    for (int j = 0; j < co.nst; ++j) {
+      const double r = val(SF * j), wa = co.ca[j] * co.dt;
+      double u[3];
+#pragma unroll
+      for (int d = 0; d < 3; ++d) u[d] = val(SF * j + 1 + d);
+      if constexpr (KIND == 0) {
+        if (j == 0) V[0] = r;
+        const double wr = wa * r;
+#pragma unroll
+        for (int i = 0; i < 3; ++i) P[0][i] = fma(wr, u[i], P[0][i]);
+      } else if constexpr (KIND == 1) {
+        const double pp = co.ct[j] * co.dt / (co.Ma * co.Ma) * val(SF * j + 4);
+        gr = fma(co.cg[j], r, gr);
+        const double wr = wa * r;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+          if (j == 0) V[d] = r * u[d];
+          const double ru = wr * u[d];
+#pragma unroll
+          for (int i = d; i < 3; ++i) P[d][i] = fma(ru, u[i], P[d][i]);  // symmetric
+          P[d][d] += pp;
+        }
+      } else {
+        const double p = val(SF * j + 4), M2 = co.Ma * co.Ma;
+        const double k = r * fma(u[0], u[0], fma(u[1], u[1], u[2] * u[2]));
+        if (j == 0) V[0] = fma(ig, p, 0.5 * M2 * k);  // rho E
+        const double ug = fma(u[0], cq[10], fma(u[1], cq[11], u[2] * cq[12]));
+        gr = fma(co.cg[j] * r, ug, gr);
+        const double h = fma(0.5 * wa * M2, k, co.ct[j] * co.dt * hgf * p);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) P[0][i] = fma(h, u[i], P[0][i]);
+      }
+    }
+    if constexpr (KIND == 1) {
+      if (fields > SF * co.nst) gr = fma(co.cg[co.nst], val(SF * co.nst), gr);
+      const double wg = co.dt / (co.Fr * co.Fr) * gr;
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        V[d] = fma(-wg, cq[10 + d], V[d]);
+#pragma unroll
+        for (int i = 0; i < d; ++i) P[d][i] = P[i][d];
+      }
+    }
+    if constexpr (KIND == 2) {
+      const double M2 = co.Ma * co.Ma, r = val(SF * co.nst);
+      double u[3];
+#pragma unroll
+      for (int d = 0; d < 3; ++d) u[d] = val(SF * co.nst + 1 + d);
+      if (hstage < 3) {  // gravity work of the density being solved for
+        const double ug = fma(u[0], cq[10], fma(u[1], cq[11], u[2] * cq[12]));
+        gr = fma(co.cg[co.nst] * r, ug, gr);
+      }
+      V[0] = fma(-0.5 * M2 * r, fma(u[0], u[0], fma(u[1], u[1], u[2] * u[2])), V[0]);
+      V[0] = fma(-co.dt * M2 / (co.Fr * co.Fr), gr, V[0]);
+    }
+#pragma unroll
+    for (int d = 0; d < NC; ++d) {
+      V[d] *= cq[9];
+#pragma unroll
+      for (int e = 0; e < 3; ++e)
+        G[d][e] = fma(cq[3 * e], P[d][0], fma(cq[3 * e + 1], P[d][1], cq[3 * e + 2] * P[d][2]));
     }
   }
   __syncthreads();
-  if (active) {  // warp-uniform: every lane of the cell's warp takes part
-    const double o = gather3(sv[lc], sf[lc], lane, T);
-    if (lane < NN) dst[(long)c * NN + lane] = o;
+  if (l < cnt) {
+    double *o = sm + l * per + q;
+#pragma unroll
+    for (int d = 0; d < NC; ++d) {
+      o[(d * 4) * NQ] = V[d];
+#pragma unroll
+      for (int e = 0; e < 3; ++e) o[(d * 4 + 1 + e) * NQ] = G[d][e];
+    }
+  }
+  __syncthreads();
+  // z, then y, then x: each task replaces its own line's values
+  for (int e = tid; e < cnt * NC * 9; e += nt) {
+    const int lo = e / (NC * 9), r = e - lo * NC * 9, d = r / 9;
+    double *v = sm + lo * per + d * 4 * NQ + (r - d * 9);
+    double a, b;
+    double *gz = v + 3 * NQ;
+    const double z = gz[0] + gz[9] + gz[18];
+    line3_t(v[0], v[9], v[18], s, t, a, b);
+    v[0] = a - z;
+    v[9] = b + z;
+#pragma unroll
+    for (int k = 1; k < 3; ++k) {
+      double *y = v + k * NQ;
+      line3_t(y[0], y[9], y[18], s, t, a, b);
+      y[0] = a;
+      y[9] = b;
+    }
+  }
+  __syncthreads();
+  for (int e = tid; e < cnt * NC * 6; e += nt) {
+    const int lo = e / (NC * 6), r = e - lo * NC * 6, d = r / 6, k = r - d * 6;
+    double *v = sm + lo * per + d * 4 * NQ + (k / 3) * 9 + k % 3;
+    double a, b;
+    const double *gy = v + 2 * NQ;
+    const double y = gy[0] + gy[3] + gy[6];
+    line3_t(v[0], v[3], v[6], s, t, a, b);
+    v[0] = a - y;
+    v[3] = b + y;
+    double *gx = v + NQ;
+    line3_t(gx[0], gx[3], gx[6], s, t, a, b);
+    gx[0] = a;
+    gx[3] = b;
+  }
+  __syncthreads();
+  for (int e = tid; e < cnt * NC * 4; e += nt) {
+    const int lo = e / (NC * 4), r = e - lo * NC * 4, d = r >> 2, y = r & 1, z = (r >> 1) & 1;
+    const double *v = sm + lo * per + d * 4 * NQ + z * 9 + y * 3;
+    double a, b;
+    const double x = v[NQ] + v[NQ + 1] + v[NQ + 2];
+    line3_t(v[0], v[1], v[2], s, t, a, b);
+    const long c = c0 + lo;
+    const double *F = Fb + (c * 6 * NC + d) * 4;  // face f at f * NC * 4
+    // vertex (x, y, z): faces x, 2 + y, 4 + z
+    const double *Fy = F + (2 + y) * NC * 4 + 2 * z, *Fz = F + (4 + z) * NC * 4 + 2 * y;
+    double *o = dst + (c * 3 * (NC == 3) + c * (NC == 1) + d) * NN + 2 * y + 4 * z;
+    o[0] = (a - x) + F[y + 2 * z] + Fy[0] + Fz[0];
+    o[1] = (b + x) + F[NC * 4 + y + 2 * z] + Fy[1] + Fz[1];
+  }
+}
+
+// ------------------------------------------------------------ B and D tables --
+// wb [nc][8][24]: B of the cell's own values, output (d, i) from vertex j:
+//   -sum_q phi_j G[.][d] . grad phi_i + half the face terms (walls: all of it)
+// nb [nc][12][24]: of the neighbours', output (d, i) from vertex k' of the face
+// along axis a that holds i (row a * 4 + k'); dm [nc][8][8]: D.
+__global__ void k3_tables(double *__restrict__ wb, double *__restrict__ nbt,
+                          double *__restrict__ dm, Geo3 g) {
+  const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= (long)g.nc * 24) return;
+  const int c = (int)(t / 24), o = (int)(t - (long)c * 24), d = o / NN, i = o - d * NN;
+  double W[NN], D[NN];
+  for (int j = 0; j < NN; ++j) W[j] = D[j] = 0.0;
+  for (int q = 0; q < NQ; ++q) {
+    const double *cq = g.cg + ((long)c * NQ + q) * 13;
+    const double s = -(cq[d] * c_dphi[q][i][0] + cq[3 + d] * c_dphi[q][i][1] +
+                       cq[6 + d] * c_dphi[q][i][2]);
+    const double m = c_phi[q][i] * cq[9] / (GAS_GAMMA - 1.0);
+    for (int j = 0; j < NN; ++j) {
+      W[j] = fma(s, c_phi[q][j], W[j]);
+      D[j] = fma(m, c_phi[q][j], D[j]);
+    }
+  }
+  for (int a = 0; a < 3; ++a) {
+    const int f = 2 * a + ((i >> a) & 1), e = c * 6 + f, nb = g.nbr[e];
+    double N[4] = {0, 0, 0, 0};
+    for (int q = 0; q < NF; ++q) {
+      const double *fq = g.fg + ((long)e * NF + q) * 4;
+      const double s = c_fphi[f][q][i] * fq[d] * fq[3] * (nb < 0 ? 1.0 : 0.5);
+      for (int k = 0; k < 4; ++k) {
+        const int j = fnode(f, k);
+        W[j] = fma(s, c_fphi[f][q][j], W[j]);
+        if (nb >= 0) N[k] = fma(s, c_psi[g.nperm[e * NF + q]][k], N[k]);
+      }
+    }
+    for (int k = 0; k < 4; ++k) nbt[((long)c * 12 + a * 4 + k) * 24 + o] = N[k];
+  }
+  for (int j = 0; j < NN; ++j) {
+    wb[((long)c * NN + j) * 24 + o] = W[j];
+    if (d == 0) dm[((long)c * NN + j) * NN + i] = D[j];
   }
 }
 
 // ------------------------------------------------------------------- B --
-// euler_operator.h:1512-1617; mode 0 dst = B p, 1 dst -= B p, 2 dst = A^{-1} B p
-__global__ void __launch_bounds__(32 * CELLS3)
+// euler_operator.h:1512-1617; mode 0 dst = cB B p, 1 dst -= cB B p,
+// 2 dst = cB A^{-1} B p.  24 threads per cell, one per output.
+constexpr int CB_B = 8;
+__global__ void __launch_bounds__(24 * CB_B)
     k3_B(double *__restrict__ dst, const double *__restrict__ p, double cB,
-         const double *__restrict__ ainv, int mode, Geo3 g) {
-  __shared__ double sp[CELLS3][NN];            // p on the cell's vertices
-  __shared__ double sgr[CELLS3][NQ][3][3];     // [q][d][e]: -cB p(q) dxi_e/dx_d JxW
-  __shared__ double sfn[CELLS3][6][NF][3];     // [f][q][d]: cB {p} n_d JxW
-  __shared__ double sout[CELLS3][3][NN];
-  const int lc = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int c = blockIdx.x * CELLS3 + lc;
+         const double *__restrict__ ainv, int mode, const double *__restrict__ wb,
+         const double *__restrict__ nbt, Geo3 g) {
+  __shared__ double so[CB_B][NN], sn[CB_B][24], sb[CB_B][24];
+  const int l = threadIdx.x / 24, o = threadIdx.x - l * 24;
+  const int c = blockIdx.x * CB_B + l;
   const bool active = c < g.nc;
-  __shared__ double stab[TAB3];
-  const Tab3S T = stage_tab3(stab);  // read after the first barrier
-  if (active && lane < NN) sp[lc][lane] = p[(long)c * NN + lane];
+  if (active) {
+    const int f = o >> 2, nb = g.nbr[c * 6 + f];  // vertex o & 3 of the neighbour across f
+    sn[l][o] = nb < 0 ? 0.0 : __ldg(p + (long)nb * NN + fnode(g.nbf[c * 6 + f], o & 3));
+    if (o < NN) so[l][o] = __ldg(p + (long)c * NN + o);
+  }
+  __syncthreads();
+  const int d = o / NN, i = o - d * NN;
+  const long gi = (long)c * 24 + o;
+  double r = 0.0;
+  if (active) {
+    const double *W = wb + (long)c * NN * 24 + o, *N = nbt + (long)c * 12 * 24 + o;
+#pragma unroll
+    for (int j = 0; j < NN; ++j) r = fma(__ldg(W + j * 24), so[l][j], r);
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      const double *v = sn[l] + (2 * a + ((i >> a) & 1)) * 4;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) r = fma(__ldg(N + (a * 4 + k) * 24), v[k], r);
+    }
+    r *= cB;
+    if (mode == 0) dst[gi] = r;
+    else if (mode == 1) dst[gi] -= r;
+    sb[l][o] = r;
+  }
+  if (mode != 2) return;  // uniform over the grid
   __syncthreads();
   if (active) {
-    if (lane < NQ) {
-      const int q = lane;
-      const double *cq = g.cg + ((long)c * NQ + q) * 13;
-      const double s = -cB * at_qs(sp[lc], q, T);
+    const double *A = ainv + (long)c * NN * NN + i;  // symmetric
+    double s = 0.0;
 #pragma unroll
-      for (int d = 0; d < 3; ++d)
-#pragma unroll
-        for (int e = 0; e < 3; ++e) sgr[lc][q][d][e] = s * cq[3 * e + d];
-    }
-    for (int e = lane; e < 6 * NF; e += 32) {
-      const int f = e / NF, q = e - f * NF;
-      const double *fq = g.fg + (((long)c * 6 + f) * NF + q) * 4;
-      const double po = at_faces(sp[lc], f, q, T);
-      const NbPt np = nb_point(g, c, f, q);
-      const double pn = np.nb < 0 ? po : nb_vals(np, p, 1, 0, T);
-      const double a = cB * 0.5 * (po + pn) * fq[3];
-#pragma unroll
-      for (int d = 0; d < 3; ++d) sfn[lc][f][q][d] = a * fq[d];
-    }
-  }
-  __syncthreads();
-  if (active) {  // warp-uniform; per component, four lanes per vertex (as gather3)
-    const int i = lane & 7, part = lane >> 3;
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      double o = 0.0;
-      for (int q = part; q < NQ; q += 4)
-        o += sgr[lc][q][d][0] * T.dphi[q][i][0] + sgr[lc][q][d][1] * T.dphi[q][i][1] +
-             sgr[lc][q][d][2] * T.dphi[q][i][2];
-      for (int t = part; t < 3 * NF; t += 4) {  // the faces holding vertex i
-        const int a = t / NF, q = t - a * NF, f = 2 * a + ((i >> a) & 1);
-        o += sfn[lc][f][q][d] * T.fphi[f][q][i];
-      }
-      o += __shfl_xor_sync(0xffffffffu, o, 8);
-      o += __shfl_xor_sync(0xffffffffu, o, 16);
-      if (lane < NN) sout[lc][d][i] = o;
-    }
-  }
-  __syncthreads();
-  if (active && lane < 3 * NN) {
-    const int d = lane / NN, i = lane - d * NN;
-    const long gi = ((long)c * 3 + d) * NN + i;
-    if (mode == 2) {
-      const double *A = ainv + (long)c * NN * NN + i * NN;
-      double s = 0.0;
-#pragma unroll
-      for (int j = 0; j < NN; ++j) s += A[j] * sout[lc][d][j];
-      dst[gi] = s;
-    } else {
-      dst[gi] = mode == 0 ? sout[lc][d][i] : dst[gi] - sout[lc][d][i];
-    }
+    for (int j = 0; j < NN; ++j) s = fma(__ldg(A + j * NN), sb[l][d * NN + j], s);
+    dst[gi] = s;
   }
 }
 
 // ----------------------------------------------------------------- C/D --
-// euler_operator.h:1386-1507.  mode 0 dst = C w; 1 dst = D p - C w;
-// 2 dst = invd .* (D p - C w); 3 dst -= C w.  D = mass / (gamma - 1).
-__global__ void __launch_bounds__(32 * CELLS3)
-    k3_CD(double *__restrict__ dst, const double *__restrict__ w,
-          const double *__restrict__ p, const double *__restrict__ pfix, double cC,
-          const double *__restrict__ invd, int mode, Geo3 g) {
-  __shared__ double swt[CELLS3][3][NN], sft[CELLS3][NN], spt[CELLS3][NN];
-  __shared__ double sv[CELLS3][NQ][4];         // [q]: V, Gr (3)
-  __shared__ double sfa[CELLS3][6][NF];        // [f][q]: face flux x JxW
-  const int lc = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int c = blockIdx.x * CELLS3 + lc;
-  const bool active = c < g.nc;
-  __shared__ double stab[TAB3];
-  const Tab3S T = stage_tab3(stab);  // read after the first barrier
-  // 1/(gamma-1) as a constant factor: a division by (gamma-1) at every point
-  // would cost an FP64 division sequence each (the values agree to rounding)
-  const double hg = GAS_GAMMA / (GAS_GAMMA - 1.0), ig = 1.0 / (GAS_GAMMA - 1.0);
-  const bool withD = mode == 1 || mode == 2;
-  const double sc = withD ? -1.0 : 1.0;  // sign of C in dst
-  if (active && lane < 3 * NN) swt[lc][lane / NN][lane % NN] = w[(long)c * 3 * NN + lane];
-  if (active && lane < NN) {
-    sft[lc][lane] = pfix[(long)c * NN + lane];
-    if (withD) spt[lc][lane] = p[(long)c * NN + lane];
+// euler_operator.h:1386-1507
+// cm [nc][24][8]: minus the volume part of C for the frozen p_fix, output i from
+// w's (d, j): gamma/(gamma-1) sum_q p_fix phi_j G[.][d] . grad phi_i.
+// 24 threads per cell: (d, i), all j.
+__global__ void __launch_bounds__(192)
+    k3_prep_C(double *__restrict__ cm, const double *__restrict__ pfix, Geo3 g) {
+  constexpr double hgf = GAS_GAMMA / (GAS_GAMMA - 1.0);
+  __shared__ double sphi[NQ][NN], sd[NQ][NN][3], spf[8][NQ];
+  for (int e = threadIdx.x; e < NQ * NN; e += blockDim.x) {
+    sphi[e / NN][e % NN] = c_phi[e / NN][e % NN];
+    for (int k = 0; k < 3; ++k) sd[e / NN][e % NN][k] = c_dphi[e / NN][e % NN][k];
   }
   __syncthreads();
-  if (active) {
-    if (lane < NQ) {
-      const int q = lane;
-      const double *cq = g.cg + ((long)c * NQ + q) * 13;
-      const double pf = at_qs(sft[lc], q, T);
-      double P[3];
+  const int c0 = blockIdx.x * 8, cnt = min(8, g.nc - c0);
+  for (int e = threadIdx.x; e < cnt * NQ; e += blockDim.x) {
+    const int l = e / NQ, q = e - l * NQ;
+    double s = 0.0;
 #pragma unroll
-      for (int d = 0; d < 3; ++d) P[d] = sc * (-cC * hg * pf * at_qs(swt[lc][d], q, T));
-      double Gr[3];
-      to_ref(cq, P, Gr);
-      sv[lc][q][0] = withD ? at_qs(spt[lc], q, T) * ig * cq[9] : 0.0;
+    for (int j = 0; j < NN; ++j) s = fma(sphi[q][j], __ldg(pfix + (long)(c0 + l) * NN + j), s);
+    spf[l][q] = hgf * s;
+  }
+  __syncthreads();
+  const int l = threadIdx.x / 24, o = threadIdx.x - l * 24, d = o / NN, i = o - d * NN;
+  if (l >= cnt) return;
+  double W[NN];
 #pragma unroll
-      for (int e = 0; e < 3; ++e) sv[lc][q][1 + e] = Gr[e];
-    }
-    for (int e = lane; e < 6 * NF; e += 32) {
-      const int f = e / NF, q = e - f * NF;
-      double a = 0.0;
-      const NbPt np = nb_point(g, c, f, q);
-      if (np.nb >= 0) {  // no boundary term
-        const double *fq = g.fg + (((long)c * 6 + f) * NF + q) * 4;
-        const double pfo = at_faces(sft[lc], f, q, T), pfn = nb_vals(np, pfix, 1, 0, T);
-        double av = 0.0, wno = 0.0, wnn = 0.0;
+  for (int j = 0; j < NN; ++j) W[j] = 0.0;
+  for (int q = 0; q < NQ; ++q) {
+    const double *cq = g.cg + ((long)(c0 + l) * NQ + q) * 13;
+    const double s = spf[l][q] * fma(__ldg(cq + d), sd[q][i][0],
+                                     fma(__ldg(cq + 3 + d), sd[q][i][1], __ldg(cq + 6 + d) * sd[q][i][2]));
 #pragma unroll
-        for (int d = 0; d < 3; ++d) {
-          const double wo = at_faces(swt[lc][d], f, q, T), wn = nb_vals(np, w, 3, d, T);
-          av += 0.5 * hg * (pfo * wo + pfn * wn) * fq[d];
-          wno += wo * fq[d];
-          wnn += wn * fq[d];
-        }
-        const double lam = fmax(fabs(wno), fabs(wnn));
-        a = sc * cC * (av + 0.5 * lam * (pfo - pfn) * ig) * fq[3];
+    for (int j = 0; j < NN; ++j) W[j] = fma(s, sphi[q][j], W[j]);
+  }
+  double *out = cm + ((long)(c0 + l) * 24 + d * NN) * NN + i;
+#pragma unroll
+  for (int j = 0; j < NN; ++j) out[j * NN] = W[j];
+}
+// face part of C: minus its nodal integrals, Fb[cell][face][4]
+__global__ void __launch_bounds__(NF * FPB)
+    k3_face_C(double *__restrict__ Fb, const double *__restrict__ w,
+              const double *__restrict__ pfix, Geo3 g) {
+  constexpr double ig = 1.0 / (GAS_GAMMA - 1.0), hgf = GAS_GAMMA * ig;
+  __shared__ double sF[FPB][1][NF];
+  const int f0 = blockIdx.x * FPB, nf = min(FPB, g.nfaces - f0);
+  const int lf = threadIdx.x / NF, q = threadIdx.x - lf * NF;
+  if (lf < nf) {
+    const FacePt P = face_point(g, g.own[f0 + lf], q);
+    double F = 0.0;
+    if (P.nb >= 0) {  // no boundary term
+      const double po = own_tr(P, pfix, 1, 0), pn = nb_tr(P, pfix, 1, 0);
+      double a = 0.0, b = 0.0;
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        a = fma(own_tr(P, w, 3, d), P.n[d], a);
+        b = fma(nb_tr(P, w, 3, d), P.n[d], b);
       }
-      sfa[lc][f][q] = a;
+      F = fma(0.5 * ig * abs_max(a, b), po - pn, 0.5 * hgf * fma(po, a, pn * b));
     }
+    sF[lf][0][q] = F;
   }
   __syncthreads();
-  if (active) {  // warp-uniform: every lane of the cell's warp takes part
-    const double o = gather3(sv[lc], sfa[lc], lane, T);
-    if (lane >= NN) return;
-    const int i = lane;
-    const long gi = (long)c * NN + i;
-    if (mode == 2) dst[gi] = invd[gi] * o;
-    else if (mode == 3) dst[gi] -= o;
-    else dst[gi] = o;
-  }
+  face_store<1>(&sF[0][0][0], g, f0, nf, Fb);
+}
+// mode 0 dst = cC C w; 1 dst = D p - cC C w; 2 dst = invd .* (D p - cC C w);
+// 3 dst -= cC C w.  A warp per cell: lane (part, i), part 0..2 the component of
+// w, part 3 p; two shuffles add the parts.
+constexpr int CB_CD = 8;
+__global__ void __launch_bounds__(32 * CB_CD)
+    k3_CD(double *__restrict__ dst, const double *__restrict__ w, const double *__restrict__ p,
+          double cC, const double *__restrict__ invd, int mode, const double *__restrict__ cm,
+          const double *__restrict__ dm, const double *__restrict__ Fb, Geo3 g) {
+  const int l = threadIdx.x >> 5, lane = threadIdx.x & 31, part = lane >> 3, i = lane & 7;
+  const int c = blockIdx.x * CB_CD + l;
+  if (c >= g.nc) return;  // warp-uniform
+  const bool withD = mode == 1 || mode == 2;
+  double in = 0.0;  // this lane's input value (part, vertex i)
+  if (part < 3) in = cC * __ldg(w + (long)c * 24 + lane);
+  else if (withD) in = __ldg(p + (long)c * NN + i);
+  const double *M = part < 3 ? cm + ((long)c * 24 + part * NN) * NN + i : dm + (long)c * NN * NN + i;
+  double o = 0.0;
+#pragma unroll
+  for (int j = 0; j < NN; ++j)
+    o = fma(__ldg(M + j * NN), __shfl_sync(0xffffffffu, in, (part << 3) + j), o);
+  o += __shfl_xor_sync(0xffffffffu, o, 8);
+  o += __shfl_xor_sync(0xffffffffu, o, 16);
+  if (lane >= NN) return;
+  const double *F = Fb + (long)c * 24;
+  const int x = i & 1, y = (i >> 1) & 1, z = i >> 2;
+  o = fma(cC, F[x * 4 + y + 2 * z] + F[(2 + y) * 4 + x + 2 * z] + F[(4 + z) * 4 + x + 2 * y], o);
+  const long gi = (long)c * NN + i;
+  if (mode == 0) dst[gi] = -o;
+  else if (mode == 1) dst[gi] = o;
+  else if (mode == 2) dst[gi] = invd[gi] * o;
+  else dst[gi] += o;
 }
 
 // ------------------------------------------------ cell-wise mass inverses --
@@ -684,7 +723,10 @@ struct atm3_ctx {
   cudaStream_t stream = nullptr;
   Geo3 g{};
   double *cg = nullptr, *fg = nullptr;
-  int *nbr = nullptr, *nbf = nullptr, *nperm = nullptr;
+  int *nbr = nullptr, *nbf = nullptr, *nperm = nullptr, *own = nullptr;
+  double *wb = nullptr, *nbt = nullptr, *dm = nullptr;  // B and D tables (k3_tables)
+  double *cm = nullptr;    // C's volume part for the frozen p_fix (k3_prep_C)
+  double *fbuf = nullptr;  // [nc][6][3][4] face integrals
   double dt = 1.0, Ma = 1.0, Fr = 1.0;
   int hstage = 1, nsstage = 1;
   Tableau tab;
@@ -751,9 +793,16 @@ int upload_tables3() {
       xi[t1] = gx[q / 3];
       q1(xi, fphi[f][q], nullptr);
     }
+  double psi[NF][4];
+  const double line[2] = {1.0 - gx[0], gx[0]};
+  for (int q = 0; q < NF; ++q)
+    for (int k = 0; k < 4; ++k)
+      psi[q][k] = ((k & 1) ? gx[q % 3] : 1.0 - gx[q % 3]) * ((k >> 1) ? gx[q / 3] : 1.0 - gx[q / 3]);
   if (cudaMemcpyToSymbol(c_phi, phi, sizeof(phi)) != cudaSuccess ||
       cudaMemcpyToSymbol(c_dphi, dphi, sizeof(dphi)) != cudaSuccess ||
-      cudaMemcpyToSymbol(c_fphi, fphi, sizeof(fphi)) != cudaSuccess) {
+      cudaMemcpyToSymbol(c_fphi, fphi, sizeof(fphi)) != cudaSuccess ||
+      cudaMemcpyToSymbol(c_psi, psi, sizeof(psi)) != cudaSuccess ||
+      cudaMemcpyToSymbol(c_line, line, sizeof(line)) != cudaSuccess) {
     set_error("failed to upload the 3D basis tables");
     return ATM_CUDA_ERROR;
   }
@@ -809,9 +858,10 @@ int alloc3(atm3_ctx &c, double **p, size_t n) {
 void free3(atm3_ctx *c) {
   if (!c) return;
   double *ds[] = {c->cg, c->fg, c->rho_fix, c->pres_fix, c->u_fix, c->minv, c->ainv, c->invd,
-                  c->wv1, c->ws1, c->ws2, c->red, c->red_out, c->dsmall, c->krylov, c->pool};
+                  c->wv1, c->ws1, c->ws2, c->red, c->red_out, c->dsmall, c->krylov, c->pool,
+                  c->wb, c->nbt, c->dm, c->cm, c->fbuf};
   for (double *d : ds) cudaFree(d);
-  cudaFree(c->nbr); cudaFree(c->nbf); cudaFree(c->nperm);
+  cudaFree(c->nbr); cudaFree(c->nbf); cudaFree(c->nperm); cudaFree(c->own);
   if (c->h_red) cudaFreeHost(c->h_red);
   delete c;
 }
@@ -843,55 +893,49 @@ Coef3 coef3(const atm3_ctx &c, int stage, bool rho_only) {
 double icoef3(const atm3_ctx &c) { return c.hstage == 1 ? c.tab.a22t : c.tab.a33t; }
 
 // ---- operators (positional source lists as the 2D entry points) -------------
-int rhs_rho3(atm3_ctx &c, double *dst, const double *const *src) {
+inline int fblocks(const atm3_ctx &c) { return (c.g.nfaces + FPB - 1) / FPB; }
+template <int KIND>
+int rhs3(atm3_ctx &c, double *dst, const double *const *src) {
+  const Coef3 co = coef3(c, c.hstage, KIND == 0);
+  const int nsrc = KIND == 0 ? 2 * co.nst : KIND == 1 ? 3 * co.nst + (c.hstage < 3) : 3 * co.nst + 2;
+  const int fields = KIND == 0 ? 4 * co.nst : KIND == 1 ? 5 * co.nst + (c.hstage < 3) : 5 * co.nst + 4;
   SrcPtrs sp{};
-  const Coef3 co = coef3(c, c.hstage, true);
-  for (int i = 0; i < 2 * co.nst; ++i) sp.p[i] = src[i];
-  k3_rhs_rho<<<(c.nc + CELLS3 - 1) / CELLS3, 32 * CELLS3, 0, c.stream>>>(dst, sp, co, c.g);
-  ATM_CHECK_LAUNCH("k3_rhs_rho");
+  for (int i = 0; i < nsrc; ++i) sp.p[i] = src[i];
+  k3_rhs_face<KIND><<<fblocks(c), NF * FPB, 0, c.stream>>>(c.fbuf, sp, co, c.hstage, c.g);
+  ATM_CHECK_LAUNCH("k3_rhs_face");
+  // 14 cells: 378 of 384 threads; small shells take small blocks
+  const int cpb = c.nc < 1500 ? 4 : 14, nc = KIND == 1 ? 3 : 1;
+  const size_t sm = sizeof(double) * (size_t)cpb * std::max(fields * 12, nc * 4 * NQ);
+  ATM_CUDA(allow_smem(k3_rhs_cell<KIND>, sm));
+  k3_rhs_cell<KIND><<<(c.nc + cpb - 1) / cpb, NQ * cpb, sm, c.stream>>>(dst, sp, co, c.hstage, fields,
+                                                                      c.g, c.fbuf, cpb);
+  ATM_CHECK_LAUNCH("k3_rhs_cell");
   return ATM_OK;
 }
+int rhs_rho3(atm3_ctx &c, double *dst, const double *const *src) { return rhs3<0>(c, dst, src); }
 // src: stage 1 {rho_old,u_old,p_old,rho_2}; 2 {.., u_2, p_2, rho_3};
 // 3 {.., u_3, p_3}
-int rhs_vel3(atm3_ctx &c, double *dst, const double *const *src) {
-  const Coef3 co = coef3(c, c.hstage, false);
-  SrcPtrs sp{}, gp{};
-  for (int i = 0; i < 3 * co.nst; ++i) sp.p[i] = src[i];
-  gp.p[0] = src[0];
-  gp.p[1] = src[3];
-  if (co.ng > 2) gp.p[2] = src[6];
-  k3_rhs_vel<<<(c.nc + CELLS3 - 1) / CELLS3, 32 * CELLS3, 0, c.stream>>>(dst, sp, gp, co, c.g);
-  ATM_CHECK_LAUNCH("k3_rhs_vel");
-  return ATM_OK;
-}
+int rhs_vel3(atm3_ctx &c, double *dst, const double *const *src) { return rhs3<1>(c, dst, src); }
 // src: stage 1 {rho_old,u_old,p_old,rho_2,u_fix}; 2 {.., u_2, p_2, rho_3,
 // u_fix}; 3 {.., u_3, p_3, rho_cur, u_cur}
-int rhs_pres3(atm3_ctx &c, double *dst, const double *const *src) {
-  const Coef3 co = coef3(c, c.hstage, false);
-  SrcPtrs sp{}, gp{};
-  for (int i = 0; i < 3 * co.nst; ++i) sp.p[i] = src[i];
-  if (c.hstage == 1) {
-    const double *g[] = {src[0], src[1], src[3], src[4], src[3], src[4]};
-    for (int i = 0; i < 6; ++i) gp.p[i] = g[i];
-  } else if (c.hstage == 2) {
-    const double *g[] = {src[0], src[1], src[3], src[4], src[6], src[7], src[6], src[7]};
-    for (int i = 0; i < 8; ++i) gp.p[i] = g[i];
-  } else {
-    const double *g[] = {src[0], src[1], src[3], src[4], src[6], src[7], src[9], src[10]};
-    for (int i = 0; i < 8; ++i) gp.p[i] = g[i];
-  }
-  k3_rhs_pres<<<(c.nc + CELLS3 - 1) / CELLS3, 32 * CELLS3, 0, c.stream>>>(dst, sp, gp, co, c.hstage, c.g);
-  ATM_CHECK_LAUNCH("k3_rhs_pres");
-  return ATM_OK;
-}
+int rhs_pres3(atm3_ctx &c, double *dst, const double *const *src) { return rhs3<2>(c, dst, src); }
 int B3(atm3_ctx &c, double *dst, const double *p, double cB, int mode) {
-  k3_B<<<(c.nc + CELLS3 - 1) / CELLS3, 32 * CELLS3, 0, c.stream>>>(dst, p, cB, c.ainv, mode, c.g);
+  k3_B<<<(c.nc + CB_B - 1) / CB_B, 24 * CB_B, 0, c.stream>>>(dst, p, cB, c.ainv, mode, c.wb, c.nbt,
+                                                           c.g);
   ATM_CHECK_LAUNCH("k3_B");
   return ATM_OK;
 }
+// after every change of pres_fix
+int prep_C3(atm3_ctx &c) {
+  k3_prep_C<<<(c.nc + 7) / 8, 192, 0, c.stream>>>(c.cm, c.pres_fix, c.g);
+  ATM_CHECK_LAUNCH("k3_prep_C");
+  return ATM_OK;
+}
 int CD3(atm3_ctx &c, double *dst, const double *w, const double *p, double cC, int mode) {
-  k3_CD<<<(c.nc + CELLS3 - 1) / CELLS3, 32 * CELLS3, 0, c.stream>>>(dst, w, p, c.pres_fix, cC, c.invd,
-                                                                      mode, c.g);
+  k3_face_C<<<fblocks(c), NF * FPB, 0, c.stream>>>(c.fbuf, w, c.pres_fix, c.g);
+  ATM_CHECK_LAUNCH("k3_face_C");
+  k3_CD<<<(c.nc + CB_CD - 1) / CB_CD, 32 * CB_CD, 0, c.stream>>>(dst, w, p, cC, c.invd, mode, c.cm,
+                                                               c.dm, c.fbuf, c.g);
   ATM_CHECK_LAUNCH("k3_CD");
   return ATM_OK;
 }
@@ -1015,6 +1059,7 @@ int set_rho_fixed3(atm3_ctx &c, const double *rho) {
 int pressure_fixed_point3(atm3_ctx &c) {
   const long ns = c.ns();
   TRY3(vec_copy(c.stream, c.pres_fix, c.p_fix_old, ns));
+  TRY3(prep_C3(c));
   if (c.hstage == 1) {
     const double *sp[] = {c.rho_old, c.u_old, c.p_old, c.rho_2, c.u_fixd};
     TRY3(rhs_pres3(c, c.rhs_p, sp));
@@ -1219,7 +1264,13 @@ int atm3_ctx_create(int n_cells, const double *nodes, int n_inner, const int *in
   cudaMemcpy(c->nbf, nbf.data(), nbf.size() * sizeof(int), cudaMemcpyHostToDevice);
   if (cudaMemcpy(c->nperm, nperm.data(), nperm.size() * sizeof(int), cudaMemcpyHostToDevice))
     return fail(cuda_fail(cudaGetLastError(), "upload shell tables"));
-  c->g = Geo3{n_cells, c->cg, c->fg, c->nbr, c->nbf, c->nperm};
+  std::vector<int> own;
+  for (int f = 0; f < n_inner; ++f) own.push_back(6 * inner[4 * f] + inner[4 * f + 1]);
+  for (int f = 0; f < n_bdry; ++f) own.push_back(6 * bdry[3 * f] + bdry[3 * f + 1]);
+  if (cudaMalloc(&c->own, own.size() * sizeof(int)) ||
+      cudaMemcpy(c->own, own.data(), own.size() * sizeof(int), cudaMemcpyHostToDevice))
+    return fail(cuda_fail(cudaGetLastError(), "upload shell tables"));
+  c->g = Geo3{n_cells, c->cg, c->fg, c->nbr, c->nbf, c->nperm, (int)own.size(), c->own};
   const long ns = c->ns(), nv = c->nv();
   double **sv[] = {&c->rho_fix, &c->pres_fix, &c->invd, &c->ws1, &c->ws2};
   for (double **p : sv)
@@ -1228,14 +1279,19 @@ int atm3_ctx_create(int n_cells, const double *nodes, int n_inner, const int *in
       (rc = alloc3(*c, &c->minv, (size_t)n_cells * 64)) ||
       (rc = alloc3(*c, &c->ainv, (size_t)n_cells * 64)) ||
       (rc = alloc3(*c, &c->red, 32 * RED_BLOCKS)) || (rc = alloc3(*c, &c->red_out, 64)) ||
-      (rc = alloc3(*c, &c->dsmall, 256)) ||
+      (rc = alloc3(*c, &c->dsmall, 256)) || (rc = alloc3(*c, &c->wb, (size_t)n_cells * 192)) ||
+      (rc = alloc3(*c, &c->nbt, (size_t)n_cells * 288)) ||
+      (rc = alloc3(*c, &c->dm, (size_t)n_cells * 64)) ||
+      (rc = alloc3(*c, &c->cm, (size_t)n_cells * 192)) ||
+      (rc = alloc3(*c, &c->fbuf, (size_t)n_cells * 72)) ||
       (rc = alloc3(*c, &c->krylov, (size_t)(RESTART3 + 1) * ns)))
     return fail(rc);
   if (cudaMallocHost(&c->h_red, 256 * sizeof(double)) != cudaSuccess)
     return fail(cuda_fail(cudaErrorMemoryAllocation, "cudaMallocHost"));
   k3_block_inverse<<<blocks(n_cells), 128, 0, c->stream>>>(c->minv, nullptr, c->g);
   k3_invdiag_D<<<blocks(n_cells), 128, 0, c->stream>>>(c->invd, c->g);
-  g_kernel_launches.fetch_add(2);
+  k3_tables<<<blocks(24 * n_cells), 128, 0, c->stream>>>(c->wb, c->nbt, c->dm, c->g);
+  g_kernel_launches.fetch_add(3);
   if (cudaStreamSynchronize(c->stream) != cudaSuccess)
     return fail(cuda_fail(cudaGetLastError(), "shell set-up kernels"));
   *out = c;
@@ -1273,7 +1329,10 @@ int atm3_set_frozen(atm3_ctx *h, const double *rho, const double *pres, const do
     int rc = rebuild_ainv3(*h);
     if (rc) return rc;
   }
-  if (pres) ATM_CUDA(cudaMemcpyAsync(h->pres_fix, pres, h->ns() * sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
+  if (pres) {
+    ATM_CUDA(cudaMemcpyAsync(h->pres_fix, pres, h->ns() * sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
+    if (int rc = prep_C3(*h)) return rc;
+  }
   if (u) ATM_CUDA(cudaMemcpyAsync(h->u_fix, u, h->nv() * sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
   return ATM_OK;
 }
