@@ -292,12 +292,13 @@ struct LevelViewT {
   cudaStream_t st;
   bool tune = false;  // the autotuner may time tile shapes on this stream
   const T *pfix = nullptr, *pfq = nullptr, *pff = nullptr;  // level p_fix (+ prepared)
+  T *fbuf = nullptr;  // [nc][4][2][nn] face integrals (the operator mesh only)
 };
 template <typename T>
 using OpView = LevelViewT<T>;
 inline OpView<double> schur_view(const atm_ctx &c) {
   return OpView<double>{c.k, c.nc, c.mesh, c.ainv, c.invdiag_D, c.stream,
-                        c.autotune && !c.capturing, c.pres_fix, c.pfq, c.pff};
+                        c.autotune && !c.capturing, c.pres_fix, c.pfq, c.pff, c.fbuf};
 }
 #define ATM_DISPATCH_K(kk, call)          \
   switch (kk) {                           \

@@ -31,8 +31,8 @@
 //
 // Measured on GB300 at 51,200 cells, k = 4 (before: the kernels of
 // schur_kernels.cuh, 2k+1 points everywhere, 9 threads per cell): FP64 B with
-// A^{-1} 0.56 -> 0.26 ms, C/D 0.55 -> 0.33 ms, the FP64 pipe busy 83-86% in
-// both; the FP32 V-cycle 1.54 -> 0.84 ms.
+// A^{-1} 0.56 -> 0.26 ms, C/D 0.55 -> 0.27 ms (53 us of it the faces), the FP64
+// pipe busy 83-88%; the FP32 V-cycle 1.54 -> 0.84 ms.
 //
 // In the Schur apply, B stores w = cB cC A^{-1} B p and C/D applies C with unit
 // coefficient: C is homogeneous of degree one in w for the positive cC
@@ -354,18 +354,122 @@ __global__ void __launch_bounds__(320)
   }
 }
 
+// nodal integrals o of C w over face f of cell c
+template <int K, typename T, bool HG>
+__device__ __forceinline__ void face_C(const T *__restrict__ w, const T *__restrict__ pfix,
+                                       const T *__restrict__ pff, const MeshT<T> &mesh, int c,
+                                       int f, T (&o)[K + 1]) {
+  constexpr int NN = K + 1, NN2 = NN * NN, NQ = 2 * K + 1;
+  const int nb = mesh.nbr[c * 4 + f], nfc = mesh.nbrf[c * 4 + f];
+  const int code = HG && nb >= 0 ? nfc >> 2 : 0;
+  const T *wc = w + (long)c * 2 * NN2;
+  if (nb < 0) {
+#pragma unroll
+    for (int i = 0; i < NN; ++i) o[i] = T(0);
+  } else if (!HG || code == 0) {
+    T t[NN], wx[NQ], wz[NQ], vx[NQ], vz[NQ], F[NQ];
+    const T *wn = w + (long)nb * 2 * NN2;
+    trace<K>(wc, f, t);
+    eo_interp<K, 2>(t, wx);
+    trace<K>(wc + NN2, f, t);
+    eo_interp<K, 2>(t, wz);
+    trace<K>(wn, nfc & 3, t);
+    eo_interp<K, 2>(t, vx);
+    trace<K>(wn + NN2, nfc & 3, t);
+    eo_interp<K, 2>(t, vz);
+    const T *hp = pff + ((long)c * 4 + f) * NQ, *hm = pff + ((long)nb * 4 + (nfc & 3)) * NQ;
+    const T *g = mesh.fC + ((long)c * 4 + f) * 2 * NQ;
+#pragma unroll
+    for (int q = 0; q < NQ; ++q)
+      F[q] = flux_C(g + 2 * q, wx[q], wz[q], vx[q], vz[q], __ldg(hp + q), __ldg(hm + q));
+    eo_integ<K, 2, NQ, true, false>(F, F, o);
+  } else {
+#pragma unroll
+    for (int i = 0; i < NN; ++i) o[i] = T(0);
+    // fine side (code 1, 2): one face, the neighbour at the shifted points;
+    // coarse side (code 3): two subfaces, this cell at the shifted points
+    for (int h = 0; h < (code == 3 ? 2 : 1); ++h) {
+      const int nc = code == 3 ? mesh.hnb[nb * 2 + h] : nb;
+      const T *wn = w + (long)nc * 2 * NN2;
+      T wx[NQ], wz[NQ], vx[NQ], vz[NQ], a[NQ], b[NQ], F[NQ];
+      own_or_sub<K>(wc, f, code == 3 ? h : -1, wx);
+      own_or_sub<K>(wc + NN2, f, code == 3 ? h : -1, wz);
+      own_or_sub<K>(pfix + (long)c * NN2, f, code == 3 ? h : -1, a);
+      own_or_sub<K>(wn, nfc & 3, code == 3 ? -1 : code - 1, vx);
+      own_or_sub<K>(wn + NN2, nfc & 3, code == 3 ? -1 : code - 1, vz);
+      own_or_sub<K>(pfix + (long)nc * NN2, nfc & 3, code == 3 ? -1 : code - 1, b);
+      const T *g = code == 3 ? mesh.hC + ((long)nb * 2 + h) * 2 * NQ
+                             : mesh.fC + ((long)c * 4 + f) * 2 * NQ;
+#pragma unroll
+      for (int q = 0; q < NQ; ++q)
+        F[q] = flux_C(g + 2 * q, wx[q], wz[q], vx[q], vz[q], a[q], b[q]);
+      if (code == 3) {
+        sub_integ_add<K, 1>(F, h, o);
+      } else {
+        eo_integ<K, 2, NQ, true, false>(F, F, o);
+      }
+    }
+  }
+}
+
+// what face_rows adds, from the face integrals of k_exact_face_C (Fb[c][f][NN]):
+// even conforming faces take the neighbour's with the sign flipped
+template <int K>
+__device__ __forceinline__ void face_rows_of(const double *__restrict__ Fb, const Mesh &mesh,
+                                             long c, int iz, double (&add)[K + 1]) {
+  constexpr int NN = K + 1;
+  const int4 nb4 = *reinterpret_cast<const int4 *>(mesh.nbr + c * 4);
+  const int4 nf4 = *reinterpret_cast<const int4 *>(mesh.nbrf + c * 4);
+  const int nb[4] = {nb4.x, nb4.y, nb4.z, nb4.w}, nf[4] = {nf4.x, nf4.y, nf4.z, nf4.w};
+#pragma unroll
+  for (int i = 0; i < NN; ++i) add[i] = 0.0;
+  // faces z = 0, 1 reach a row only at the first and last row
+  const int fz = iz == 0 ? 2 : 3;
+  const bool edge = iz == 0 || iz == K;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const int f = k < 2 ? k : fz;
+    const int b = k == 0 ? nb[0] : k == 1 ? nb[1] : fz == 2 ? nb[2] : nb[3];
+    const int n = k == 0 ? nf[0] : k == 1 ? nf[1] : fz == 2 ? nf[2] : nf[3];
+    if (b < 0 || (k == 2 && !edge)) continue;
+    const bool theirs = !(f & 1) && (n >> 2) == 0;
+    const double *F = Fb + (theirs ? (long)b * 4 + (n & 3) : c * 4 + f) * NN;
+    const long long flip = theirs ? (long long)0x8000000000000000ull : 0;
+    if (k < 2) {
+      const double v = __longlong_as_double(__double_as_longlong(F[iz]) ^ flip);
+      if (k == 0) add[0] = v;
+      else add[K] = v;
+    } else {
+#pragma unroll
+      for (int i = 0; i < NN; ++i)
+        add[i] += __longlong_as_double(__double_as_longlong(F[i]) ^ flip);
+    }
+  }
+}
+template <int K>
+__device__ __forceinline__ void face_rows_of(const float *, const MeshT<float> &, long, int,
+                                             float (&)[K + 1]) {}
+
 // ===================================================================== CD ===
 // MODE 0: dst = cC C w ; 3: dst -= cC C w
 // MODE 1: dst = D p - C w ; 2: dst = invd .* (D p - C w)
 // MODE 4: t = D p - C w with p = ch.x, then the Chebyshev update of ch
-// Threads (cell, column), column < NC; `cpb` cells per block, a multiple of 8, at
-// most 32.  Three blocks per SM in FP64 (80 registers, k = 4): two leave the
-// SM's quarters with 4, 4, 3 and 3 warps (51,200 cells: S apply 577 -> 572 us).
-template <int K, int MODE, typename T, bool HG>
-__global__ void __launch_bounds__(32 * Ex<K>::NC, sizeof(T) == 8 ? 3 : 1)
+//
+// Large FP64 meshes (FB): a face takes 256 FP64 instructions at k = 4, the rest
+// of a cell 2150, so k_exact_face_C integrates every conforming face once and
+// this kernel reads the integrals; without its own faces it fills blocks of
+// whole warps.  Smaller meshes (EXACT_FB_UNKNOWNS) and the FP32 levels (not
+// bound by arithmetic) integrate their own four faces.
+//
+// Threads (cell, column), column < NC; `cpb` cells per block, without FB a
+// multiple of 8, at most 32.  Three blocks per SM in FP64 (80 registers, k = 4):
+// two leave the SM's quarters with 4, 4, 3 and 3 warps (51,200 cells: S apply 577 -> 572 us).
+template <int K, int MODE, typename T, bool HG, bool FB>
+__global__ void __launch_bounds__(FB ? 256 : 32 * Ex<K>::NC, FB || (sizeof(T) == 8 && !HG) ? 3 : 1)
     k_exact_CD(T *__restrict__ dst, const T *__restrict__ w, const T *__restrict__ p,
                const T *__restrict__ pfix, const T *__restrict__ hq, const T *__restrict__ pff,
-               T cC, const T *__restrict__ invd, MeshT<T> mesh, ChebArgs<T> ch, int cpb) {
+               const T *__restrict__ Fb, T cC, const T *__restrict__ invd, MeshT<T> mesh,
+               ChebArgs<T> ch, int cpb) {
   using E = Ex<K>;
   constexpr int NN = E::NN, NN2 = E::NN2, NC = E::NC, NC2 = E::NC2, NQ = E::NQ;
   constexpr bool WITH_D = MODE == 1 || MODE == 2 || MODE == 4;
@@ -381,7 +485,7 @@ __global__ void __launch_bounds__(32 * Ex<K>::NC, sizeof(T) == 8 ? 3 : 1)
   T *sJ = sH + (STG ? cpb * 4 * NC2 : 0);      // [cpb][NC][NC]
   T *sV = sJ + (STG ? cpb * NC2 : 0);          // [NV][cpb][NN2]: rhs, invd, d, x
   T *X = sV + (STG ? NV * cpb * NN2 : 0);      // [cpb][NF][NN][NC] x-interpolated w, p; then xa, xb
-  T *Fs = X + cpb * NF * XS;                   // [cpb][4][NN] face integrals of C w
+  T *Fs = X + cpb * NF * XS;                   // [cpb][4][NN] face integrals of C w (not FB)
   const int tid = threadIdx.x, nt = blockDim.x;
   const int c0 = blockIdx.x * cpb;
   const int cnt = min(cpb, mesh.nc - c0);
@@ -402,65 +506,16 @@ __global__ void __launch_bounds__(32 * Ex<K>::NC, sizeof(T) == 8 ? 3 : 1)
   }
   // faces: one thread per (cell, face); with NC > 4 the first 4 cpb threads
   // (whole warps) take them while the others interpolate the rows
-  for (int e = tid; e < 4 * cnt; e += nt) {
+  for (int e = tid; !FB && e < 4 * cnt; e += nt) {
     const int l = e >> 2, f = e & 3, c = c0 + l;
-    const int nb = mesh.nbr[c * 4 + f], nfc = mesh.nbrf[c * 4 + f];
-    const int code = HG && nb >= 0 ? nfc >> 2 : 0;
-    const T *wc = w + (long)c * 2 * NN2;
     T o[NN];
-    if (nb < 0) {
-#pragma unroll
-      for (int i = 0; i < NN; ++i) o[i] = T(0);
-    } else if (!HG || code == 0) {
-      T t[NN], wx[NQ], wz[NQ], vx[NQ], vz[NQ], F[NQ];
-      const T *wn = w + (long)nb * 2 * NN2;
-      trace<K>(wc, f, t);
-      eo_interp<K, 2>(t, wx);
-      trace<K>(wc + NN2, f, t);
-      eo_interp<K, 2>(t, wz);
-      trace<K>(wn, nfc & 3, t);
-      eo_interp<K, 2>(t, vx);
-      trace<K>(wn + NN2, nfc & 3, t);
-      eo_interp<K, 2>(t, vz);
-      const T *hp = pff + ((long)c * 4 + f) * NQ, *hm = pff + ((long)nb * 4 + (nfc & 3)) * NQ;
-      const T *g = mesh.fC + ((long)c * 4 + f) * 2 * NQ;
-#pragma unroll
-      for (int q = 0; q < NQ; ++q)
-        F[q] = flux_C(g + 2 * q, wx[q], wz[q], vx[q], vz[q], __ldg(hp + q), __ldg(hm + q));
-      eo_integ<K, 2, NQ, true, false>(F, F, o);
-    } else {
-#pragma unroll
-      for (int i = 0; i < NN; ++i) o[i] = T(0);
-      // fine side (code 1, 2): one face, the neighbour at the shifted points;
-      // coarse side (code 3): two subfaces, this cell at the shifted points
-      for (int h = 0; h < (code == 3 ? 2 : 1); ++h) {
-        const int nc = code == 3 ? mesh.hnb[nb * 2 + h] : nb;
-        const T *wn = w + (long)nc * 2 * NN2;
-        T wx[NQ], wz[NQ], vx[NQ], vz[NQ], a[NQ], b[NQ], F[NQ];
-        own_or_sub<K>(wc, f, code == 3 ? h : -1, wx);
-        own_or_sub<K>(wc + NN2, f, code == 3 ? h : -1, wz);
-        own_or_sub<K>(pfix + (long)c * NN2, f, code == 3 ? h : -1, a);
-        own_or_sub<K>(wn, nfc & 3, code == 3 ? -1 : code - 1, vx);
-        own_or_sub<K>(wn + NN2, nfc & 3, code == 3 ? -1 : code - 1, vz);
-        own_or_sub<K>(pfix + (long)nc * NN2, nfc & 3, code == 3 ? -1 : code - 1, b);
-        const T *g = code == 3 ? mesh.hC + ((long)nb * 2 + h) * 2 * NQ
-                               : mesh.fC + ((long)c * 4 + f) * 2 * NQ;
-#pragma unroll
-        for (int q = 0; q < NQ; ++q)
-          F[q] = flux_C(g + 2 * q, wx[q], wz[q], vx[q], vz[q], a[q], b[q]);
-        if (code == 3) {
-          sub_integ_add<K, 1>(F, h, o);
-        } else {
-          eo_integ<K, 2, NQ, true, false>(F, F, o);
-        }
-      }
-    }
+    face_C<K, T, HG>(w, pfix, pff, mesh, c, f, o);
 #pragma unroll
     for (int i = 0; i < NN; ++i) Fs[(l * 4 + f) * NN + i] = o[i];
   }
   // rows (cell, field, iz): x-interpolation to the NC points
   {
-    constexpr bool SPLIT = NC > 4;
+    constexpr bool SPLIT = NC > 4 && !FB;
     const int first = SPLIT ? 4 * cpb : 0, stride = nt - first;
     for (int e = tid - first; e >= 0 && e < cnt * NF * NN; e += stride) {
       const int l = e / (NF * NN), r = e - l * (NF * NN);
@@ -526,7 +581,8 @@ __global__ void __launch_bounds__(32 * Ex<K>::NC, sizeof(T) == 8 ? 3 : 1)
       b[q] = x[XS + q];
     }
     eo_integ<K, 1, NC, true, true>(a, b, out);
-    face_rows<K>(Fs + l * 4 * NN, iz, add);
+    if constexpr (FB) face_rows_of<K>(Fb, mesh, c0 + l, iz, add);
+    else face_rows<K>(Fs + l * 4 * NN, iz, add);
     const long g0 = (long)(c0 + l) * NN2 + iz * NN;
     T s = cC;
     if (!WITH_D && mesh.dts) s *= mesh.dts[c0 + l];
@@ -558,6 +614,27 @@ __global__ void __launch_bounds__(32 * Ex<K>::NC, sizeof(T) == 8 ? 3 : 1)
       }
     }
   }
+}
+
+// Fb[c][f][k+1]: nodal integrals of C w over the odd local faces, whose conforming
+// neighbours read them with the opposite sign; with hanging faces also over
+// the even faces that are not the other side of a conforming one.
+template <int K, typename T, bool HG>
+__global__ void __launch_bounds__(64)
+    k_exact_face_C(T *__restrict__ Fb, const T *__restrict__ w, const T *__restrict__ pfix,
+                   const T *__restrict__ pff, MeshT<T> mesh) {
+  constexpr int NN = K + 1;
+  const long g = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  const bool even = HG && g >= 2L * mesh.nc;
+  const long e = even ? g - 2L * mesh.nc : g;
+  if (e >= 2L * mesh.nc) return;
+  const int c = (int)(e >> 1), f = (int)(e & 1) * 2 + (even ? 0 : 1);
+  const int nb = mesh.nbr[c * 4 + f];
+  if (nb < 0 || (even && (mesh.nbrf[c * 4 + f] >> 2) == 0)) return;
+  T o[NN];
+  face_C<K, T, HG>(w, pfix, pff, mesh, c, f, o);
+#pragma unroll
+  for (int i = 0; i < NN; ++i) Fb[((long)c * 4 + f) * NN + i] = o[i];
 }
 
 // ========================================================== p_fix prep ===
@@ -610,6 +687,11 @@ __global__ void __launch_bounds__(32 * Ex<K>::NC)
 // ============================================================ launchers ===
 // The autotuner's cells per block, rounded up to a multiple of 8 so that the
 // face threads of C/D fill whole warps.
+// Scalar unknowns from which FP64 C/D takes its face integrals from a kernel of
+// their own.  S apply without / with it: 37 / 43 us at 4140 cells, k = 3 (66,000
+// unknowns); 32 / 33 at 8192, k = 2 (74,000); 100 / 96 at 4140, k = 5 (149,000);
+// 109 / 102 at 8192, k = 4 (205,000); 573 / 530 at 51,200, k = 4.
+constexpr long EXACT_FB_UNKNOWNS = 140000;
 inline int exact_cells(int cpb) { return (cpb + 7) / 8 * 8; }
 
 template <int K, typename T, bool HG>
@@ -636,35 +718,53 @@ int exact_B_launch(const OpView<T> &v, T *dst, const T *p, T cB, T cC, int mode)
   return ATM_OK;
 }
 
+template <int K, int MODE, typename T, bool HG>
+auto exact_CD_kernel(bool fb) {
+  // FP32 has no FB form
+  if constexpr (sizeof(T) == 8)
+    return fb ? k_exact_CD<K, MODE, T, HG, true> : k_exact_CD<K, MODE, T, HG, false>;
+  else
+    return k_exact_CD<K, MODE, T, HG, false>;
+}
+
 template <int K, typename T, bool HG>
 int exact_CD_launch(const OpView<T> &v, T *dst, const T *w, const T *p, T cC, int mode,
                     const ChebArgs<T> *cheb) {
   using E = Ex<K>;
   const T *pfix = v.pfix;
   const ChebArgs<T> ch = cheb ? *cheb : ChebArgs<T>{};
+  const bool fb = sizeof(T) == 8 && v.fbuf && (long)v.nc * E::NN2 >= EXACT_FB_UNKNOWNS;
   bool overlap = false;  // not while the tuner times the kernel
   auto launch = [&](int tuned) -> cudaError_t {
     int cpb = v.nc < 2048 ? 8 : exact_cells(tuned);
     if (cpb > 32) cpb = 32;
+    // FB: the tuner's candidates are 64, 128 and 256 threads' worth of columns
+    if (fb) cpb = (tuned >= 256 / E::NQ ? 256 : tuned >= 128 / E::NQ ? 128 : 64) / E::NC;
     const int staged = sizeof(T) == 4 ? 5 * E::NC2 + (mode == 4 ? 4 * E::NN2 : 0) : 0;
     const size_t sm = sizeof(T) * (size_t)cpb *
                       ((mode == 0 || mode == 3 ? 2 : 3) * E::NN * E::NC + 4 * E::NN + staged);
-    void (*fn)(T *, const T *, const T *, const T *, const T *, const T *, T, const T *, MeshT<T>,
-               ChebArgs<T>, int) = mode == 0   ? k_exact_CD<K, 0, T, HG>
-                                   : mode == 1 ? k_exact_CD<K, 1, T, HG>
-                                   : mode == 2 ? k_exact_CD<K, 2, T, HG>
-                                   : mode == 3 ? k_exact_CD<K, 3, T, HG>
-                                               : k_exact_CD<K, 4, T, HG>;
+    auto fn = mode == 0   ? exact_CD_kernel<K, 0, T, HG>(fb)
+              : mode == 1 ? exact_CD_kernel<K, 1, T, HG>(fb)
+              : mode == 2 ? exact_CD_kernel<K, 2, T, HG>(fb)
+              : mode == 3 ? exact_CD_kernel<K, 3, T, HG>(fb)
+                          : exact_CD_kernel<K, 4, T, HG>(fb);
     if (cudaError_t e = allow_smem(fn, sm); e != cudaSuccess) return e;
-    return launch_overlapped(overlap, fn, (v.nc + cpb - 1) / cpb, cpb * E::NC, sm, v.st, dst, w, p, pfix,
-                             v.pfq, v.pff, cC, v.invd, v.mesh, ch, cpb);
+    return launch_overlapped(overlap, fn, (v.nc + cpb - 1) / cpb, cpb * E::NC, sm, v.st, dst, w, p,
+                             pfix, v.pfq, v.pff, (const T *)v.fbuf, cC, v.invd, v.mesh, ch, cpb);
   };
+  if constexpr (sizeof(T) == 8)
+    if (fb) {
+      const long n = (long)v.nc * (HG ? 4 : 2);
+      k_exact_face_C<K, T, HG><<<(unsigned)((n + 63) / 64), 64, 0, v.st>>>(v.fbuf, w, pfix, v.pff,
+                                                                         v.mesh);
+      ATM_CHECK_LAUNCH("k_exact_face_C");
+    }
   // modes 3 (dst -= C w) and 4 (x += d) are not idempotent: they use the
   // choices made for modes 0 and 1
   const bool idem = mode < 3 && dst != w && dst != p && dst != pfix;
   const int key = mode == 3 ? 0 : (mode == 4 ? 1 : mode);
   const int cpb = tuned_cpb(v.tune, v.st, TF_CD, K, key, HG, (int)sizeof(T), v.nc, idem, launch);
-  overlap = !HG;
+  overlap = !HG && !fb;
   ATM_CUDA(launch(cpb));
   g_kernel_launches.fetch_add(1);
   return ATM_OK;

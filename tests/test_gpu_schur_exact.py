@@ -57,6 +57,28 @@ def test_operators_at_block_edges(cuda_ok, nx, nz, degree, mapping_degree):
     assert rel(s, o.vmult(p)) < 1e-11
 
 
+@pytest.mark.parametrize("nx,nz,degree,adaptive", [(74, 52, 5, False), (75, 52, 5, False),
+                                                   (98, 90, 3, True)])
+def test_face_integrals_of_their_own(cuda_ok, nx, nz, degree, adaptive):
+    """Just below and above the size from which C/D reads its face integrals
+    from k_exact_face_C (140,000 unknowns), walls, and hanging faces above it."""
+    p = HillParams(nx=nx, nz=nz, degree=degree, cfl=3.0, periodic=adaptive)
+    case = build_case(p)
+    if adaptive:
+        from atmospheric_flows_gb300 import amr
+
+        case = amr.adaptive_case(p, amr.example_tree(nx, nz, True))
+        assert case.n_cells * (degree + 1) ** 2 > 140000
+    g, o, rng = operators(case)
+    w = case.u + rng.standard_normal(case.u.shape)
+    s = torch.full((g.n_scalar,), np.nan, dtype=torch.float64, device="cuda")
+    g.vmult_enthalpy(s, dev(w))
+    assert rel(s, o.vmult_enthalpy(w)) < 1e-12
+    q = case.p * (1 + 0.01 * rng.standard_normal(case.p.shape))
+    g.vmult(s, dev(q))
+    assert rel(s, o.vmult(q)) < 1e-11
+
+
 def test_upload_mesh_changes_the_route(cuda_ok):
     """A mapping of degree 2, then 3, then 2 in one context: p_fix set once."""
     from atmospheric_flows_gb300 import _lib
