@@ -45,7 +45,7 @@ struct MGLevelT {
   int *children = nullptr;  // [nc][4] cells of level-1 (levels >= 1)
   T *ainv = nullptr, *invd = nullptr, *rho = nullptr, *pfix = nullptr;
   T *pfq = nullptr, *pff = nullptr;  // p_fix at quadrature points / face traces
-  T *x = nullptr, *b = nullptr, *r = nullptr, *t = nullptr, *d = nullptr, *wv = nullptr;
+  T *x = nullptr, *b = nullptr, *t = nullptr, *d = nullptr, *wv = nullptr;
   double lam = 0.0;
 };
 
@@ -99,19 +99,16 @@ __global__ void k_convert(A *__restrict__ o, const B *__restrict__ i, long n) {
   for (long k = (long)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (long)gridDim.x * blockDim.x)
     o[k] = (A)i[k];
 }
-// Chebyshev update with r = rhs - t (t ignored when `zero_t`):
-//   mode 0: d = b invd r, x = d        (start from x = 0)
-//   mode 1: d = b invd r, x += d       (first step from a given x)
-//   mode 2: d = a d + b invd r, x += d (later steps)
+// V-cycle input and the first Chebyshev step from zero on the finest level:
+// b = v, d = x = cb invd b
 template <typename T>
-__global__ void k_cheb(T *__restrict__ x, T *__restrict__ d, const T *__restrict__ rhs,
-                       const T *__restrict__ t, const T *__restrict__ invd, T a, T b,
-                       int zero_t, int mode, long n) {
+__global__ void k_mg_start(T *__restrict__ b, T *__restrict__ d, T *__restrict__ x,
+                           const double *__restrict__ v, const T *__restrict__ invd, T cb, long n) {
   for (long k = (long)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (long)gridDim.x * blockDim.x) {
-    const T r = zero_t ? rhs[k] : rhs[k] - t[k];
-    const T dk = (mode == 2 ? a * d[k] : T(0)) + b * invd[k] * r;
+    const T r = (T)v[k], dk = cb * invd[k] * r;
+    b[k] = r;
     d[k] = dk;
-    x[k] = mode == 0 ? dk : x[k] + dk;
+    x[k] = dk;
   }
 }
 template <typename T>
@@ -173,58 +170,107 @@ __global__ void k_hash_init(T *__restrict__ v, long n) {
   }
 }
 
+// Transfers: blocks of whole cells (XFER_CELLS fine cells, or as many coarse
+// ones), one thread per node, the 1D contractions in two passes through shared
+// memory with the tables staged there (indexed by lane, constant memory would
+// serialise them).  Bound by their vectors' traffic and their launch: 1.28 M
+// nodes, k = 4, FP32: prolongation 25 -> 8 us, residual and restriction
+// together 20 -> 9 us.
+constexpr int XFER_CELLS = 8;
 template <int K, typename T>
-__global__ void k_prolong_add(T *__restrict__ fine, const T *__restrict__ coarse,
-                              const int *__restrict__ parent, const int *__restrict__ ppos,
-                              int ncf, XferTabT<T> tb) {
-  constexpr int NN = K + 1, NN2 = NN * NN;
-  const long g = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= (long)ncf * NN2) return;
-  const int cf = (int)(g / NN2), i = (int)(g - (long)cf * NN2);
-  const int iz = i / NN, ix = i - iz * NN;
-  const int pos = ppos[cf], a = pos & 1, b = pos >> 1;
-  const T *u = coarse + (long)parent[cf] * NN2;
-  if (pos == 4) {  // cell unchanged on the coarser level
-    fine[g] += u[i];
-    return;
+__device__ __forceinline__ void xfer_stage(T (&sE)[2][K + 1][K + 1], const XferTabT<T> &tb) {
+  constexpr int NN = K + 1;
+  for (int e = threadIdx.x; e < 2 * NN * NN; e += blockDim.x) {
+    const int a = e / (NN * NN), r = e - a * NN * NN;
+    sE[a][r / NN][r % NN] = tb.E[a][r / NN][r % NN];
   }
-  T s = 0;
-#pragma unroll
-  for (int jz = 0; jz < NN; ++jz) {
-    T t = 0;
-#pragma unroll
-    for (int jx = 0; jx < NN; ++jx) t = fma(tb.E[a][ix][jx], u[jz * NN + jx], t);
-    s = fma(tb.E[b][iz][jz], t, s);
-  }
-  fine[g] += s;
 }
 
 template <int K, typename T>
-__global__ void k_restrict(T *__restrict__ coarse, const T *__restrict__ fine,
-                           const int *__restrict__ children, int ncc, XferTabT<T> tb) {
+__global__ void __launch_bounds__(XFER_CELLS *(K + 1) * (K + 1))
+    k_prolong_add(T *__restrict__ fine, const T *__restrict__ coarse,
+                  const int *__restrict__ parent, const int *__restrict__ ppos, int ncf,
+                  XferTabT<T> tb) {
   constexpr int NN = K + 1, NN2 = NN * NN;
-  const long g = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= (long)ncc * NN2) return;
-  const int cc = (int)(g / NN2), j = (int)(g - (long)cc * NN2);
-  const int jz = j / NN, jx = j - jz * NN;
-  if (children[cc * 4 + 1] < 0) {  // cell unchanged on this level
-    coarse[g] = fine[(long)children[cc * 4] * NN2 + j];
-    return;
+  __shared__ T sE[2][NN][NN], sT[XFER_CELLS][NN2];
+  xfer_stage<K, T>(sE, tb);
+  const int l = threadIdx.x / NN2, i = threadIdx.x - l * NN2, iz = i / NN, ix = i - iz * NN;
+  const int cf = blockIdx.x * XFER_CELLS + l;
+  const bool active = cf < ncf;
+  const int pos = active ? ppos[cf] : 4;
+  const T *u = coarse + (long)(active ? parent[cf] : 0) * NN2;
+  __syncthreads();
+  if (pos != 4) {  // row iz of the parent along x
+    T t = 0;
+#pragma unroll
+    for (int jx = 0; jx < NN; ++jx) t = fma(sE[pos & 1][ix][jx], u[iz * NN + jx], t);
+    sT[l][i] = t;
   }
+  __syncthreads();
+  if (!active) return;
   T s = 0;
+  if (pos == 4) {  // cell unchanged on the coarser level
+    s = u[i];
+  } else {
 #pragma unroll
-  for (int pos = 0; pos < 4; ++pos) {
-    const int a = pos & 1, b = pos >> 1;
-    const T *r = fine + (long)children[cc * 4 + pos] * NN2;
+    for (int jz = 0; jz < NN; ++jz) s = fma(sE[pos >> 1][iz][jz], sT[l][jz * NN + ix], s);
+  }
+  fine[(long)cf * NN2 + i] += s;
+}
+
+// coarse = R (b - t), the restricted residual, and the first Chebyshev step
+// from zero on the coarse level: d = x = cb invd coarse
+template <int K, typename T>
+__global__ void __launch_bounds__(XFER_CELLS *(K + 1) * (K + 1))
+    k_restrict(T *__restrict__ coarse, const T *__restrict__ b, const T *__restrict__ t,
+               const int *__restrict__ children, int ncc, XferTabT<T> tb,
+               const T *__restrict__ invd, T cb, T *__restrict__ x, T *__restrict__ d) {
+  constexpr int NN = K + 1, NN2 = NN * NN;
+  __shared__ T sE[2][NN][NN], sR[XFER_CELLS][4][NN2], sT[XFER_CELLS][2][NN2];
+  xfer_stage<K, T>(sE, tb);
+  const int l = threadIdx.x / NN2, j = threadIdx.x - l * NN2, jz = j / NN, jx = j - jz * NN;
+  const int cc = blockIdx.x * XFER_CELLS + l;
+  const bool active = cc < ncc;
+  bool same = false;  // cell unchanged on this level
+  if (active) {
+    const int4 ch = *reinterpret_cast<const int4 *>(children + (long)cc * 4);
+    const int c4[4] = {ch.x, ch.y, ch.z, ch.w};
+    same = c4[1] < 0;
 #pragma unroll
-    for (int iz = 0; iz < NN; ++iz) {
-      T t = 0;
+    for (int p = 0; p < 4; ++p)
+      if (p == 0 || !same) {
+        const long g = (long)c4[p] * NN2 + j;
+        sR[l][p][j] = b[g] - t[g];
+      }
+  }
+  __syncthreads();
+  if (active && !same) {  // row jz of both halves in z, contracted along x
 #pragma unroll
-      for (int ix = 0; ix < NN; ++ix) t = fma(tb.E[a][ix][jx], r[iz * NN + ix], t);
-      s = fma(tb.E[b][iz][jz], t, s);
+    for (int h = 0; h < 2; ++h) {
+      T s = 0;
+#pragma unroll
+      for (int a = 0; a < 2; ++a)
+#pragma unroll
+        for (int ix = 0; ix < NN; ++ix) s = fma(sE[a][ix][jx], sR[l][a + 2 * h][jz * NN + ix], s);
+      sT[l][h][j] = s;
     }
   }
+  __syncthreads();
+  if (!active) return;
+  T s = 0;
+  if (same) {
+    s = sR[l][0][j];
+  } else {
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int iz = 0; iz < NN; ++iz) s = fma(sE[h][iz][jz], sT[l][h][iz * NN + jx], s);
+  }
+  const long g = (long)cc * NN2 + j;
+  const T dk = cb * invd[g] * s;
   coarse[g] = s;
+  d[g] = dk;
+  x[g] = dk;
 }
 
 template <int K, typename T>
@@ -272,6 +318,20 @@ inline int gsz(long n) {
     default: kern<5, T><<<grid, 256, 0, c.stream>>>(__VA_ARGS__); break;     \
   }
 
+// the transfers' launches (blocks of whole cells)
+#define MG_XFER(kk, T, kern, cells, ...)                                                      \
+  do {                                                                                        \
+    const int grid_ = ((cells) + XFER_CELLS - 1) / XFER_CELLS;                                \
+    switch (kk) {                                                                             \
+      case 1: kern<1, T><<<grid_, XFER_CELLS * 4, 0, c.stream>>>(__VA_ARGS__); break;         \
+      case 2: kern<2, T><<<grid_, XFER_CELLS * 9, 0, c.stream>>>(__VA_ARGS__); break;         \
+      case 3: kern<3, T><<<grid_, XFER_CELLS * 16, 0, c.stream>>>(__VA_ARGS__); break;        \
+      case 4: kern<4, T><<<grid_, XFER_CELLS * 25, 0, c.stream>>>(__VA_ARGS__); break;        \
+      default: kern<5, T><<<grid_, XFER_CELLS * 36, 0, c.stream>>>(__VA_ARGS__); break;       \
+    }                                                                                         \
+    LAUNCHED();                                                                               \
+  } while (0)
+
 template <typename T>
 LevelViewT<T> lview(const atm_ctx &c, const MGLevelT<T> &L) {
   return LevelViewT<T>{c.k, L.nc, L.mesh, L.ainv, L.invd, c.stream, c.autotune && !c.capturing,
@@ -293,7 +353,7 @@ void level_free(MGLevelT<T> &L) {
   cudaFree(L.parent); cudaFree(L.ppos); cudaFree(L.children);
   cudaFree(L.ainv); cudaFree(L.invd); cudaFree(L.rho); cudaFree(L.pfix);
   cudaFree(L.pfq); cudaFree(L.pff);
-  cudaFree(L.x); cudaFree(L.b); cudaFree(L.r); cudaFree(L.t); cudaFree(L.d); cudaFree(L.wv);
+  cudaFree(L.x); cudaFree(L.b); cudaFree(L.t); cudaFree(L.d); cudaFree(L.wv);
   L = MGLevelT<T>();
 }
 
@@ -376,7 +436,7 @@ int level_alloc(atm_ctx &c, MGLevelT<T> &L, const HostMesh &hm) {
       ATM_CUDA(cudaStreamSynchronize(c.stream));
     }
   }
-  T **vecs[] = {&L.invd, &L.rho, &L.pfix, &L.x, &L.b, &L.r, &L.t, &L.d};
+  T **vecs[] = {&L.invd, &L.rho, &L.pfix, &L.x, &L.b, &L.t, &L.d};
   for (T **v : vecs) {
     ATM_CUDA(cudaMalloc(v, ns * sizeof(T)));
     ATM_CUDA(cudaMemsetAsync(*v, 0, ns * sizeof(T), c.stream));
@@ -539,21 +599,24 @@ int estimate_lambda(atm_ctx &c, MGLevelT<T> &L, int its) {
   return ATM_OK;
 }
 
-// Chebyshev smoothing of S_l x = b on [1.2 lam / range, 1.2 lam]
+// Chebyshev on [1.2 lam / range, 1.2 lam]: centre and half width
 template <typename T>
-int chebyshev(atm_ctx &c, MGLevelT<T> &L, int degree, double range, bool zero_start) {
-  const long n = (long)L.nc * c.nn2;
+void cheb_interval(const MGLevelT<T> &L, double range, double &theta, double &delta) {
   const double hi = 1.2 * L.lam, lo = hi / range;
-  const double theta = 0.5 * (hi + lo), delta = 0.5 * (hi - lo), sigma = theta / delta;
+  theta = 0.5 * (hi + lo);
+  delta = 0.5 * (hi - lo);
+}
+
+// Chebyshev smoothing of S_l x = b from the given x, or, with `begun`, from zero
+// with the first step already done (k_mg_start, k_restrict)
+template <typename T>
+int chebyshev(atm_ctx &c, MGLevelT<T> &L, int degree, double range, bool begun) {
+  double theta, delta;
+  cheb_interval(L, range, theta, delta);
+  const double sigma = theta / delta;
   double rho = 1.0 / sigma;
   int rc;
-  if (zero_start) {
-    k_cheb<T><<<gsz(n), 256, 0, c.stream>>>(L.x, L.d, L.b, L.t, L.invd, T(0),
-                                             (T)(1.0 / theta), 1, 0, n);
-    LAUNCHED();
-  } else if ((rc = level_apply_cheb<T>(c, L, 0.0, 1.0 / theta, true))) {
-    return rc;
-  }
+  if (!begun && (rc = level_apply_cheb<T>(c, L, 0.0, 1.0 / theta, true))) return rc;
   for (int k = 1; k < degree; ++k) {
     const double rho_new = 1.0 / (2.0 * sigma - rho);
     if ((rc = level_apply_cheb<T>(c, L, rho_new * rho, 2.0 * rho_new / delta, false))) return rc;
@@ -565,24 +628,20 @@ int chebyshev(atm_ctx &c, MGLevelT<T> &L, int degree, double range, bool zero_st
 template <typename T>
 int vcycle(atm_ctx &c, MG &mg, MGHier<T> &H, int l) {
   MGLevelT<T> &L = H.lv[l];
-  const long n = (long)L.nc * c.nn2;
+  const int last = (int)H.lv.size() - 1;
   int rc;
   // the vector work of this level (transfers, Chebyshev updates) is timed
   // as a whole by the caller's KF_MG_OTHER region minus the level applies
-  if (l == (int)H.lv.size() - 1) return chebyshev<T>(c, L, mg.coarse_deg, mg.coarse_range, true);
+  if (l == last) return chebyshev<T>(c, L, mg.coarse_deg, mg.coarse_range, true);
   if ((rc = chebyshev<T>(c, L, mg.cheb_deg, mg.range, true))) return rc;
   if ((rc = level_apply<T>(c, L, L.t, L.x))) return rc;
-  k_sub<T><<<gsz(n), 256, 0, c.stream>>>(L.r, L.b, L.t, n);
-  LAUNCHED();
   MGLevelT<T> &Cl = H.lv[l + 1];
-  const long nc2 = (long)Cl.nc * c.nn2;
-  MG_DISPATCH(c.k, T, k_restrict, (int)((nc2 + 255) / 256), Cl.b, L.r, Cl.children, Cl.nc,
-              H.tab);
-  LAUNCHED();
+  double theta, delta;
+  cheb_interval(Cl, l + 1 == last ? mg.coarse_range : mg.range, theta, delta);
+  MG_XFER(c.k, T, k_restrict, Cl.nc, Cl.b, L.b, L.t, Cl.children, Cl.nc, H.tab, Cl.invd,
+          (T)(1.0 / theta), Cl.x, Cl.d);
   if ((rc = vcycle<T>(c, mg, H, l + 1))) return rc;
-  MG_DISPATCH(c.k, T, k_prolong_add, (int)((n + 255) / 256), L.x, Cl.x, L.parent, L.ppos, L.nc,
-              H.tab);
-  LAUNCHED();
+  MG_XFER(c.k, T, k_prolong_add, L.nc, L.x, Cl.x, L.parent, L.ppos, L.nc, H.tab);
   return chebyshev<T>(c, L, mg.cheb_deg, mg.range, false);
 }
 
@@ -625,7 +684,8 @@ int prepare(atm_ctx &c, MG &mg) {
   return ATM_OK;
 }
 
-// Record one V-cycle (input L0.b, output L0.x) into H.graph.  The capture
+// Record one V-cycle (input L0.b, its first step in L0.x and L0.d; output L0.x)
+// into H.graph.  The capture
 // runs on the hierarchy's private non-blocking stream (the legacy default
 // stream cannot be captured) in thread-local mode, so members captured or
 // running on other threads are not affected; the kernels counted while
@@ -671,7 +731,9 @@ int precondition(atm_ctx &c, MG &mg, double *z, const double *v) {
   MGHier<T> &H = hier<T>(mg);
   MGLevelT<T> &L0 = H.lv[0];
   const long n = c.n_scalar();
-  k_convert<T, double><<<gsz(n), 256, 0, c.stream>>>(L0.b, v, n);
+  double theta, delta;
+  cheb_interval(L0, mg.range, theta, delta);
+  k_mg_start<T><<<gsz(n), 256, 0, c.stream>>>(L0.b, L0.d, L0.x, v, L0.invd, (T)(1.0 / theta), n);
   LAUNCHED();
   int rc = ATM_OK;
   bool replayed = false;

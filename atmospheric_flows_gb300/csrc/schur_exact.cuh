@@ -463,9 +463,9 @@ __device__ __forceinline__ void face_rows_of(const float *, const MeshT<float> &
 //
 // Threads (cell, column), column < NC; `cpb` cells per block, without FB a
 // multiple of 8, at most 32.  Three blocks per SM in FP64 (80 registers, k = 4):
-// two leave the SM's quarters with 4, 4, 3 and 3 warps (51,200 cells: S apply 577 -> 572 us).
+// two leave the SM's quarters with 4, 4, 3 and 3 warps (51,200 cells: S apply 577 -> 572 us); five in FP32.
 template <int K, int MODE, typename T, bool HG, bool FB>
-__global__ void __launch_bounds__(FB ? 256 : 32 * Ex<K>::NC, FB || (sizeof(T) == 8 && !HG) ? 3 : 1)
+__global__ void __launch_bounds__(FB ? 256 : 32 * Ex<K>::NC, FB ? 3 : HG ? 1 : sizeof(T) == 8 ? 3 : 5)
     k_exact_CD(T *__restrict__ dst, const T *__restrict__ w, const T *__restrict__ p,
                const T *__restrict__ pfix, const T *__restrict__ hq, const T *__restrict__ pff,
                const T *__restrict__ Fb, T cC, const T *__restrict__ invd, MeshT<T> mesh,
