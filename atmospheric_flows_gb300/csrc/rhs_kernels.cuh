@@ -45,33 +45,53 @@ struct RhsKind {
 };
 
 // =============================================================== faces ===
-// F[comp][q] += numerical flux of all stage states at the points of one face,
-// outward of cell c, times the face weight.  n0, n1: normal times weight.
-// sub_o / sub_n >= 0: this cell's / the neighbour's trace on that subface.
-template <int K, int ST, int KIND, bool HG>
-__device__ __forceinline__ void face_flux(const SrcPtrs &src, const StageCoef &co, int c, int f,
-                                          int sub_o, int nb, int nf, int sub_n,
-                                          const double (&n0)[2 * K + 1],
-                                          const double (&n1)[2 * K + 1],
-                                          double (&F)[RhsKind<KIND>::NCOMP][2 * K + 1]) {
-  constexpr int NN2 = (K + 1) * (K + 1), NQ = 2 * K + 1, PER = RhsKind<KIND>::PER;
+// Traces of a cell's field on a face: at all 2k+1 points of the face or of its
+// subface `sub` (>= 0), or at one point of it whose basis row is given.
+template <int K>
+struct LineTrace {
+  int f, sub;
+  __device__ __forceinline__ void operator()(const double *cell, double (&v)[2 * K + 1]) const {
+    own_or_sub<K>(cell, f, sub, v);
+  }
+};
+template <int K>
+struct PointTrace {
+  int f;
+  const double *row;
+  __device__ __forceinline__ void operator()(const double *cell, double (&v)[1]) const {
+    double t[K + 1], s = 0.0;
+    trace<K>(cell, f, t);
+#pragma unroll
+    for (int i = 0; i <= K; ++i) s = fma(row[i], t[i], s);
+    v[0] = s;
+  }
+};
+
+// F[comp][q] += numerical flux of all stage states at NQ points of one face,
+// outward of cell c, times the face weight.  n0, n1: normal times weight; to,
+// tn: traces of this cell and of the neighbour.
+template <int K, int ST, int KIND, int NQ, typename Trace>
+__device__ __forceinline__ void face_flux(const SrcPtrs &src, const StageCoef &co, int c, int nb,
+                                          const Trace &to, const Trace &tn,
+                                          const double (&n0)[NQ], const double (&n1)[NQ],
+                                          double (&F)[RhsKind<KIND>::NCOMP][NQ]) {
+  constexpr int NN2 = (K + 1) * (K + 1), PER = RhsKind<KIND>::PER;
   constexpr double IG = 1.0 / (GAS_GAMMA - 1.0), HGF = GAS_GAMMA * IG;
   constexpr bool MIXED = KIND == 2 && ST == 2;  // stage 2 mixes the states' velocities
-  if (!HG) sub_o = sub_n = -1;
   double xo[MIXED ? NQ : 1], zo[MIXED ? NQ : 1], xn[MIXED ? NQ : 1], zn[MIXED ? NQ : 1];
 #pragma unroll
   for (int j = 0; j < ST; ++j) {
     const double *sr = src.p[PER * j], *su = src.p[PER * j + 1];
     double r[NQ], ux[NQ], uz[NQ], p[NQ], un[NQ];
-    own_or_sub<K>(sr + (long)c * NN2, f, sub_o, r);
-    own_or_sub<K>(su + (long)c * 2 * NN2, f, sub_o, ux);
-    own_or_sub<K>(su + ((long)c * 2 + 1) * NN2, f, sub_o, uz);
-    if (KIND > 0) own_or_sub<K>(src.p[PER * j + 2] + (long)c * NN2, f, sub_o, p);
+    to(sr + (long)c * NN2, r);
+    to(su + (long)c * 2 * NN2, ux);
+    to(su + ((long)c * 2 + 1) * NN2, uz);
+    if (KIND > 0) to(src.p[PER * j + 2] + (long)c * NN2, p);
     double vr[NQ], vx[NQ], vz[NQ], vp[NQ];
-    own_or_sub<K>(sr + (long)nb * NN2, nf, sub_n, vr);
-    own_or_sub<K>(su + (long)nb * 2 * NN2, nf, sub_n, vx);
-    own_or_sub<K>(su + ((long)nb * 2 + 1) * NN2, nf, sub_n, vz);
-    if (KIND > 0) own_or_sub<K>(src.p[PER * j + 2] + (long)nb * NN2, nf, sub_n, vp);
+    tn(sr + (long)nb * NN2, vr);
+    tn(su + (long)nb * 2 * NN2, vx);
+    tn(su + ((long)nb * 2 + 1) * NN2, vz);
+    if (KIND > 0) tn(src.p[PER * j + 2] + (long)nb * NN2, vp);
 #pragma unroll
     for (int q = 0; q < NQ; ++q) un[q] = fma(ux[q], n0[q], uz[q] * n1[q]);
     if constexpr (KIND == 0) {
@@ -167,7 +187,8 @@ __global__ void __launch_bounds__(64)
         }
       }
     } else {
-      face_flux<K, ST, KIND, HG>(src, co, c, f, -1, nb, nf, code - 1, n0, n1, F);
+      face_flux<K, ST, KIND>(src, co, c, nb, LineTrace<K>{f, -1},
+                             LineTrace<K>{nf, HG ? code - 1 : -1}, n0, n1, F);
     }
 #pragma unroll
     for (int d = 0; d < NCOMP; ++d) eo_integ<K, 2, NQ, true, false>(F[d], F[d], o[d]);
@@ -185,7 +206,8 @@ __global__ void __launch_bounds__(64)
 #pragma unroll
         for (int d = 0; d < NCOMP; ++d) F[d][q] = 0.0;
       }
-      face_flux<K, ST, KIND, HG>(src, co, c, f, h, mesh.hnb[nb * 2 + h], nf, -1, n0, n1, F);
+      face_flux<K, ST, KIND>(src, co, c, mesh.hnb[nb * 2 + h], LineTrace<K>{f, h},
+                             LineTrace<K>{nf, -1}, n0, n1, F);
 #pragma unroll
       for (int d = 0; d < NCOMP; ++d) sub_integ_add<K, 1>(F[d], h, o[d]);
     }
@@ -195,6 +217,73 @@ __global__ void __launch_bounds__(64)
   for (int d = 0; d < NCOMP; ++d)
 #pragma unroll
     for (int i = 0; i < NN; ++i) out[d * NN + i] = o[d][i];
+}
+
+// The same on a conforming mesh with one thread per face point, RHS_FPB faces
+// per block: 5 instead of 4 FP64 instructions per trace value at k = 4, but nine
+// times the threads.  A face per thread needs tens of thousands of faces to
+// reach every quarter of every SM, each of which takes 64 clocks for an FP64
+// instruction whether one warp issues it or many.
+constexpr int RHS_FPB = 16;
+template <int K, int ST, int KIND>
+__global__ void __launch_bounds__(RHS_FPB *(2 * K + 1))
+    k_rhs_face_points(double *__restrict__ Fb, SrcPtrs src, StageCoef co, Mesh mesh) {
+  constexpr int NN = K + 1, NN2 = NN * NN, NQ = 2 * K + 1, NCOMP = RhsKind<KIND>::NCOMP;
+  __shared__ double sS[NQ][NN], sF[RHS_FPB][NCOMP][NQ];
+  for (int e = threadIdx.x; e < NQ * NN; e += blockDim.x) {  // S from its even-odd halves
+    const int q = e / NN, i = e - q * NN, qq = q <= K ? q : NQ - 1 - q;
+    const int ii = q <= K ? i : K - i, a = ii <= K / 2 ? ii : K - ii;
+    const double E = CEo<double>::get(K, 2, 0, qq, a), O = CEo<double>::get(K, 2, 1, qq, a);
+    sS[q][i] = ii <= K / 2 ? E + O : E - O;
+  }
+  __syncthreads();
+  // odd faces first, then (momentum) the even walls
+  const long total = (KIND == 1 ? 4L : 2L) * mesh.nc, g0 = (long)blockIdx.x * RHS_FPB;
+  const int lf = threadIdx.x / NQ, q = threadIdx.x - lf * NQ;
+  const long g = g0 + lf;
+  auto face_of = [&](long id, int &c, int &f) {  // false: nothing to integrate
+    if (id >= total) return false;
+    const bool even = id >= 2L * mesh.nc;
+    const long e = even ? id - 2L * mesh.nc : id;
+    c = (int)(e >> 1);
+    f = (int)(e & 1) * 2 + (even ? 0 : 1);
+    const int nb = mesh.nbr[c * 4 + f];
+    return nb < 0 ? KIND == 1 : !even;
+  };
+  int c, f;
+  if (face_of(g, c, f)) {
+    const int nb = mesh.nbr[c * 4 + f], nf = mesh.nbrf[c * 4 + f] & 3;
+    if (mesh.dts) co.dt *= mesh.dts[c];  // per-member time step
+    const double *fg = mesh.fgeo + ((long)c * 4 + f) * 3 * NQ + q;
+    const double n0[1] = {fg[0] * fg[2 * NQ]}, n1[1] = {fg[NQ] * fg[2 * NQ]};
+    double F[NCOMP][1];
+#pragma unroll
+    for (int d = 0; d < NCOMP; ++d) F[d][0] = 0.0;
+    const PointTrace<K> to{f, sS[q]};
+    if (nb < 0) {  // no-flux wall: only the pressure term with p_D = p
+#pragma unroll
+      for (int j = 0; j < ST; ++j) {
+        double p[1];
+        to(src.p[RhsKind<KIND>::PER * j + 2] + (long)c * NN2, p);
+        const double w = co.ct[j] * co.dt / (co.Ma * co.Ma) * p[0];
+        F[0][0] = fma(w, n0[0], F[0][0]);
+        F[NCOMP - 1][0] = fma(w, n1[0], F[NCOMP - 1][0]);
+      }
+    } else {
+      face_flux<K, ST, KIND>(src, co, c, nb, to, PointTrace<K>{nf, sS[q]}, n0, n1, F);
+    }
+#pragma unroll
+    for (int d = 0; d < NCOMP; ++d) sF[lf][d][q] = F[d][0];
+  }
+  __syncthreads();
+  for (int t = threadIdx.x; t < RHS_FPB * NCOMP * NN; t += blockDim.x) {
+    const int l = t / (NCOMP * NN), r = t - l * NCOMP * NN, d = r / NN, i = r - d * NN;
+    if (!face_of(g0 + l, c, f)) continue;
+    double o = 0.0;
+#pragma unroll
+    for (int k = 0; k < NQ; ++k) o = fma(sS[k][i], sF[l][d][k], o);
+    Fb[((long)c * 4 + f) * NCOMP * NN + r] = o;
+  }
 }
 
 // =============================================================== cells ===
@@ -479,10 +568,25 @@ inline void rhs_sources(SrcPtrs &sp, int &nsrc, int kind, int stage, const doubl
   for (int i = 0; i < nsrc; ++i) sp.p[i] = src[i];
 }
 
+// Conforming meshes below this many cells integrate faces point by point.  The
+// second stage's three right-hand sides, a face per thread / a point per thread:
+// 231 / 158 us at 800 cells, k = 4; 182 / 146 at 2304, k = 3; 554 / 535 at 4140,
+// k = 5; 197 / 207 at 8192, k = 2; 554 / 561 at 8192, k = 4.
+constexpr int RHS_POINT_CELLS = 6000;
 template <int K, int KIND, bool HG>
 int rhs_face_launch(const atm_ctx &c, int stage, const SrcPtrs &sp, const StageCoef &co) {
   // even faces: the momentum walls, and hanging faces
   const long n = (long)c.nc * (HG || KIND == 1 ? 4 : 2);
+  if constexpr (!HG)
+    if (c.nc < RHS_POINT_CELLS) {
+      void (*fn)(double *, SrcPtrs, StageCoef, Mesh) =
+          stage == 1 ? k_rhs_face_points<K, 1, KIND>
+                     : (stage == 2 ? k_rhs_face_points<K, 2, KIND> : k_rhs_face_points<K, 3, KIND>);
+      fn<<<(unsigned)((n + RHS_FPB - 1) / RHS_FPB), RHS_FPB * (2 * K + 1), 0, c.stream>>>(c.fbuf, sp,
+                                                                                        co, c.mesh);
+      ATM_CHECK_LAUNCH("k_rhs_face_points");
+      return ATM_OK;
+    }
   void (*fn)(double *, SrcPtrs, StageCoef, Mesh) =
       stage == 1 ? k_rhs_face<K, 1, KIND, HG>
                  : (stage == 2 ? k_rhs_face<K, 2, KIND, HG> : k_rhs_face<K, 3, KIND, HG>);
