@@ -154,6 +154,72 @@ struct ExB {
   }
 };
 
+// nodal integrals of the face term of B over face f of cell cf, both
+// components: F[0..k] and F[4(k+1)..]; without HG the face is conforming or a wall
+template <int K, typename T, bool HG>
+__device__ __forceinline__ void face_B(const T *__restrict__ p, const MeshT<T> &mesh, int cf,
+                                       int f, T *__restrict__ F) {
+  constexpr int NN = K + 1, NN2 = NN * NN;
+  // fB, hB hold half the outward normal times the weight; what is added to
+  // the rows is half the jump times it
+  const int nb = mesh.nbr[cf * 4 + f], nfc = mesh.nbrf[cf * 4 + f];
+  const int code = HG && nb >= 0 ? nfc >> 2 : 0;
+  T own[NN], o0[NN], o1[NN];
+#pragma unroll
+  for (int i = 0; i < NN; ++i) o0[i] = o1[i] = T(0);
+  if (nb >= 0) {
+    trace<K>(p + (long)cf * NN2, f, own);
+    if (!HG || code < 3) {
+      T nbt[NN], s[NN], F0[NN], F1[NN];
+      trace<K>(p + (long)nb * NN2, nfc & 3, nbt);
+      if (!HG || code == 0) {
+#pragma unroll
+        for (int i = 0; i < NN; ++i) nbt[i] -= own[i];
+        eo_interp<K, 0>(nbt, s);
+      } else {  // fine side: the coarse neighbour at the shifted points
+        T sn[NN];
+        eo_interp<K, 0>(own, sn);
+        sub_interp<K, 0>(nbt, code - 1, s);
+#pragma unroll
+        for (int q = 0; q < NN; ++q) s[q] -= sn[q];
+      }
+      const T *g = mesh.fB + ((long)cf * 4 + f) * 2 * NN;
+#pragma unroll
+      for (int q = 0; q < NN; ++q) {
+        T n0, n1;
+        load2(g + 2 * q, n0, n1);
+        F0[q] = n0 * s[q];
+        F1[q] = n1 * s[q];
+      }
+      eo_integ<K, 0, NN, true, false>(F0, F0, o0);
+      eo_integ<K, 0, NN, true, false>(F1, F1, o1);
+    } else {  // coarse side: two subfaces
+      for (int h = 0; h < 2; ++h) {
+        T nbt[NN], s[NN], sn[NN], F0[NN], F1[NN];
+        trace<K>(p + (long)mesh.hnb[nb * 2 + h] * NN2, nfc & 3, nbt);
+        sub_interp<K, 0>(own, h, sn);
+        eo_interp<K, 0>(nbt, s);
+        const T *g = mesh.hB + ((long)nb * 2 + h) * 2 * NN;
+#pragma unroll
+        for (int q = 0; q < NN; ++q) {
+          T n0, n1;
+          load2(g + 2 * q, n0, n1);
+          s[q] -= sn[q];
+          F0[q] = n0 * s[q];
+          F1[q] = n1 * s[q];
+        }
+        sub_integ_add<K, 0>(F0, h, o0);
+        sub_integ_add<K, 0>(F1, h, o1);
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < NN; ++i) {
+    F[i] = o0[i];
+    F[4 * NN + i] = o1[i];
+  }
+}
+
 template <int K, int MODE, typename T, bool HG>
 __global__ void __launch_bounds__(320)
     k_exact_B(T *__restrict__ dst, const T *__restrict__ p, T cB, T cC,
@@ -167,6 +233,7 @@ __global__ void __launch_bounds__(320)
   T *Xs = sm + (STAGE ? cpb * AS : 0);       // [cpb][2][NN2] p, d_xi p at (iz, qx); then B p pairs
   T *Y = Xs + cpb * XV;                      // [cpb][2 comp][NN2]; then the result
   T *Fs = Y + cpb * XV;                      // [cpb][2 comp][4][NN]
+  int *hlist = reinterpret_cast<int *>(Fs + cpb * FV);  // count, hanging faces (HG)
   const int tid = threadIdx.x;
   const int c0 = blockIdx.x * cpb;
   const int cnt = min(cpb, mesh.nc - c0);
@@ -181,6 +248,10 @@ __global__ void __launch_bounds__(320)
   }
   // up to here only A^{-1}, which no kernel of the overlapping chain writes
   pdl_wait();
+  if constexpr (HG) {
+    if (tid == 0) hlist[0] = 0;
+    __syncthreads();
+  }
   const int rt = tid - 4 * cpb;             // row/column threads: rt >= 0
   const int lc = rt / NN, j = rt - lc * NN;
   const bool active = rt >= 0 && lc < cnt;
@@ -199,68 +270,18 @@ __global__ void __launch_bounds__(320)
       x[NN2 + i] = d[i];
     }
   } else if (rt < 0 && tid < 4 * cnt) {
-    // fB, hB hold half the outward normal times the weight; what is added to
-    // the rows is half the jump times it
-    const int l = tid >> 2, f = tid & 3, cf = c0 + l;
-    const int nb = mesh.nbr[cf * 4 + f], nfc = mesh.nbrf[cf * 4 + f];
-    const int code = HG && nb >= 0 ? nfc >> 2 : 0;
-    T own[NN], o0[NN], o1[NN];
-#pragma unroll
-    for (int i = 0; i < NN; ++i) o0[i] = o1[i] = T(0);
-    if (nb >= 0) {
-      trace<K>(p + (long)cf * NN2, f, own);
-      if (!HG || code < 3) {
-        T nbt[NN], s[NN], F0[NN], F1[NN];
-        trace<K>(p + (long)nb * NN2, nfc & 3, nbt);
-        if (!HG || code == 0) {
-#pragma unroll
-          for (int i = 0; i < NN; ++i) nbt[i] -= own[i];
-          eo_interp<K, 0>(nbt, s);
-        } else {  // fine side: the coarse neighbour at the shifted points
-          T sn[NN];
-          eo_interp<K, 0>(own, sn);
-          sub_interp<K, 0>(nbt, code - 1, s);
-#pragma unroll
-          for (int q = 0; q < NN; ++q) s[q] -= sn[q];
-        }
-        const T *g = mesh.fB + ((long)cf * 4 + f) * 2 * NN;
-#pragma unroll
-        for (int q = 0; q < NN; ++q) {
-          T n0, n1;
-          load2(g + 2 * q, n0, n1);
-          F0[q] = n0 * s[q];
-          F1[q] = n1 * s[q];
-        }
-        eo_integ<K, 0, NN, true, false>(F0, F0, o0);
-        eo_integ<K, 0, NN, true, false>(F1, F1, o1);
-      } else {  // coarse side: two subfaces
-        for (int h = 0; h < 2; ++h) {
-          T nbt[NN], s[NN], sn[NN], F0[NN], F1[NN];
-          trace<K>(p + (long)mesh.hnb[nb * 2 + h] * NN2, nfc & 3, nbt);
-          sub_interp<K, 0>(own, h, sn);
-          eo_interp<K, 0>(nbt, s);
-          const T *g = mesh.hB + ((long)nb * 2 + h) * 2 * NN;
-#pragma unroll
-          for (int q = 0; q < NN; ++q) {
-            T n0, n1;
-            load2(g + 2 * q, n0, n1);
-            s[q] -= sn[q];
-            F0[q] = n0 * s[q];
-            F1[q] = n1 * s[q];
-          }
-          sub_integ_add<K, 0>(F0, h, o0);
-          sub_integ_add<K, 0>(F1, h, o1);
-        }
-      }
-    }
-    T *F = Fs + l * FV + f * NN;
-#pragma unroll
-    for (int i = 0; i < NN; ++i) {
-      F[i] = o0[i];
-      F[4 * NN + i] = o1[i];
-    }
+    const int l = tid >> 2, f = tid & 3;
+    if (HG && mesh.nbr[(c0 + l) * 4 + f] >= 0 && (mesh.nbrf[(c0 + l) * 4 + f] >> 2) != 0)
+      hlist[1 + atomicAdd(hlist, 1)] = tid;
+    else
+      face_B<K, T, false>(p, mesh, c0 + l, f, Fs + l * FV + f * NN);
   }
   __syncthreads();
+  if constexpr (HG)
+    for (int t = tid; t < hlist[0]; t += blockDim.x) {
+      const int l = hlist[1 + t] >> 2, f = hlist[1 + t] & 3;
+      face_B<K, T, true>(p, mesh, c0 + l, f, Fs + l * FV + f * NN);
+    }
   if (active) {
     // column j: gradient at the points, z-integration of both components
     T t[NN], px[NN], pe[NN], G0[NN], G1[NN], b[NN];
@@ -486,6 +507,7 @@ __global__ void __launch_bounds__(FB ? 256 : 32 * Ex<K>::NC, FB ? 3 : HG ? 1 : s
   T *sV = sJ + (STG ? cpb * NC2 : 0);          // [NV][cpb][NN2]: rhs, invd, d, x
   T *X = sV + (STG ? NV * cpb * NN2 : 0);      // [cpb][NF][NN][NC] x-interpolated w, p; then xa, xb
   T *Fs = X + cpb * NF * XS;                   // [cpb][4][NN] face integrals of C w (not FB)
+  int *hlist = reinterpret_cast<int *>(Fs + cpb * 4 * NN);  // count, hanging faces (HG)
   const int tid = threadIdx.x, nt = blockDim.x;
   const int c0 = blockIdx.x * cpb;
   const int cnt = min(cpb, mesh.nc - c0);
@@ -504,14 +526,25 @@ __global__ void __launch_bounds__(FB ? 256 : 32 * Ex<K>::NC, FB ? 3 : HG ? 1 : s
     }
     cp_async_commit();
   }
+  if constexpr (HG && !FB) {
+    if (tid == 0) hlist[0] = 0;
+    __syncthreads();
+  }
   // faces: one thread per (cell, face); with NC > 4 the first 4 cpb threads
-  // (whole warps) take them while the others interpolate the rows
+  // (whole warps) take them while the others interpolate the rows.  Hanging
+  // faces take several times as long: they are put on a list and done by
+  // consecutive threads, instead of holding up a warp each (S apply of 6300
+  // cells with 12% hanging faces, k = 3: 84 -> 74 us)
   for (int e = tid; !FB && e < 4 * cnt; e += nt) {
-    const int l = e >> 2, f = e & 3, c = c0 + l;
+    const int f = e & 3, c = c0 + (e >> 2);
+    if (HG && mesh.nbr[c * 4 + f] >= 0 && (mesh.nbrf[c * 4 + f] >> 2) != 0) {
+      hlist[1 + atomicAdd(hlist, 1)] = e;
+      continue;
+    }
     T o[NN];
-    face_C<K, T, HG>(w, pfix, pff, mesh, c, f, o);
+    face_C<K, T, false>(w, pfix, pff, mesh, c, f, o);
 #pragma unroll
-    for (int i = 0; i < NN; ++i) Fs[(l * 4 + f) * NN + i] = o[i];
+    for (int i = 0; i < NN; ++i) Fs[e * NN + i] = o[i];
   }
   // rows (cell, field, iz): x-interpolation to the NC points
   {
@@ -531,6 +564,14 @@ __global__ void __launch_bounds__(FB ? 256 : 32 * Ex<K>::NC, FB ? 3 : HG ? 1 : s
   }
   if constexpr (STG) cp_async_wait_all();
   __syncthreads();
+  if constexpr (HG && !FB)
+    for (int t = tid; t < hlist[0]; t += nt) {
+      const int e = hlist[1 + t];
+      T o[NN];
+      face_C<K, T, true>(w, pfix, pff, mesh, c0 + (e >> 2), e & 3, o);
+#pragma unroll
+      for (int i = 0; i < NN; ++i) Fs[e * NN + i] = o[i];
+    }
   // columns: z-interpolation, fluxes, z-integration; xa and xb replace the
   // column's own x-interpolated values
   {
@@ -617,22 +658,30 @@ __global__ void __launch_bounds__(FB ? 256 : 32 * Ex<K>::NC, FB ? 3 : HG ? 1 : s
 }
 
 // Fb[c][f][k+1]: nodal integrals of C w over the odd local faces, whose conforming
-// neighbours read them with the opposite sign; with hanging faces also over
-// the even faces that are not the other side of a conforming one.
+// neighbours read them with the opposite sign, and over both sides of hanging
+// faces.
 template <int K, typename T, bool HG>
 __global__ void __launch_bounds__(64)
     k_exact_face_C(T *__restrict__ Fb, const T *__restrict__ w, const T *__restrict__ pfix,
                    const T *__restrict__ pff, MeshT<T> mesh) {
   constexpr int NN = K + 1;
   const long g = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  const bool even = HG && g >= 2L * mesh.nc;
-  const long e = even ? g - 2L * mesh.nc : g;
-  if (e >= 2L * mesh.nc) return;
-  const int c = (int)(e >> 1), f = (int)(e & 1) * 2 + (even ? 0 : 1);
-  const int nb = mesh.nbr[c * 4 + f];
-  if (nb < 0 || (even && (mesh.nbrf[c * 4 + f] >> 2) == 0)) return;
   T o[NN];
-  face_C<K, T, HG>(w, pfix, pff, mesh, c, f, o);
+  int c, f;
+  if (!HG || g < 2L * mesh.nc) {  // conforming odd faces
+    if (g >= 2L * mesh.nc) return;
+    c = (int)(g >> 1);
+    f = (int)(g & 1) * 2 + 1;
+    if (mesh.nbr[c * 4 + f] < 0 || (HG && (mesh.nbrf[c * 4 + f] >> 2) != 0)) return;
+    face_C<K, T, false>(w, pfix, pff, mesh, c, f, o);
+  } else {  // hanging faces, each from its own side
+    const long e = g - 2L * mesh.nc;
+    if (e >= 4L * mesh.nc) return;
+    c = (int)(e >> 2);
+    f = (int)(e & 3);
+    if (mesh.nbr[c * 4 + f] < 0 || (mesh.nbrf[c * 4 + f] >> 2) == 0) return;
+    face_C<K, T, true>(w, pfix, pff, mesh, c, f, o);
+  }
 #pragma unroll
   for (int i = 0; i < NN; ++i) Fb[((long)c * 4 + f) * NN + i] = o[i];
 }
@@ -701,7 +750,8 @@ int exact_B_launch(const OpView<T> &v, T *dst, const T *p, T cB, T cC, int mode)
     int cpb = v.nc < 2048 ? 8 : exact_cells(tuned);
     if (cpb * ExB<K>::TPC > 320) cpb = 320 / ExB<K>::TPC / 8 * 8;
     const size_t sm =
-        sizeof(T) * (size_t)cpb * ExB<K>::template values<T>(mode == 2 && sizeof(T) == 4);
+        sizeof(T) * (size_t)cpb * ExB<K>::template values<T>(mode == 2 && sizeof(T) == 4) +
+        (HG ? sizeof(int) * (4 * cpb + 1) : 0);
     void (*fn)(T *, const T *, T, T, const T *, MeshT<T>, int) =
         mode == 0 ? k_exact_B<K, 0, T, HG>
                   : (mode == 1 ? k_exact_B<K, 1, T, HG> : k_exact_B<K, 2, T, HG>);
@@ -742,7 +792,8 @@ int exact_CD_launch(const OpView<T> &v, T *dst, const T *w, const T *p, T cC, in
     if (fb) cpb = (tuned >= 256 / E::NQ ? 256 : tuned >= 128 / E::NQ ? 128 : 64) / E::NC;
     const int staged = sizeof(T) == 4 ? 5 * E::NC2 + (mode == 4 ? 4 * E::NN2 : 0) : 0;
     const size_t sm = sizeof(T) * (size_t)cpb *
-                      ((mode == 0 || mode == 3 ? 2 : 3) * E::NN * E::NC + 4 * E::NN + staged);
+                      ((mode == 0 || mode == 3 ? 2 : 3) * E::NN * E::NC + 4 * E::NN + staged) +
+                      (HG ? sizeof(int) * (4 * cpb + 1) : 0);
     auto fn = mode == 0   ? exact_CD_kernel<K, 0, T, HG>(fb)
               : mode == 1 ? exact_CD_kernel<K, 1, T, HG>(fb)
               : mode == 2 ? exact_CD_kernel<K, 2, T, HG>(fb)
@@ -754,7 +805,7 @@ int exact_CD_launch(const OpView<T> &v, T *dst, const T *w, const T *p, T cC, in
   };
   if constexpr (sizeof(T) == 8)
     if (fb) {
-      const long n = (long)v.nc * (HG ? 4 : 2);
+      const long n = (long)v.nc * (HG ? 6 : 2);
       k_exact_face_C<K, T, HG><<<(unsigned)((n + 63) / 64), 64, 0, v.st>>>(v.fbuf, w, pfix, v.pff,
                                                                          v.mesh);
       ATM_CHECK_LAUNCH("k_exact_face_C");
