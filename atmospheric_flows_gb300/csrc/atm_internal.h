@@ -407,6 +407,24 @@ inline double fl_integrate(int k, bool grad) {  // one output component
 inline double fl_face(int k) {  // one field trace at the points of one face
   return 2.0 * (2 * k + 1) * (k + 1);
 }
+// FP64 flops per cell of the contractions of B (`apply`: with A^{-1}) and of C
+// (`d`: with D), on the point sets the kernels use
+inline double fl_B(int k, bool exact, bool apply) {
+  const double nn = k + 1, n2 = nn * nn;
+  const double a = apply ? 4.0 * n2 * n2 : 0.0;
+  if (!exact) return fl_eval(k) + 2 * fl_integrate(k, true) + 4.0 * 4 * fl_face(k) + a;
+  // value and derivative along x, then z; values of two components back along
+  // both; the faces' jump and two components
+  return 2.0 * nn * n2 * (2 + 2 + 4) + 4.0 * 3 * 2.0 * n2 + a;
+}
+inline double fl_CD(int k, bool exact, bool d) {
+  const double nn = k + 1, nc = (3 * k + 3) / 2;
+  if (!exact) return (d ? 4 : 3) * fl_eval(k) + fl_integrate(k, true) + 4.0 * 7 * fl_face(k);
+  // w (2) and p to the points; value (with D) and two derivatives back along z,
+  // two quantities along x; four traces and one integration per face and side
+  return 2.0 * ((d ? 3 : 2) * (nn * nn * nc + nn * nc * nc) + (d ? 3 : 2) * nn * nc * nc +
+                2 * nn * nn * nc) + 4.0 * 5 * fl_face(k);
+}
 StageCoef stage_coef_rho(const atm_ctx &c, int stage);
 StageCoef stage_coef_flux(const atm_ctx &c, int stage);
 double implicit_coeff(const atm_ctx &c);

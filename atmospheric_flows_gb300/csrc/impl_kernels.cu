@@ -363,9 +363,7 @@ int launch_B(const atm_ctx &c, double *dst, const double *p, double cB, int mode
   // p read; B p written (2 comps); mode 1 reads dst too; mode 2 reads A^{-1}
   const double bytes = 8.0 * ns * (1 + 2 + (mode == 1 ? 2 : 0)) +
                        (mode == 2 ? 8.0 * c.nc * c.nn2 * c.nn2 : 0.0);
-  const double flops = c.nc * (fl_eval(c.k) + 2 * fl_integrate(c.k, true) +
-                               4.0 * (2 * fl_face(c.k) + 2 * fl_face(c.k)) +
-                               (mode == 2 ? 4.0 * c.nn2 * c.nn2 : 0.0));
+  const double flops = c.nc * fl_B(c.k, c.mesh.exact, mode == 2);
   TimedRegion tr(c, KF_B, bytes, flops);
   if (c.mesh.exact) return exact_B(schur_view(c), dst, p, cB, cC, mode);
   if (c.mesh.nhang > 0) return launch_B_hang(c, dst, p, cB, mode);
@@ -377,8 +375,7 @@ int launch_CD(const atm_ctx &c, double *dst, const double *w, const double *p, d
   const bool wd = (mode == 1 || mode == 2);
   // w (2 comps) + pfix read, [p], [inverse diagonal], [dst read], dst written
   const double bytes = 8.0 * ns * (3 + (wd ? 1 : 0) + (mode == 2 ? 1 : 0) + (mode == 3 ? 1 : 0) + 1);
-  const double flops = c.nc * ((wd ? 4 : 3) * fl_eval(c.k) + fl_integrate(c.k, true) +
-                               4.0 * (2 * 3 * fl_face(c.k) + fl_face(c.k)));
+  const double flops = c.nc * fl_CD(c.k, c.mesh.exact, wd);
   TimedRegion tr(c, KF_CD, bytes, flops);
   if (c.mesh.exact) return exact_CD(schur_view(c), dst, w, p, coeff, mode, nullptr);
   if (c.mesh.nhang > 0) return launch_CD_hang(c, dst, w, p, coeff, mode);

@@ -520,13 +520,11 @@ int level_apply(atm_ctx &c, MGLevelT<T> &L, T *out, const T *x) {
   const double co = implicit_coeff(c);
   LevelViewT<T> v = lview(c, L);
   // algorithmic bytes: x, pfix, invd-free D/C read + B/A^{-1} intermediate
-  // (2 comps written + read) + A^{-1} as stored (FP32: its triangle) + out; flops: the FP64 formulas of
+  // (2 comps written + read) + A^{-1} as stored (FP32: its triangle) + out; flops as
   // launch_B (mode 2) and launch_CD (mode 1)
   const double ns = (double)L.nc * c.nn2, sz = sizeof(T);
   const double bytes = sz * (ns * (1 + 2 + 2 + 1 + 1 + 1) + (double)L.nc * ainv_stride_rt(c.k, sz));
-  const double flops = L.nc * (fl_eval(c.k) + 2 * fl_integrate(c.k, true) + 4.0 * 4 * fl_face(c.k) +
-                               4.0 * c.nn2 * c.nn2 + 4 * fl_eval(c.k) + fl_integrate(c.k, true) +
-                               4.0 * 7 * fl_face(c.k));
+  const double flops = L.nc * (fl_B(c.k, L.mesh.exact, true) + fl_CD(c.k, L.mesh.exact, true));
   TimedRegion tr(c, KF_MG_APPLY, bytes, flops);
   int rc = level_B<T>(v, L.wv, x, (T)(co * c.dt / (c.Ma * c.Ma)), (T)(co * c.dt));
   if (rc) return rc;
@@ -543,9 +541,7 @@ int level_apply_cheb(atm_ctx &c, MGLevelT<T> &L, double a, double b_coef, bool f
   const double ns = (double)L.nc * c.nn2, sz = sizeof(T);
   // as level_apply, plus rhs, invd, d read and d, x written in the update
   const double bytes = sz * (ns * (1 + 2 + 2 + 1 + 1 + 5) + (double)L.nc * ainv_stride_rt(c.k, sz));
-  const double flops = L.nc * (fl_eval(c.k) + 2 * fl_integrate(c.k, true) + 4.0 * 4 * fl_face(c.k) +
-                               4.0 * c.nn2 * c.nn2 + 4 * fl_eval(c.k) + fl_integrate(c.k, true) +
-                               4.0 * 7 * fl_face(c.k));
+  const double flops = L.nc * (fl_B(c.k, L.mesh.exact, true) + fl_CD(c.k, L.mesh.exact, true));
   TimedRegion tr(c, KF_MG_APPLY, bytes, flops);
   int rc = level_B<T>(v, L.wv, L.x, (T)(co * c.dt / (c.Ma * c.Ma)), (T)(co * c.dt));
   if (rc) return rc;

@@ -247,10 +247,10 @@ def measured_peaks():
 # independent-chain DFMA probe of `bench.py --fma-probe`)
 FP64_PEAK_TFLOPS = 1.255
 # DRAM bytes (read + write) per cell and launch of the dominant kernel families,
-# from single-kernel `ncu` captures of this bench at 320x160 Q4: 311.0 MB per
-# k_CD<4,2> launch and 469.6 MB per k_B<4,2> launch over 51,200 cells; the
-# traffic grows in proportion to the cell count.
-NCU_TRAFFIC_PER_CELL = {4: {"CD": 311.0e6 / 51200, "B": 469.6e6 / 51200}}
+# from single-kernel `ncu` captures of the S apply at 320x160 Q4: 207.4 MB per
+# k_exact_face_C and k_exact_CD pair and 339.1 MB per k_exact_B<4,2> launch over
+# 51,200 cells; the traffic grows in proportion to the cell count.
+NCU_TRAFFIC_PER_CELL = {4: {"CD": 207.4e6 / 51200, "B": 339.1e6 / 51200}}
 
 
 def cpu_baseline(case, eps, gpu_state=None):
@@ -322,7 +322,7 @@ def level_roofline(case, eps):
     avg = ms[i] / max(cnt[i], 1)
     gbs = byt[i] / max(cnt[i], 1) / (avg * 1e-3) / 1e9
     peak, kind = measured_peaks()
-    return {"bound": "hbm", "kernel": "mg_level_apply (FP32 k_B<K,2,float> + k_CD<K,1|4,float>, "
+    return {"bound": "hbm", "kernel": "mg_level_apply (FP32 k_exact_B<K,2,float> + k_exact_CD<K,1|4,float>, "
             "all levels)", "achieved": gbs, "peak": peak, "unit": "GB/s", "frac": gbs / peak,
             "peak_source": kind, "avg_pair_ms": avg, "pairs": int(cnt[i]),
             "algorithmic_bytes_per_pair": byt[i] / max(cnt[i], 1),
