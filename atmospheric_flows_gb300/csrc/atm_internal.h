@@ -239,7 +239,7 @@ int vec_xmy_scaled(cudaStream_t st, double *dst, const double *d, const double *
                    const double *t, long n);  // dst = d .* (b - t)
 int vec_scale_by_inv_norm(cudaStream_t st, double *dst, const double *src,
                           const double *normsq, long n);  // dst = src/sqrt(*normsq)
-// partial-sum buffer `red` must hold 29*RED_BLOCKS doubles
+// partial-sum buffer `red` must hold 32*RED_BLOCKS doubles
 constexpr int RED_BLOCKS = 608;
 int vec_dot(cudaStream_t st, const double *x, const double *y, long n, double *red,
             double *out);  // out[0] = x.y (device)
@@ -266,8 +266,6 @@ int arnoldi_step(cudaStream_t st, double *V, long n, int j, double *w, double *r
 int arnoldi_blocks(long n, int m, int segments);
 int arnoldi_sweeps(cudaStream_t st, double *V, long n, int j, double *w, const long *eoff,
                    int segments, double *red, double *coef, unsigned *ticket, double *host);
-int vec_multidot(cudaStream_t st, const double *V, long ldv, int m, const double *w, long n,
-                 double *red, double *out);  // out[l] = V_l . w, l < m
 // w += sign * sum_l h[l] V_l  (h device)
 int vec_multiaxpy(cudaStream_t st, double *w, const double *V, long ldv, int m,
                   const double *h, double sign, long n);
@@ -495,7 +493,7 @@ int members_set(atm_ctx &c, int n, const int *cell_off, const double *dt);
 void members_free(atm_ctx &c);
 int members_refresh_dt(atm_ctx &c);  // after a change of c.dt
 // member-wise reductions: out[col * n + m] (device, then copied to h_out)
-int seg_multidot(atm_ctx &c, const double *V, long ldv, int m, const double *w);
+int seg_dot(atm_ctx &c, const double *v, const double *w);
 int seg_maxdiff(atm_ctx &c, const double *a, const double *b);  // rows 0, 1
 int seg_read(atm_ctx &c, int rows);                             // out -> h_out (sync)
 // member-wise vector updates with coefficients coef[col * n + m] (host

@@ -97,43 +97,6 @@ __global__ void k_finalize(const double *__restrict__ red, double *__restrict__ 
   if (threadIdx.x == 0) out[blockIdx.x] = acc;
 }
 
-// M vectors per pass: fixed-size accumulators stay in registers
-template <int M>
-__global__ void k_multidot_partial(const double *__restrict__ V, long ldv,
-                                   const double *__restrict__ w, long n,
-                                   double *__restrict__ red) {
-  __shared__ double sh[RT / 32];
-  double acc[M];
-#pragma unroll
-  for (int l = 0; l < M; ++l) acc[l] = 0.0;
-  for (long i = (long)blockIdx.x * RT + threadIdx.x; i < n; i += (long)RED_BLOCKS * RT) {
-    const double wi = w[i];
-#pragma unroll
-    for (int l = 0; l < M; ++l) acc[l] = fma(V[l * ldv + i], wi, acc[l]);
-  }
-#pragma unroll
-  for (int l = 0; l < M; ++l) {
-    const double s = block_reduce<0>(acc[l], sh);
-    if (threadIdx.x == 0) red[(long)l * RED_BLOCKS + blockIdx.x] = s;
-  }
-}
-
-// up to 8 vectors per launch; larger m is split into chunks of 8
-void multidot_chunk(cudaStream_t st, const double *V, long ldv, int m, const double *w,
-                    long n, double *red) {
-  switch (m) {
-    case 1: k_multidot_partial<1><<<RED_BLOCKS, RT, 0, st>>>(V, ldv, w, n, red); break;
-    case 2: k_multidot_partial<2><<<RED_BLOCKS, RT, 0, st>>>(V, ldv, w, n, red); break;
-    case 3: k_multidot_partial<3><<<RED_BLOCKS, RT, 0, st>>>(V, ldv, w, n, red); break;
-    case 4: k_multidot_partial<4><<<RED_BLOCKS, RT, 0, st>>>(V, ldv, w, n, red); break;
-    case 5: k_multidot_partial<5><<<RED_BLOCKS, RT, 0, st>>>(V, ldv, w, n, red); break;
-    case 6: k_multidot_partial<6><<<RED_BLOCKS, RT, 0, st>>>(V, ldv, w, n, red); break;
-    case 7: k_multidot_partial<7><<<RED_BLOCKS, RT, 0, st>>>(V, ldv, w, n, red); break;
-    default: k_multidot_partial<8><<<RED_BLOCKS, RT, 0, st>>>(V, ldv, w, n, red); break;
-  }
-  g_kernel_launches.fetch_add(1);
-}
-
 __global__ void k_multiaxpy(double *__restrict__ w, const double *__restrict__ V, long ldv,
                             int m, const double *__restrict__ h, double sign, long n) {
   for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
@@ -367,17 +330,6 @@ int vec_dot(cudaStream_t st, const double *x, const double *y, long n, double *r
   k_dot_partial<<<RED_BLOCKS, RT, 0, st>>>(x, y, n, red);
   k_finalize<0><<<1, RT, 0, st>>>(red, out);
   ATM_CHECK_LAUNCH("vec_dot");
-  return ATM_OK;
-}
-int vec_multidot(cudaStream_t st, const double *V, long ldv, int m, const double *w, long n,
-                 double *red, double *out) {
-  if (m < 1 || m > MAXM) return ATM_BAD_ARG;
-  for (int l0 = 0; l0 < m; l0 += 8) {
-    const int mm = m - l0 < 8 ? m - l0 : 8;
-    multidot_chunk(st, V + (long)l0 * ldv, ldv, mm, w, n, red + (long)l0 * RED_BLOCKS);
-  }
-  k_finalize<0><<<m, RT, 0, st>>>(red, out);
-  ATM_CHECK_LAUNCH("vec_multidot");
   return ATM_OK;
 }
 int vec_multiaxpy(cudaStream_t st, double *w, const double *V, long ldv, int m,

@@ -49,27 +49,17 @@ __device__ double block_red(double v, double *sh) {
 }
 
 // block (b, m) reduces its share of member m's elements eoff[m]..eoff[m+1];
-// partials red[(l * nm + m) * sb + b]
-template <int M>
-__global__ void k_seg_multidot(const double *__restrict__ V, long ldv,
-                               const double *__restrict__ w, const long *__restrict__ eoff,
-                               int nm, int sb, double *__restrict__ red) {
+// partials red[m * sb + b]
+__global__ void k_seg_dot(const double *__restrict__ v, const double *__restrict__ w,
+                          const long *__restrict__ eoff, int sb, double *__restrict__ red) {
   __shared__ double sh[RT / 32];
   const int m = blockIdx.y, b = blockIdx.x;
   const long lo = eoff[m], hi = eoff[m + 1];
-  double acc[M];
-#pragma unroll
-  for (int l = 0; l < M; ++l) acc[l] = 0.0;
-  for (long i = lo + (long)b * RT + threadIdx.x; i < hi; i += (long)sb * RT) {
-    const double wi = w[i];
-#pragma unroll
-    for (int l = 0; l < M; ++l) acc[l] = fma(V[l * ldv + i], wi, acc[l]);
-  }
-#pragma unroll
-  for (int l = 0; l < M; ++l) {
-    const double s = block_red<0>(acc[l], sh);
-    if (threadIdx.x == 0) red[((long)l * nm + m) * sb + b] = s;
-  }
+  double acc = 0.0;
+  for (long i = lo + (long)b * RT + threadIdx.x; i < hi; i += (long)sb * RT)
+    acc = fma(v[i], w[i], acc);
+  acc = block_red<0>(acc, sh);
+  if (threadIdx.x == 0) red[(long)m * sb + b] = acc;
 }
 
 // rows 0: max |a - b|, 1: max |a| per member
@@ -139,21 +129,6 @@ inline int gs(long n) {
   long g = (n + 255) / 256;
   if (g > 152L * 16) g = 152L * 16;
   return (int)(g < 1 ? 1 : g);
-}
-
-void multidot_chunk(cudaStream_t st, dim3 grid, const double *V, long ldv, int m,
-                    const double *w, const long *eoff, int nm, int sb, double *red) {
-  switch (m) {
-    case 1: k_seg_multidot<1><<<grid, RT, 0, st>>>(V, ldv, w, eoff, nm, sb, red); break;
-    case 2: k_seg_multidot<2><<<grid, RT, 0, st>>>(V, ldv, w, eoff, nm, sb, red); break;
-    case 3: k_seg_multidot<3><<<grid, RT, 0, st>>>(V, ldv, w, eoff, nm, sb, red); break;
-    case 4: k_seg_multidot<4><<<grid, RT, 0, st>>>(V, ldv, w, eoff, nm, sb, red); break;
-    case 5: k_seg_multidot<5><<<grid, RT, 0, st>>>(V, ldv, w, eoff, nm, sb, red); break;
-    case 6: k_seg_multidot<6><<<grid, RT, 0, st>>>(V, ldv, w, eoff, nm, sb, red); break;
-    case 7: k_seg_multidot<7><<<grid, RT, 0, st>>>(V, ldv, w, eoff, nm, sb, red); break;
-    default: k_seg_multidot<8><<<grid, RT, 0, st>>>(V, ldv, w, eoff, nm, sb, red); break;
-  }
-  g_kernel_launches.fetch_add(1);
 }
 }  // namespace
 
@@ -249,8 +224,8 @@ int members_set(atm_ctx &c, int n, const int *cell_off, const double *dt) {
     if ((e = cudaMalloc(&M->cell_mem, c.nc * sizeof(int)))) return fail(e, "cudaMalloc members");
     if ((e = cudaMalloc(&M->eoff, (n + 1) * sizeof(long)))) return fail(e, "cudaMalloc members");
     if ((e = cudaMalloc(&M->dts, c.nc * sizeof(double)))) return fail(e, "cudaMalloc members");
-    // 8 columns of sb blocks, or the Arnoldi sweeps' 32
-    const size_t nred = (size_t)n * std::max(8 * M->sb, 32 * 304);
+    // two rows of sb blocks, or the Arnoldi sweeps' 32 of arnoldi_blocks()
+    const size_t nred = std::max((size_t)2 * n * M->sb, (size_t)32 * std::max(304, n));
     if ((e = cudaMalloc(&M->red, nred * sizeof(double))))
       return fail(e, "cudaMalloc members");
     if ((e = cudaMalloc(&M->ticket, n * sizeof(unsigned))) ||
@@ -293,16 +268,12 @@ int seg_read(atm_ctx &c, int rows) {
   return ATM_OK;
 }
 
-int seg_multidot(atm_ctx &c, const double *V, long ldv, int m, const double *w) {
+int seg_dot(atm_ctx &c, const double *v, const double *w) {
   Members &M = *c.mem;
-  const dim3 grid(M.sb, M.n);
-  for (int l0 = 0; l0 < m; l0 += 8) {
-    const int cols = std::min(8, m - l0);
-    multidot_chunk(c.stream, grid, V + (long)l0 * ldv, ldv, cols, w, M.eoff, M.n, M.sb, M.red);
-    ATM_CUDA(cudaGetLastError());
-    k_seg_finalize<0><<<cols * M.n, RT, 0, c.stream>>>(M.red, M.sb, M.out + (long)l0 * M.n);
-    ATM_CHECK_LAUNCH("k_seg_finalize");
-  }
+  k_seg_dot<<<dim3(M.sb, M.n), RT, 0, c.stream>>>(v, w, M.eoff, M.sb, M.red);
+  ATM_CHECK_LAUNCH("k_seg_dot");
+  k_seg_finalize<0><<<M.n, RT, 0, c.stream>>>(M.red, M.sb, M.out);
+  ATM_CHECK_LAUNCH("k_seg_finalize");
   return ATM_OK;
 }
 
@@ -376,7 +347,7 @@ int krylov_members(atm_ctx &c, int precision, double *x, const double *b,
     } else if ((rc = vec_xmy_scaled(c.stream, V, c.invdiag_D, b, t, n))) {
       return rc;
     }
-    if ((rc = seg_multidot(c, V, n, 1, V)) || (rc = seg_read(c, 1))) return rc;
+    if ((rc = seg_dot(c, V, V)) || (rc = seg_read(c, 1))) return rc;
     bool any = false;
     for (int m = 0; m < nm; ++m) {
       run[m] = 0;

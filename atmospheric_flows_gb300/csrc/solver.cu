@@ -122,7 +122,7 @@ int members_check_finite(atm_ctx &c, Solver &s, const double *v) {
 int schur_solve_members(atm_ctx &c, Solver &s) {
   Members &M = *c.mem;
   const long ns = c.n_scalar();
-  TRY(seg_multidot(c, s.rhs_pres, ns, 1, s.rhs_pres));
+  TRY(seg_dot(c, s.rhs_pres, s.rhs_pres));
   TRY(seg_read(c, 1));
   std::vector<double> tol(M.n);
   std::vector<int> st(M.n);
