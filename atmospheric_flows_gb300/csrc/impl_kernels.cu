@@ -153,7 +153,6 @@ __global__ void __launch_bounds__(Cfg<K>::THREADS)
 // kernel and 325 triangle entries left 8% of the lanes idle.  Four cells per
 // warp share the division's instructions and fill the lanes.  Fewer than 4096
 // cells leave SMs without warps; there a warp per cell is the shorter chain.
-constexpr int BI_WARPS = 4;
 
 template <int K>
 struct BlockInvCfg {
@@ -179,7 +178,7 @@ __device__ __forceinline__ int sym_index(int i, int j) {
   return i >= j ? tri_index(i, j) : tri_index(j, i);
 }
 
-template <int K, typename T, int G>
+template <int K, typename T, int G, int BI_WARPS>
 __global__ void __launch_bounds__(32 * BI_WARPS)
     k_block_inverse(T *__restrict__ out, const T *__restrict__ weight, MeshT<T> mesh) {
   using B = BlockInvCfg<K>;
@@ -336,12 +335,18 @@ int invdiag_launch(const OpView<T> &v, T *out, int ncomp, const T *weight, T sca
 
 template <int K, typename T>
 int block_inverse_launch(const OpView<T> &v, T *out, const T *weight) {
-  const bool one = v.nc < 4096;  // a warp per cell, or four cells per warp
-  const int cells = BI_WARPS * (one ? 1 : 4);
+  // a warp per cell, or several.  At k = 5 four cells per warp take 33 KB of shared
+  // memory, so that an SM holds one block of four warps: slower than a warp per
+  // cell.  Two cells keep twelve warps: 2254 us at 28800 cells, a warp per cell
+  // 2476.  Their lines cross between 4700 cells (564 / 447 us) and 7200 (589 / 694)
+  const bool one = v.nc < (K == 5 ? 6000 : 4096);
+  constexpr int G = K == 5 ? 16 : 8, W = 4;
+  const int warps = one ? 2 : W, cells = one ? 2 : W * (32 / G);
   const size_t sm = BlockInvCfg<K>::template smem<T>(cells);
-  void (*fn)(T *, const T *, MeshT<T>) = one ? k_block_inverse<K, T, 32> : k_block_inverse<K, T, 8>;
+  void (*fn)(T *, const T *, MeshT<T>) =
+      one ? k_block_inverse<K, T, 32, 2> : k_block_inverse<K, T, G, W>;
   ATM_CUDA(allow_smem(fn, sm));
-  fn<<<(v.nc + cells - 1) / cells, 32 * BI_WARPS, sm, v.st>>>(out, weight, v.mesh);
+  fn<<<(v.nc + cells - 1) / cells, 32 * warps, sm, v.st>>>(out, weight, v.mesh);
   ATM_CHECK_LAUNCH("k_block_inverse");
   return ATM_OK;
 }
