@@ -219,69 +219,95 @@ __global__ void __launch_bounds__(64)
     for (int i = 0; i < NN; ++i) out[d * NN + i] = o[d][i];
 }
 
-// The same on a conforming mesh with one thread per face point, RHS_FPB faces
-// per block: 5 instead of 4 FP64 instructions per trace value at k = 4, but nine
-// times the threads.  A face per thread needs tens of thousands of faces to
-// reach every quarter of every SM, each of which takes 64 clocks for an FP64
-// instruction whether one warp issues it or many.
+// The same with one thread per face point, RHS_FPB faces per block: 5 instead of
+// 4 FP64 instructions per trace value at k = 4, but nine times the threads.  A
+// face per thread needs tens of thousands of faces to reach every quarter of
+// every SM, each of which takes 64 clocks for an FP64 instruction whether one
+// warp issues it or many.
 constexpr int RHS_FPB = 16;
-template <int K, int ST, int KIND>
+template <int K, int ST, int KIND, bool HG>
 __global__ void __launch_bounds__(RHS_FPB *(2 * K + 1))
     k_rhs_face_points(double *__restrict__ Fb, SrcPtrs src, StageCoef co, Mesh mesh) {
   constexpr int NN = K + 1, NN2 = NN * NN, NQ = 2 * K + 1, NCOMP = RhsKind<KIND>::NCOMP;
-  __shared__ double sS[NQ][NN], sF[RHS_FPB][NCOMP][NQ];
+  constexpr int NT = HG ? 3 : 1, NH = HG ? 2 : 1;
+  // basis rows at the face's points, and at those of its two subfaces
+  __shared__ double sS[NT][NQ][NN], sF[RHS_FPB][NH][NCOMP][NQ];
   for (int e = threadIdx.x; e < NQ * NN; e += blockDim.x) {  // S from its even-odd halves
     const int q = e / NN, i = e - q * NN, qq = q <= K ? q : NQ - 1 - q;
     const int ii = q <= K ? i : K - i, a = ii <= K / 2 ? ii : K - ii;
     const double E = CEo<double>::get(K, 2, 0, qq, a), O = CEo<double>::get(K, 2, 1, qq, a);
-    sS[q][i] = ii <= K / 2 ? E + O : E - O;
+    sS[0][q][i] = ii <= K / 2 ? E + O : E - O;
+    if (HG)
+      for (int h = 0; h < 2; ++h) sS[HG ? 1 + h : 0][q][i] = CEo<double>::sub(K, 1, h, q, i);
   }
   __syncthreads();
-  // odd faces first, then (momentum) the even walls
-  const long total = (KIND == 1 ? 4L : 2L) * mesh.nc, g0 = (long)blockIdx.x * RHS_FPB;
+  // odd conforming faces and walls; (momentum) even walls; hanging faces
+  const long nodd = 2L * mesh.nc, neven = KIND == 1 ? nodd : 0;
+  const long g0 = (long)blockIdx.x * RHS_FPB;
   const int lf = threadIdx.x / NQ, q = threadIdx.x - lf * NQ;
-  const long g = g0 + lf;
-  auto face_of = [&](long id, int &c, int &f) {  // false: nothing to integrate
-    if (id >= total) return false;
-    const bool even = id >= 2L * mesh.nc;
-    const long e = even ? id - 2L * mesh.nc : id;
-    c = (int)(e >> 1);
-    f = (int)(e & 1) * 2 + (even ? 0 : 1);
+  auto face_of = [&](long id, int &c, int &f, int &code) {  // false: nothing to integrate
+    const bool hang = id >= nodd + neven;
+    if (hang) {
+      id -= nodd + neven;
+      if (!HG || id >= 2 * nodd) return false;
+      c = (int)(id >> 2);
+      f = (int)(id & 3);
+    } else {
+      const bool even = id >= nodd;
+      const long e = even ? id - nodd : id;
+      c = (int)(e >> 1);
+      f = (int)(e & 1) * 2 + (even ? 0 : 1);
+    }
     const int nb = mesh.nbr[c * 4 + f];
-    return nb < 0 ? KIND == 1 : !even;
+    code = HG && nb >= 0 ? mesh.nbrf[c * 4 + f] >> 2 : 0;
+    if (hang) return code != 0;
+    return nb < 0 ? KIND == 1 : (f & 1) && code == 0;
   };
-  int c, f;
-  if (face_of(g, c, f)) {
+  int c, f, code;
+  if (face_of(g0 + lf, c, f, code)) {
     const int nb = mesh.nbr[c * 4 + f], nf = mesh.nbrf[c * 4 + f] & 3;
     if (mesh.dts) co.dt *= mesh.dts[c];  // per-member time step
-    const double *fg = mesh.fgeo + ((long)c * 4 + f) * 3 * NQ + q;
-    const double n0[1] = {fg[0] * fg[2 * NQ]}, n1[1] = {fg[NQ] * fg[2 * NQ]};
-    double F[NCOMP][1];
+    for (int h = 0; h < (HG && code == 3 ? 2 : 1); ++h) {
+      const double *fg = (HG && code == 3 ? mesh.hgeo + ((long)nb * 2 + h) * 3 * NQ
+                                          : mesh.fgeo + ((long)c * 4 + f) * 3 * NQ) + q;
+      const double n0[1] = {fg[0] * fg[2 * NQ]}, n1[1] = {fg[NQ] * fg[2 * NQ]};
+      double F[NCOMP][1];
 #pragma unroll
-    for (int d = 0; d < NCOMP; ++d) F[d][0] = 0.0;
-    const PointTrace<K> to{f, sS[q]};
-    if (nb < 0) {  // no-flux wall: only the pressure term with p_D = p
+      for (int d = 0; d < NCOMP; ++d) F[d][0] = 0.0;
+      const PointTrace<K> to{f, sS[HG && code == 3 ? 1 + h : 0][q]};
+      if (nb < 0) {  // no-flux wall: only the pressure term with p_D = p
 #pragma unroll
-      for (int j = 0; j < ST; ++j) {
-        double p[1];
-        to(src.p[RhsKind<KIND>::PER * j + 2] + (long)c * NN2, p);
-        const double w = co.ct[j] * co.dt / (co.Ma * co.Ma) * p[0];
-        F[0][0] = fma(w, n0[0], F[0][0]);
-        F[NCOMP - 1][0] = fma(w, n1[0], F[NCOMP - 1][0]);
+        for (int j = 0; j < ST; ++j) {
+          double p[1];
+          to(src.p[RhsKind<KIND>::PER * j + 2] + (long)c * NN2, p);
+          const double w = co.ct[j] * co.dt / (co.Ma * co.Ma) * p[0];
+          F[0][0] = fma(w, n0[0], F[0][0]);
+          F[NCOMP - 1][0] = fma(w, n1[0], F[NCOMP - 1][0]);
+        }
+      } else {
+        const int cn = HG && code == 3 ? mesh.hnb[nb * 2 + h] : nb;
+        face_flux<K, ST, KIND>(src, co, c, cn, to,
+                               PointTrace<K>{nf, sS[HG && (code == 1 || code == 2) ? code : 0][q]},
+                               n0, n1, F);
       }
-    } else {
-      face_flux<K, ST, KIND>(src, co, c, nb, to, PointTrace<K>{nf, sS[q]}, n0, n1, F);
-    }
 #pragma unroll
-    for (int d = 0; d < NCOMP; ++d) sF[lf][d][q] = F[d][0];
+      for (int d = 0; d < NCOMP; ++d) sF[lf][HG ? h : 0][d][q] = F[d][0];
+    }
   }
   __syncthreads();
   for (int t = threadIdx.x; t < RHS_FPB * NCOMP * NN; t += blockDim.x) {
     const int l = t / (NCOMP * NN), r = t - l * NCOMP * NN, d = r / NN, i = r - d * NN;
-    if (!face_of(g0 + l, c, f)) continue;
+    if (!face_of(g0 + l, c, f, code)) continue;
     double o = 0.0;
+    if (HG && code == 3) {
+      for (int h = 0; h < 2; ++h)
 #pragma unroll
-    for (int k = 0; k < NQ; ++k) o = fma(sS[k][i], sF[l][d][k], o);
+        for (int k = 0; k < NQ; ++k)
+          o = fma(sS[HG ? 1 + h : 0][k][i], sF[l][HG ? h : 0][d][k], o);
+    } else {
+#pragma unroll
+      for (int k = 0; k < NQ; ++k) o = fma(sS[0][k][i], sF[l][0][d][k], o);
+    }
     Fb[((long)c * 4 + f) * NCOMP * NN + r] = o;
   }
 }
@@ -568,25 +594,30 @@ inline void rhs_sources(SrcPtrs &sp, int &nsrc, int kind, int stage, const doubl
   for (int i = 0; i < nsrc; ++i) sp.p[i] = src[i];
 }
 
-// Conforming meshes below this many cells integrate faces point by point.  The
-// second stage's three right-hand sides, a face per thread / a point per thread:
+// Meshes below this many cells integrate faces point by point.  The second
+// stage's three right-hand sides, a face per thread / a point per thread:
 // 231 / 158 us at 800 cells, k = 4; 182 / 146 at 2304, k = 3; 554 / 535 at 4140,
-// k = 5; 197 / 207 at 8192, k = 2; 554 / 561 at 8192, k = 4.
-constexpr int RHS_POINT_CELLS = 6000;
+// k = 5; 197 / 207 at 8192, k = 2; 554 / 561 at 8192, k = 4.  With hanging faces,
+// which are of either parity, a mesh has more faces per cell and a thread more
+// registers: third stage at k = 3, 788 / 638 us at 9120 cells, 1300 / 1345 at
+// 22000; at k = 5 1792 / 1540 and 3256 / 3480.
+constexpr int RHS_POINT_CELLS = 6000, RHS_POINT_CELLS_HANG = 12000;
 template <int K, int KIND, bool HG>
 int rhs_face_launch(const atm_ctx &c, int stage, const SrcPtrs &sp, const StageCoef &co) {
   // even faces: the momentum walls, and hanging faces
   const long n = (long)c.nc * (HG || KIND == 1 ? 4 : 2);
-  if constexpr (!HG)
-    if (c.nc < RHS_POINT_CELLS) {
-      void (*fn)(double *, SrcPtrs, StageCoef, Mesh) =
-          stage == 1 ? k_rhs_face_points<K, 1, KIND>
-                     : (stage == 2 ? k_rhs_face_points<K, 2, KIND> : k_rhs_face_points<K, 3, KIND>);
-      fn<<<(unsigned)((n + RHS_FPB - 1) / RHS_FPB), RHS_FPB * (2 * K + 1), 0, c.stream>>>(c.fbuf, sp,
-                                                                                        co, c.mesh);
-      ATM_CHECK_LAUNCH("k_rhs_face_points");
-      return ATM_OK;
-    }
+  if (c.nc < (HG ? RHS_POINT_CELLS_HANG : RHS_POINT_CELLS)) {
+    // odd faces; even walls of the momentum equation; hanging faces
+    const long m = (long)c.nc * (2 + (KIND == 1 ? 2 : 0) + (HG ? 4 : 0));
+    void (*fp)(double *, SrcPtrs, StageCoef, Mesh) =
+        stage == 1 ? k_rhs_face_points<K, 1, KIND, HG>
+                   : (stage == 2 ? k_rhs_face_points<K, 2, KIND, HG>
+                                 : k_rhs_face_points<K, 3, KIND, HG>);
+    fp<<<(unsigned)((m + RHS_FPB - 1) / RHS_FPB), RHS_FPB * (2 * K + 1), 0, c.stream>>>(c.fbuf, sp, co,
+                                                                                      c.mesh);
+    ATM_CHECK_LAUNCH("k_rhs_face_points");
+    return ATM_OK;
+  }
   void (*fn)(double *, SrcPtrs, StageCoef, Mesh) =
       stage == 1 ? k_rhs_face<K, 1, KIND, HG>
                  : (stage == 2 ? k_rhs_face<K, 2, KIND, HG> : k_rhs_face<K, 3, KIND, HG>);
