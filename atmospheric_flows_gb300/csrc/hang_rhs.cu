@@ -7,11 +7,12 @@ namespace atm {
 
 int upload_contract_hang_rhs(const double *t) { return upload_exact_here(t); }
 
-int rhs_face_hang(const atm_ctx &c, int kind, int stage, const SrcPtrs &sp, const StageCoef &co) {
+int rhs_face_hang(const atm_ctx &c, int kind, int stage, double *dst, int way, const SrcPtrs &sp,
+                  const StageCoef &co) {
   switch (kind) {
-    case 0: return rhs_face_dispatch<0, true>(c, stage, sp, co);
-    case 1: return rhs_face_dispatch<1, true>(c, stage, sp, co);
-    default: return rhs_face_dispatch<2, true>(c, stage, sp, co);
+    case 0: return rhs_face_dispatch<0, true>(c, stage, dst, way, sp, co);
+    case 1: return rhs_face_dispatch<1, true>(c, stage, dst, way, sp, co);
+    default: return rhs_face_dispatch<2, true>(c, stage, dst, way, sp, co);
   }
 }
 

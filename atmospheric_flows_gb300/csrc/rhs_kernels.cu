@@ -7,16 +7,18 @@ namespace atm {
 int upload_contract_rhs(const double *t) { return upload_exact_here(t); }
 
 // face kernels of meshes with hanging faces (hang_rhs.cu)
-int rhs_face_hang(const atm_ctx &c, int kind, int stage, const SrcPtrs &sp, const StageCoef &co);
+int rhs_face_hang(const atm_ctx &c, int kind, int stage, double *dst, int way, const SrcPtrs &sp,
+                  const StageCoef &co);
 
 namespace {
 template <int K, int KIND>
-int rhs_cell_launch(const atm_ctx &c, int stage, double *dst, const SrcPtrs &sp,
-                    const StageCoef &co, bool idem) {
+int rhs_passes(const atm_ctx &c, int stage, double *dst, const SrcPtrs &sp, const StageCoef &co,
+               bool aliased) {
   using E = Ex<K>;
   const bool ex = KIND == 0 && c.mesh.exact;
   const int np = ex ? E::NC : E::NQ;
-  void (*fn)(double *, SrcPtrs, StageCoef, Mesh, const double *, int);
+  const bool held = !aliased;
+  void (*fn)(double *, SrcPtrs, StageCoef, Mesh, bool, int);
   if (ex) {
     constexpr bool X = KIND == 0;
     fn = stage == 1 ? k_rhs_cell<K, 1, KIND, X>
@@ -30,16 +32,29 @@ int rhs_cell_launch(const atm_ctx &c, int stage, double *dst, const SrcPtrs &sp,
     // below 2048 cells it has no say: small blocks reach more SMs
     const int threads = tuned >= 256 / E::NQ ? 256 : (tuned >= 128 / E::NQ ? 128 : 64);
     const int cpb = (c.nc < 2048 ? 64 : threads) / np;
-    const size_t sm = sizeof(double) * (size_t)cpb * RhsKind<KIND>::NF * E::NN * np;
+    const size_t sm = sizeof(double) * (size_t)cpb *
+                      (RhsKind<KIND>::NF * E::NN * np + (held ? RhsKind<KIND>::NCOMP * FACE_VALUES<K> : 0));
     if (cudaError_t e = allow_smem(fn, sm); e != cudaSuccess) return e;
-    fn<<<(c.nc + cpb - 1) / cpb, cpb * np, sm, c.stream>>>(dst, sp, co, c.mesh, c.fbuf, cpb);
+    fn<<<(c.nc + cpb - 1) / cpb, cpb * np, sm, c.stream>>>(dst, sp, co, c.mesh, held, cpb);
     return cudaGetLastError();
   };
+  auto faces = [&](int way) {
+    return c.mesh.nhang > 0 ? rhs_face_hang(c, KIND, stage, dst, way, sp, co)
+                            : rhs_face_launch<K, KIND, false>(c, stage, dst, way, sp, co);
+  };
+  // the tuner runs the cell kernel on whatever dst holds, before the faces fill it
   const int cpb = tuned_cpb(c.autotune && !c.capturing, c.stream, TF_RHS_RHO + KIND, K, stage,
-                            c.mesh.nhang > 0, 8, c.nc, idem, launch);
+                            c.mesh.nhang > 0, 8, c.nc, !aliased, launch);
+  if (held) {
+    if (!FACE_SLOTS<K>)
+      ATM_CUDA(cudaMemsetAsync(dst, 0, RhsKind<KIND>::NCOMP * c.n_scalar() * sizeof(double), c.stream));
+    if (int rc = faces(FACE_HELD)) return rc;
+  }
   ATM_CUDA(launch(cpb));
   g_kernel_launches.fetch_add(1);
-  return ATM_OK;
+  if (held) return ATM_OK;
+  if (int rc = faces(FACE_ADD_X)) return rc;
+  return faces(FACE_ADD_Z);
 }
 
 template <int KIND>
@@ -49,8 +64,14 @@ int rhs_launch(const atm_ctx &c, int stage, double *dst, const double *const *sr
   SrcPtrs sp{};
   int nsrc;
   rhs_sources(sp, nsrc, KIND, stage, src);
-  bool idem = true;  // the kernel only writes dst: safe to run repeatedly
-  for (int i = 0; i < nsrc; ++i) idem = idem && src[i] != dst;
+  // dst may overlap a source that only the cell kernel reads
+  bool aliased = false;
+  for (int i = 0; i < nsrc; ++i) {
+    const bool velocity = i % RhsKind<KIND>::PER == 1;
+    const uintptr_t a = (uintptr_t)src[i], d = (uintptr_t)dst;
+    aliased = aliased || (a < d + RhsKind<KIND>::NCOMP * c.n_scalar() * sizeof(double) &&
+                          d < a + (velocity ? 2 : 1) * c.n_scalar() * sizeof(double) && src[i]);
+  }
   // algorithmic bytes: every source field read once, the result written once
   const int k = c.k, nout = KIND == 1 ? 2 : 1;
   const int nfields =
@@ -63,10 +84,7 @@ int rhs_launch(const atm_ctx &c, int stage, double *dst, const double *const *sr
   const double flops = c.nc * (nfields * fl_eval(k) + nout * fl_integrate(k, true) +
                                2.0 * (2 * ntrace * fl_face(k) + nout * fl_face(k)));
   TimedRegion tr(c, KF_RHS_RHO + KIND, bytes, flops);
-  if (int rc = c.mesh.nhang > 0 ? rhs_face_hang(c, KIND, stage, sp, co)
-                                : rhs_face_dispatch<KIND, false>(c, stage, sp, co))
-    return rc;
-  ATM_DISPATCH_K(k, (rhs_cell_launch<K, KIND>(c, stage, dst, sp, co, idem)));
+  ATM_DISPATCH_K(k, (rhs_passes<K, KIND>(c, stage, dst, sp, co, aliased)));
 }
 }  // namespace
 

@@ -8,17 +8,22 @@
 // 2D form of the reference's 3D operators: gravity acts along -e_z with the
 // factor a^2/r^2 = 1 (euler_operator.h:790-811 on a Cartesian domain).
 //
-// Each right-hand side is two kernels, bound by their FP64 instructions:
+// Each right-hand side has face and cell kernels, bound by their FP64
+// instructions:
 //   * k_rhs_face integrates the numerical flux of every face once.  The fluxes
 //     are conservative (the reference's "+" and "-" contributions are one
 //     expression with the sides swapped and n -> -n), so of the two sides of a
 //     conforming face only the odd local face (1: x = 1, 3: z = 1) is
-//     integrated and the cell on the other side adds the same nodal integrals
-//     with the opposite sign.  Walls and hanging faces are integrated from
-//     each of their sides, with that side's geometry.
+//     integrated and its nodal integrals go to both cells, with opposite
+//     signs.  Walls and hanging faces are integrated from each of their sides,
+//     with that side's geometry.
 //   * k_rhs_cell evaluates the fields row by row and column by column (one
 //     thread per 1D contraction, contract.cuh), forms the cell integrals and
 //     adds the face integrals.
+//
+// The integrals pass from one kernel to the other in dst itself (FaceWay): a
+// right-hand side writes nothing but its destination, so that calls on one
+// handle may overlap, on several streams, threads or branches of a graph.
 // A face trace takes 35 FP64 instructions per field and stage state, a face
 // point about 20: integrating a face from both cells would cost a quarter of
 // the whole right-hand side.  No atomics; runs are bitwise reproducible.
@@ -66,6 +71,41 @@ struct PointTrace {
     v[0] = s;
   }
 };
+
+// How the face integrals reach dst.
+//   FACE_HELD: all faces are integrated first and the cell kernel reads its cells'
+//     values before it overwrites them.  With k >= 3 a cell's (k+1)^2 values hold
+//     its 4 (k+1) face integrals in slots of their own.  With k <= 2 they do not
+//     fit: dst is zeroed and a node gets the sum of its face integrals, at most
+//     two (in a corner), by atomics; 0 + a + b does not depend on their order.
+//   FACE_ADD_X, FACE_ADD_Z: for a dst that is also a source, which must not be
+//     written before the cell kernel has read it.  The cell kernel goes first,
+//     then the x-faces and the z-faces add to the nodes they touch, in two
+//     launches (the two meet in the corner nodes).  For k <= 2 this order took 310
+//     instead of 250 us at 8192 cells, k = 2, third stage.
+enum FaceWay { FACE_HELD = 0, FACE_ADD_X = 1, FACE_ADD_Z = 2 };
+template <int K>
+constexpr bool FACE_SLOTS = K >= 3;
+template <int K>  // values per cell and component that hold face integrals
+constexpr int FACE_VALUES = FACE_SLOTS<K> ? 4 * (K + 1) : (K + 1) * (K + 1);
+
+// local faces that a launch takes of each parity and cell, and the n-th of them
+__device__ __forceinline__ int way_faces(int way) { return way == FACE_HELD ? 2 : 1; }
+__device__ __forceinline__ int way_face(int way, int n, int odd) {
+  return (way == FACE_HELD ? 2 * n : way == FACE_ADD_X ? 0 : 2) + odd;
+}
+
+// nodal integral i of component `comp` over face f of cell c
+template <int K, int NCOMP>
+__device__ __forceinline__ void face_put(double *__restrict__ dst, int way, int c, int f, int comp,
+                                         int i, double v) {
+  constexpr int NN = K + 1, NN2 = NN * NN;
+  double *b = dst + ((long)c * NCOMP + comp) * NN2;
+  double *node = b + (f < 2 ? i * NN + f * K : (f - 2) * K * NN + i);
+  if (way != FACE_HELD) *node += v;
+  else if (FACE_SLOTS<K>) b[f * NN + i] = v;
+  else atomicAdd(node, v);
+}
 
 // F[comp][q] += numerical flux of all stage states at NQ points of one face,
 // outward of cell c, times the face weight.  n0, n1: normal times weight; to,
@@ -146,18 +186,20 @@ __device__ __forceinline__ void face_flux(const SrcPtrs &src, const StageCoef &c
   }
 }
 
-// Fb[c][f][comp][k+1]: nodal integrals of the outward flux; one thread per
-// face, the odd local faces first, then (`all`) the even ones that are not
-// the other side of a conforming face.
+// Nodal integrals of the outward flux; one thread per face, the odd local faces
+// first, then the even ones that are not the other side of a conforming face
+// (walls of the momentum equation, hanging faces).
 template <int K, int ST, int KIND, bool HG>
 __global__ void __launch_bounds__(64)
-    k_rhs_face(double *__restrict__ Fb, SrcPtrs src, StageCoef co, Mesh mesh) {
+    k_rhs_face(double *__restrict__ dst, int way, SrcPtrs src, StageCoef co, Mesh mesh) {
   constexpr int NN = K + 1, NN2 = NN * NN, NQ = 2 * K + 1, NCOMP = RhsKind<KIND>::NCOMP;
   const long g = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  const bool even = g >= 2L * mesh.nc;
-  const long e = even ? g - 2L * mesh.nc : g;
-  if (e >= 2L * mesh.nc) return;
-  const int c = (int)(e >> 1), f = (int)(e & 1) * 2 + (even ? 0 : 1);
+  const long half = (long)way_faces(way) * mesh.nc;
+  const bool even = g >= half;
+  const long e = even ? g - half : g;
+  if (e >= half) return;
+  const int c = (int)(way == FACE_HELD ? e >> 1 : e);
+  const int f = way_face(way, (int)(e & 1), even ? 0 : 1);
   const int nb = mesh.nbr[c * 4 + f], nfc = mesh.nbrf[c * 4 + f], nf = nfc & 3;
   if (nb < 0 && KIND != 1) return;
   const int code = HG && nb >= 0 ? nfc >> 2 : 0;
@@ -212,11 +254,13 @@ __global__ void __launch_bounds__(64)
       for (int d = 0; d < NCOMP; ++d) sub_integ_add<K, 1>(F[d], h, o[d]);
     }
   }
-  double *out = Fb + ((long)c * 4 + f) * NCOMP * NN;
 #pragma unroll
   for (int d = 0; d < NCOMP; ++d)
 #pragma unroll
-    for (int i = 0; i < NN; ++i) out[d * NN + i] = o[d][i];
+    for (int i = 0; i < NN; ++i) {
+      face_put<K, NCOMP>(dst, way, c, f, d, i, -o[d][i]);
+      if (nb >= 0 && code == 0) face_put<K, NCOMP>(dst, way, nb, nf, d, i, o[d][i]);
+    }
 }
 
 // The same with one thread per face point, RHS_FPB faces per block: 5 instead of
@@ -227,7 +271,7 @@ __global__ void __launch_bounds__(64)
 constexpr int RHS_FPB = 16;
 template <int K, int ST, int KIND, bool HG>
 __global__ void __launch_bounds__(RHS_FPB *(2 * K + 1))
-    k_rhs_face_points(double *__restrict__ Fb, SrcPtrs src, StageCoef co, Mesh mesh) {
+    k_rhs_face_points(double *__restrict__ dst, int way, SrcPtrs src, StageCoef co, Mesh mesh) {
   constexpr int NN = K + 1, NN2 = NN * NN, NQ = 2 * K + 1, NCOMP = RhsKind<KIND>::NCOMP;
   constexpr int NT = HG ? 3 : 1, NH = HG ? 2 : 1;
   // basis rows at the face's points, and at those of its two subfaces
@@ -242,7 +286,8 @@ __global__ void __launch_bounds__(RHS_FPB *(2 * K + 1))
   }
   __syncthreads();
   // odd conforming faces and walls; (momentum) even walls; hanging faces
-  const long nodd = 2L * mesh.nc, neven = KIND == 1 ? nodd : 0;
+  const int per = way_faces(way);
+  const long nodd = (long)per * mesh.nc, neven = KIND == 1 ? nodd : 0;
   const long g0 = (long)blockIdx.x * RHS_FPB;
   const int lf = threadIdx.x / NQ, q = threadIdx.x - lf * NQ;
   auto face_of = [&](long id, int &c, int &f, int &code) {  // false: nothing to integrate
@@ -250,13 +295,13 @@ __global__ void __launch_bounds__(RHS_FPB *(2 * K + 1))
     if (hang) {
       id -= nodd + neven;
       if (!HG || id >= 2 * nodd) return false;
-      c = (int)(id >> 2);
-      f = (int)(id & 3);
+      c = (int)(per == 2 ? id >> 2 : id >> 1);
+      f = way_face(way, (int)(id >> 1) & 1, (int)(id & 1));
     } else {
       const bool even = id >= nodd;
       const long e = even ? id - nodd : id;
-      c = (int)(e >> 1);
-      f = (int)(e & 1) * 2 + (even ? 0 : 1);
+      c = (int)(per == 2 ? e >> 1 : e);
+      f = way_face(way, (int)(e & 1), even ? 0 : 1);
     }
     const int nb = mesh.nbr[c * 4 + f];
     code = HG && nb >= 0 ? mesh.nbrf[c * 4 + f] >> 2 : 0;
@@ -308,7 +353,10 @@ __global__ void __launch_bounds__(RHS_FPB *(2 * K + 1))
 #pragma unroll
       for (int k = 0; k < NQ; ++k) o = fma(sS[0][k][i], sF[l][0][d][k], o);
     }
-    Fb[((long)c * 4 + f) * NCOMP * NN + r] = o;
+    face_put<K, NCOMP>(dst, way, c, f, d, i, -o);
+    const int nb = mesh.nbr[c * 4 + f];
+    if (nb >= 0 && code == 0)
+      face_put<K, NCOMP>(dst, way, nb, mesh.nbrf[c * 4 + f] & 3, d, i, o);
   }
 }
 
@@ -342,53 +390,53 @@ __device__ __forceinline__ void rhs_col(const double *__restrict__ x, double (&v
   eo_interp<K, SET>(t, v);
 }
 
-// face integrals of component `comp` that output row iz adds
-template <int K, int KIND>
-__device__ __forceinline__ void rhs_face_rows(const double *__restrict__ Fb, const Mesh &mesh,
-                                              long c, int comp, int iz, double (&add)[K + 1]) {
-  constexpr int NN = K + 1, NCOMP = RhsKind<KIND>::NCOMP;
-  const int4 nb4 = *reinterpret_cast<const int4 *>(mesh.nbr + c * 4);
-  const int4 nf4 = *reinterpret_cast<const int4 *>(mesh.nbrf + c * 4);
-  const int nb[4] = {nb4.x, nb4.y, nb4.z, nb4.w}, nf[4] = {nf4.x, nf4.y, nf4.z, nf4.w};
+// face integrals that output row iz adds; F: the cell's held values, [4][k+1]
+// slots or node sums
+template <int K>
+__device__ __forceinline__ void rhs_face_rows(const double *__restrict__ F, int iz,
+                                              double (&add)[K + 1]) {
+  constexpr int NN = K + 1;
+  if constexpr (FACE_SLOTS<K>) {
 #pragma unroll
-  for (int i = 0; i < NN; ++i) add[i] = 0.0;
+    for (int i = 0; i < NN; ++i) add[i] = 0.0;
+    add[0] += F[iz];
+    add[K] += F[NN + iz];
+    if (iz == 0 || iz == K) {
+      const double *Fz = iz == 0 ? F + 2 * NN : F + 3 * NN;
 #pragma unroll
-  for (int f = 0; f < 4; ++f) {
-    if (f == 2 ? iz != 0 : f == 3 ? iz != K : false) continue;
-    if (nb[f] < 0 && KIND != 1) continue;
-    // even conforming faces: the neighbour's integrals, as they are; the
-    // others: this cell's own with the sign flipped (on the integer pipe)
-    const bool theirs = !(f & 1) && nb[f] >= 0 && (nf[f] >> 2) == 0;
-    const double *F =
-        Fb + (theirs ? (long)nb[f] * 4 + (nf[f] & 3) : c * 4 + f) * NCOMP * NN + comp * NN;
-    const long long flip = theirs ? 0 : (long long)0x8000000000000000ull;
-    if (f < 2) {
-      const double v = __longlong_as_double(__double_as_longlong(F[iz]) ^ flip);
-      if (f == 0) add[0] += v;
-      else add[K] += v;
-    } else {
-#pragma unroll
-      for (int i = 0; i < NN; ++i)
-        add[i] += __longlong_as_double(__double_as_longlong(F[i]) ^ flip);
+      for (int i = 0; i < NN; ++i) add[i] += Fz[i];
     }
+  } else {
+#pragma unroll
+    for (int i = 0; i < NN; ++i) add[i] = F[iz * NN + i];
   }
 }
 
-// Threads (cell, column); `cpb` cells per block.
+// Threads (cell, column); `cpb` cells per block.  With `held`, dst holds the
+// face integrals of its cells (FaceWay).
 template <int K, int ST, int KIND, bool EX>
 __global__ void __launch_bounds__(256)
-    k_rhs_cell(double *__restrict__ dst, SrcPtrs src, StageCoef co, Mesh mesh,
-               const double *__restrict__ Fb, int cpb) {
+    k_rhs_cell(double *dst, SrcPtrs src, StageCoef co, Mesh mesh, bool held, int cpb) {
   using E = Ex<K>;
   using R = RhsKind<KIND>;
   constexpr int NN = E::NN, NN2 = E::NN2, NCOMP = R::NCOMP, PER = R::PER;
   constexpr int SET = EX ? 1 : 2, NP = EX ? E::NC : E::NQ, XS = NN * NP, XC = R::NF * XS;
   constexpr double IG = 1.0 / (GAS_GAMMA - 1.0), HGF = GAS_GAMMA * IG;
-  extern __shared__ double sm[];  // [cpb][NF][NN][NP]
+  constexpr int FV = FACE_VALUES<K>;
+  extern __shared__ double sm[];  // [cpb][NF][NN][NP], then (held) [cpb][NCOMP][FV]
   const int tid = threadIdx.x, l = tid / NP, col = tid - l * NP;
   const int c0 = blockIdx.x * cpb, cnt = min(cpb, mesh.nc - c0);
   const bool active = l < cnt;
   const long c = c0 + l;
+  double *sF = sm + cpb * XC;
+  if (held) {
+    for (int e = tid; e < cnt * NCOMP * FV; e += blockDim.x) {
+      const int lc = e / FV, i = e - lc * FV;
+      // (density and energy have no boundary term: nothing is in a wall's slot)
+      const bool wall = FACE_SLOTS<K> && KIND != 1 && mesh.nbr[(c0 + lc / NCOMP) * 4 + i / NN] < 0;
+      sF[e] = wall ? 0.0 : dst[((long)c0 * NCOMP + lc) * NN2 + i];
+    }
+  }
   if (mesh.dts && active) co.dt *= mesh.dts[c];  // per-member time step
   const double M2 = co.Ma * co.Ma;
   double *x = sm + l * XC + col;
@@ -532,11 +580,15 @@ __global__ void __launch_bounds__(256)
       a[q] = y[q];
       b[q] = y[XS + q];
     }
-    rhs_face_rows<K, KIND>(Fb, mesh, c0 + lo, comp, iz, add);
     eo_integ<K, SET, NP, true, true>(a, b, out);
     double *d = dst + ((long)(c0 + lo) * NCOMP + comp) * NN2 + iz * NN;
+    if (held) {
+      rhs_face_rows<K>(sF + (lo * NCOMP + comp) * FV, iz, add);
 #pragma unroll
-    for (int q = 0; q < NN; ++q) d[q] = out[q] + add[q];
+      for (int q = 0; q < NN; ++q) out[q] += add[q];
+    }
+#pragma unroll
+    for (int q = 0; q < NN; ++q) d[q] = out[q];
   }
 }
 
@@ -603,32 +655,35 @@ inline void rhs_sources(SrcPtrs &sp, int &nsrc, int kind, int stage, const doubl
 // 22000; at k = 5 1792 / 1540 and 3256 / 3480.
 constexpr int RHS_POINT_CELLS = 6000, RHS_POINT_CELLS_HANG = 12000;
 template <int K, int KIND, bool HG>
-int rhs_face_launch(const atm_ctx &c, int stage, const SrcPtrs &sp, const StageCoef &co) {
+int rhs_face_launch(const atm_ctx &c, int stage, double *dst, int way, const SrcPtrs &sp,
+                    const StageCoef &co) {
+  const int per = way == FACE_HELD ? 2 : 1;  // as way_faces
   // even faces: the momentum walls, and hanging faces
-  const long n = (long)c.nc * (HG || KIND == 1 ? 4 : 2);
+  const long n = (long)c.nc * per * (HG || KIND == 1 ? 2 : 1);
   if (c.nc < (HG ? RHS_POINT_CELLS_HANG : RHS_POINT_CELLS)) {
     // odd faces; even walls of the momentum equation; hanging faces
-    const long m = (long)c.nc * (2 + (KIND == 1 ? 2 : 0) + (HG ? 4 : 0));
-    void (*fp)(double *, SrcPtrs, StageCoef, Mesh) =
+    const long m = (long)c.nc * per * (1 + (KIND == 1 ? 1 : 0) + (HG ? 2 : 0));
+    void (*fp)(double *, int, SrcPtrs, StageCoef, Mesh) =
         stage == 1 ? k_rhs_face_points<K, 1, KIND, HG>
                    : (stage == 2 ? k_rhs_face_points<K, 2, KIND, HG>
                                  : k_rhs_face_points<K, 3, KIND, HG>);
-    fp<<<(unsigned)((m + RHS_FPB - 1) / RHS_FPB), RHS_FPB * (2 * K + 1), 0, c.stream>>>(c.fbuf, sp, co,
-                                                                                      c.mesh);
+    fp<<<(unsigned)((m + RHS_FPB - 1) / RHS_FPB), RHS_FPB * (2 * K + 1), 0, c.stream>>>(
+        dst, way, sp, co, c.mesh);
     ATM_CHECK_LAUNCH("k_rhs_face_points");
     return ATM_OK;
   }
-  void (*fn)(double *, SrcPtrs, StageCoef, Mesh) =
+  void (*fn)(double *, int, SrcPtrs, StageCoef, Mesh) =
       stage == 1 ? k_rhs_face<K, 1, KIND, HG>
                  : (stage == 2 ? k_rhs_face<K, 2, KIND, HG> : k_rhs_face<K, 3, KIND, HG>);
-  fn<<<(unsigned)((n + 63) / 64), 64, 0, c.stream>>>(c.fbuf, sp, co, c.mesh);
+  fn<<<(unsigned)((n + 63) / 64), 64, 0, c.stream>>>(dst, way, sp, co, c.mesh);
   ATM_CHECK_LAUNCH("k_rhs_face");
   return ATM_OK;
 }
 
 template <int KIND, bool HG>
-int rhs_face_dispatch(const atm_ctx &c, int stage, const SrcPtrs &sp, const StageCoef &co) {
-  ATM_DISPATCH_K(c.k, (rhs_face_launch<K, KIND, HG>(c, stage, sp, co)));
+int rhs_face_dispatch(const atm_ctx &c, int stage, double *dst, int way, const SrcPtrs &sp,
+                      const StageCoef &co) {
+  ATM_DISPATCH_K(c.k, (rhs_face_launch<K, KIND, HG>(c, stage, dst, way, sp, co)));
 }
 
 }  // namespace atm
