@@ -120,7 +120,10 @@ struct atm_ctx {
   double *ainv = nullptr;       // [nc][nn2*nn2] inverse of rho_fix-weighted mass
   double *invdiag_D = nullptr;  // inverse diagonal of D (Schur Jacobi)
   // workspace
-  double *fbuf = nullptr;  // [nc][4][2][nn] face integrals of the explicit right-hand sides
+  // [nc][4][nn] face integrals of C/D on large meshes (from EXACT_FB_UNKNOWNS, null
+  // below).  Workspace like wv1: only S and the solver, which use that too, may touch
+  // it, so that every other operator call can overlap any call of the handle.
+  double *fbuf = nullptr;
   double *wv1 = nullptr, *wv2 = nullptr;  // velocity-sized
   double *ws1 = nullptr, *ws2 = nullptr;  // scalar-sized
   double *red = nullptr;                  // reduction partials (device)
@@ -213,8 +216,10 @@ int launch_B(const atm_ctx &c, double *dst, const double *p, double cB, int mode
 //   mode 2: dst = invdiag .* (sD*D p - C w)
 //   mode 3: dst -= C w
 // (C uses the context's frozen p_fix, prepared by launch_pfix_prep)
+// `workspace`: the call belongs to one that uses the handle's workspace anyway,
+// and may use its face buffer
 int launch_CD(const atm_ctx &c, double *dst, const double *w, const double *p, double coeff,
-              int mode);
+              int mode, bool workspace = false);
 // values of p_fix at the quadrature points and its face traces (after every
 // change of p_fix)
 int launch_pfix_prep(const atm_ctx &c);
@@ -290,14 +295,20 @@ struct LevelViewT {
   cudaStream_t st;
   bool tune = false;  // the autotuner may time tile shapes on this stream
   const T *pfix = nullptr, *pfq = nullptr, *pff = nullptr;  // level p_fix (+ prepared)
-  T *fbuf = nullptr;  // [nc][4][2][nn] face integrals (the operator mesh only)
+  T *fbuf = nullptr;  // face integrals of C/D: atm_ctx::fbuf, where the call may use it
 };
 template <typename T>
 using OpView = LevelViewT<T>;
-inline OpView<double> schur_view(const atm_ctx &c) {
+inline OpView<double> schur_view(const atm_ctx &c, bool workspace = false) {
   return OpView<double>{c.k, c.nc, c.mesh, c.ainv, c.invdiag_D, c.stream,
-                        c.autotune && !c.capturing, c.pres_fix, c.pfq, c.pff, c.fbuf};
+                        c.autotune && !c.capturing, c.pres_fix, c.pfq, c.pff,
+                        workspace ? c.fbuf : nullptr};
 }
+// Scalar unknowns from which FP64 C/D takes its face integrals from a kernel of
+// their own.  S apply without / with it: 37 / 43 us at 4140 cells, k = 3 (66,000
+// unknowns); 32 / 33 at 8192, k = 2 (74,000); 100 / 96 at 4140, k = 5 (149,000);
+// 109 / 102 at 8192, k = 4 (205,000); 573 / 530 at 51,200, k = 4.
+constexpr long EXACT_FB_UNKNOWNS = 140000;
 #define ATM_DISPATCH_K(kk, call)          \
   switch (kk) {                           \
     case 1: { constexpr int K = 1; return call; } \

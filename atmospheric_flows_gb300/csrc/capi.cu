@@ -146,7 +146,7 @@ int atm_ctx_create(int dim, int degree, int n_cells, int mapping_degree,
   ALLOC(c->u_fix, nv);
   ALLOC(c->ainv, blk);
   ALLOC(c->invdiag_D, ns);
-  ALLOC(c->fbuf, (long)n_cells * 8 * c->nn);
+  if (ns >= EXACT_FB_UNKNOWNS) ALLOC(c->fbuf, (long)n_cells * 4 * c->nn);
   ALLOC(c->wv1, nv);
   ALLOC(c->wv2, nv);
   ALLOC(c->ws1, ns);

@@ -375,14 +375,14 @@ int launch_B(const atm_ctx &c, double *dst, const double *p, double cB, int mode
   ATM_DISPATCH_K(c.k, (B_launch<K, double, false>(schur_view(c), dst, p, cB, mode)));
 }
 int launch_CD(const atm_ctx &c, double *dst, const double *w, const double *p, double coeff,
-              int mode) {
+              int mode, bool workspace) {
   const double ns = (double)c.nc * c.nn2;
   const bool wd = (mode == 1 || mode == 2);
   // w (2 comps) + pfix read, [p], [inverse diagonal], [dst read], dst written
   const double bytes = 8.0 * ns * (3 + (wd ? 1 : 0) + (mode == 2 ? 1 : 0) + (mode == 3 ? 1 : 0) + 1);
   const double flops = c.nc * fl_CD(c.k, c.mesh.exact, wd);
   TimedRegion tr(c, KF_CD, bytes, flops);
-  if (c.mesh.exact) return exact_CD(schur_view(c), dst, w, p, coeff, mode, nullptr);
+  if (c.mesh.exact) return exact_CD(schur_view(c, workspace), dst, w, p, coeff, mode, nullptr);
   if (c.mesh.nhang > 0) return launch_CD_hang(c, dst, w, p, coeff, mode);
   ATM_DISPATCH_K(c.k, (CD_launch<K, double, false>(schur_view(c), dst, w, p, coeff, mode)));
 }

@@ -479,8 +479,9 @@ __device__ __forceinline__ void face_rows_of(const float *, const MeshT<float> &
 // Large FP64 meshes (FB): a face takes 256 FP64 instructions at k = 4, the rest
 // of a cell 2150, so k_exact_face_C integrates every conforming face once and
 // this kernel reads the integrals; without its own faces it fills blocks of
-// whole warps.  Smaller meshes (EXACT_FB_UNKNOWNS) and the FP32 levels (not
-// bound by arithmetic) integrate their own four faces.
+// whole warps.  Smaller meshes (EXACT_FB_UNKNOWNS), calls that may not use the
+// handle's workspace (C alone, the static-scratch S) and the FP32 levels (not bound
+// by arithmetic) integrate their own four faces.
 //
 // Threads (cell, column), column < NC; `cpb` cells per block, without FB a
 // multiple of 8, at most 32.  Three blocks per SM in FP64 (80 registers, k = 4):
@@ -736,11 +737,6 @@ __global__ void __launch_bounds__(32 * Ex<K>::NC)
 // ============================================================ launchers ===
 // The autotuner's cells per block, rounded up to a multiple of 8 so that the
 // face threads of C/D fill whole warps.
-// Scalar unknowns from which FP64 C/D takes its face integrals from a kernel of
-// their own.  S apply without / with it: 37 / 43 us at 4140 cells, k = 3 (66,000
-// unknowns); 32 / 33 at 8192, k = 2 (74,000); 100 / 96 at 4140, k = 5 (149,000);
-// 109 / 102 at 8192, k = 4 (205,000); 573 / 530 at 51,200, k = 4.
-constexpr long EXACT_FB_UNKNOWNS = 140000;
 inline int exact_cells(int cpb) { return (cpb + 7) / 8 * 8; }
 
 template <int K, typename T, bool HG>
@@ -783,7 +779,7 @@ int exact_CD_launch(const OpView<T> &v, T *dst, const T *w, const T *p, T cC, in
   using E = Ex<K>;
   const T *pfix = v.pfix;
   const ChebArgs<T> ch = cheb ? *cheb : ChebArgs<T>{};
-  const bool fb = sizeof(T) == 8 && v.fbuf && (long)v.nc * E::NN2 >= EXACT_FB_UNKNOWNS;
+  const bool fb = sizeof(T) == 8 && v.fbuf;
   bool overlap = false;  // not while the tuner times the kernel
   auto launch = [&](int tuned) -> cudaError_t {
     int cpb = v.nc < 2048 ? 8 : exact_cells(tuned);

@@ -8,7 +8,8 @@
 // device, which a latency-sensitive caller sharing the GPU with other streams
 // cannot afford.  This entry point computes the same S p = D p - C A^{-1} B p
 // as atm_vmult in NS stage 2, but keeps A^{-1} B p in the file-scope array
-// below instead of the context's workspace, and calls no allocating routine.
+// below instead of the context's workspace (C/D integrates its own faces, without
+// the context's face buffer), and calls no allocating routine.
 //
 // Limits and sharing rules:
 //   * the array holds SCHUR_SCRATCH_DOUBLES doubles (8 MiB); a context whose

@@ -177,7 +177,7 @@ int pressure_fixed_point(atm_ctx &c, Solver &s) {
                          c.hstage == 1 ? s.rho_tmp_2 : s.rho_tmp_3, s.u_fixed, co));
   // rhs_pres -= C A^{-1} rhs_u
   const double cc = implicit_coeff(c);
-  TRY(launch_CD(c, s.rhs_pres, s.tmp_1, nullptr, cc * c.dt, 3));
+  TRY(launch_CD(c, s.rhs_pres, s.tmp_1, nullptr, cc * c.dt, 3, true));
   if (c.mem) return schur_solve_members(c, s);
   TRY(vec_dot(c.stream, s.rhs_pres, s.rhs_pres, ns, c.red, c.red_out));
   TRY(read_scalars(c, 1));

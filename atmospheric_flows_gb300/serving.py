@@ -107,7 +107,9 @@ def member_bytes(p: HillParams, precision: int = 1) -> int:
     schur = 4 * nn2 + 8 * (k + 1) + 9 * ncp * ncp + 12 * nq
     geo = nc * (5 * nq * nq + 12 * nq + schur) * 8 + nc * 8 * 4 * 2
     blocks = 2 * nc * nn2 * nn2 * 8           # M^{-1}, A^{-1}
-    ctx_vec = (4 + 4 + 2 + 1 + 29) * ns * 8 + nc * 8 * (k + 1) * 8  # frozen fields, work, GMRES basis, face integrals
+    ctx_vec = (4 + 4 + 2 + 1 + 29) * ns * 8   # frozen fields, work, GMRES basis
+    if ns >= 140000:
+        ctx_vec += nc * 4 * (k + 1) * 8       # face integrals of C/D
     solver_vec = (13 + 16) * ns * 8
     total = geo + blocks + ctx_vec + solver_vec
     if precision in (1, 2):

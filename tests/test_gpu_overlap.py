@@ -141,3 +141,41 @@ def test_energy_rhs_into_its_density(cuda_ok, nx, nz, degree, adaptive):
     err = (own - ref).abs().max().item() / ref.abs().max().item()
     assert err < 1e-12, err
     op.close()
+
+
+@pytest.mark.parametrize("nx,nz,degree,adaptive", [(101, 60, 4, False), (60, 40, 4, False),
+                                                   (94, 96, 3, True)])
+def test_operators_beside_the_schur_apply(cuda_ok, nx, nz, degree, adaptive):
+    """B, C, the static-scratch S and a right-hand side, each on a stream of its
+    own, beside the one call that uses the handle's workspace: S (with a face
+    buffer from 140,000 unknowns on, first and last mesh)."""
+    from atmospheric_flows_gb300 import _lib
+
+    op, case, rng = setup(nx, nz, degree, adaptive)
+    rho, _, p = state(case, rng)
+    op.set_rho_for_fixed(rho)
+    op.set_pres_fixed(p)
+    op.set_NS_stage(2)
+    q, w = state(case, rng)[2], state(case, rng)[1]
+    rhs, src, mom, _ = rhs_calls(op, case, rng)[1]
+    out = [torch.empty_like(q), torch.empty_like(w), torch.empty_like(q), torch.empty_like(q), mom]
+    static = lambda d, s: _lib.call("atm_schur_vmult_static_scratch", op.handle,  # noqa: E731
+                                    ctypes.c_void_p(d.data_ptr()), ctypes.c_void_p(s.data_ptr()))
+    calls = [(op.vmult, q), (op.vmult_pressure, q), (op.vmult_enthalpy, w), (static, q), (rhs, src)]
+    for (fn, s), d in zip(calls, out):
+        fn(d, s)
+        torch.cuda.synchronize()
+    ref = [d.clone() for d in out]
+    streams = [torch.cuda.Stream() for _ in calls]
+    for _ in range(40):
+        for d in out:
+            d.fill_(float("nan"))
+        torch.cuda.synchronize()
+        for st, (fn, s), d in zip(streams, calls, out):
+            set_stream(op, st)
+            fn(d, s)
+        torch.cuda.synchronize()
+        for d, r in zip(out, ref):
+            assert torch.equal(d, r)
+    set_stream(op, None)
+    op.close()
