@@ -13,6 +13,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
+#include <mutex>
 #include <vector>
 
 #include "atm_device.cuh"
@@ -726,7 +727,11 @@ struct atm3_ctx {
   int *nbr = nullptr, *nbf = nullptr, *nperm = nullptr, *own = nullptr;
   double *wb = nullptr, *nbt = nullptr, *dm = nullptr;  // B and D tables (k3_tables)
   double *cm = nullptr;    // C's volume part for the frozen p_fix (k3_prep_C)
-  double *fbuf = nullptr;  // [nc][6][3][4] face integrals
+  // [nc][6][3][4] face integrals, from a face kernel to the cell kernel behind it.
+  // Everything runs on the one stream; `pair` keeps host threads that share the
+  // handle from launching between the two
+  double *fbuf = nullptr;
+  std::mutex pair;
   double dt = 1.0, Ma = 1.0, Fr = 1.0;
   int hstage = 1, nsstage = 1;
   Tableau tab;
@@ -901,6 +906,7 @@ int rhs3(atm3_ctx &c, double *dst, const double *const *src) {
   const int fields = KIND == 0 ? 4 * co.nst : KIND == 1 ? 5 * co.nst + (c.hstage < 3) : 5 * co.nst + 4;
   SrcPtrs sp{};
   for (int i = 0; i < nsrc; ++i) sp.p[i] = src[i];
+  std::lock_guard<std::mutex> lock(c.pair);
   k3_rhs_face<KIND><<<fblocks(c), NF * FPB, 0, c.stream>>>(c.fbuf, sp, co, c.hstage, c.g);
   ATM_CHECK_LAUNCH("k3_rhs_face");
   // 14 cells: 378 of 384 threads; small shells take small blocks
@@ -932,6 +938,7 @@ int prep_C3(atm3_ctx &c) {
   return ATM_OK;
 }
 int CD3(atm3_ctx &c, double *dst, const double *w, const double *p, double cC, int mode) {
+  std::lock_guard<std::mutex> lock(c.pair);
   k3_face_C<<<fblocks(c), NF * FPB, 0, c.stream>>>(c.fbuf, w, c.pres_fix, c.g);
   ATM_CHECK_LAUNCH("k3_face_C");
   k3_CD<<<(c.nc + CB_CD - 1) / CB_CD, 32 * CB_CD, 0, c.stream>>>(dst, w, p, cC, c.invd, mode, c.cm,

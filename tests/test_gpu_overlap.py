@@ -179,3 +179,37 @@ def test_operators_beside_the_schur_apply(cuda_ok, nx, nz, degree, adaptive):
             assert torch.equal(d, r)
     set_stream(op, None)
     op.close()
+
+
+def test_threads_share_a_shell(cuda_ok):
+    """Host threads that call the right-hand sides and C of one shell handle."""
+    from atmospheric_flows_gb300.shell import ShellSolver, build_shell
+
+    case = build_shell(n=4, nr=2, r_in=6.36122e6, r_out=6.37122e6, rotate_every=5)
+    op, rng = ShellSolver(case), np.random.default_rng(3)
+    op.set_stage(1, 2)
+    op.set_frozen(dev(case.rho), dev(case.p))
+    calls = []
+    for which in (0, 1, 2, 0, 3):
+        rho, u, p = state(case, rng)
+        src = [[rho, u], [rho, u, p, rho], [rho, u, p, rho, u]][which] if which < 3 else u
+        dst = torch.empty_like(u if which == 1 else rho)
+        fn = (lambda d, s, w=which: op.rhs(w, d, s)) if which < 3 else (
+            lambda d, s: op.apply(1, d, s))
+        fn(dst, src)
+        calls.append((fn, src, dst, dst.clone()))
+    bad = []
+
+    def work(fn, src, dst, ref):
+        for _ in range(60):
+            fn(dst, src)
+            torch.cuda.synchronize()
+            if not torch.equal(dst, ref):
+                bad.append(1)
+
+    threads = [threading.Thread(target=work, args=c) for c in calls]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad
