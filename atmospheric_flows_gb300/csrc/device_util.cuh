@@ -25,7 +25,9 @@ __device__ __forceinline__ float abs_max(float a, float b) {
 
 // Values between two cells' A^{-1} blocks ([nc][stride]).  FP64: the full
 // (k+1)^2 x (k+1)^2 block.  FP32 (multigrid levels): A^{-1} is symmetric, so
-// only its lower triangle of (k+1) x (k+1) tiles is stored: tile (a, b), b <= a,
+// only its lower triangle is stored, for the general kernels row by row ((r, c <= r)
+// at r (r+1)/2 + c, padded to a multiple of four values) and for the `exact` ones
+// as (k+1) x (k+1) tiles: tile (a, b), b <= a,
 // couples the node rows iz = a and iz = b.  Off-diagonal tiles come first
 // (row by row, each padded to a multiple of four values), then the diagonal
 // ones as packed lower triangles.  The B kernel stages the blocks of its cells
@@ -42,8 +44,9 @@ struct ATile {
   static constexpr int STRIDE = USED % 8 == 4 ? USED : USED + 4;
 };
 template <int K, typename T>
-__host__ __device__ constexpr int ainv_stride() {
-  return sizeof(T) == 4 ? ATile<K>::STRIDE : (K + 1) * (K + 1) * (K + 1) * (K + 1);
+__host__ __device__ constexpr int ainv_stride(bool exact = true) {
+  constexpr int N2 = (K + 1) * (K + 1);
+  return sizeof(T) == 8 ? N2 * N2 : exact ? ATile<K>::STRIDE : (N2 * (N2 + 1) / 2 + 3) / 4 * 4;
 }
 // offset of entry (i, j), i >= j, in the FP32 tiles
 template <int K>
@@ -53,14 +56,14 @@ __device__ __forceinline__ int atile_index(int i, int j) {
   if (a == b) return ATile<K>::D0 + a * ATile<K>::DIA + r * (r + 1) / 2 + c;
   return (a * (a - 1) / 2 + b) * ATile<K>::OFF + r * NN + c;
 }
-inline long ainv_stride_rt(int k, size_t elem) {
+inline long ainv_stride_rt(int k, size_t elem, bool exact) {
   if (elem != 4) return (long)(k + 1) * (k + 1) * (k + 1) * (k + 1);
   switch (k) {
-    case 1: return ATile<1>::STRIDE;
-    case 2: return ATile<2>::STRIDE;
-    case 3: return ATile<3>::STRIDE;
-    case 4: return ATile<4>::STRIDE;
-    default: return ATile<5>::STRIDE;
+    case 1: return ainv_stride<1, float>(exact);
+    case 2: return ainv_stride<2, float>(exact);
+    case 3: return ainv_stride<3, float>(exact);
+    case 4: return ainv_stride<4, float>(exact);
+    default: return ainv_stride<5, float>(exact);
   }
 }
 

@@ -27,6 +27,10 @@ int level_B_hang(const OpView<T> &o, T *dst, const T *p, T cB, int mode);
 template <typename T>
 int level_CD_hang(const OpView<T> &o, T *dst, const T *w, const T *p, T cC, int mode,
                   const ChebArgs<T> *ch);
+// general_schur_f.cu (FP32 levels, conforming)
+int general_B_f(const OpView<float> &o, float *dst, const float *p, float cB);
+int general_CD_f(const OpView<float> &o, float *dst, const float *w, const float *p, float cC,
+                 int mode, const ChebArgs<float> *ch);
 
 // ============================================================ mass apply ===
 // dst = M_w src for NCOMP components; weight tile (rho) or constant scale
@@ -274,10 +278,11 @@ __global__ void __launch_bounds__(32 * BI_WARPS)
     __syncwarp();
   }
   for (int g = 0; g < CPW && cw + g < mesh.nc; ++g) {
-    T *o = out + (long)(cw + g) * ainv_stride<K, T>();
+    T *o = out + (long)(cw + g) * ainv_stride<K, T>(mesh.exact);
     const T *Mg = wsm + (warp * CPW + g) * B::PER;
-    if constexpr (sizeof(T) == 4) {  // lower triangle of tiles (ATile)
-      for (int e = wl; e < NTRI; e += 32) o[atile_index<K>(ti[e], tj[e])] = -Mg[e];
+    if constexpr (sizeof(T) == 4) {  // lower triangle, by rows or by tiles (ainv_stride)
+      for (int e = wl; e < NTRI; e += 32)
+        o[mesh.exact ? atile_index<K>(ti[e], tj[e]) : e] = -Mg[e];
     } else {
       for (int e = wl; e < NN2 * NN2; e += 32) {
         const int j = e / NN2, i = e - j * NN2;
@@ -430,19 +435,22 @@ template <typename T>
 int level_B(const LevelViewT<T> &v, T *dst, const T *p, T cB, T cC) {
   if (v.mesh.exact) return exact_B(v, dst, p, cB, cC, 2);
   if (v.mesh.nhang > 0) return level_B_hang<T>(v, dst, p, cB, 2);
-  ATM_DISPATCH_K(v.k, (B_launch<K, T, false>(v, dst, p, cB, 2)));
+  if constexpr (sizeof(T) == 4) return general_B_f(v, dst, p, cB);
+  else ATM_DISPATCH_K(v.k, (B_launch<K, T, false>(v, dst, p, cB, 2)));
 }
 template <typename T>
 int level_CD(const LevelViewT<T> &v, T *dst, const T *w, const T *p, T cC, int mode) {
   if (v.mesh.exact) return exact_CD(v, dst, w, p, cC, mode, nullptr);
   if (v.mesh.nhang > 0) return level_CD_hang<T>(v, dst, w, p, cC, mode, nullptr);
-  ATM_DISPATCH_K(v.k, (CD_launch<K, T, false>(v, dst, w, p, cC, mode)));
+  if constexpr (sizeof(T) == 4) return general_CD_f(v, dst, w, p, cC, mode, nullptr);
+  else ATM_DISPATCH_K(v.k, (CD_launch<K, T, false>(v, dst, w, p, cC, mode)));
 }
 template <typename T>
 int level_CD_cheb(const LevelViewT<T> &v, const T *w, T cC, const ChebArgs<T> &ch) {
   if (v.mesh.exact) return exact_CD(v, (T *)nullptr, w, ch.x, cC, 4, &ch);
   if (v.mesh.nhang > 0) return level_CD_hang<T>(v, nullptr, w, ch.x, cC, 4, &ch);
-  ATM_DISPATCH_K(v.k, (CD_launch<K, T, false>(v, nullptr, w, ch.x, cC, 4, &ch)));
+  if constexpr (sizeof(T) == 4) return general_CD_f(v, nullptr, w, ch.x, cC, 4, &ch);
+  else ATM_DISPATCH_K(v.k, (CD_launch<K, T, false>(v, nullptr, w, ch.x, cC, 4, &ch)));
 }
 template <typename T>
 int level_pfix_prep(const LevelViewT<T> &v) {

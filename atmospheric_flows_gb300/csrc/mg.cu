@@ -442,9 +442,9 @@ int level_alloc(atm_ctx &c, MGLevelT<T> &L, const HostMesh &hm) {
     ATM_CUDA(cudaMemsetAsync(*v, 0, ns * sizeof(T), c.stream));
   }
   ATM_CUDA(cudaMalloc(&L.wv, 2 * ns * sizeof(T)));
-  ATM_CUDA(cudaMalloc(&L.ainv, (size_t)L.nc * ainv_stride_rt(c.k, sizeof(T)) * sizeof(T)));
-  // the padding after each FP32 triangle is copied but never used
-  ATM_CUDA(cudaMemsetAsync(L.ainv, 0, (size_t)L.nc * ainv_stride_rt(c.k, sizeof(T)) * sizeof(T),
+  ATM_CUDA(cudaMalloc(&L.ainv, (size_t)L.nc * ainv_stride_rt(c.k, sizeof(T), hm.exact) * sizeof(T)));
+  // the padding in each FP32 block is copied but never used
+  ATM_CUDA(cudaMemsetAsync(L.ainv, 0, (size_t)L.nc * ainv_stride_rt(c.k, sizeof(T), hm.exact) * sizeof(T),
                            c.stream));
   if (hm.exact)
     if (int rc = exact_mesh_build(L.mesh, hm.map2.data(), hm.hcf, c.stream)) return rc;
@@ -523,7 +523,7 @@ int level_apply(atm_ctx &c, MGLevelT<T> &L, T *out, const T *x) {
   // (2 comps written + read) + A^{-1} as stored (FP32: its triangle) + out; flops as
   // launch_B (mode 2) and launch_CD (mode 1)
   const double ns = (double)L.nc * c.nn2, sz = sizeof(T);
-  const double bytes = sz * (ns * (1 + 2 + 2 + 1 + 1 + 1) + (double)L.nc * ainv_stride_rt(c.k, sz));
+  const double bytes = sz * (ns * (1 + 2 + 2 + 1 + 1 + 1) + (double)L.nc * ainv_stride_rt(c.k, sz, L.mesh.exact));
   const double flops = L.nc * (fl_B(c.k, L.mesh.exact, true) + fl_CD(c.k, L.mesh.exact, true));
   TimedRegion tr(c, KF_MG_APPLY, bytes, flops);
   int rc = level_B<T>(v, L.wv, x, (T)(co * c.dt / (c.Ma * c.Ma)), (T)(co * c.dt));
@@ -540,7 +540,7 @@ int level_apply_cheb(atm_ctx &c, MGLevelT<T> &L, double a, double b_coef, bool f
   LevelViewT<T> v = lview(c, L);
   const double ns = (double)L.nc * c.nn2, sz = sizeof(T);
   // as level_apply, plus rhs, invd, d read and d, x written in the update
-  const double bytes = sz * (ns * (1 + 2 + 2 + 1 + 1 + 5) + (double)L.nc * ainv_stride_rt(c.k, sz));
+  const double bytes = sz * (ns * (1 + 2 + 2 + 1 + 1 + 5) + (double)L.nc * ainv_stride_rt(c.k, sz, L.mesh.exact));
   const double flops = L.nc * (fl_B(c.k, L.mesh.exact, true) + fl_CD(c.k, L.mesh.exact, true));
   TimedRegion tr(c, KF_MG_APPLY, bytes, flops);
   int rc = level_B<T>(v, L.wv, L.x, (T)(co * c.dt / (c.Ma * c.Ma)), (T)(co * c.dt));

@@ -19,6 +19,7 @@ namespace atm {
 int upload_basis_impl(const double *t);
 int upload_basis_hang_schur(const double *t);
 int upload_basis_hang_schur_f(const double *t);
+int upload_basis_general_f(const double *t);
 
 // Legendre P_n(x) and P_n'(x) by the three-term recurrence
 static void legendre_pd(int n, double x, double *p, double *dp) {
@@ -152,7 +153,8 @@ int upload_basis_all() {
     }
   }
   if (upload_basis_impl(tab.data()) || upload_basis_hang_schur(tab.data()) ||
-      upload_basis_hang_schur_f(tab.data()) || upload_exact_all()) {
+      upload_basis_hang_schur_f(tab.data()) || upload_basis_general_f(tab.data()) ||
+      upload_exact_all()) {
     set_error("failed to upload basis tables to constant memory");
     return ATM_CUDA_ERROR;
   }
