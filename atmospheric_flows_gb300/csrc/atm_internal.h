@@ -222,7 +222,7 @@ int launch_CD(const atm_ctx &c, double *dst, const double *w, const double *p, d
               int mode, bool workspace = false);
 // values of p_fix at the quadrature points and its face traces (after every
 // change of p_fix)
-int launch_pfix_prep(const atm_ctx &c);
+int launch_pfix_prep(const atm_ctx &c, const double *p);  // pres_fix = p, and what C keeps of it
 // matrix-free mass apply: dst = M_w src, weight = tile field or constant scale
 int launch_mass(const atm_ctx &c, double *dst, const double *src, int ncomp,
                 const double *weight, double scale);
@@ -342,8 +342,8 @@ int exact_CD(const OpView<double> &o, double *dst, const double *w, const double
              int mode, const ChebArgs<double> *ch);
 int exact_CD(const OpView<float> &o, float *dst, const float *w, const float *p, float cC,
              int mode, const ChebArgs<float> *ch);
-int exact_pfix(const OpView<double> &o);
-int exact_pfix(const OpView<float> &o);
+int exact_pfix(const OpView<double> &o, const double *src);
+int exact_pfix(const OpView<float> &o, const float *src);
 int upload_exact_all();
 template <typename T>
 int exact_mesh_build(MeshT<T> &m, const double *map2, const std::vector<int> &hcf,

@@ -287,8 +287,7 @@ int atm_set_rho_for_fixed(atm_handle h, const double *rho) {
 int atm_set_pres_fixed(atm_handle h, const double *p) {
   CHECK_H(h);
   CHECK_PTR(p, "pres");
-  int rc = vec_copy(h->stream, h->pres_fix, p, h->n_scalar());
-  return rc ? rc : launch_pfix_prep(*h);
+  return launch_pfix_prep(*h, p);
 }
 int atm_set_u_fixed(atm_handle h, const double *u) {
   CHECK_H(h);

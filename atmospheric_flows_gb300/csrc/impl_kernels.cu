@@ -391,12 +391,16 @@ int launch_CD(const atm_ctx &c, double *dst, const double *w, const double *p, d
   if (c.mesh.nhang > 0) return launch_CD_hang(c, dst, w, p, coeff, mode);
   ATM_DISPATCH_K(c.k, (CD_launch<K, double, false>(schur_view(c), dst, w, p, coeff, mode)));
 }
-int launch_pfix_prep(const atm_ctx &c) {
-  // p_fix read; its values at the quadrature points and face traces written
-  const double bytes = 8.0 * c.nc * (c.nn2 + c.nq2 + 4.0 * c.nq);
-  const double flops = c.nc * (fl_eval(c.k) + 4.0 * fl_face(c.k));
-  TimedRegion tr(c, KF_PFIX_PREP, bytes, flops);
-  if (c.mesh.exact) return exact_pfix(schur_view(c));
+int launch_pfix_prep(const atm_ctx &c, const double *p) {
+  // p read and copied; its products with the cofactors at the points of C (general
+  // kernels: its values at the quadrature points) and its face traces written
+  const double nc = (3 * c.k + 3) / 2, nn = c.nn;
+  const double bytes =
+      8.0 * c.nc * (2.0 * c.nn2 + (c.mesh.exact ? 4.0 * nc * nc : c.nq2) + 4.0 * c.nq);
+  const double volume = c.mesh.exact ? 2.0 * (nn * nn * nc + nn * nc * nc) + 4.0 * nc * nc : fl_eval(c.k);
+  TimedRegion tr(c, KF_PFIX_PREP, bytes, c.nc * (volume + 4.0 * fl_face(c.k)));
+  if (c.mesh.exact) return exact_pfix(schur_view(c), p);
+  if (int rc = vec_copy(c.stream, c.pres_fix, p, c.n_scalar())) return rc;
   ATM_DISPATCH_K(c.k, (pfix_prep_launch<K, double>(schur_view(c))));
 }
 int launch_mass(const atm_ctx &c, double *dst, const double *src, int ncomp,
@@ -454,7 +458,7 @@ int level_CD_cheb(const LevelViewT<T> &v, const T *w, T cC, const ChebArgs<T> &c
 }
 template <typename T>
 int level_pfix_prep(const LevelViewT<T> &v) {
-  if (v.mesh.exact) return exact_pfix(v);
+  if (v.mesh.exact) return exact_pfix(v, v.pfix);
   ATM_DISPATCH_K(v.k, (pfix_prep_launch<K, T>(v)));
 }
 template <typename T>

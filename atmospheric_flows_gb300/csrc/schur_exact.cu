@@ -251,8 +251,8 @@ int exact_CD(const OpView<double> &o, double *dst, const double *w, const double
   if (o.mesh.nhang > 0) return exact_CD_hang(o, dst, w, p, cC, mode, ch);
   ATM_DISPATCH_K(o.k, (exact_CD_launch<K, double, false>(o, dst, w, p, cC, mode, ch)));
 }
-int exact_pfix(const OpView<double> &o) {
-  ATM_DISPATCH_K(o.k, (exact_pfix_launch<K, double>(o)));
+int exact_pfix(const OpView<double> &o, const double *src) {
+  ATM_DISPATCH_K(o.k, (exact_pfix_launch<K, double>(o, src)));
 }
 
 }  // namespace atm

@@ -691,10 +691,13 @@ __global__ void __launch_bounds__(64)
 // H = gamma/(gamma-1) p_fix cof at the NC x NC points ([c][qx][qz][4]) and the
 // face traces of p_fix at the 2k+1 points.  Threads (cell, column).  Bound by
 // its stores at large meshes (1,568 + 288 bytes per cell at k = 4 in FP64).
+// `copy` (may be null) receives p_fix itself: on small meshes a launch of its own
+// for the copy is 4 us of the 25-75 that freezing rho and p takes (800 cells,
+// k = 2: 30.7 -> 26.6 us).
 template <int K, typename T>
 __global__ void __launch_bounds__(32 * Ex<K>::NC)
     k_exact_pfix(T *__restrict__ hq, T *__restrict__ pff, const T *__restrict__ pfix,
-                 MeshT<T> mesh, int cpb) {
+                 T *__restrict__ copy, MeshT<T> mesh, int cpb) {
   using E = Ex<K>;
   constexpr int NN = E::NN, NN2 = E::NN2, NC = E::NC, NQ = E::NQ;
   extern __shared__ __align__(16) unsigned char sm_raw[];
@@ -706,6 +709,10 @@ __global__ void __launch_bounds__(32 * Ex<K>::NC)
     T t[NN], v[NC];
 #pragma unroll
     for (int i = 0; i < NN; ++i) t[i] = __ldg(pfix + ((long)c0 * NN + e) * NN + i);
+    if (copy) {
+#pragma unroll
+      for (int i = 0; i < NN; ++i) copy[((long)c0 * NN + e) * NN + i] = t[i];
+    }
     eo_interp<K, 1>(t, v);
 #pragma unroll
     for (int q = 0; q < NC; ++q) X[e * NC + q] = v[q];
@@ -817,12 +824,14 @@ int exact_CD_launch(const OpView<T> &v, T *dst, const T *w, const T *p, T cC, in
   return ATM_OK;
 }
 
+// p_fix from `src` (also copied to v.pfix when that is another vector)
 template <int K, typename T>
-int exact_pfix_launch(const OpView<T> &v) {
+int exact_pfix_launch(const OpView<T> &v, const T *src) {
   using E = Ex<K>;
   const int cpb = v.nc < 4096 ? 8 : 32;
   k_exact_pfix<K, T><<<(v.nc + cpb - 1) / cpb, cpb * E::NC, sizeof(T) * cpb * E::NN * E::NC, v.st>>>(
-      const_cast<T *>(v.pfq), const_cast<T *>(v.pff), v.pfix, v.mesh, cpb);
+      const_cast<T *>(v.pfq), const_cast<T *>(v.pff), src,
+      src == v.pfix ? nullptr : const_cast<T *>(v.pfix), v.mesh, cpb);
   ATM_CHECK_LAUNCH("k_exact_pfix");
   return ATM_OK;
 }

@@ -20,8 +20,8 @@ int exact_CD(const OpView<float> &o, float *dst, const float *w, const float *p,
   if (o.mesh.nhang > 0) return exact_CD_hang(o, dst, w, p, cC, mode, ch);
   ATM_DISPATCH_K(o.k, (exact_CD_launch<K, float, false>(o, dst, w, p, cC, mode, ch)));
 }
-int exact_pfix(const OpView<float> &o) {
-  ATM_DISPATCH_K(o.k, (exact_pfix_launch<K, float>(o)));
+int exact_pfix(const OpView<float> &o, const float *src) {
+  ATM_DISPATCH_K(o.k, (exact_pfix_launch<K, float>(o, src)));
 }
 
 }  // namespace atm

@@ -420,7 +420,7 @@ int mesh_upload(atm_ctx &c, int mapdeg, const double *nodes, int n_inner, const 
   rc = launch_inv_diag(c, c.invdiag_D, 1, nullptr, 1.0 / (GAS_GAMMA - 1.0));
   if (rc) return rc;
   // what C keeps of p_fix holds geometry: prepare it again on the new mesh
-  if ((rc = launch_pfix_prep(c))) return rc;
+  if ((rc = launch_pfix_prep(c, c.pres_fix))) return rc;
   ATM_CUDA(cudaStreamSynchronize(c.stream));
   return ATM_OK;
 }

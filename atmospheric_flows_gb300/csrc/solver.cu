@@ -170,8 +170,7 @@ int picard_prepare(atm_ctx &c, Solver &s) {
 // Atmospheric_Flow.cc:544-673
 int pressure_fixed_point(atm_ctx &c, Solver &s) {
   const long ns = c.n_scalar();
-  TRY(vec_copy(c.stream, c.pres_fix, s.pres_fixed_old, ns));  // set_pres_fixed
-  TRY(launch_pfix_prep(c));
+  TRY(launch_pfix_prep(c, s.pres_fixed_old));  // set_pres_fixed
   const StageCoef co = stage_coef_flux(c, c.hstage);
   TRY(launch_rhs_kinetic(c, c.hstage, s.rhs_pres, s.rhs_pres0,
                          c.hstage == 1 ? s.rho_tmp_2 : s.rho_tmp_3, s.u_fixed, co));
