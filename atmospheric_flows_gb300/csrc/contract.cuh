@@ -185,15 +185,17 @@ __device__ __forceinline__ void eo_integ(const T (&V)[NP], const T (&G)[NP], T (
   }
 }
 
+// how four values are loaded: from a table that does not change, from shared
+// memory, or (FP64) from global memory that the launch before may have written
+enum LoadFrom { FROM_TABLE, FROM_SHARED, FROM_LATE };
 template <typename T>
 struct Vec4;
 template <>
 struct Vec4<float> {
   float v[4];
-  // 16-byte aligned, in global memory or (shared) in shared memory
-  __device__ __forceinline__ explicit Vec4(const float *p, bool shared = false) {
+  __device__ __forceinline__ explicit Vec4(const float *p, LoadFrom from = FROM_TABLE) {  // 16-byte aligned
     const float4 *s = reinterpret_cast<const float4 *>(p);
-    const float4 a = shared ? *s : __ldg(s);
+    const float4 a = from == FROM_SHARED ? *s : __ldg(s);
     v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
   }
   __device__ __forceinline__ void store(float *p) const {
@@ -203,10 +205,18 @@ struct Vec4<float> {
 template <>
 struct Vec4<double> {
   double v[4];
-  __device__ __forceinline__ explicit Vec4(const double *p, bool = false) {  // 16-byte aligned
-    const double2 a = __ldg(reinterpret_cast<const double2 *>(p));
-    const double2 b = __ldg(reinterpret_cast<const double2 *>(p) + 1);
-    v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
+  __device__ __forceinline__ explicit Vec4(const double *p, LoadFrom from = FROM_TABLE) {  // 16-byte aligned
+    if (from == FROM_LATE) {
+#pragma unroll
+      for (int i = 0; i < 4; i += 2)
+        asm volatile("ld.global.v2.f64 {%0, %1}, [%2];"
+                     : "=d"(v[i]), "=d"(v[i + 1])
+                     : "l"(__cvta_generic_to_global(p + i)));
+    } else {
+      const double2 a = __ldg(reinterpret_cast<const double2 *>(p));
+      const double2 b = __ldg(reinterpret_cast<const double2 *>(p) + 1);
+      v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
+    }
   }
   __device__ __forceinline__ void store(double *p) const {
     reinterpret_cast<double2 *>(p)[0] = make_double2(v[0], v[1]);
@@ -222,14 +232,14 @@ __device__ __forceinline__ void load2(const double *p, double &a, double &b) {  
   a = x.x; b = x.y;
 }
 
-// nodal trace of a cell's field on face f
-template <int K, typename T>
+// nodal trace of a cell's field on face f (LATE: load_late)
+template <int K, bool LATE = false, typename T>
 __device__ __forceinline__ void trace(const T *__restrict__ cell, int f, T (&t)[K + 1]) {
   constexpr int NN = K + 1;
   const T *b = cell + (f == 1 ? K : f == 3 ? K * NN : 0);
   const int st = f < 2 ? NN : 1;
 #pragma unroll
-  for (int i = 0; i < NN; ++i) t[i] = __ldg(b + i * st);
+  for (int i = 0; i < NN; ++i) t[i] = LATE ? load_late(b + i * st) : __ldg(b + i * st);
 }
 // the same trace at the points of subface s (point set PS: 0 k+1, 1 2k+1)
 template <int K, int PS, int NP, typename T>

@@ -88,8 +88,14 @@ __device__ __forceinline__ void cp_async_wait_all() {
 // become resident while its predecessor in the stream drains, so that launch
 // latency and the predecessor's tail overlap.  Such a kernel calls
 // pdl_trigger() (its own successor may do the same) and must call pdl_wait()
-// before it touches anything that an earlier kernel writes or reads: the wait
-// returns when the predecessor, and with it everything before, has completed.
+// before it touches anything that an overlapped kernel or the launch directly
+// before it writes or reads: the wait returns when the predecessor, and with it
+// everything before, has completed.  What earlier launches wrote may be read
+// sooner, provided that at least one kernel launched without overlap lies between
+// (it started after they had completed, and this one starts after it).
+// Values that the launch directly before may have written are loaded with
+// load_late: the read-only path (__ldg, const __restrict__) is for data that nobody
+// writes during the kernel's lifetime, which begins before the wait.
 // A kernel triggers only if its successor's blocks then spread well: early
 // blocks of a grid that fits the GPU in a wave pack the SMs that are free first.
 // C/D does not trigger: the next operator's B packed itself that way and S took
@@ -101,6 +107,16 @@ __device__ __forceinline__ void pdl_trigger() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ double load_late(const double *p) {
+  double v;
+  asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(__cvta_generic_to_global(p)));
+  return v;
+}
+__device__ __forceinline__ float load_late(const float *p) {
+  float v;
+  asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(__cvta_generic_to_global(p)));
+  return v;
+}
 template <typename... P, typename... A>
 inline cudaError_t launch_overlapped(bool overlap, void (*fn)(P...), long grid, int block, size_t smem,
                                      cudaStream_t st, A... args) {

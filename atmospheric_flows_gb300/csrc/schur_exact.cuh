@@ -168,10 +168,10 @@ __device__ __forceinline__ void face_B(const T *__restrict__ p, const MeshT<T> &
 #pragma unroll
   for (int i = 0; i < NN; ++i) o0[i] = o1[i] = T(0);
   if (nb >= 0) {
-    trace<K>(p + (long)cf * NN2, f, own);
+    trace<K, !HG>(p + (long)cf * NN2, f, own);
     if (!HG || code < 3) {
       T nbt[NN], s[NN], F0[NN], F1[NN];
-      trace<K>(p + (long)nb * NN2, nfc & 3, nbt);
+      trace<K, !HG>(p + (long)nb * NN2, nfc & 3, nbt);
       if (!HG || code == 0) {
 #pragma unroll
         for (int i = 0; i < NN; ++i) nbt[i] -= own[i];
@@ -246,7 +246,9 @@ __global__ void __launch_bounds__(320)
     for (int e = tid; e < n16; e += blockDim.x) cp_async16(as + 4 * e, src + 4 * e);
     cp_async_commit();
   }
-  // up to here only A^{-1}, which no kernel of the overlapping chain writes
+  // up to here only A^{-1} (FP32): on a level at least one kernel launched without
+  // overlap (k_mg_start, k_restrict, k_hash_init) lies between k_block_inverse and
+  // every B
   pdl_wait();
   if constexpr (HG) {
     if (tid == 0) hlist[0] = 0;
@@ -261,7 +263,7 @@ __global__ void __launch_bounds__(320)
     T t[NN], v[NN], d[NN];
     const T *row = p + (long)c * NN2 + j * NN;
 #pragma unroll
-    for (int i = 0; i < NN; ++i) t[i] = __ldg(row + i);
+    for (int i = 0; i < NN; ++i) t[i] = load_late(row + i);
     eo_interp_d<K, 0>(t, v, d);
     T *x = Xs + lc * XV + j * NN;
 #pragma unroll
@@ -363,7 +365,7 @@ __global__ void __launch_bounds__(320)
         const T *Ab = ainv + (long)(c0 + l) * AS + i;
 #pragma unroll
         for (int jj = 0; jj < NN2; ++jj) {
-          const T a = __ldg(Ab + jj * NN2);
+          const T a = load_late(Ab + jj * NN2);
           s0 = fma(a, b[2 * jj], s0);
           s1 = fma(a, b[2 * jj + 1], s1);
         }
@@ -390,19 +392,19 @@ __device__ __forceinline__ void face_C(const T *__restrict__ w, const T *__restr
   } else if (!HG || code == 0) {
     T t[NN], wx[NQ], wz[NQ], vx[NQ], vz[NQ], F[NQ];
     const T *wn = w + (long)nb * 2 * NN2;
-    trace<K>(wc, f, t);
+    trace<K, !HG>(wc, f, t);
     eo_interp<K, 2>(t, wx);
-    trace<K>(wc + NN2, f, t);
+    trace<K, !HG>(wc + NN2, f, t);
     eo_interp<K, 2>(t, wz);
-    trace<K>(wn, nfc & 3, t);
+    trace<K, !HG>(wn, nfc & 3, t);
     eo_interp<K, 2>(t, vx);
-    trace<K>(wn + NN2, nfc & 3, t);
+    trace<K, !HG>(wn + NN2, nfc & 3, t);
     eo_interp<K, 2>(t, vz);
     const T *hp = pff + ((long)c * 4 + f) * NQ, *hm = pff + ((long)nb * 4 + (nfc & 3)) * NQ;
     const T *g = mesh.fC + ((long)c * 4 + f) * 2 * NQ;
 #pragma unroll
     for (int q = 0; q < NQ; ++q)
-      F[q] = flux_C(g + 2 * q, wx[q], wz[q], vx[q], vz[q], __ldg(hp + q), __ldg(hm + q));
+      F[q] = flux_C(g + 2 * q, wx[q], wz[q], vx[q], vz[q], load_late(hp + q), load_late(hm + q));
     eo_integ<K, 2, NQ, true, false>(F, F, o);
   } else {
 #pragma unroll
@@ -513,7 +515,8 @@ __global__ void __launch_bounds__(FB ? 256 : 32 * Ex<K>::NC, FB ? 3 : HG ? 1 : s
   const int c0 = blockIdx.x * cpb;
   const int cnt = min(cpb, mesh.nc - c0);
   if constexpr (STG) {
-    // no kernel of the overlapping chain writes these two
+    // H and det J: as A^{-1} in k_exact_B, a kernel launched without overlap lies
+    // between k_exact_pfix and every C/D of a level
     stage(sH, hq + (long)c0 * 4 * NC2, cnt * 4 * NC2);
     if (WITH_D) stage(sJ, mesh.gJ + (long)c0 * NC2, cnt * NC2);
   }
@@ -557,7 +560,7 @@ __global__ void __launch_bounds__(FB ? 256 : 32 * Ex<K>::NC, FB ? 3 : HG ? 1 : s
                                 : p + ((long)(c0 + l) * NN + (r - 2 * NN)) * NN;
       T t[NN], v[NC];
 #pragma unroll
-      for (int i = 0; i < NN; ++i) t[i] = row[i];
+      for (int i = 0; i < NN; ++i) t[i] = load_late(row + i);
       eo_interp<K, 1>(t, v);
 #pragma unroll
       for (int q = 0; q < NC; ++q) X[l * NF * XS + r * NC + q] = v[q];
@@ -597,7 +600,7 @@ __global__ void __launch_bounds__(FB ? 256 : 32 * Ex<K>::NC, FB ? 3 : HG ? 1 : s
       const T *h = STG ? sH + (l * NC + j) * NC * 4 : hq + ((long)(c0 + l) * NC + j) * NC * 4;
 #pragma unroll
       for (int q = 0; q < NC; ++q) {
-        const Vec4<T> H(h + 4 * q, STG);  // (xi, eta) from w_x, then from w_z
+        const Vec4<T> H(h + 4 * q, STG ? FROM_SHARED : FROM_LATE);  // (xi, eta) from w_x, then from w_z
         Gx[q] = fma(H.v[0], wx[q], H.v[2] * wz[q]);
         Ge[q] = fma(H.v[1], wx[q], H.v[3] * wz[q]);
       }

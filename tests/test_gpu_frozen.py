@@ -44,3 +44,40 @@ def test_frozen_fields_are_copies(cuda_ok, degree, adaptive, mapping_degree):
         r = ref(x)
         assert np.max(np.abs(s.cpu().numpy() - r)) < bar * np.max(np.abs(r))
     g.close()
+
+
+@pytest.mark.parametrize("nx,nz,degree", [(40, 20, 2), (96, 50, 4), (160, 80, 3)])
+def test_apply_directly_behind_a_rebuild(cuda_ok, nx, nz, degree):
+    """S launched right behind new frozen fields, and behind each other, gives
+    the bits of the same calls with the device idle in between."""
+    from atmospheric_flows_gb300.euler_operator import EULEROperator, MatrixFreeStorage
+
+    case = build_case(HillParams(nx=nx, nz=nz, degree=degree, cfl=3.0))
+    g = EULEROperator(MatrixFreeStorage.from_case(case), case.dt, case.Ma, case.Fr)
+    g.set_NS_stage(2)
+    rng = np.random.default_rng(12)
+    field = lambda a: dev(a * (1 + 0.01 * rng.standard_normal(a.shape)))  # noqa: E731
+    sets = [(field(case.rho), field(case.p), field(case.p)) for _ in range(3)]
+    out = [torch.empty(2, g.n_scalar, dtype=torch.float64, device="cuda") for _ in sets]
+
+    def run(wait):
+        for (rho, p, x), s in zip(sets, out):
+            g.set_rho_for_fixed(rho)
+            wait()
+            g.set_pres_fixed(p)
+            wait()
+            g.vmult(s[0], x)
+            wait()
+            g.vmult(s[1], s[0])
+            wait()
+
+    run(torch.cuda.synchronize)
+    ref = [s.clone() for s in out]
+    for _ in range(20):
+        for s in out:
+            s.fill_(float("nan"))
+        run(lambda: None)
+        torch.cuda.synchronize()
+        for s, r in zip(out, ref):
+            assert torch.equal(s, r)
+    g.close()
