@@ -134,7 +134,8 @@ def call(name: str, *args) -> None:
     check(getattr(load(), name)(*args), name)
 
 
-TUNE_FAMILIES = ("rhs_rho", "rhs_vel", "rhs_pres", "B", "CD")
+TUNE_FAMILIES = ("rhs_rho", "rhs_vel", "rhs_pres", "B", "CD",
+                 "B_general", "CD_general", "CD_faces", "rhs_rho_general")
 
 
 def autotune_table():

@@ -378,7 +378,13 @@ long mg_vcycles(const atm_ctx &c);
 // for meshes below 2048 cells, and when tuning is off the default 128/NQ is
 // used.  The choice never changes results: every cell is computed by its own
 // threads whatever the block grouping.
-enum TuneFamily { TF_RHS_RHO = 0, TF_RHS_VEL, TF_RHS_PRES, TF_B, TF_CD };
+// Kernels that take a candidate for another block have families of their own: the
+// general ones beside those of mapping degree <= 2 (for the density, 2k+1 beside
+// fewer points), and C/D with its face integrals from k_exact_face_C.
+enum TuneFamily {
+  TF_RHS_RHO = 0, TF_RHS_VEL, TF_RHS_PRES, TF_B, TF_CD,
+  TF_B_GENERAL, TF_CD_GENERAL, TF_CD_FACES, TF_RHS_RHO_GENERAL
+};
 int tuned_cpb(bool tune, cudaStream_t st, int family, int k, int mode, bool hg, int tsize,
               int nc, bool idempotent, const std::function<cudaError_t(int)> &launch);
 int tune_table(int *out, int max_entries);

@@ -43,7 +43,8 @@ int rhs_passes(const atm_ctx &c, int stage, double *dst, const SrcPtrs &sp, cons
                             : rhs_face_launch<K, KIND, false>(c, stage, dst, way, sp, co);
   };
   // the tuner runs the cell kernel on whatever dst holds, before the faces fill it
-  const int cpb = tuned_cpb(c.autotune && !c.capturing, c.stream, TF_RHS_RHO + KIND, K, stage,
+  const int family = KIND == 0 && !ex ? TF_RHS_RHO_GENERAL : TF_RHS_RHO + KIND;
+  const int cpb = tuned_cpb(c.autotune && !c.capturing, c.stream, family, K, stage,
                             c.mesh.nhang > 0, 8, c.nc, !aliased, launch);
   if (held) {
     if (!FACE_SLOTS<K>)

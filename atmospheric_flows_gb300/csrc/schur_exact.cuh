@@ -820,7 +820,8 @@ int exact_CD_launch(const OpView<T> &v, T *dst, const T *w, const T *p, T cC, in
   // choices made for modes 0 and 1
   const bool idem = mode < 3 && dst != w && dst != p && dst != pfix;
   const int key = mode == 3 ? 0 : (mode == 4 ? 1 : mode);
-  const int cpb = tuned_cpb(v.tune, v.st, TF_CD, K, key, HG, (int)sizeof(T), v.nc, idem, launch);
+  const int cpb = tuned_cpb(v.tune, v.st, fb ? TF_CD_FACES : TF_CD, K, key, HG, (int)sizeof(T),
+                            v.nc, idem, launch);
   overlap = !HG && !fb;
   ATM_CUDA(launch(cpb));
   g_kernel_launches.fetch_add(1);

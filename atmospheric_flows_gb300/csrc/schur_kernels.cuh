@@ -360,8 +360,8 @@ int B_launch(const OpView<T> &v, T *dst, const T *p, T cB, int mode) {
     return cudaGetLastError();
   };
   // mode 1 (dst -= B p) is not idempotent: it uses the choice made for mode 0
-  const int cpb = tuned_cpb(v.tune, v.st, TF_B, K, mode == 1 ? 0 : mode, HG, (int)sizeof(T),
-                            v.nc, mode != 1 && dst != p, launch);
+  const int cpb = tuned_cpb(v.tune, v.st, TF_B_GENERAL, K, mode == 1 ? 0 : mode, HG,
+                            (int)sizeof(T), v.nc, mode != 1 && dst != p, launch);
   ATM_CUDA(launch(cpb));
   g_kernel_launches.fetch_add(1);
   return ATM_OK;
@@ -406,7 +406,8 @@ int CD_launch(const OpView<T> &v, T *dst, const T *w, const T *p, T cC, int mode
   // choices made for modes 0 and 1
   const bool idem = mode < 3 && dst != w && dst != p && dst != pfix;
   const int key = mode == 3 ? 0 : (mode == 4 ? 1 : mode);
-  const int cpb = tuned_cpb(v.tune, v.st, TF_CD, K, key, HG, (int)sizeof(T), v.nc, idem, launch);
+  const int cpb = tuned_cpb(v.tune, v.st, TF_CD_GENERAL, K, key, HG, (int)sizeof(T), v.nc, idem,
+                            launch);
   ATM_CUDA(launch(cpb));
   g_kernel_launches.fetch_add(1);
   return ATM_OK;

@@ -230,7 +230,8 @@ int atm_mg_stats(atm_handle h, long *out);
  * cell batch size at compile time, Atmospheric_Flow.cc:337-344). */
 int atm_set_autotune(atm_handle h, int on);
 /* The choices made so far in this process: up to max_entries rows of 8 ints
- * (device, family 0 rhs_rho / 1 rhs_vel / 2 rhs_pres / 3 B / 4 C/D, degree,
+ * (device, family 0 rhs_rho / 1 rhs_vel / 2 rhs_pres / 3 B / 4 C/D, and
+ * for mappings of degree >= 3 5 B / 6 C/D / 8 rhs_rho; 7 C/D of large meshes, degree,
  * mode or stage, hanging faces, bytes per value, log2 of the cell count,
  * cells per block).  Returns the number of entries (may exceed max_entries). */
 int atm_autotune_table(int *out, int max_entries);
