@@ -749,6 +749,35 @@ __global__ void __launch_bounds__(32 * Ex<K>::NC)
 // face threads of C/D fill whole warps.
 inline int exact_cells(int cpb) { return (cpb + 7) / 8 * 8; }
 
+// The modes that are used: FP32 (multigrid levels) B mode 2 and C/D modes 1 and 4;
+// FP64 C/D with FB (S and the solver) modes 1, 2 and 3.  Null for the others.
+template <int K, typename T, bool HG>
+auto exact_B_kernel(int mode) {
+  decltype(&k_exact_B<K, 2, T, HG>) fn = mode == 2 ? k_exact_B<K, 2, T, HG> : nullptr;
+  if constexpr (sizeof(T) == 8) {
+    if (mode == 0) fn = k_exact_B<K, 0, T, HG>;
+    if (mode == 1) fn = k_exact_B<K, 1, T, HG>;
+  }
+  return fn;
+}
+template <int K, typename T, bool HG>
+auto exact_CD_kernel(int mode, bool fb) {
+  decltype(&k_exact_CD<K, 1, T, HG, false>) fn = nullptr;
+  if constexpr (sizeof(T) == 8) {
+    if (fb)
+      return mode == 1   ? k_exact_CD<K, 1, T, HG, true>
+             : mode == 2 ? k_exact_CD<K, 2, T, HG, true>
+             : mode == 3 ? k_exact_CD<K, 3, T, HG, true>
+                         : fn;
+    if (mode == 0) fn = k_exact_CD<K, 0, T, HG, false>;
+    if (mode == 2) fn = k_exact_CD<K, 2, T, HG, false>;
+    if (mode == 3) fn = k_exact_CD<K, 3, T, HG, false>;
+  }
+  if (mode == 1) fn = k_exact_CD<K, 1, T, HG, false>;
+  if (mode == 4) fn = k_exact_CD<K, 4, T, HG, false>;
+  return fn;
+}
+
 template <int K, typename T, bool HG>
 int exact_B_launch(const OpView<T> &v, T *dst, const T *p, T cB, T cC, int mode) {
   bool overlap = false;  // not while the tuner times the kernel
@@ -758,9 +787,8 @@ int exact_B_launch(const OpView<T> &v, T *dst, const T *p, T cB, T cC, int mode)
     const size_t sm =
         sizeof(T) * (size_t)cpb * ExB<K>::template values<T>(mode == 2 && sizeof(T) == 4) +
         (HG ? sizeof(int) * (4 * cpb + 1) : 0);
-    void (*fn)(T *, const T *, T, T, const T *, MeshT<T>, int) =
-        mode == 0 ? k_exact_B<K, 0, T, HG>
-                  : (mode == 1 ? k_exact_B<K, 1, T, HG> : k_exact_B<K, 2, T, HG>);
+    auto fn = exact_B_kernel<K, T, HG>(mode);
+    if (!fn) return cudaErrorInvalidValue;
     if (cudaError_t e = allow_smem(fn, sm); e != cudaSuccess) return e;
     return launch_overlapped(overlap, fn, (v.nc + cpb - 1) / cpb, cpb * ExB<K>::TPC, sm, v.st, dst, p, cB,
                              cC, v.ainv, v.mesh, cpb);
@@ -772,15 +800,6 @@ int exact_B_launch(const OpView<T> &v, T *dst, const T *p, T cB, T cC, int mode)
   ATM_CUDA(launch(cpb));
   g_kernel_launches.fetch_add(1);
   return ATM_OK;
-}
-
-template <int K, int MODE, typename T, bool HG>
-auto exact_CD_kernel(bool fb) {
-  // FP32 has no FB form
-  if constexpr (sizeof(T) == 8)
-    return fb ? k_exact_CD<K, MODE, T, HG, true> : k_exact_CD<K, MODE, T, HG, false>;
-  else
-    return k_exact_CD<K, MODE, T, HG, false>;
 }
 
 template <int K, typename T, bool HG>
@@ -800,11 +819,8 @@ int exact_CD_launch(const OpView<T> &v, T *dst, const T *w, const T *p, T cC, in
     const size_t sm = sizeof(T) * (size_t)cpb *
                       ((mode == 0 || mode == 3 ? 2 : 3) * E::NN * E::NC + 4 * E::NN + staged) +
                       (HG ? sizeof(int) * (4 * cpb + 1) : 0);
-    auto fn = mode == 0   ? exact_CD_kernel<K, 0, T, HG>(fb)
-              : mode == 1 ? exact_CD_kernel<K, 1, T, HG>(fb)
-              : mode == 2 ? exact_CD_kernel<K, 2, T, HG>(fb)
-              : mode == 3 ? exact_CD_kernel<K, 3, T, HG>(fb)
-                          : exact_CD_kernel<K, 4, T, HG>(fb);
+    auto fn = exact_CD_kernel<K, T, HG>(mode, fb);
+    if (!fn) return cudaErrorInvalidValue;
     if (cudaError_t e = allow_smem(fn, sm); e != cudaSuccess) return e;
     return launch_overlapped(overlap, fn, (v.nc + cpb - 1) / cpb, cpb * E::NC, sm, v.st, dst, w, p,
                              pfix, v.pfq, v.pff, (const T *)v.fbuf, cC, v.invd, v.mesh, ch, cpb);

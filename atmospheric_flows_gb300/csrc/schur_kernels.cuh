@@ -353,8 +353,13 @@ int B_launch(const OpView<T> &v, T *dst, const T *p, T cB, int mode) {
     const int grid = (v.nc + cpb - 1) / cpb, th = cpb * C::NQ;
     const size_t sm = smem_bytes<K, T>(cpb, 1, 2, HG) + sizeof(T) * cpb * 2 * C::NN2 +
                       (mode == 2 && sizeof(T) == 4 ? sizeof(T) * cpb * ainv_stride<K, T>(false) : 0);
-    void (*fn)(T *, const T *, T, const T *, MeshT<T>) =
-        mode == 0 ? k_B<K, 0, T, HG> : (mode == 1 ? k_B<K, 1, T, HG> : k_B<K, 2, T, HG>);
+    // FP32 (multigrid levels): mode 2 only
+    decltype(&k_B<K, 2, T, HG>) fn = mode == 2 ? k_B<K, 2, T, HG> : nullptr;
+    if constexpr (sizeof(T) == 8) {
+      if (mode == 0) fn = k_B<K, 0, T, HG>;
+      if (mode == 1) fn = k_B<K, 1, T, HG>;
+    }
+    if (!fn) return cudaErrorInvalidValue;
     if (cudaError_t e = allow_smem(fn, sm); e != cudaSuccess) return e;
     fn<<<grid, th, sm, v.st>>>(dst, p, cB, v.ainv, v.mesh);
     return cudaGetLastError();
@@ -391,13 +396,15 @@ int CD_launch(const OpView<T> &v, T *dst, const T *w, const T *p, T cC, int mode
                                                           (mode == 4 ? 3 * C::NN2 : 0)) + 3) / 4 * 4)
                            : 0;
     const size_t sm = smem_bytes<K, T>(cpb, 4, 1, HG) + stg;
-    void (*fn)(T *, const T *, const T *, const T *, const T *, const T *, T, const T *,
-               MeshT<T>, ChebArgs<T>) =
-        mode == 0 ? k_CD<K, 0, T, HG>
-        : mode == 1 ? k_CD<K, 1, T, HG>
-        : mode == 2 ? k_CD<K, 2, T, HG>
-        : mode == 3 ? k_CD<K, 3, T, HG>
-                    : k_CD<K, 4, T, HG>;
+    // FP32 (multigrid levels): modes 1 and 4 only
+    decltype(&k_CD<K, 1, T, HG>) fn = mode == 1 ? k_CD<K, 1, T, HG> : nullptr;
+    if (mode == 4) fn = k_CD<K, 4, T, HG>;
+    if constexpr (sizeof(T) == 8) {
+      if (mode == 0) fn = k_CD<K, 0, T, HG>;
+      if (mode == 2) fn = k_CD<K, 2, T, HG>;
+      if (mode == 3) fn = k_CD<K, 3, T, HG>;
+    }
+    if (!fn) return cudaErrorInvalidValue;
     if (cudaError_t e = allow_smem(fn, sm); e != cudaSuccess) return e;
     fn<<<grid, th, sm, v.st>>>(dst, w, p, pfix, v.pfq, v.pff, cC, v.invd, v.mesh, ch);
     return cudaGetLastError();
