@@ -448,8 +448,8 @@ int level_alloc(atm_ctx &c, MGLevelT<T> &L, const HostMesh &hm) {
                            c.stream));
   if (hm.exact)
     if (int rc = exact_mesh_build(L.mesh, hm.map2.data(), hm.hcf, c.stream)) return rc;
-  const size_t ncp = (3 * c.k + 3) / 2;  // H of the exact Schur kernels, or pfq
-  ATM_CUDA(cudaMalloc(&L.pfq, (size_t)L.nc * 4 * ncp * ncp * sizeof(T)));
+  const size_t ncp = (3 * c.k + 3) / 2, npf = hm.exact ? 4 * ncp * ncp : c.nq2;  // H, or pfq
+  ATM_CUDA(cudaMalloc(&L.pfq, (size_t)L.nc * npf * sizeof(T)));
   ATM_CUDA(cudaMalloc(&L.pff, (size_t)L.nc * 4 * c.nq * sizeof(T)));
   return level_inv_diag<T>(lview(c, L), L.invd, (T)(1.0 / (GAS_GAMMA - 1.0)));
 }

@@ -114,8 +114,16 @@ def member_bytes(p: HillParams, precision: int = 1) -> int:
     total = geo + blocks + ctx_vec + solver_vec
     if precision in (1, 2):
         w = 4 if precision == 1 else 8
-        # FGMRES basis + levels (geometry, A^{-1}, vectors) over a 4/3 series
-        lv = (nc * (5 * nq * nq + 12 * nq + schur) * w + nc * nn2 * nn2 * w + 10 * ns * w) * 4 // 3
+        # FGMRES basis + levels (geometry, A^{-1}, vectors) over a 4/3 series.  On a
+        # mapping of degree <= 2 a level keeps JxW and the Schur kernels' tables, and
+        # an FP32 one the lower triangle of A^{-1} in padded tiles
+        inv, tables = nn2 * nn2, nq * nq + schur
+        if p.mapping_degree > 2:
+            tables = 5 * nq * nq + 12 * nq + schur
+        elif precision == 1:
+            off, dia = (nn2 + 3) // 4 * 4, ((k + 1) * (k + 2) // 2 + 3) // 4 * 4
+            inv = k * (k + 1) // 2 * off + (k + 1) * dia + 4
+        lv = nc * (tables + inv + 10 * nn2) * w * 4 // 3
         total += 16 * ns * 8 + lv
     return int(total * 1.15) + (16 << 20)
 
