@@ -1,6 +1,7 @@
 // Device-side helpers: per-degree launch configuration, constant basis tables
-// and the column-wise sum-factorisation primitives shared by every operator
-// kernel.
+// and the column-wise sum-factorisation primitives of the general operator
+// kernels (contract.cuh has those of the right-hand sides and of the Schur
+// kernels for mappings of degree <= 2).
 //
 // Thread layout of the operator kernels ("column" layout): a block holds CPB
 // cells; each cell is served by NQ = 2k+1 threads.  Thread `col` owns the

@@ -32,7 +32,7 @@ static __constant__ float c_sub_f[KMAX + 1][2][2][NQ_MAX][NN_MAX];
 constexpr int EO_DOUBLES = (KMAX + 1) * EO_SETS * 4 * EO_Q * EO_I;
 constexpr int SUB_DOUBLES = (KMAX + 1) * 4 * NQ_MAX * NN_MAX;
 
-// `table`: c_eo followed by c_sub (make_exact_basis)
+// `table`: c_eo followed by c_sub (upload_exact_all)
 static inline int upload_exact_here(const double *table) {
   std::vector<float> f(table, table + EO_DOUBLES + SUB_DOUBLES);
   if (cudaMemcpyToSymbol(c_eo, table, sizeof(c_eo)) != cudaSuccess) return 1;

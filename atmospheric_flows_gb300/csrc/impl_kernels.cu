@@ -155,8 +155,9 @@ __global__ void __launch_bounds__(Cfg<K>::THREADS)
 // Bound by FP64 instructions, which cost a warp the same with one useful lane
 // as with 32: with a warp per cell the pivots' divisions were a third of the
 // kernel and 325 triangle entries left 8% of the lanes idle.  Four cells per
-// warp share the division's instructions and fill the lanes.  Fewer than 4096
-// cells leave SMs without warps; there a warp per cell is the shorter chain.
+// warp share the division's instructions and fill the lanes (12,800 cells, k = 4:
+// 0.47 -> 0.39 ms, the FP64 pipe 87% busy).  Fewer than 4096 cells leave SMs without
+// warps; there a warp per cell is the shorter chain.
 
 template <int K>
 struct BlockInvCfg {

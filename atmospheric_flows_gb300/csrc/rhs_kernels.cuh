@@ -26,12 +26,12 @@
 // handle may overlap, on several streams, threads or branches of a graph.
 // A face trace takes 35 FP64 instructions per field and stage state, a face
 // point about 20: integrating a face from both cells would cost a quarter of
-// the whole right-hand side.  No atomics; runs are bitwise reproducible.
+// the whole right-hand side.  Runs are bitwise reproducible.
 // Measured on GB300, the three right-hand sides of the last stage at 51,200
-// cells, k = 4: 5.82 -> 4.20 ms against one kernel per equation with every
-// face integrated twice and the x-contractions done point by point (the energy
-// cell kernel keeps the FP64 pipe 82-85% busy); 3239 cells, k = 3, second
-// stage: 232 -> 214 us.
+// cells, k = 4: 5.82 -> 3.99 ms against one kernel per equation with every
+// face integrated twice and the x-contractions done point by point (the cell
+// kernels keep the FP64 pipe 83-85% busy); 3239 cells, k = 3, second stage:
+// 232 -> 192 us.
 //
 // The reference integrates with 2k+1 points.  The momentum flux (degree 4k+1
 // on a degree-2 mapping) needs them all, the energy flux more; the density

@@ -31,8 +31,8 @@
 //
 // Measured on GB300 at 51,200 cells, k = 4 (before: the kernels of
 // schur_kernels.cuh, 2k+1 points everywhere, 9 threads per cell): FP64 B with
-// A^{-1} 0.56 -> 0.26 ms, C/D 0.55 -> 0.27 ms (53 us of it the faces), the FP64
-// pipe busy 83-88%; the FP32 V-cycle 1.54 -> 0.84 ms.
+// A^{-1} 0.56 -> 0.24 ms, C/D 0.55 -> 0.28 ms (63 us of it the faces), the FP64
+// pipe busy 80-89%; the FP32 V-cycle 1.54 -> 0.80 ms.
 //
 // In the Schur apply, B stores w = cB cC A^{-1} B p and C/D applies C with unit
 // coefficient: C is homogeneous of degree one in w for the positive cC
@@ -488,6 +488,9 @@ __device__ __forceinline__ void face_rows_of(const float *, const MeshT<float> &
 // Threads (cell, column), column < NC; `cpb` cells per block, without FB a
 // multiple of 8, at most 32.  Three blocks per SM in FP64 (80 registers, k = 4):
 // two leave the SM's quarters with 4, 4, 3 and 3 warps (51,200 cells: S apply 577 -> 572 us); five in FP32.
+// Measured at k = 4 and applied to every order: at k = 5 the FP32 form has 40
+// registers and spills 224 bytes, with a V-cycle of 0.55 ms at 160x80 (0.92 by the
+// general kernels).
 template <int K, int MODE, typename T, bool HG, bool FB>
 __global__ void __launch_bounds__(FB ? 256 : 32 * Ex<K>::NC, FB ? 3 : HG ? 1 : sizeof(T) == 8 ? 3 : 5)
     k_exact_CD(T *__restrict__ dst, const T *__restrict__ w, const T *__restrict__ p,

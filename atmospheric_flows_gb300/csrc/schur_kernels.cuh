@@ -9,7 +9,8 @@
 // mappings of degree 3 and higher (and FP32 levels of such meshes), where no
 // smaller point set gives the same integrals.  Degree <= 2 runs
 // schur_exact.cuh.
-// Included by impl_kernels.cu (HG = false) and hang_rhs_*.cu / hang_schur.cu (HG = true).
+// Included by impl_kernels.cu and general_schur_f.cu (HG = false), hang_schur.cu and
+// hang_schur_f.cu (HG = true).
 #pragma once
 #include "atm_device.cuh"
 

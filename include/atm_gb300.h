@@ -19,6 +19,14 @@
  *   - The solver-level entry points (atm_solver_*) take HOST pointers.
  *   - A handle is not thread-safe; several handles may be used from one
  *     host thread.
+ *   - What may overlap on the GPU (calls of one handle on several streams, or in
+ *     parallel branches of a captured graph): the right-hand sides, B, C, the mass
+ *     operators and diagonals use the caller's vectors and the frozen fields alone.
+ *     S (atm_vmult in NS stage 2), atm_solve, the multigrid calls and atm_solver_*
+ *     share the handle's workspace; the caller orders them among each other, and
+ *     every call after the atm_set_*_fixed that it reads.
+ *   - The destination of a right-hand side must not overlap a source, except that
+ *     the energy's may be the density that it takes last (read cell by cell).
  */
 #ifndef ATM_GB300_H
 #define ATM_GB300_H
