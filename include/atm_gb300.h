@@ -62,7 +62,9 @@ const char *atm_version(void);
  *                   degree-m tensor Lagrange mapping (MappingQ(m)), x fastest
  *   inner_faces   : [n_inner][5] host: cell+, face+, cell-, face-, o
  *                   (local faces 0:x=0 1:x=1 2:z=0 3:z=1; face+ and face- opposite).
- *                   o = 0: conforming face.  o = 1, 2: hanging face of a 2:1
+ *                   o = 0: conforming face; the two cells' faces are the same
+ *                   curve, up to a periodic translation (a flux is integrated with
+ *                   the geometry of one of them).  o = 1, 2: hanging face of a 2:1
  *                   adaptive mesh -- cell+ is the fine cell and its face is
  *                   subface o-1 (the half at the lower face parameter for o = 1)
  *                   of face- of the coarse cell cell-; both subfaces must be
